@@ -380,8 +380,7 @@ __global__ void VENU_TRACE_MULTI_BOUNDS k_trace_shade_multi(const DevJob* __rest
                                                            Queue q0, Queue q1) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
-    sm.node = reinterpret_cast<int*>(smem);
-    sm.tn = reinterpret_cast<float*>(smem + sizeof(int) * kShared * blockDim.x);
+    sm.e = reinterpret_cast<int2*>(smem);
     const int in = (int)(ctl->parity & 1u), out = 1 - in;
     const Queue qin = in ? q1 : q0, qout = in ? q0 : q1;
     const uint32_t lane = threadIdx.x & 31;

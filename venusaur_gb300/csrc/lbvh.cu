@@ -38,14 +38,19 @@ __device__ __forceinline__ float u2f(uint32_t u) {
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
+// The hoisted leaves, slots ascending.
+struct HoistList {
+    uint32_t n;
+    int32_t slot[kMaxHoisted];
+};
+
 // Build-time control block: centroid bounds (order-preserving encoded),
 // the bounds used for quantisation, and the hoisted-sphere list.
 struct LbvhCtl {
     uint32_t b0[6];       // all centroids: lo.xyz, hi.xyz
     float bounds[6];      // the same bounds as floats
     uint32_t hoist_cnt;   // huge spheres found
-    uint32_t nhoist;      // hoisted (<= kMaxHoisted), 0 if more than kHoistCandidates
-    int32_t hoist[kMaxHoisted];
+    HoistList hoisted;    // n <= kMaxHoisted, 0 if more than kHoistCandidates
     uint32_t hoist_buf[64];
     uint32_t bad_words;   // child words k_trav_layout had to replace (never, for a sound build)
 };
@@ -67,7 +72,7 @@ __global__ void k_lbvh_init(LbvhCtl* c) {
             c->b0[3 + a] = 0u;
         }
         c->hoist_cnt = 0;
-        c->nhoist = 0;
+        c->hoisted.n = 0;
         c->bad_words = 0;
     }
 }
@@ -162,7 +167,7 @@ __global__ void k_hoist_finalize(LbvhCtl* c, const int32_t* __restrict__ pleaf, 
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const uint32_t cnt = c->hoist_cnt;
     if (cnt == 0 || cnt > kHoistCandidates) {
-        c->nhoist = 0;
+        c->hoisted.n = 0;
         return;
     }
     uint32_t buf[kHoistCandidates];
@@ -179,7 +184,7 @@ __global__ void k_hoist_finalize(LbvhCtl* c, const int32_t* __restrict__ pleaf, 
     for (uint32_t i = 0; i < nh; ++i) {
         const uint32_t k = buf[i];
         const int32_t p = pleaf[k];
-        c->hoist[i] = (int32_t)k;
+        c->hoisted.slot[i] = (int32_t)k;
         if (p < 0 || (uint32_t)p >= n - 1) continue;
         const int32_t want = (int32_t)k | kLeaf;
         if (__float_as_int(nodes[2 * p].w) == want)
@@ -187,7 +192,7 @@ __global__ void k_hoist_finalize(LbvhCtl* c, const int32_t* __restrict__ pleaf, 
         else if (__float_as_int(nodes[2 * p + 1].w) == want)
             nodes[2 * p + 1].w = __int_as_float(want | kHoisted);
     }
-    c->nhoist = nh;
+    c->hoisted.n = nh;
 }
 
 // Per-tile digit histogram, digit-major: hist[d * ntiles + tile].
@@ -601,23 +606,98 @@ __global__ void k_gather(const venu_sphere* __restrict__ s, const uint32_t* ids,
     meta[k] = id | (type << 30);
 }
 
+// Box of a leaf: the sphere's box rounded outwards (as k_refit makes it).
+__device__ __forceinline__ void leaf_box(float4 s4, float4& lo, float4& hi) {
+    const float r = fabsf(s4.w);
+    lo = make_float4(__fsub_rd(s4.x, r) + 0.0f, __fsub_rd(s4.y, r) + 0.0f, __fsub_rd(s4.z, r) + 0.0f, 0.0f);
+    hi = make_float4(__fadd_ru(s4.x, r), __fadd_ru(s4.y, r), __fadd_ru(s4.z, r), 0.0f);
+}
+
+// ---------------------------------------------------------------------------
 // Traversal layout: internal node p becomes one 64-byte record holding both
-// children, child c in float4s 4p+2c and 4p+2c+1:
-//   internal child q: {lo.xyz, q}, {hi.xyz, 0}   (q's box from nodes)
-//   leaf child:       {center, word}, {radius, 0, 0, 0}   (word keeps the
-//                     leaf and hoisted flags; the sphere is inlined)
-// A step of the traversal then reads one record instead of two boxes or
-// spheres at two addresses.  Runs after k_hoist_finalize, so the flags are
-// final; the canonical nodes array stays the exported form.
+// children, child c in the 32 bytes at float4s 4p + 2c and 4p + 2c + 1:
+//   {c.x, c.y, h.x, h.y}, {c.z, h.z, word, 0}
+// with the centre and the half extents of the child's box (an internal
+// node's, or a leaf's sphere box rounded outwards) and its word (leaf and
+// hoisted flags kept).  A step of the traversal then reads one record with
+// two 32-byte loads instead of two boxes at two addresses, tests nodes and
+// leaves by the same instructions, and finds the operands of the packed FMAs
+// in adjacent registers.  c +- h encloses the box widened by e (the fast
+// walk's bound, venu_device.cuh) under any rounding.  The canonical nodes
+// array stays the exported form.
+//
+// Behind the n - 1 records stands the root's: {c.x, c.y, h.x, h.y},
+// {c.z, h.z, E, 0}.
+//
+// A hoisted leaf is tested before the walk, so its box is empty here
+// (h = -inf is never met), and k_hoist_clean takes it out of the boxes above
+// it: the r = 1000 ground sphere would otherwise make every box on its way
+// to the root one that every ray meets.
 //
 // Every word written here is in range by construction -- an internal child
 // in [1, n-1), a leaf slot below n -- so the traversal needs no per-step
 // index checks: a word that is not (which a sound build never produces) is
 // replaced by a skipped leaf and counted in *bad.
+// ---------------------------------------------------------------------------
+// |C| + |r| of a sphere, 0 unless finite: the bits of non-negative floats
+// order like the values.
+__device__ __forceinline__ uint32_t extent_bits(float4 s4) {
+    const float e = sqrtf(s4.x * s4.x + s4.y * s4.y + s4.z * s4.z) * 1.000001f + fabsf(s4.w);
+    return e <= 3.0e38f ? __float_as_uint(e) : 0u;
+}
+
+__device__ __forceinline__ float widen_of(float E) { return E * 2.86102294921875e-06f; }  // 1.5 2^-19
+
+__device__ __forceinline__ void centre_half(float lo, float hi, float e, float& c, float& h) {
+    c = 0.5f * lo + 0.5f * hi;
+    h = __fadd_ru(fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo)), e);
+    if (!(lo <= hi)) h = __int_as_float(0x7fc00000);  // a NaN box is always met
+}
+
+__device__ __forceinline__ void write_child(float4* rec, float4 lo, float4 hi, float e, int32_t w) {
+    float cx, cy, cz, hx, hy, hz;
+    centre_half(lo.x, hi.x, e, cx, hx);
+    centre_half(lo.y, hi.y, e, cy, hy);
+    centre_half(lo.z, hi.z, e, cz, hz);
+    if ((w & kLeaf) && (w & kHoisted)) {
+        cx = cy = cz = 0.0f;
+        hx = hy = hz = -INFINITY;
+    }
+    rec[0] = make_float4(cx, cy, hx, hy);
+    rec[1] = make_float4(cz, hz, __int_as_float(w), 0.0f);
+}
+
+// E into the root's record (zeroed before): over all leaves but the listed
+// slots.
+__global__ void k_extent(const float4* __restrict__ sph, uint32_t n, const HoistList* __restrict__ ctl_list,
+                         HoistList list, uint32_t* __restrict__ extent) {
+    const HoistList H = ctl_list ? *ctl_list : list;
+    uint32_t ext = 0;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        bool hoisted = false;
+        for (uint32_t i = 0; i < H.n; ++i) hoisted = hoisted || H.slot[i] == (int32_t)k;
+        if (!hoisted) ext = max(ext, extent_bits(sph[k]));
+    }
+    ext = __reduce_max_sync(0xffffffffu, ext);
+    if ((threadIdx.x & 31u) == 0 && ext) atomicMax(extent, ext);
+}
+
 __global__ void k_trav_layout(const float4* __restrict__ nodes, const float4* __restrict__ sph, uint32_t n,
                               float4* __restrict__ trav, uint32_t* bad) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2u * (n - 1u)) return;
+    float4* const root = trav + 4 * (size_t)(n - 1u);
+    const float e = widen_of(root[1].z);
+    if (i == 0) {
+        float4 c;
+        const float4 lo = nodes[0], hi = nodes[1];
+        float cz, hz;
+        centre_half(lo.x, hi.x, e, c.x, c.z);
+        centre_half(lo.y, hi.y, e, c.y, c.w);
+        centre_half(lo.z, hi.z, e, cz, hz);
+        root[0] = c;
+        reinterpret_cast<float2*>(root + 1)[0] = make_float2(cz, hz);  // E beside it stays
+    }
     const uint32_t p = i >> 1, c = i & 1u;
     int32_t w = __float_as_int(nodes[2 * p + c].w);
     const bool ok = (w & kLeaf) ? (uint32_t)(w & kSlotMask) < n && !(w & ~(kLeaf | kHoisted | kSlotMask))
@@ -626,18 +706,81 @@ __global__ void k_trav_layout(const float4* __restrict__ nodes, const float4* __
         w = kLeaf | kHoisted;  // slot 0, never tested
         if (bad) atomicAdd(bad, 1u);
     }
-    float4 a, b;
+    float4 lo, hi;
     if (w & kLeaf) {
-        const float4 s4 = sph[w & kSlotMask];
-        a = make_float4(s4.x, s4.y, s4.z, __int_as_float(w));
-        b = make_float4(s4.w, 0.0f, 0.0f, 0.0f);
+        leaf_box(sph[w & kSlotMask], lo, hi);
     } else {
-        const float4 lo = nodes[2 * w], hi = nodes[2 * w + 1];
-        a = make_float4(lo.x, lo.y, lo.z, __int_as_float(w));
-        b = make_float4(hi.x, hi.y, hi.z, 0.0f);
+        lo = nodes[2 * w];
+        hi = nodes[2 * w + 1];
     }
-    trav[4 * (size_t)p + 2 * c] = a;
-    trav[4 * (size_t)p + 2 * c + 1] = b;
+    write_child(trav + 4 * (size_t)p + 2 * c, lo, hi, e, w);
+}
+
+// Takes the hoisted leaves out of the boxes of the nodes above them, in the
+// records only: one thread per scene walks up from each hoisted leaf; a
+// node's box becomes the union of its record's two children (rounded
+// outwards), written into its parent's record, or the root's.  Walks of
+// several leaves run one after another, so a node above two of them is
+// written last by the later walk, with both taken out.  The widening is in
+// the children already.
+__global__ void k_hoist_clean(float4* trav, const int32_t* __restrict__ pint, const int32_t* __restrict__ pleaf,
+                              uint32_t n, const HoistList* __restrict__ ctl_list, HoistList list) {
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    const HoistList H = ctl_list ? *ctl_list : list;
+    for (uint32_t i = 0; i < H.n; ++i) {
+        int32_t p = pleaf[H.slot[i]];
+        for (uint32_t level = 0; p >= 0 && (uint32_t)p < n - 1u && level < n; ++level) {
+            const float4* T = trav + 4 * (size_t)p;
+            const float4 a0 = T[0], b0 = T[1], a1 = T[2], b1 = T[3];
+            const int32_t q = pint[p];
+            const float c0[3] = {a0.x, a0.y, b0.x}, h0[3] = {a0.z, a0.w, b0.y};
+            const float c1[3] = {a1.x, a1.y, b1.x}, h1[3] = {a1.z, a1.w, b1.y};
+            float c[3], h[3];
+            for (int ax = 0; ax < 3; ++ax) {
+                const bool e0 = h0[ax] == -INFINITY, e1 = h1[ax] == -INFINITY;
+                if (e0) {
+                    c[ax] = c1[ax];
+                    h[ax] = h1[ax];
+                } else if (e1) {
+                    c[ax] = c0[ax];
+                    h[ax] = h0[ax];
+                } else {
+                    const float l0 = __fsub_rd(c0[ax], h0[ax]), u0 = __fadd_ru(c0[ax], h0[ax]);
+                    const float l1 = __fsub_rd(c1[ax], h1[ax]), u1 = __fadd_ru(c1[ax], h1[ax]);
+                    centre_half(fminf(l0, l1), fmaxf(u0, u1), 0.0f, c[ax], h[ax]);
+                    // a NaN box is always met, and so is every box above it
+                    if (!(l0 <= u0) || !(l1 <= u1)) h[ax] = __int_as_float(0x7fc00000);
+                }
+            }
+            if (q >= 0 && (uint32_t)q < n - 1u) {
+                float4* Q = trav + 4 * (size_t)q;
+                const int side = __float_as_int(Q[1].z) == p ? 0 : (__float_as_int(Q[3].z) == p ? 1 : -1);
+                if (side < 0) break;  // never for a sound tree
+                Q[2 * side] = make_float4(c[0], c[1], h[0], h[1]);
+                reinterpret_cast<float2*>(Q + 2 * side + 1)[0] = make_float2(c[2], h[2]);
+            } else {
+                float4* root = trav + 4 * (size_t)(n - 1u);
+                root[0] = make_float4(c[0], c[1], h[0], h[1]);
+                reinterpret_cast<float2*>(root + 1)[0] = make_float2(c[2], h[2]);
+            }
+            p = q;
+        }
+    }
+}
+
+// The records of a built (or refit) tree, on `st`.  The hoisted slots come
+// from the build's control block (ctl_list) or by value.
+cudaError_t launch_trav_layout(const float4* nodes, const float4* sph, uint32_t n, float4* trav, const int32_t* pint,
+                               const int32_t* pleaf, const HoistList* ctl_list, HoistList list, uint32_t* bad,
+                               cudaStream_t st) {
+    float4* const root = trav + 4 * (size_t)(n - 1);
+    const cudaError_t e = cudaMemsetAsync(root, 0, 2 * sizeof(float4), st);
+    if (e != cudaSuccess) return e;
+    k_extent<<<std::min((n + 255) / 256, (uint32_t)(sm_count() * 4)), 256, 0, st>>>(
+        sph, n, ctl_list, list, reinterpret_cast<uint32_t*>(&root[1].z));
+    k_trav_layout<<<(2 * (n - 1) + 255) / 256, 256, 0, st>>>(nodes, sph, n, trav, bad);
+    if (ctl_list || list.n) k_hoist_clean<<<1, 32, 0, st>>>(trav, pint, pleaf, n, ctl_list, list);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -707,13 +850,6 @@ __global__ void k_wide_frontier(const float4* __restrict__ nodes, const int32_t*
         flag[w[j]] = 1u;
         fout[atomicAdd(nout, 1u)] = w[j];
     }
-}
-
-// Box of a leaf: the sphere's box rounded outwards (as k_refit makes it).
-__device__ __forceinline__ void leaf_box(float4 s4, float4& lo, float4& hi) {
-    const float r = fabsf(s4.w);
-    lo = make_float4(__fsub_rd(s4.x, r) + 0.0f, __fsub_rd(s4.y, r) + 0.0f, __fsub_rd(s4.z, r) + 0.0f, 0.0f);
-    hi = make_float4(__fadd_ru(s4.x, r), __fadd_ru(s4.y, r), __fadd_ru(s4.z, r), 0.0f);
 }
 
 // Writes wide node w from the binary words of its children (src[0..7];
@@ -852,7 +988,11 @@ cudaError_t launch_lbvh(const venu_sphere* s, uint32_t n, cudaStream_t st, const
     if (n > 1) {
         k_hoist_collect<<<cdiv(n, 256), 256, 0, st>>>(B.sph, n, B.ctl);
         k_hoist_finalize<<<1, 32, 0, st>>>(B.ctl, B.pleaf, B.nodes, n);
-        if (B.trav) k_trav_layout<<<cdiv(2 * (n - 1), 256), 256, 0, st>>>(B.nodes, B.sph, n, B.trav, &B.ctl->bad_words);
+        if (B.trav) {
+            e = launch_trav_layout(B.nodes, B.sph, n, B.trav, B.pint, B.pleaf, &B.ctl->hoisted, HoistList{},
+                                   &B.ctl->bad_words, st);
+            if (e != cudaSuccess) return e;
+        }
     }
     return cudaGetLastError();
 }
@@ -966,7 +1106,7 @@ venu_status build_scene(const venu_sphere* spheres_dev, uint32_t n, cudaStream_t
     };
     const uint32_t nint = n > 1 ? n - 1 : 1;
     VENU_CUDA(alloc((void**)&S->nodes, sizeof(float4) * 2 * nint));
-    VENU_CUDA(alloc((void**)&S->trav, sizeof(float4) * 4 * nint));
+    VENU_CUDA(alloc((void**)&S->trav, sizeof(float4) * (4 * (size_t)nint + 2)));
     VENU_CUDA(alloc((void**)&S->sph, sizeof(float4) * n));
     VENU_CUDA(alloc((void**)&S->mat, sizeof(float4) * n));
     VENU_CUDA(alloc((void**)&S->meta, sizeof(uint32_t) * n));
@@ -1012,8 +1152,8 @@ venu_status build_scene(const venu_sphere* spheres_dev, uint32_t n, cudaStream_t
         STEP(cudaEventElapsedTime(&ms, e0, e1));
         S->build_ms = ms;
         std::memcpy(S->bounds, hc.bounds, sizeof(S->bounds));
-        S->nhoist = n > 1 ? hc.nhoist : 0u;
-        for (int i = 0; i < kMaxHoisted; ++i) S->hoist[i] = hc.hoist[i];
+        S->nhoist = n > 1 ? hc.hoisted.n : 0u;
+        for (int i = 0; i < kMaxHoisted; ++i) S->hoist[i] = hc.hoisted.slot[i];
         if (n > 1 && hc.bad_words) {
             set_error("venu_scene_create: the LBVH build produced " + std::to_string(hc.bad_words) +
                       " out-of-range child words");
@@ -1071,10 +1211,13 @@ venu_status update_scene(venu_scene* S, const venu_sphere* s, cudaStream_t st) {
     if (e == cudaSuccess) {
         k_refit<<<cdiv(n, 256), 256, 0, st>>>(s, S->meta, 0x3fffffffu, (int)n, S->nodes, S->parents,
                                               S->parents + (n - 1), leafbox, arrive);
-        k_trav_layout<<<cdiv(2 * (n - 1), 256), 256, 0, st>>>(S->nodes, S->sph, n, S->trav, nullptr);
-        if (S->nwide) k_wide_refit<<<cdiv(S->nwide, 128), 128, 0, st>>>(S->nodes, S->sph, S->nwide, S->wide_src,
+        HoistList list{S->nhoist, {}};
+        for (int i = 0; i < kMaxHoisted; ++i) list.slot[i] = S->hoist[i];
+        e = launch_trav_layout(S->nodes, S->sph, n, S->trav, S->parents, S->parents + (n - 1), nullptr, list, nullptr,
+                               st);
+        if (e == cudaSuccess && S->nwide) k_wide_refit<<<cdiv(S->nwide, 128), 128, 0, st>>>(S->nodes, S->sph, S->nwide, S->wide_src,
                                                                       S->wide);
-        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaGetLastError();
     }
     cudaFreeAsync(leafbox, st);
     if (arrive) cudaFreeAsync(arrive, st);

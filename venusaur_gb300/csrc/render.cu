@@ -83,8 +83,7 @@ __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const ui
                                                   unsigned long long* __restrict__ stats) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
-    sm.node = reinterpret_cast<int*>(smem);
-    sm.tn = reinterpret_cast<float*>(smem + sizeof(int) * kShared * blockDim.x);
+    sm.e = reinterpret_cast<int2*>(smem);
     const uint32_t n = *cnt;
     const uint32_t lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats, (unsigned long long)n);
@@ -121,8 +120,7 @@ __global__ void __launch_bounds__(256) k_traverse_dyn(SceneView S, Queue q, cons
                                                       unsigned long long* __restrict__ stats, uint32_t refill_min) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
-    sm.node = reinterpret_cast<int*>(smem);
-    sm.tn = reinterpret_cast<float*>(smem + sizeof(int) * kShared * blockDim.x);
+    sm.e = reinterpret_cast<int2*>(smem);
     const uint32_t n = *cnt;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
@@ -130,8 +128,7 @@ __global__ void __launch_bounds__(256) k_traverse_dyn(SceneView S, Queue q, cons
     TraceCounters K{0, 0};
     bool overflow = false;
     Tracer<COUNT> T;
-    int spill[kSpill];
-    float spill_tn[kSpill];
+    int2 spill[kSpill];
     uint32_t ray = 0;
     bool active = false, exhausted = false;
     for (;;) {
@@ -149,15 +146,17 @@ __global__ void __launch_bounds__(256) k_traverse_dyn(SceneView S, Queue q, cons
                     const float4 o4 = __ldcs(q.o + my), d4 = __ldcs(q.d + my);
                     RayPre R = prep(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
                     R.from = packed_from(d4.w);
-                    if (R.axis) {
-                        // a near-axis-parallel ray (rare): traced to the end now with
-                        // the per-axis loop, on this lane's free stack; the lane
-                        // stays idle
+                    const float m = COUNT ? 0.0f : ray_margin(S, R);
+                    if (COUNT ? R.axis : !(m <= kFarMarginMax)) {
+                        // a ray that needs per-axis margins (rare): traced to the
+                        // end now with the canonical loop, on this lane's free
+                        // stack; the lane stays idle
+                        axis_margins(R);
                         float t;
-                        const int32_t kk = trace_closest_as<COUNT, true>(S, R, 0.001f, 1e16f, t, sm, threadIdx.x,
-                                                                         blockDim.x, overflow, K);
+                        const int32_t kk = trace_with<Tracer<COUNT, true, true>>(
+                            S, R, 0.0f, 0.001f, 1e16f, t, sm, threadIdx.x, blockDim.x, overflow, K);
                         __stcs(hits + my, make_int2(__float_as_int(t), kk));
-                    } else if (T.begin(S, R, 0.001f, 1e16f, K)) {
+                    } else if (T.begin(S, R, m, 0.001f, 1e16f, K)) {
                         active = true;
                     } else {
                         float t;
@@ -171,7 +170,7 @@ __global__ void __launch_bounds__(256) k_traverse_dyn(SceneView S, Queue q, cons
             if (exhausted) break;
             continue;
         }
-        if (active && !T.step(S, sm, threadIdx.x, blockDim.x, spill, spill_tn, overflow, K)) {
+        if (active && !T.step(S, sm, threadIdx.x, blockDim.x, spill, overflow, K)) {
             active = false;
             float t;
             const int32_t kk = T.result(t);
@@ -443,8 +442,7 @@ __device__ __forceinline__ void trace_shade_body(const SceneView& S, const Queue
                                                  WaveCtl* ctl, cudaGraphConditionalHandle handle) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
-    sm.node = reinterpret_cast<int*>(smem);
-    sm.tn = reinterpret_cast<float*>(smem + sizeof(int) * KS * blockDim.x);
+    sm.e = reinterpret_cast<int2*>(smem);
     __shared__ DevCamera cam;  // the primary rays' camera basis, once per block
     if (gen.path_seeds) {      // a kernel parameter: the same in every thread
         if (threadIdx.x == 0) cam = load_camera(gen.cam);
@@ -554,8 +552,7 @@ __global__ void __launch_bounds__(128) k_trace_rays(SceneView S, const float* __
                                                     uint32_t* __restrict__ err) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
-    sm.node = reinterpret_cast<int*>(smem);
-    sm.tn = reinterpret_cast<float*>(smem + sizeof(int) * kShared * blockDim.x);
+    sm.e = reinterpret_cast<int2*>(smem);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     f3 o = mk(rays[6 * (size_t)i], rays[6 * (size_t)i + 1], rays[6 * (size_t)i + 2]);
@@ -591,10 +588,14 @@ SceneView view_of(const venu_scene* s) {
     v.n = s->n;
     v.nhoist = s->nhoist;
     for (int i = 0; i < kMaxHoisted; ++i) v.hoist[i] = s->hoist[i];
+    if (s->n == 1) {  // no tree: the only sphere is tested up front
+        v.nhoist = 1;
+        v.hoist[0] = 0;
+    }
     return v;
 }
 
-size_t traverse_smem(int block, int entries) { return (size_t)block * entries * (sizeof(int) + sizeof(float)); }
+size_t traverse_smem(int block, int entries) { return (size_t)block * entries * sizeof(int2); }
 size_t traverse_smem(int block) { return traverse_smem(block, kShared); }
 
 }  // namespace venu

@@ -266,6 +266,20 @@ struct RayPre {
 
 constexpr float kSharedMarginMax = 1.0f;
 
+// The same ray with per-axis margins (for the canonical walk's AXIS form).
+__device__ __forceinline__ void axis_margins(RayPre& R) {
+    const float px = R.o.x * R.inv.x, py = R.o.y * R.inv.y, pz = R.o.z * R.inv.z;
+    const float mx = fabsf(px) * 4.76837158203125e-07f;  // 2^-21
+    const float my = fabsf(py) * 4.76837158203125e-07f;
+    const float mz = fabsf(pz) * 4.76837158203125e-07f;
+    const float lx = -px - mx, hx = -px + mx;
+    const float ly = -py - my, hy = -py + my;
+    const float lz = -pz - mz, hz = -pz + mz;
+    R.n0 = mk(R.inv.x >= 0.0f ? lx : hx, R.inv.y >= 0.0f ? ly : hy, R.inv.z >= 0.0f ? lz : hz);
+    R.n1 = mk(R.inv.x >= 0.0f ? hx : lx, R.inv.y >= 0.0f ? hy : ly, R.inv.z >= 0.0f ? hz : lz);
+    R.axis = true;
+}
+
 __device__ __forceinline__ RayPre prep(f3 o, f3 d) {
     RayPre R;
     R.from = -1;
@@ -281,16 +295,8 @@ __device__ __forceinline__ RayPre prep(f3 o, f3 d) {
     const float mz = fabsf(pz) * 4.76837158203125e-07f;
     const float m = fmaxf(fmaxf(mx, my), mz);
     R.axis = m > kSharedMarginMax;
-    if (!R.axis) {
-        R.n0 = mk(-px, -py, -pz);
-        R.n1 = mk(m, 0.0f, 0.0f);
-    } else {
-        const float lx = -px - mx, hx = -px + mx;
-        const float ly = -py - my, hy = -py + my;
-        const float lz = -pz - mz, hz = -pz + mz;
-        R.n0 = mk(R.inv.x >= 0.0f ? lx : hx, R.inv.y >= 0.0f ? ly : hy, R.inv.z >= 0.0f ? lz : hz);
-        R.n1 = mk(R.inv.x >= 0.0f ? hx : lx, R.inv.y >= 0.0f ? hy : ly, R.inv.z >= 0.0f ? hz : lz);
-    }
+    R.n0 = mk(-px, -py, -pz);
+    R.n1 = mk(m, 0.0f, 0.0f);
     R.a = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
     R.inv_a = 1.0f / R.a;
     return R;
@@ -341,6 +347,28 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     float bp = s - a;
     float ap = s - bp;
     e = (a - ap) + (b - bp);
+}
+
+// Two floats in one 64-bit register pair, and the packed FMA of sm_100 and
+// later (each half is one ordinary fmaf).
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// 32 bytes with one instruction (32-byte aligned, read-only data).
+__device__ __forceinline__ void ldg32(const void* p, f2& a, f2& b, f2& c, f2& d) {
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
 }
 
 // Ray/sphere: the discriminant is formed from the perpendicular distance of
@@ -449,8 +477,7 @@ constexpr int kSharedShallow = 4;  // the fused kernel's choice for shallow tree
 constexpr int kSpill = 64;   // local-memory entries beyond those
 
 struct StackSmem {
-    int* node;   // [kShared][block]
-    float* tn;   // [kShared][block]
+    int2* e;     // [kShared][block]: {node, entry distance}
 };
 
 // Counting builds only.  lane_steps / warp_steps: traversal steps summed over
@@ -479,46 +506,111 @@ __device__ __forceinline__ void flush_counters(const TraceCounters& K, unsigned 
     }
 }
 
+// Tested up front, with the whole warp converged: first the sphere the
+// ray leaves (R.from; its origin lies within r/16 of that surface, so its
+// test takes sphere_test's long refined branch, which in the walk would
+// run at a different step in each lane), then the huge hoisted spheres
+// (the ground) but that one.  Both are skipped during traversal, and
+// their hit distances already cull boxes behind them.  The closest hit
+// does not depend on the order of the tests.  (A scene of one sphere has
+// it hoisted, see view_of.)  One copy of the test for all of them.
+template <typename T>
+__device__ __forceinline__ void up_front(T& W, const SceneView& S, TraceCounters& K) {
+#pragma unroll 1
+    for (int h = W.R.from >= 0 ? -1 : 0; h < (int)S.nhoist; ++h) {
+        const int32_t k = h < 0 ? W.R.from : S.hoist[h];
+        if (h >= 0 && k == W.R.from) continue;
+        ++K.spheres;
+        W.leaf(k, __ldg(S.sph + k));
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Two walks over the same tree.
+//
+// The canonical walk (CANON) tests the boxes of the canonical nodes with the
+// slab test above, and every leaf's sphere; the host walk does the same, so
+// its counts can be checked exactly.  It serves the counting builds and rays
+// that start far outside the scene.
+//
+// Every other ray takes the fast walk over the traversal records (lbvh.cu):
+// a box is kept as centre c and half extent h per axis, so its entry and exit
+// are fma(h, -|1/d|, tc) and fma(h, |1/d|, tc) with tc = fma(c, 1/d, -o/d)
+// and need no minimum and maximum per slab.  What bounds a step is issue and
+// the ALU pipe (minima, maxima, compares and selects run at half the rate of
+// the FMAs), and whatever one lane of a warp needs all of them pay for; so
+// the x and y slabs are packed FMAs, leaves are tested by their boxes with
+// the same instructions as nodes, and a sphere itself only where its box is
+// hit, by one copy of the test for both children.
+//
+// Nothing is lost by it: '// the records' half extents are widened by
+// e = 1.5 2^-19 E, where E is the largest |C| + |r| of the leaves.
+// sphere_test may accept a point that lies off the sphere by up to
+// 12 2^-24 (|h| + r) (h = o - C; roundings of h, of h.d, of the products with
+// d and of the root), and the slab parameters above are off by at most
+// 4 2^-24 (|o| + E) |1/d|: together 16 2^-24 (|o| + E) in units of length,
+// which is 2^-19 E for |o| = E.  For origins further out the rest, at most
+// 2 2^-20 (|o| - E) max|1/d|, is added to the exit parameter with a factor of
+// two (m); where that exceeds kFarMarginMax the ray takes the canonical walk
+// with margins per axis.  A sphere that is not finite is not part of E; its
+// box is NaN or infinite, and such a box is always met.
+// ---------------------------------------------------------------------------
+constexpr float kFarMarginMax = 1.0f;
+
+__device__ __forceinline__ float far_margin(f3 o, f3 inv, float E) {
+    const float out = fmaxf((fabsf(o.x) + fabsf(o.y) + fabsf(o.z)) - E, 0.0f);
+    return out * fmax3(fabsf(inv.x), fabsf(inv.y), fabsf(inv.z)) * 3.814697265625e-06f;  // 2^-18
+}
+
+// The root's record behind the n - 1 node records: {c.x, c.y, h.x, h.y},
+// {c.z, h.z, E, 0}.
+__device__ __forceinline__ const float4* root_record(const SceneView& S) { return S.trav + 4 * (size_t)(S.n - 1u); }
+
+__device__ __forceinline__ float ray_margin(const SceneView& S, const RayPre& R) {
+    return S.n > 1u ? far_margin(R.o, R.inv, __ldg(&root_record(S)[1].z)) : 0.0f;
+}
+
 // Per-lane traversal state.  begin() prepares a ray and tests the root;
-// step() tests both children of the current node (from its 64-byte record in
-// the traversal layout: boxes of internal children, spheres of leaf children
-// inline) and descends or pops; both return whether more work remains.  The
-// same state machine serves the one-ray-per-thread kernels (trace_closest)
-// and the persistent kernels that refill idle lanes.
-template <bool COUNT, bool AXIS = false, int KS = kShared>
+// step() tests both children of the current node (from its 64-byte record)
+// and descends or pops; both return whether more work remains.  The same
+// state machine serves the one-ray-per-thread kernels (trace_closest) and
+// the persistent kernels that refill idle lanes.
+// AXIS (canonical walk only): R carries per-axis margins.
+template <bool COUNT, bool CANON = COUNT, bool AXIS = false, int KS = kShared>
 struct Tracer {
     RayPre R;
-    float tmin, tmax, best_t;
+    float tmin, tmax, best_t, m;
+    f2 inv_xy, n0_xy, a_xy, na_xy;  // 1/d, -o/d, |1/d|, -|1/d| of x and y
     int32_t best, cur;
     int sp;
     uint32_t guard;
 
-    __device__ __forceinline__ void leaf(int32_t k, float4 s4, TraceCounters& K) {
+    __device__ __forceinline__ void leaf(int32_t k, float4 s4) {
         float t;
-        if (COUNT) ++K.spheres;
         if (sphere_test(R, s4, tmin, tmax, t) && (t < best_t || (t == best_t && k < best))) {
             best_t = t;
             best = k;
         }
     }
 
-    // Tested up front, with the whole warp converged: first the sphere the
-    // ray leaves (R.from; its origin lies within r/16 of that surface, so its
-    // test takes sphere_test's long refined branch, which in the walk would
-    // run at a different step in each lane), then the huge hoisted spheres
-    // (the ground) but that one.  Both are skipped during traversal, and
-    // their hit distances already cull boxes behind them.  The closest hit
-    // does not depend on the order of the tests.
-    __device__ __forceinline__ void from_first(const SceneView& S, TraceCounters& K) {
-        if (R.from >= 0) leaf(R.from, __ldg(S.sph + R.from), K);
-        for (uint32_t h = 0; h < S.nhoist; ++h)
-            if (S.hoist[h] != R.from) leaf(S.hoist[h], __ldg(S.sph + S.hoist[h]), K);
+    // Entry (clipped to tmin) and exit (margin included) of a record's box.
+    __device__ __forceinline__ void interval(f2 c_xy, f2 h_xy, float c_z, float h_z, float& tn, float& tf) const {
+        const f2 tc = fma2(c_xy, inv_xy, n0_xy);
+        float nx, ny, fx, fy;
+        unpack2(fma2(h_xy, na_xy, tc), nx, ny);
+        unpack2(fma2(h_xy, a_xy, tc), fx, fy);
+        const float tcz = fmaf(c_z, R.inv.z, R.n0.z);
+        const float nz = fmaf(h_z, -fabsf(R.inv.z), tcz), fz = fmaf(h_z, fabsf(R.inv.z), tcz);
+        tn = fmaxf(fmax3(nx, ny, nz), tmin);
+        tf = fmin3(fx, fy, fz);
     }
+    __device__ __forceinline__ bool meets(float tn, float tf) const { return tn <= fminf(tf, best_t) + m; }
 
-    // R_ from prep(); its axis flag must equal AXIS.
-    __device__ __forceinline__ bool begin(const SceneView& S, const RayPre& R_, float tmin_, float tmax_,
+    // R_ from prep(); AXIS: with per-axis margins.  m_: far_margin (fast walk).
+    __device__ __forceinline__ bool begin(const SceneView& S, const RayPre& R_, float m_, float tmin_, float tmax_,
                                           TraceCounters& K) {
         R = R_;
+        m = m_;
         tmin = tmin_;
         tmax = tmax_;
         best_t = tmax_;
@@ -526,15 +618,23 @@ struct Tracer {
         sp = 0;
         const uint32_t n = S.n;
         if (n == 0) return false;
-        from_first(S, K);
-        if (n == 1) {
-            if (R.from != 0) leaf(0, __ldg(S.sph), K);
-            return false;
-        }
+        up_front(*this, S, K);
+        if (n == 1) return false;
         float tn;
-        float4 rlo = __ldg(S.nodes + 0), rhi = __ldg(S.nodes + 1);
-        if (COUNT) ++K.nodes;
-        if (!box_test<AXIS>(R, rlo, rhi, tmin, best_t, tn)) return false;
+        if (CANON) {
+            float4 rlo = __ldg(S.nodes + 0), rhi = __ldg(S.nodes + 1);
+            if (COUNT) ++K.nodes;
+            if (!box_test<AXIS>(R, rlo, rhi, tmin, best_t, tn)) return false;
+        } else {
+            inv_xy = pack2(R.inv.x, R.inv.y);
+            n0_xy = pack2(R.n0.x, R.n0.y);
+            a_xy = pack2(fabsf(R.inv.x), fabsf(R.inv.y));
+            na_xy = pack2(-fabsf(R.inv.x), -fabsf(R.inv.y));
+            const float4 r0 = __ldg(root_record(S)), r1 = __ldg(root_record(S) + 1);
+            float tf;
+            interval(pack2(r0.x, r0.y), pack2(r0.z, r0.w), r1.x, r1.y, tn, tf);
+            if (!meets(tn, tf)) return false;
+        }
         cur = 0;
         // A tree has n-1 internal nodes and each step expands a different one;
         // the guard turns a cyclic (corrupt) tree into an error flag instead
@@ -543,10 +643,10 @@ struct Tracer {
         return true;
     }
 
-    // spill / spill_tn: this thread's local-memory stack entries beyond the
-    // kShared in shared memory.
+    // spill: this thread's local-memory stack entries beyond the KS in shared
+    // memory.
     __device__ __forceinline__ bool step(const SceneView& S, StackSmem sm, uint32_t tid, uint32_t bdim,
-                                         int* spill, float* spill_tn, bool& overflow, TraceCounters& K) {
+                                         int2* spill, bool& overflow, TraceCounters& K) {
         // Every word of the traversal records is in range (checked when the
         // records are written), so only termination needs guarding here.
         if (--guard == 0u) {
@@ -558,71 +658,89 @@ struct Tracer {
             const uint32_t am = __activemask();
             if ((tid & 31u) == (uint32_t)(__ffs(am) - 1)) ++K.warp_steps;
         }
+        f2 c0, h0_, z0, q0, c1, h1_, z1, q1;
         const float4* T = S.trav + 4 * (size_t)cur;
-        const float4 a0 = __ldg(T), b0 = __ldg(T + 1), a1 = __ldg(T + 2), b1 = __ldg(T + 3);
-        const int32_t w0 = __float_as_int(a0.w), w1 = __float_as_int(a1.w);
+        ldg32(T, c0, h0_, z0, q0);
+        ldg32(T + 2, c1, h1_, z1, q1);
+        const int32_t w0 = (int32_t)(uint32_t)q0, w1 = (int32_t)(uint32_t)q1;
         bool h0 = false, h1 = false;
         float tn0 = 0.0f, tn1 = 0.0f;
-        if (w0 & kLeaf) {
-            if (!(w0 & kHoisted) && (w0 & kSlotMask) != R.from)
-                leaf(w0 & kSlotMask, make_float4(a0.x, a0.y, a0.z, b0.x), K);
-        } else {
-            if (COUNT) ++K.nodes;
-            h0 = box_test<AXIS>(R, a0, b0, tmin, best_t, tn0);
-        }
-        if (w1 & kLeaf) {
-            if (!(w1 & kHoisted) && (w1 & kSlotMask) != R.from)
-                leaf(w1 & kSlotMask, make_float4(a1.x, a1.y, a1.z, b1.x), K);
-        } else {
-            if (COUNT) ++K.nodes;
-            h1 = box_test<AXIS>(R, a1, b1, tmin, best_t, tn1);
-        }
-        if (h0 && h1) {
-            int32_t far;
-            float far_tn;
-            if (tn1 < tn0) {
-                far = w0;
-                far_tn = tn0;
-                cur = w1;
-            } else {
-                far = w1;
-                far_tn = tn1;
-                cur = w0;
-            }
-            const uint32_t j = (uint32_t)(sp & (KS - 1)) * bdim + tid;
-            if (sp >= KS) {
-                const int g = sp - KS;
-                if (g >= kSpill) {
-                    overflow = true;
-                    return false;
+        if (CANON) {
+#pragma unroll 1
+            for (int c = 0; c < 2; ++c) {
+                const int32_t w = c ? w1 : w0;
+                bool h = false;
+                float tn = 0.0f;
+                if (w < 0) {
+                    const int32_t k = w & kSlotMask;
+                    if (!(w & kHoisted) && k != R.from) {
+                        if (COUNT) ++K.spheres;
+                        leaf(k, __ldg(S.sph + k));
+                    }
+                } else {
+                    if (COUNT) ++K.nodes;
+                    h = box_test<AXIS>(R, __ldg(S.nodes + 2 * (size_t)w), __ldg(S.nodes + 2 * (size_t)w + 1), tmin,
+                                       best_t, tn);
                 }
-                spill[g] = sm.node[j];
-                spill_tn[g] = sm.tn[j];
+                if (c) {
+                    h1 = h;
+                    tn1 = tn;
+                } else {
+                    h0 = h;
+                    tn0 = tn;
+                }
             }
-            sm.node[j] = far;
-            sm.tn[j] = far_tn;
-            ++sp;
-            return true;
+        } else {
+            float tf0, tf1, cz, hz;
+            unpack2(z0, cz, hz);
+            interval(c0, h0_, cz, hz, tn0, tf0);
+            unpack2(z1, cz, hz);
+            interval(c1, h1_, cz, hz, tn1, tf1);
+            h0 = meets(tn0, tf0);
+            h1 = meets(tn1, tf1);
+            // a hoisted leaf's box is empty
+            bool l0 = h0 && w0 < 0, l1 = h1 && w1 < 0;
+            h0 = h0 && w0 >= 0;
+            h1 = h1 && w1 >= 0;
+            if (l0 || l1) {
+                for (;;) {
+                    const int32_t k = (l0 ? w0 : w1) & kSlotMask;
+                    if (k != R.from) leaf(k, __ldg(S.sph + k));
+                    if (!l0) break;
+                    l0 = false;
+                    // the other child against the shortened ray
+                    const bool ok = meets(tn1, tf1);
+                    h1 = h1 && ok;
+                    l1 = l1 && ok;
+                    if (!l1) break;
+                }
+            }
         }
-        if (h0) {
-            cur = w0;
-            return true;
-        }
-        if (h1) {
-            cur = w1;
+        if (h0 || h1) {
+            const bool second = h1 && (!h0 || tn1 < tn0);
+            cur = second ? w1 : w0;
+            if (h0 && h1) {
+                const int2 e = make_int2(second ? w0 : w1, __float_as_int(second ? tn0 : tn1));
+                if (sp < KS) {
+                    sm.e[(uint32_t)sp * bdim + tid] = e;
+                } else {
+                    if (sp >= KS + kSpill) {
+                        overflow = true;
+                        return false;
+                    }
+                    spill[sp - KS] = e;
+                }
+                ++sp;
+            }
             return true;
         }
         while (sp > 0) {
             --sp;
-            const uint32_t j = (uint32_t)(sp & (KS - 1)) * bdim + tid;
-            const int32_t e = sm.node[j];
-            const float etn = sm.tn[j];
-            if (sp >= KS) {
-                sm.node[j] = spill[sp - KS];
-                sm.tn[j] = spill_tn[sp - KS];
-            }
-            if (etn <= best_t) {
-                cur = e;
+            int2 e;
+            if (sp < KS) e = sm.e[(uint32_t)sp * bdim + tid];
+            else e = spill[sp - KS];
+            if (__int_as_float(e.y) <= (CANON ? best_t : best_t + m)) {
+                cur = e.x;
                 return true;
             }
         }
@@ -694,23 +812,15 @@ struct WideTracer {
     int sp;
     uint32_t guard;
 
-    __device__ __forceinline__ void leaf(int32_t k, float4 s4, TraceCounters& K) {
+    __device__ __forceinline__ void leaf(int32_t k, float4 s4) {
         float t;
-        if (COUNT) ++K.spheres;
         if (sphere_test(R, s4, tmin, tmax, t) && (t < best_t || (t == best_t && k < best))) {
             best_t = t;
             best = k;
         }
     }
 
-    // as Tracer::from_first
-    __device__ __forceinline__ void from_first(const SceneView& S, TraceCounters& K) {
-        if (R.from >= 0) leaf(R.from, __ldg(S.sph + R.from), K);
-        for (uint32_t h = 0; h < S.nhoist; ++h)
-            if (S.hoist[h] != R.from) leaf(S.hoist[h], __ldg(S.sph + S.hoist[h]), K);
-    }
-
-    __device__ __forceinline__ bool begin(const SceneView& S, const RayPre& R_, float tmin_, float tmax_,
+    __device__ __forceinline__ bool begin(const SceneView& S, const RayPre& R_, float, float tmin_, float tmax_,
                                           TraceCounters& K) {
         R = R_;
         tmin = tmin_;
@@ -720,11 +830,8 @@ struct WideTracer {
         sp = 0;
         const uint32_t n = S.n;
         if (n == 0) return false;
-        from_first(S, K);
-        if (n == 1) {
-            if (R.from != 0) leaf(0, __ldg(S.sph), K);
-            return false;
-        }
+        up_front(*this, S, K);
+        if (n == 1) return false;
         float tn;
         float4 rlo = __ldg(S.nodes + 0), rhi = __ldg(S.nodes + 1);
         if (COUNT) ++K.nodes;
@@ -736,25 +843,23 @@ struct WideTracer {
         return true;
     }
 
-    __device__ __forceinline__ void push(StackSmem sm, uint32_t tid, uint32_t bdim, int* spill, float* spill_tn,
-                                         bool& overflow, int32_t node, float tn) {
-        const uint32_t j = (uint32_t)(sp & (KS - 1)) * bdim + tid;
+    __device__ __forceinline__ void push(StackSmem sm, uint32_t tid, uint32_t bdim, int2* spill, bool& overflow,
+                                         int32_t node, float tn) {
+        int2* const e = sm.e + ((uint32_t)(sp & (KS - 1)) * bdim + tid);
         if (sp >= KS) {
             const int g = sp - KS;
             if (g >= kSpill) {
                 overflow = true;
                 return;
             }
-            spill[g] = sm.node[j];
-            spill_tn[g] = sm.tn[j];
+            spill[g] = *e;
         }
-        sm.node[j] = node;
-        sm.tn[j] = tn;
+        *e = make_int2(node, __float_as_int(tn));
         ++sp;
     }
 
     __device__ __forceinline__ bool step(const SceneView& S, StackSmem sm, uint32_t tid, uint32_t bdim,
-                                         int* spill, float* spill_tn, bool& overflow, TraceCounters& K) {
+                                         int2* spill, bool& overflow, TraceCounters& K) {
         if (--guard == 0u) {
             overflow = true;
             return false;
@@ -808,14 +913,14 @@ struct WideTracer {
                 uint32_t kmax = 0;
 #pragma unroll
                 for (int c = 0; c < kWideW; ++c) kmax = key[c] != 0xffffffffu ? max(kmax, key[c]) : kmax;
-                push(sm, tid, bdim, spill, spill_tn, overflow, __ldg(words + (kmax & 7u)),
+                push(sm, tid, bdim, spill, overflow, __ldg(words + (kmax & 7u)),
                      __uint_as_float(kmax & ~7u));
             } else if (nhit > 2u) {
                 if (kWideW == 8) sort8(key); else sort4(key);
 #pragma unroll
                 for (int i = kWideW - 1; i >= 1; --i) {
                     if (key[i] != 0xffffffffu)
-                        push(sm, tid, bdim, spill, spill_tn, overflow, __ldg(words + (key[i] & 7u)),
+                        push(sm, tid, bdim, spill, overflow, __ldg(words + (key[i] & 7u)),
                              __uint_as_float(key[i] & ~7u));
                 }
             }
@@ -825,7 +930,10 @@ struct WideTracer {
         // ray and cull the pushed entries and the nearest child
         for (uint32_t lm = lhit; lm; lm &= lm - 1u) {
             const int32_t k = __ldg(words + (__ffs(lm) - 1)) & kSlotMask;
-            if (k != R.from) leaf(k, __ldg(S.sph + k), K);
+            if (k != R.from) {
+                if (COUNT) ++K.spheres;
+                leaf(k, __ldg(S.sph + k));
+            }
         }
         if (kmin != 0xffffffffu && __uint_as_float(kmin & ~7u) <= best_t) {
             cur = __ldg(words + (kmin & 7u));
@@ -833,15 +941,11 @@ struct WideTracer {
         }
         while (sp > 0) {
             --sp;
-            const uint32_t j = (uint32_t)(sp & (KS - 1)) * bdim + tid;
-            const int32_t e = sm.node[j];
-            const float etn = sm.tn[j];
-            if (sp >= KS) {
-                sm.node[j] = spill[sp - KS];
-                sm.tn[j] = spill_tn[sp - KS];
-            }
-            if (etn <= best_t) {
-                cur = e;
+            int2* const p = sm.e + ((uint32_t)(sp & (KS - 1)) * bdim + tid);
+            const int2 e = *p;
+            if (sp >= KS) *p = spill[sp - KS];
+            if (__int_as_float(e.y) <= best_t) {
+                cur = e.x;
                 return true;
             }
         }
@@ -858,31 +962,43 @@ struct WideTracer {
     }
 };
 
-template <bool COUNT, bool AXIS, int KS = kShared, bool WIDE = false>
-__device__ __forceinline__ int32_t trace_closest_as(const SceneView& S, const RayPre& R, float tmin,
-                                                    float tmax, float& t_out, StackSmem sm,
-                                                    uint32_t tid, uint32_t bdim, bool& overflow,
-                                                    TraceCounters& K) {
-    typename std::conditional<WIDE, WideTracer<COUNT, AXIS, KS>, Tracer<COUNT, AXIS, KS>>::type T;
-    int spill[kSpill];
-    float spill_tn[kSpill];
-    if (T.begin(S, R, tmin, tmax, K))
-        while (T.step(S, sm, tid, bdim, spill, spill_tn, overflow, K)) {
+template <class T>
+__device__ __forceinline__ int32_t trace_with(const SceneView& S, const RayPre& R, float m, float tmin, float tmax,
+                                              float& t_out, StackSmem sm, uint32_t tid, uint32_t bdim,
+                                              bool& overflow, TraceCounters& K) {
+    T W;
+    int2 spill[kSpill];
+    if (W.begin(S, R, m, tmin, tmax, K))
+        while (W.step(S, sm, tid, bdim, spill, overflow, K)) {
         }
-    return T.result(t_out);
+    return W.result(t_out);
 }
 
-// Closest hit of one ray (R from prep): the shared-margin loop, or the
-// per-axis one for the rare near-axis-parallel ray.  KS: shared-memory stack
-// entries per thread (the kernel's StackSmem holds KS of them).
+// Closest hit of one ray (R from prep).  The binary tree: the fast walk,
+// unless the ray starts far outside the scene (rare) or the build counts;
+// those, and the wide tree, take the shared-margin loop, or the per-axis one
+// for the rare near-axis-parallel ray.  KS: shared-memory stack entries per
+// thread (the kernel's StackSmem holds KS of them).
 template <bool COUNT, int KS = kShared, bool WIDE = false>
 __device__ __forceinline__ int32_t trace_closest(const SceneView& S, const RayPre& R, float tmin,
                                                  float tmax, float& t_out, StackSmem sm,
                                                  uint32_t tid, uint32_t bdim, bool& overflow,
                                                  TraceCounters& K) {
-    if (R.axis)
-        return trace_closest_as<COUNT, true, KS, WIDE>(S, R, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
-    return trace_closest_as<COUNT, false, KS, WIDE>(S, R, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
+    if (WIDE) {
+        if (R.axis) {
+            RayPre A = R;
+            axis_margins(A);
+            return trace_with<WideTracer<COUNT, true, KS>>(S, A, 0.0f, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
+        }
+        return trace_with<WideTracer<COUNT, false, KS>>(S, R, 0.0f, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
+    }
+    const float m = COUNT ? 0.0f : ray_margin(S, R);
+    if (COUNT ? R.axis : !(m <= kFarMarginMax)) {
+        RayPre A = R;
+        axis_margins(A);
+        return trace_with<Tracer<COUNT, true, true, KS>>(S, A, 0.0f, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
+    }
+    return trace_with<Tracer<COUNT, COUNT, false, KS>>(S, R, m, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
 }
 
 // ---------------------------------------------------------------------------
