@@ -231,12 +231,17 @@ __device__ __forceinline__ void trace_shade_loop(const SceneView& S, const Queue
 
 // The in-place launch (no more rays than the grid has threads): block b
 // takes rays [b * blockDim, (b + 1) * blockDim) and finishes them bounce by
-// bounce.  Between bounces the block's surviving paths are compacted to its
-// first threads (their state staged through the unused output queue, at the
-// block's own positions), so its warps stay full while paths end at
-// different bounces instead of idling around the few long paths.  Each path
-// goes through exactly the same arithmetic as in the ordinary loop; only
-// the thread that runs it changes.
+// bounce.  After bounces 1, 2, 4, 8, ... the block's surviving paths are
+// compacted to its first threads where that frees a warp (their state staged
+// through the unused output queue, at the block's own positions), so its
+// warps stay full while paths end at different bounces instead of idling
+// around the few long paths; in between each warp runs at its own pace.
+// This launch waits for its longest path (28-31 % of the issue slots used),
+// so a barrier at every bounce cost more than the fuller warps gave: against
+// that, 256x144 x 4 RTIOW 319 -> 303 us, 400x225 x 16 692 -> 679 us, larger
+// frames unchanged; after every 4th or 8th bounce only, 400x225 x 16 takes
+// 804 and 1073 us.  Each path goes through exactly the same arithmetic as in
+// the ordinary loop; only the thread that runs it changes.
 template <bool COUNT, int KS, bool WIDE>
 __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Queue& qin, uint32_t n,
                                                      const Queue& qout, float4* __restrict__ slots,
@@ -260,10 +265,11 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
         }
     }
     uint32_t held = (uint32_t)__syncthreads_count(live);  // threads holding a state, from thread 0 on
-    for (bool first = true;; first = false) {
+    uint32_t done = 0;                                    // bounces traced in place
+    for (;;) {
         const uint32_t cnt = (uint32_t)__syncthreads_count(live);
         if (cnt == 0) break;
-        if (cnt < held) {
+        if ((cnt + 31u) / 32u < (held + 31u) / 32u) {
             // compaction: the live states to threads [0, cnt)
             const uint32_t m = __ballot_sync(0xffffffffu, live);
             if (lane == 0) warp_live[w] = (uint32_t)__popc(m);
@@ -285,13 +291,16 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
             }
             held = cnt;
         }
-        if (live) {
+        // as many bounces as were traced before, by each warp at its own pace
+        const uint32_t until = done ? 2u * done : 1u;
+        for (; done < until && __any_sync(0xffffffffu, live); ++done) {
+            if (!live) continue;
             RayPre R = prep(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float th;
             const int32_t k = trace_closest<COUNT, KS, WIDE>(S, R, 0.001f, 1e16f, th, sm, t, blockDim.x, overflow, K);
             const ShadeOut r = shade_one<true>(S, o4, d4, qout.t[i], make_int2(__float_as_int(th), k));
-            if (!first) ++extra;
+            if (done) ++extra;
             if (r.cont) {
                 o4 = r.o;
                 d4 = r.d;
@@ -301,6 +310,7 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
                 live = false;
             }
         }
+        done = until;
     }
 }
 
