@@ -347,20 +347,49 @@ __global__ void k_refit(const venu_sphere* __restrict__ s, const uint32_t* __res
 }
 
 // ---------------------------------------------------------------------------
-// Treelet restructuring (Karras & Aila, HPG 2013), one bottom-up pass after
-// the refit: at every internal node N, once both of its subtrees are final,
-// a treelet of up to 7 leaves is grown from N's children by opening the
-// internal treelet leaf with the largest surface area (first on ties); a
-// dynamic program over the 2^7 subsets finds the topology with the least
-// total internal surface area, and the treelet is rewired that way if that
-// is strictly less than its current total.  Leaves keep their Morton slots,
-// N stays the treelet root, the treelet's internal nodes are reused in the
-// order they were opened and handed out in depth-first order of the new
+// Refit and treelet restructuring (Karras & Aila, HPG 2013) in one bottom-up
+// pass: at every internal node N, once both of its subtrees are final, its
+// box is made and a treelet of up to 7 leaves is grown from N's children by
+// opening the internal treelet leaf with the largest surface area (first on
+// ties); a dynamic program over the 2^7 subsets finds the topology with the
+// least total internal surface area, and the treelet is rewired that way if
+// that is strictly less than its current total.  Leaves keep their Morton
+// slots, N stays the treelet root, the treelet's internal nodes are reused in
+// the order they were opened and handed out in depth-first order of the new
 // topology.  Same arithmetic, same order as the host LBVH of the oracle, so
-// the tree stays bit-exact.  One thread per leaf walks up as in k_refit;
-// the second thread to reach a node restructures it.
+// the tree stays bit-exact.
+//
+// Small scenes are bound by the chain of dependent steps from a leaf to the
+// root, large ones by issue; both by the work of one treelet.  So a node's
+// record is read once (its box and its child words are the same 32 bytes),
+// the growth step is one load and one warp maximum, the 966 (subset,
+// partition) pairs of the program are spread over the lanes by subset size
+// (about 45 evaluations deep instead of 180), the rewired nodes are written
+// by a lane each, and a node whose children are both leaves needs no warp.
+// Whole builds against the earlier form (one lane a subset, a refit pass
+// before): 485 spheres 530 -> 204 us, 40k 904 -> 420, 300k 2229 -> 1228,
+// 1M 5725 -> 3285.
 // ---------------------------------------------------------------------------
 constexpr int kTreeletLeaves = 7;
+
+// The subsets of 7 entries with 2 .. 7 members, by size.
+struct SubsetTable {
+    uint8_t s[120];
+};
+constexpr SubsetTable make_subsets() {
+    SubsetTable t{};
+    int at = 0;
+    for (int k = 2; k <= kTreeletLeaves; ++k)
+        for (int S = 1; S < (1 << kTreeletLeaves); ++S) {
+            int c = 0;
+            for (int b = 0; b < kTreeletLeaves; ++b) c += S >> b & 1;
+            if (c == k) t.s[at++] = (uint8_t)S;
+        }
+    return t;
+}
+__device__ const SubsetTable kSubsets = make_subsets();
+// sizes 2, 3, 4, 5, 6, 7: 21, 35, 35, 21, 7, 1 subsets
+constexpr int kSub2 = 0, kSub3 = 21, kSub4 = 56, kSub5 = 91, kSub6 = 112;
 
 struct TBox {
     float lo[3], hi[3];
@@ -371,203 +400,297 @@ __device__ __forceinline__ float tbox_area(const TBox& b) {
     return 2.0f * ((dx * dy + dy * dz) + dz * dx);
 }
 
-__device__ __forceinline__ TBox tbox_of(const float4* nodes, const float4* leafbox, int32_t c) {
-    const float4 lo = (c & kLeaf) ? __ldcg(leafbox + 2 * (c & kSlotMask)) : __ldcg(nodes + 2 * c);
-    const float4 hi = (c & kLeaf) ? __ldcg(leafbox + 2 * (c & kSlotMask) + 1) : __ldcg(nodes + 2 * c + 1);
+__device__ __forceinline__ void tbox_add(TBox& u, const TBox& b) {
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        u.lo[ax] = fminf(u.lo[ax], b.lo[ax]);
+        u.hi[ax] = fmaxf(u.hi[ax], b.hi[ax]);
+    }
+}
+
+// An entry of a treelet: a child word, its box, and its own child words when
+// it is an internal node.
+struct TEntry {
     TBox b;
-    b.lo[0] = lo.x;
-    b.lo[1] = lo.y;
-    b.lo[2] = lo.z;
-    b.hi[0] = hi.x;
-    b.hi[1] = hi.y;
-    b.hi[2] = hi.z;
-    return b;
+    int32_t word, left, right;
+};
+
+__device__ __forceinline__ void tentry_load(TEntry& e, const float4* nodes, const float4* leafbox, int32_t word) {
+    const float4* src = (word & kLeaf) ? leafbox + 2 * (size_t)(word & kSlotMask) : nodes + 2 * (size_t)word;
+    const float4 lo = __ldcg(src), hi = __ldcg(src + 1);
+    e.word = word;
+    e.b.lo[0] = lo.x;
+    e.b.lo[1] = lo.y;
+    e.b.lo[2] = lo.z;
+    e.b.hi[0] = hi.x;
+    e.b.hi[1] = hi.y;
+    e.b.hi[2] = hi.z;
+    e.left = __float_as_int(lo.w);
+    e.right = __float_as_int(hi.w);
 }
 
-__device__ __forceinline__ int32_t child_word(const float4* nodes, int32_t p, int side) {
-    return __float_as_int(__ldcg(&nodes[2 * p + side].w));
+__device__ __forceinline__ bool word_ok(int32_t w, int n) {
+    return (w & kLeaf) ? (w & kSlotMask) < n : (uint32_t)w < (uint32_t)(n - 1);
 }
 
-// Restructures the treelet rooted at N with the whole warp.  The treelet's
-// entries are spread over lanes 0..6 (lane i holds entry i), so every
-// memory round trip serves all entries at once: the growth step reads the
-// open entries' boxes in parallel and picks the largest area (first on
-// ties) with a warp reduction; the DP's subsets of one size are shared out
-// over the lanes (each subset's cost computed exactly as a single thread
-// would: the same members in the same order, the same partition order and
-// tie rule); lane 0 rewires the treelet, and each rewired node's box is the
-// union of its subset's entry boxes (min / max are exact, so this equals
-// refitting it from its children).  Every lane of the warp calls it with
-// the same N.  cost / split: this warp's shared-memory DP tables.
-__device__ void restructure_treelet_warp(int32_t N, int n, float4* nodes, int32_t* parent_int,
-                                         int32_t* parent_leaf, const float4* leafbox, float* cost,
-                                         uint8_t* split) {
+// A warp's shared memory.
+struct TreeletSmem {
+    float4 box[kTreeletLeaves][2];
+    float area[1 << kTreeletLeaves];
+    float cost[1 << kTreeletLeaves];
+    uint8_t split[1 << kTreeletLeaves];
+};
+
+// One partition of S: cost of its two sides; kept when strictly less.
+__device__ __forceinline__ void try_partition(const TreeletSmem& T, int S, int P, float& bc, int& bp) {
+    const float c = T.cost[P] + T.cost[S ^ P];
+    if (c < bc) {
+        bc = c;
+        bp = P;
+    }
+}
+
+// The least partition of S by one lane: the side with the lowest member runs
+// over low | Q, Q the proper subsets of the rest, largest first.
+__device__ __forceinline__ void solve_subset(TreeletSmem& T, int S) {
+    const int low = S & -S, rest = S ^ low;
+    float bc = INFINITY;
+    int bp = 0;
+    for (int Q = (rest - 1) & rest;; Q = (Q - 1) & rest) {
+        try_partition(T, S, Q | low, bc, bp);
+        if (Q == 0) break;
+    }
+    T.cost[S] = T.area[S] + bc;
+    T.split[S] = (uint8_t)bp;
+}
+
+// Restructures the treelet rooted at N with the whole warp.  Lane `who` holds
+// N's two children in c0 and c1 and N's area.  Every lane calls it with the
+// same N.
+__device__ void restructure_treelet_warp(int32_t N, int n, int who, const TEntry& c0, const TEntry& c1, float area_n,
+                                         float4* nodes, int32_t* parent_int, int32_t* parent_leaf,
+                                         const float4* leafbox, TreeletSmem& T) {
+    constexpr uint32_t kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    int32_t internals[kTreeletLeaves - 1];
-    int nl = 2, ni = 0;
-    int32_t mine = lane < 2 ? child_word(nodes, N, lane) : 0;  // entry `lane` of the treelet
-    internals[ni++] = N;
-    bool bad = false;
+    // lane i < nl holds entry i, lane i < ni internal node i of the treelet
+    TEntry e;
+    {
+        const bool second = lane == 1;
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            const float l0 = __shfl_sync(kAll, c0.b.lo[ax], who), l1 = __shfl_sync(kAll, c1.b.lo[ax], who);
+            const float h0 = __shfl_sync(kAll, c0.b.hi[ax], who), h1 = __shfl_sync(kAll, c1.b.hi[ax], who);
+            e.b.lo[ax] = second ? l1 : l0;
+            e.b.hi[ax] = second ? h1 : h0;
+        }
+        const int32_t w0 = __shfl_sync(kAll, c0.word, who), w1 = __shfl_sync(kAll, c1.word, who);
+        const int32_t a0 = __shfl_sync(kAll, c0.left, who), a1 = __shfl_sync(kAll, c1.left, who);
+        const int32_t b0 = __shfl_sync(kAll, c0.right, who), b1 = __shfl_sync(kAll, c1.right, who);
+        e.word = second ? w1 : w0;
+        e.left = second ? a1 : a0;
+        e.right = second ? b1 : b0;
+    }
+    float current = 0.0f + __shfl_sync(kAll, area_n, who);  // the treelet's internal area, in the order opened
+    int32_t my_int = N;
+    int nl = 2, ni = 1;
+    float area = lane < 2 && !(e.word & kLeaf) ? tbox_area(e.b) : -1.0f;
     while (nl < kTreeletLeaves) {
-        float a = -1.0f;
-        if (lane < nl && !(mine & kLeaf)) a = tbox_area(tbox_of(nodes, leafbox, mine));
-        float ba = a;
-        int bi = lane;
-        for (int off = 16; off > 0; off >>= 1) {
-            const float oa = __shfl_xor_sync(0xffffffffu, ba, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-            if (oa > ba || (oa == ba && oi < bi)) {
-                ba = oa;
-                bi = oi;
-            }
+        const uint32_t key = area >= 0.0f ? __float_as_uint(area) + 1u : 0u;  // orders like the area
+        const uint32_t top = __reduce_max_sync(kAll, key);
+        if (top == 0u) break;  // no internal entry left
+        const int bi = __ffs(__ballot_sync(kAll, key == top)) - 1;
+        current = current + __uint_as_float(top - 1u);
+        const int32_t c = __shfl_sync(kAll, e.word, bi);
+        const int32_t left = __shfl_sync(kAll, e.left, bi), right = __shfl_sync(kAll, e.right, bi);
+        if (!word_ok(left, n) || !word_ok(right, n)) return;  // never for a sound tree
+        if (lane == ni) my_int = c;
+        ++ni;
+        if (lane == bi || lane == nl) {
+            tentry_load(e, nodes, leafbox, lane == bi ? left : right);
+            area = (e.word & kLeaf) ? -1.0f : tbox_area(e.b);
         }
-        if (ba < 0.0f) break;  // no internal entry left
-        const int32_t c = __shfl_sync(0xffffffffu, mine, bi);
-        if ((uint32_t)c >= (uint32_t)(n - 1)) {  // never for a sound tree
-            bad = true;
-            break;
-        }
-        internals[ni++] = c;
-        if (lane == bi) mine = child_word(nodes, c, 0);
-        if (lane == nl) mine = child_word(nodes, c, 1);
         ++nl;
     }
-    const bool my_bad = lane < nl && ((mine & kLeaf) ? (mine & kSlotMask) >= n : (uint32_t)mine >= (uint32_t)(n - 1));
-    if (__any_sync(0xffffffffu, my_bad)) bad = true;
-    if (bad || nl < 3) return;  // the same decision in every lane
+    if (nl < 3) return;  // the same decision in every lane
     const int full = (1 << nl) - 1;
-    TBox bx[kTreeletLeaves];
-    {
-        TBox b{};
-        if (lane < nl) b = tbox_of(nodes, leafbox, mine);
-        for (int i = 0; i < nl; ++i)
-            for (int ax = 0; ax < 3; ++ax) {
-                bx[i].lo[ax] = __shfl_sync(0xffffffffu, b.lo[ax], i);
-                bx[i].hi[ax] = __shfl_sync(0xffffffffu, b.hi[ax], i);
-            }
+    __syncwarp();  // the previous treelet's reads of T are done
+    if (lane < nl) {
+        T.box[lane][0] = make_float4(e.b.lo[0], e.b.lo[1], e.b.lo[2], 0.0f);
+        T.box[lane][1] = make_float4(e.b.hi[0], e.b.hi[1], e.b.hi[2], 0.0f);
+        T.cost[1 << lane] = 0.0f;
     }
-    for (int S = 1 + lane; S <= full; S += 32)
-        if ((S & (S - 1)) == 0) {
-            cost[S] = 0.0f;
-            split[S] = 0;
+    __syncwarp();
+    auto box_of = [&](int i) {
+        const float4 lo = T.box[i][0], hi = T.box[i][1];
+        return TBox{{lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}};
+    };
+    // areas of the subsets: the members among the first five from the lane's
+    // bits, then the four choices of the last two
+    {
+        TBox u{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+            if (i < nl && (lane >> i & 1)) tbox_add(u, box_of(i));
+        if (lane <= full && lane) T.area[lane] = tbox_area(u);
+        if (nl > 5) {
+            TBox v = u;
+            tbox_add(v, box_of(5));
+            T.area[32 | lane] = tbox_area(v);
+            if (nl > 6) {
+                tbox_add(u, box_of(6));
+                T.area[64 | lane] = tbox_area(u);
+                tbox_add(v, box_of(6));
+                T.area[96 | lane] = tbox_area(v);
+            }
         }
-    for (int k = 2; k <= nl; ++k) {
+    }
+    __syncwarp();
+    // subsets by size; those with entries the treelet does not have are skipped
+    if (lane < 21) {
+        const int S = kSubsets.s[kSub2 + lane];
+        if (S <= full) {
+            T.cost[S] = T.area[S] + 0.0f;
+            T.split[S] = (uint8_t)(S & -S);
+        }
+    }
+    __syncwarp();
+    for (int i = lane; i < 35; i += 32) {
+        const int S = kSubsets.s[kSub3 + i];
+        if (S <= full) solve_subset(T, S);
+    }
+    __syncwarp();
+    if (nl >= 4) {
+        for (int i = lane; i < 35; i += 32) {
+            const int S = kSubsets.s[kSub4 + i];
+            if (S <= full) solve_subset(T, S);
+        }
         __syncwarp();
-        for (int S = 1 + lane; S <= full; S += 32) {
-            if (__popc(S) != k) continue;
-            TBox u;
-            for (int ax = 0; ax < 3; ++ax) {
-                u.lo[ax] = INFINITY;
-                u.hi[ax] = -INFINITY;
-            }
-            for (int i = 0; i < nl; ++i)
-                if (S >> i & 1)
-                    for (int ax = 0; ax < 3; ++ax) {
-                        u.lo[ax] = fminf(u.lo[ax], bx[i].lo[ax]);
-                        u.hi[ax] = fmaxf(u.hi[ax], bx[i].hi[ax]);
-                    }
-            const float area = tbox_area(u);
-            const int low = S & -S, rest = S ^ low;
-            float bc = INFINITY;
-            int bp = 0;
-            for (int Q = (rest - 1) & rest;; Q = (Q - 1) & rest) {  // the subsets of rest but rest, largest first
-                const int P = Q | low;
-                const float c = cost[P] + cost[S ^ P];
-                if (c < bc) {
-                    bc = c;
-                    bp = P;
-                }
-                if (Q == 0) break;
-            }
-            cost[S] = area + bc;
-            split[S] = (uint8_t)bp;
+    }
+    if (nl >= 5) {
+        if (lane < 21) {
+            const int S = kSubsets.s[kSub5 + lane];
+            if (S <= full) solve_subset(T, S);
         }
+        __syncwarp();
     }
-    __syncwarp();
-    // the treelet's current internal area, summed in the same order as a
-    // single thread would (internals[0], [1], ...)
-    float my_area = 0.0f;
-    {
-        int32_t my_int = 0;
-        for (int i = 0; i < ni; ++i)
-            if (lane == i) my_int = internals[i];
-        if (lane < ni) my_area = tbox_area(tbox_of(nodes, leafbox, my_int));
-    }
-    float current = 0.0f;
-    for (int i = 0; i < ni; ++i) current = current + __shfl_sync(0xffffffffu, my_area, i);
-    const bool better = cost[full] < current;
-    int32_t L[kTreeletLeaves];
-    for (int i = 0; i < nl; ++i) L[i] = __shfl_sync(0xffffffffu, mine, i);
-    __syncwarp();
-    if (better && lane == 0) {
-        // order[i]: the subset of the i-th internal node in depth-first
-        // preorder; it is given internals[i]
-        int order[kTreeletLeaves - 1];
-        int no = 0;
-        {
-            int stack[kTreeletLeaves];
-            int sp = 0;
-            stack[sp++] = full;
-            while (sp > 0) {
-                const int S = stack[--sp];
-                if ((S & (S - 1)) == 0) continue;
-                order[no++] = S;
-                stack[sp++] = S ^ split[S];
-                stack[sp++] = split[S];
+    if (nl >= 6) {  // 7 subsets of 31 partitions: four lanes each
+        const int S = kSubsets.s[kSub6 + min(lane >> 2, 6)];
+        const int low = S & -S, rest = S ^ low;
+        float bc = INFINITY;
+        int bp = 0;
+        if (S <= full && lane < 28) {
+            int Q = rest;
+            for (int j = lane & 3; j >= 0; --j) Q = (Q - 1) & rest;
+            for (int i = lane & 3; i < 31; i += 4) {
+                try_partition(T, S, Q | low, bc, bp);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) Q = (Q - 1) & rest;
             }
         }
-        auto word = [&](int T) -> int32_t {
-            if ((T & (T - 1)) == 0) return L[__ffs(T) - 1];
-            for (int i = 0; i < no; ++i)
-                if (order[i] == T) return internals[i];
-            return internals[0];  // unreachable: every internal subset is in order[]
-        };
-        for (int i = 0; i < no; ++i) {
-            const int S = order[i];
-            const int32_t me = internals[i];
-            const int32_t l = word(split[S]), r = word(S ^ split[S]);
-            TBox u;
-            for (int ax = 0; ax < 3; ++ax) {
-                u.lo[ax] = INFINITY;
-                u.hi[ax] = -INFINITY;
+#pragma unroll
+        for (int off = 1; off <= 2; off <<= 1) {
+            const float oc = __shfl_xor_sync(kAll, bc, off);
+            const int op = __shfl_xor_sync(kAll, bp, off);
+            if (oc < bc || (oc == bc && op > bp)) {  // the first of equal ones: the largest side
+                bc = oc;
+                bp = op;
             }
-            for (int j = 0; j < nl; ++j)
-                if (S >> j & 1)
-                    for (int ax = 0; ax < 3; ++ax) {
-                        u.lo[ax] = fminf(u.lo[ax], bx[j].lo[ax]);
-                        u.hi[ax] = fmaxf(u.hi[ax], bx[j].hi[ax]);
-                    }
-            nodes[2 * me] = make_float4(u.lo[0], u.lo[1], u.lo[2], __int_as_float(l));
-            nodes[2 * me + 1] = make_float4(u.hi[0], u.hi[1], u.hi[2], __int_as_float(r));
-            if (l & kLeaf) parent_leaf[l & kSlotMask] = me;
-            else parent_int[l] = me;
-            if (r & kLeaf) parent_leaf[r & kSlotMask] = me;
-            else parent_int[r] = me;
         }
+        if (S <= full && lane < 28 && (lane & 3) == 0) {
+            T.cost[S] = T.area[S] + bc;
+            T.split[S] = (uint8_t)bp;
+        }
+        __syncwarp();
     }
-    // lane 0's rewiring is published before any lane moves on (the arrival
-    // atomics order it for the other warps)
-    __syncwarp();
-    __threadfence();
+    if (nl == 7) {  // 63 partitions of the whole set over the warp
+        float bc = INFINITY;
+        int bp = 0;
+        try_partition(T, full, ((62 - lane) << 1) | 1, bc, bp);
+        if (lane < 31) try_partition(T, full, ((30 - lane) << 1) | 1, bc, bp);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const float oc = __shfl_xor_sync(kAll, bc, off);
+            const int op = __shfl_xor_sync(kAll, bp, off);
+            if (oc < bc || (oc == bc && op > bp)) {
+                bc = oc;
+                bp = op;
+            }
+        }
+        if (lane == 0) {
+            T.cost[full] = T.area[full] + bc;
+            T.split[full] = (uint8_t)bp;
+        }
+        __syncwarp();
+    }
+    if (!(T.cost[full] < current)) return;
+    // order: byte i is the subset of the i-th internal node in depth-first
+    // preorder; it is given internal node i
+    unsigned long long order = 0, stack = (unsigned long long)full;
+    int no = 0;
+    while (stack) {
+        const int S = (int)(stack & 0xffu);
+        stack >>= 8;
+        order |= (unsigned long long)S << (8 * no++);
+        const int P = T.split[S], O = S ^ P;
+        if (O & (O - 1)) stack = stack << 8 | (unsigned)O;
+        if (P & (P - 1)) stack = stack << 8 | (unsigned)P;
+    }
+    const int S = lane < no ? (int)(order >> (8 * lane) & 0xffu) : full;
+    const int P = T.split[S], O = S ^ P;
+    auto word = [&](int X) -> int32_t {
+        int at = 0;  // the internal node that X is given
+        for (int i = 1; i < no; ++i)
+            if ((int)(order >> (8 * i) & 0xffu) == X) at = i;
+        const int32_t leaf_word = __shfl_sync(kAll, e.word, __ffs(X) - 1);
+        const int32_t int_word = __shfl_sync(kAll, my_int, at);
+        return (X & (X - 1)) == 0 ? leaf_word : int_word;
+    };
+    const int32_t l = word(P), r = word(O);
+    TBox u{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
+    for (int i = 0; i < nl; ++i)
+        if (S >> i & 1) tbox_add(u, box_of(i));
+    if (lane < no) {
+        const int32_t me = my_int;
+        nodes[2 * (size_t)me] = make_float4(u.lo[0], u.lo[1], u.lo[2], __int_as_float(l));
+        nodes[2 * (size_t)me + 1] = make_float4(u.hi[0], u.hi[1], u.hi[2], __int_as_float(r));
+        if (l & kLeaf) parent_leaf[l & kSlotMask] = me;
+        else parent_int[l] = me;
+        if (r & kLeaf) parent_leaf[r & kSlotMask] = me;
+        else parent_int[r] = me;
+    }
 }
 
-// One thread per leaf walks up as in k_refit; a node is restructured once
-// both of its subtrees are final, by the warp of the thread that arrived
-// second.  Every lane of a warp stays in the loop until none of them is
-// walking, so that it can help: the lanes that won a node in a round are
-// served one after another by the whole warp.
+// A warp starts from `per_warp` leaves (a power of two, at most 32), one a
+// lane; each walks up as in k_refit, and the lane that reaches a node second
+// makes its box from its final children.  Nodes that need restructuring are
+// then served one after another by the whole warp: the lanes stay in the
+// loop until none of them is walking.  Fewer leaves a warp make fewer nodes
+// to serve in turn (31 of them for 32 leaves) and more warps.
 constexpr int kTreeletBlock = 128;
-__global__ void __launch_bounds__(kTreeletBlock) k_treelets(int n, float4* nodes, int32_t* parent_int,
-                                                             int32_t* parent_leaf, const float4* __restrict__ leafbox,
-                                                             uint32_t* __restrict__ arrive) {
-    __shared__ float s_cost[kTreeletBlock / 32][1 << kTreeletLeaves];
-    __shared__ uint8_t s_split[kTreeletBlock / 32][1 << kTreeletLeaves];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int w = threadIdx.x >> 5;
-    int p = k < n ? parent_leaf[k] : -1;
-    bool walking = k < n;
+__global__ void __launch_bounds__(kTreeletBlock)
+    k_treelets(const venu_sphere* __restrict__ s, const uint32_t* __restrict__ ids, int n, int per_warp, float4* nodes,
+               int32_t* parent_int, int32_t* parent_leaf, float4* leafbox, uint32_t* __restrict__ arrive) {
+    __shared__ TreeletSmem smem[kTreeletBlock / 32];
+    TreeletSmem& T = smem[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const long long first = (long long)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp;
+    bool walking = lane < per_warp && first + lane < n;
+    int p = -1;
+    if (walking) {
+        const int k = (int)first + lane;
+        const venu_sphere& sp = s[ids[k]];
+        const float r = fabsf(sp.radius);
+        // as in k_refit: outwards, never a signed zero
+        leafbox[2 * (size_t)k] = make_float4(__fsub_rd(sp.center[0], r) + 0.0f, __fsub_rd(sp.center[1], r) + 0.0f,
+                                             __fsub_rd(sp.center[2], r) + 0.0f, 0.0f);
+        leafbox[2 * (size_t)k + 1] = make_float4(__fadd_ru(sp.center[0], r), __fadd_ru(sp.center[1], r),
+                                                 __fadd_ru(sp.center[2], r), 0.0f);
+        p = parent_leaf[k];
+    }
     for (int level = 0; level < 128; ++level) {
         bool want = false;
+        TEntry c0{}, c1{};
+        float area = 0.0f;
         if (walking) {
             if (p < 0 || p >= n - 1) {
                 walking = false;
@@ -577,15 +700,33 @@ __global__ void __launch_bounds__(kTreeletBlock) k_treelets(int n, float4* nodes
                     walking = false;  // the other subtree is not final yet
                 } else {
                     __threadfence();
-                    want = true;
+                    const int32_t w0 = __float_as_int(__ldcg(&nodes[2 * (size_t)p].w));
+                    const int32_t w1 = __float_as_int(__ldcg(&nodes[2 * (size_t)p + 1].w));
+                    if (word_ok(w0, n) && word_ok(w1, n)) {
+                        tentry_load(c0, nodes, leafbox, w0);
+                        tentry_load(c1, nodes, leafbox, w1);
+                        TBox u = c0.b;
+                        tbox_add(u, c1.b);
+                        nodes[2 * (size_t)p] = make_float4(u.lo[0], u.lo[1], u.lo[2], __int_as_float(w0));
+                        nodes[2 * (size_t)p + 1] = make_float4(u.hi[0], u.hi[1], u.hi[2], __int_as_float(w1));
+                        area = tbox_area(u);
+                        want = !(w0 & kLeaf) || !(w1 & kLeaf);
+                    } else {
+                        walking = false;  // never for a sound tree
+                    }
                 }
             }
         }
+        __syncwarp();
         for (uint32_t m = __ballot_sync(0xffffffffu, want); m; m &= m - 1u) {
-            const int32_t q = __shfl_sync(0xffffffffu, p, __ffs(m) - 1);
-            restructure_treelet_warp(q, n, nodes, parent_int, parent_leaf, leafbox, s_cost[w], s_split[w]);
+            const int who = __ffs(m) - 1;
+            const int32_t q = __shfl_sync(0xffffffffu, p, who);
+            restructure_treelet_warp(q, n, who, c0, c1, area, nodes, parent_int, parent_leaf, leafbox, T);
         }
-        if (want) p = __ldcg(parent_int + p);
+        // the rewiring by the other lanes comes before this lane's fence and
+        // arrival at the parent
+        __syncwarp();
+        if (walking) p = __ldcg(parent_int + p);
         if (!__any_sync(0xffffffffu, walking)) break;
     }
 }
@@ -952,6 +1093,17 @@ struct LbvhBuffers {
     float4* leafbox;
 };
 
+// Leaves a warp of k_treelets starts from: few while that still leaves warps
+// to spare (the nodes a warp serves in turn are then the chain that counts),
+// 32 once the whole GPU is busy.  Whole builds at 4 / 8 / 16 / 32: 485 spheres
+// 204 / 213 / 232 / 250 us, 40k 428 / 420 / 424 / 445, 100k 679 / 646 / 622 /
+// 602, 1M 4122 / 3736 / 3459 / 3285.
+uint32_t treelet_leaves_per_warp(uint32_t n) {
+    uint32_t per = 4;
+    while (per < 32u && n / per > 4096u) per *= 2;
+    return per;
+}
+
 // The whole build, asynchronously on `st`; both venu_scene_create and
 // venu_lbvh_build_noalloc run exactly this sequence.
 cudaError_t launch_lbvh(const venu_sphere* s, uint32_t n, cudaStream_t st, const LbvhBuffers& B) {
@@ -977,12 +1129,9 @@ cudaError_t launch_lbvh(const venu_sphere* s, uint32_t n, cudaStream_t st, const
     // four passes: the sorted codes / ids are back in B.keys / B.vals
     if (n > 1) {
         k_karras<<<cdiv(n - 1, 256), 256, 0, st>>>(B.keys, (int)n, B.nodes, B.pint, B.pleaf);
-        k_refit<<<cdiv(n, 256), 256, 0, st>>>(s, B.vals, 0xffffffffu, (int)n, B.nodes, B.pint, B.pleaf, B.leafbox,
-                                              B.arrive);
-        e = cudaMemsetAsync(B.arrive, 0, sizeof(uint32_t) * nint, st);
-        if (e != cudaSuccess) return e;
-        k_treelets<<<cdiv(n, kTreeletBlock), kTreeletBlock, 0, st>>>((int)n, B.nodes, B.pint, B.pleaf, B.leafbox,
-                                                                     B.arrive);
+        const uint32_t per_warp = treelet_leaves_per_warp(n);
+        k_treelets<<<cdiv(cdiv(n, per_warp), kTreeletBlock / 32), kTreeletBlock, 0, st>>>(
+            s, B.vals, (int)n, (int)per_warp, B.nodes, B.pint, B.pleaf, B.leafbox, B.arrive);
     }
     k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, B.vals, 0xffffffffu, n, B.sph, B.mat, B.meta);
     if (n > 1) {
