@@ -4,11 +4,13 @@
 //   1. centroid bounds (order-preserving integer atomics: exact min/max),
 //   2. 30-bit Morton codes of the centroids quantised to 10 bits per axis,
 //   3. stable LSD radix sort of (code, original index), 4 passes of 8 bits,
-//      one warp per 512-key tile, stable ranking with __match_any_sync,
+//      one warp per tile, stable ranking with __match_any_sync (small scenes:
+//      one block for 1 to 3, a bitonic sort),
 //   4. Karras 2012 hierarchy ("Maximizing Parallelism in the Construction of
 //      BVHs, Octrees, and k-d Trees"), ties on equal codes broken by index,
-//   5. bottom-up refit with per-node arrival counters; leaf boxes are the
-//      sphere AABBs rounded outward (__fsub_rd / __fadd_ru, |radius|),
+//   5. bottom-up refit with per-node arrival counters and treelet
+//      restructuring in one pass; leaf boxes are the sphere AABBs rounded
+//      outward (__fsub_rd / __fadd_ru, |radius|),
 //   6. gather of spheres and materials into Morton (slot) order.
 // Every step is integer work or exact float min/max, so the result is
 // bit-identical to a host build of the same algorithm.
@@ -17,6 +19,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -25,7 +28,7 @@
 namespace venu {
 namespace {
 
-constexpr int kTileKeys = 512;  // keys per warp tile
+constexpr int kMaxTileKeys = 512;  // keys per warp tile, at most (see sort_rounds)
 constexpr int kWarpsPerBlock = 8;
 constexpr int kRadixBits = 8;
 constexpr int kBuckets = 1 << kRadixBits;
@@ -53,6 +56,7 @@ struct LbvhCtl {
     HoistList hoisted;    // n <= kMaxHoisted, 0 if more than kHoistCandidates
     uint32_t hoist_buf[64];
     uint32_t bad_words;   // child words k_trav_layout had to replace (never, for a sound build)
+    uint32_t totals[4 * kBuckets];  // digits of all codes, per radix pass
 };
 constexpr uint32_t kHoistCandidates = 64;
 
@@ -65,8 +69,12 @@ __device__ __forceinline__ float huge_threshold(const uint32_t* b0) {
     return 0.25f * m;
 }
 
-__global__ void k_lbvh_init(LbvhCtl* c) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
+// What must start from a known value: the control block, the arrival counters
+// and the parent links.  One launch instead of four.
+__global__ void k_lbvh_init(LbvhCtl* c, uint32_t n, uint32_t nint, uint32_t* __restrict__ arrive,
+                            int32_t* __restrict__ pint, int32_t* __restrict__ pleaf) {
+    const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    if (i0 == 0) {
         for (int a = 0; a < 3; ++a) {
             c->b0[a] = 0xffffffffu;
             c->b0[3 + a] = 0u;
@@ -75,10 +83,21 @@ __global__ void k_lbvh_init(LbvhCtl* c) {
         c->hoisted.n = 0;
         c->bad_words = 0;
     }
+    for (uint32_t i = i0; i < 4u * kBuckets; i += step) c->totals[i] = 0u;
+    for (uint32_t i = i0; i < nint; i += step) {
+        arrive[i] = 0u;
+        pint[i] = -1;
+    }
+    for (uint32_t i = i0; i < n; i += step) pleaf[i] = -1;
 }
 
-// Centroid bounds (exact min/max through order-preserving integer atomics).
-__global__ void k_bounds(const venu_sphere* __restrict__ s, uint32_t n, uint32_t* __restrict__ bu) {
+// Centroid bounds (exact min/max through order-preserving integer atomics,
+// one set a block: a set a warp kept 300k spheres' launch at 40 us).
+__global__ void __launch_bounds__(256) k_bounds(const venu_sphere* __restrict__ s, uint32_t n,
+                                                uint32_t* __restrict__ bu) {
+    __shared__ uint32_t ends[6];
+    if (threadIdx.x < 6) ends[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
+    __syncthreads();
     uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0, 0, 0};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 #pragma unroll
@@ -90,19 +109,15 @@ __global__ void k_bounds(const venu_sphere* __restrict__ s, uint32_t n, uint32_t
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            lo[a] = min(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
-            hi[a] = max(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+        const uint32_t l = __reduce_min_sync(0xffffffffu, lo[a]), h = __reduce_max_sync(0xffffffffu, hi[a]);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&ends[a], l);
+            atomicMax(&ends[3 + a], h);
         }
     }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(bu + a, lo[a]);
-            atomicMax(bu + 3 + a, hi[a]);
-        }
-    }
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMin(bu + threadIdx.x, ends[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(bu + threadIdx.x, ends[threadIdx.x]);
 }
 
 // Karras's bit spreading: bit i of v goes to bit 3i.
@@ -127,8 +142,12 @@ __device__ __forceinline__ uint32_t quant10(float c, float lo, float ext) {
 // instead of its thin axis being stretched over 1024 levels.  (Measured on
 // the oracle: 27 % fewer box tests per segment on a 200 000-sphere scene and
 // 18 % on 1 M spheres than per-axis scaling, equal on the RTIOW scene.)
-__global__ void k_morton(const venu_sphere* __restrict__ s, uint32_t n, LbvhCtl* c, uint32_t* __restrict__ keys,
-                         uint32_t* __restrict__ vals) {
+// Also counts the digits of each radix pass (the same for all orders).
+__global__ void __launch_bounds__(256) k_morton(const venu_sphere* __restrict__ s, uint32_t n, LbvhCtl* c,
+                                                uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+    __shared__ uint32_t digits[4 * kBuckets];
+    for (int i = threadIdx.x; i < 4 * kBuckets; i += blockDim.x) digits[i] = 0u;
+    __syncthreads();
     const uint32_t* bu = c->b0;
     float lo[3], ext = 0.0f;
 #pragma unroll
@@ -145,19 +164,84 @@ __global__ void k_morton(const venu_sphere* __restrict__ s, uint32_t n, LbvhCtl*
         uint32_t qx = quant10(s[i].center[0], lo[0], ext);
         uint32_t qy = quant10(s[i].center[1], lo[1], ext);
         uint32_t qz = quant10(s[i].center[2], lo[2], ext);
-        keys[i] = (spread10(qx) << 2) | (spread10(qy) << 1) | spread10(qz);
+        const uint32_t key = (spread10(qx) << 2) | (spread10(qy) << 1) | spread10(qz);
+        keys[i] = key;
         vals[i] = i;
+#pragma unroll
+        for (int d = 0; d < 4; ++d) atomicAdd(&digits[d * kBuckets + ((key >> (8 * d)) & (kBuckets - 1))], 1u);
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 4 * kBuckets; i += blockDim.x)
+        if (digits[i]) atomicAdd(&c->totals[i], digits[i]);
 }
 
-// Huge spheres in slot order -> candidates (unordered, at most 64).
-__global__ void k_hoist_collect(const float4* __restrict__ sph, uint32_t n, LbvhCtl* c) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const float thr = huge_threshold(c->b0);
-    if (fabsf(sph[k].w) > thr) {
-        const uint32_t i = atomicAdd(&c->hoist_cnt, 1u);
-        if (i < kHoistCandidates) c->hoist_buf[i] = k;
+// Bounds, codes and sort of a small scene in one block (in place of 15
+// launches, each of which costs more than its work here): a bitonic sort of
+// (code, index) pairs in shared memory, whose order is that of the stable
+// sort by code.  Builds of 485 / 2000 / 4000 spheres with it 134 / 178 / 207 us;
+// 485 and 2000 through the general path 204 / 254.
+constexpr uint32_t kSmallScene = 4096;
+__global__ void __launch_bounds__(1024) k_small_codes(const venu_sphere* __restrict__ s, uint32_t n, uint32_t n2,
+                                                      LbvhCtl* c, uint32_t* __restrict__ keys,
+                                                      uint32_t* __restrict__ vals) {
+    __shared__ unsigned long long pair[kSmallScene];
+    __shared__ uint32_t ends[6];
+    const uint32_t t = threadIdx.x, nt = blockDim.x;
+    if (t < 6) ends[t] = t < 3 ? 0xffffffffu : 0u;
+    __syncthreads();
+    uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0, 0, 0};
+    for (uint32_t i = t; i < n; i += nt)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const uint32_t u = f2u(s[i].center[a]);
+            lo[a] = min(lo[a], u);
+            hi[a] = max(hi[a], u);
+        }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const uint32_t l = __reduce_min_sync(0xffffffffu, lo[a]), h = __reduce_max_sync(0xffffffffu, hi[a]);
+        if ((t & 31u) == 0) {
+            atomicMin(&ends[a], l);
+            atomicMax(&ends[3 + a], h);
+        }
+    }
+    __syncthreads();
+    float base[3], ext = 0.0f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        base[a] = u2f(ends[a]);
+        ext = fmaxf(ext, u2f(ends[3 + a]) - base[a]);
+    }
+    if (t < 6) {
+        c->b0[t] = ends[t];
+        c->bounds[t] = u2f(ends[t]);
+    }
+    for (uint32_t i = t; i < n2; i += nt) {
+        unsigned long long v = ~0ull;
+        if (i < n) {
+            const uint32_t qx = quant10(s[i].center[0], base[0], ext);
+            const uint32_t qy = quant10(s[i].center[1], base[1], ext);
+            const uint32_t qz = quant10(s[i].center[2], base[2], ext);
+            v = (unsigned long long)((spread10(qx) << 2) | (spread10(qy) << 1) | spread10(qz)) << 32 | i;
+        }
+        pair[i] = v;
+    }
+    for (uint32_t k = 2; k <= n2; k <<= 1)
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            __syncthreads();
+            for (uint32_t q = t; q < n2 / 2; q += nt) {
+                const uint32_t i = (q & ~(j - 1u)) << 1 | (q & (j - 1u));
+                const unsigned long long x = pair[i], y = pair[i + j];
+                if ((x > y) == ((i & k) == 0u)) {
+                    pair[i] = y;
+                    pair[i + j] = x;
+                }
+            }
+        }
+    __syncthreads();
+    for (uint32_t i = t; i < n; i += nt) {
+        keys[i] = (uint32_t)(pair[i] >> 32);
+        vals[i] = (uint32_t)pair[i];
     }
 }
 
@@ -196,7 +280,7 @@ __global__ void k_hoist_finalize(LbvhCtl* c, const int32_t* __restrict__ pleaf, 
 }
 
 // Per-tile digit histogram, digit-major: hist[d * ntiles + tile].
-__global__ void k_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift, uint32_t ntiles,
+__global__ void k_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift, uint32_t ntiles, uint32_t rounds,
                        uint32_t* __restrict__ hist) {
     __shared__ uint32_t cnt[kWarpsPerBlock][kBuckets];
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -204,8 +288,8 @@ __global__ void k_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift,
     for (int d = lane; d < kBuckets; d += 32) cnt[w][d] = 0;
     __syncwarp();
     if (tile < ntiles) {
-        for (int j = 0; j < kTileKeys / 32; ++j) {
-            uint32_t idx = tile * kTileKeys + j * 32 + lane;
+        for (uint32_t j = 0; j < rounds; ++j) {
+            uint32_t idx = (tile * rounds + j) * 32 + lane;
             if (idx < n) atomicAdd(&cnt[w][(keys[idx] >> shift) & (kBuckets - 1)], 1u);
         }
         __syncwarp();
@@ -237,9 +321,45 @@ __global__ void k_scan(uint32_t* __restrict__ a, uint32_t total) {
     }
 }
 
+// The radix pass's offsets: block d turns row d of the tile histogram into
+// where each tile's keys of digit d go, from the digit totals and a scan of
+// its row.  (One block scanning all 256 x ntiles counters took 17 us of a 40k
+// build and 129 us of a 300k one, per pass.)
+__global__ void __launch_bounds__(256) k_scan_rows(uint32_t* __restrict__ hist, uint32_t ntiles,
+                                                   const uint32_t* __restrict__ totals) {
+    __shared__ uint32_t part[8], below[8];
+    const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5, d = blockIdx.x;
+    uint32_t* const row = hist + (size_t)d * ntiles;
+    const uint32_t per = (ntiles + 255u) / 256u;
+    const uint32_t b = min(ntiles, t * per), e = min(ntiles, b + per);
+    uint32_t sum = 0;
+    for (uint32_t i = b; i < e; ++i) sum += row[i];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= (uint32_t)off) incl += v;
+    }
+    const uint32_t under = __reduce_add_sync(0xffffffffu, t < d ? totals[t] : 0u);
+    if (lane == 31) part[w] = incl;
+    if (lane == 0) below[w] = under;
+    __syncthreads();
+    uint32_t run = incl - sum;
+#pragma unroll
+    for (uint32_t v = 0; v < 8; ++v) {
+        run += below[v];
+        if (v < w) run += part[v];
+    }
+    for (uint32_t i = b; i < e; ++i) {
+        const uint32_t v = row[i];
+        row[i] = run;
+        run += v;
+    }
+}
+
 // Stable scatter: keys of a tile are ranked in tile order within their digit.
 __global__ void k_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t n,
-                          int shift, uint32_t ntiles, const uint32_t* __restrict__ offs,
+                          int shift, uint32_t ntiles, uint32_t rounds, const uint32_t* __restrict__ offs,
                           uint32_t* __restrict__ kout, uint32_t* __restrict__ vout) {
     __shared__ uint32_t base[kWarpsPerBlock][kBuckets];
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -248,8 +368,8 @@ __global__ void k_scatter(const uint32_t* __restrict__ kin, const uint32_t* __re
     for (int d = lane; d < kBuckets; d += 32) base[w][d] = offs[(size_t)d * ntiles + tile];
     __syncwarp();
     const uint32_t lt = (1u << lane) - 1u;
-    for (int j = 0; j < kTileKeys / 32; ++j) {
-        uint32_t idx = tile * kTileKeys + j * 32 + lane;
+    for (uint32_t j = 0; j < rounds; ++j) {
+        uint32_t idx = (tile * rounds + j) * 32 + lane;
         bool valid = idx < n;
         uint32_t k = valid ? kin[idx] : 0u;
         uint32_t d = valid ? ((k >> shift) & (kBuckets - 1)) : (uint32_t)kBuckets + lane;
@@ -303,9 +423,18 @@ __global__ void k_karras(const uint32_t* __restrict__ keys, int n, float4* __res
     if (i == 0) parent_int[0] = -1;
 }
 
-// Leaf boxes + bottom-up refit.  The second thread to arrive at a node
-// computes its box; a __threadfence before each arrival publishes the
-// children's boxes, and they are read back through L2 (__ldcg).
+// Arrival at a node: publishes what this thread (and, before a __syncwarp,
+// its warp) has written, and sees what the earlier arrival published.
+__device__ __forceinline__ uint32_t arrive_acq_rel(uint32_t* counter) {
+    uint32_t old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
+    return old;
+}
+
+// Leaf boxes + bottom-up refit of moved spheres.  The second thread to
+// arrive at a node computes its box; the arrivals publish the children's
+// boxes, which are read back through L2 (__ldcg).  The tree itself does not
+// change, so a node's child words and parent are read beside its arrival.
 // ids[k] & id_mask = original index of the sphere in slot k (the sorted
 // values during a build, the meta words during a refit of moved spheres).
 // Leaf words may carry the hoisted flag (refit after a build).
@@ -328,11 +457,10 @@ __global__ void k_refit(const venu_sphere* __restrict__ s, const uint32_t* __res
     // A Karras tree over unique (code, index) keys is at most 63 levels deep;
     // the bound only guards against a corrupt parent chain.
     for (int level = 0; p >= 0 && p < n - 1 && level < 128; ++level) {
-        __threadfence();
-        if (atomicAdd(arrive + p, 1u) == 0u) return;
-        __threadfence();
-        int32_t cl = __float_as_int(__ldcg(&nodes[2 * p].w));
-        int32_t cr = __float_as_int(__ldcg(&nodes[2 * p + 1].w));
+        const int32_t cl = __float_as_int(__ldcg(&nodes[2 * p].w));
+        const int32_t cr = __float_as_int(__ldcg(&nodes[2 * p + 1].w));
+        const int32_t up = parent_int[p];
+        if (arrive_acq_rel(arrive + p) == 0u) return;
         const bool ok_l = (cl & kLeaf) ? (cl & kSlotMask) < n : cl < n - 1;
         const bool ok_r = (cr & kLeaf) ? (cr & kSlotMask) < n : cr < n - 1;
         if (!ok_l || !ok_r) return;
@@ -342,7 +470,7 @@ __global__ void k_refit(const venu_sphere* __restrict__ s, const uint32_t* __res
         float4 h1 = (cr & kLeaf) ? __ldcg(leafbox + 2 * (cr & kSlotMask) + 1) : __ldcg(nodes + 2 * cr + 1);
         nodes[2 * p] = make_float4(fminf(l0.x, l1.x), fminf(l0.y, l1.y), fminf(l0.z, l1.z), __int_as_float(cl));
         nodes[2 * p + 1] = make_float4(fmaxf(h0.x, h1.x), fmaxf(h0.y, h1.y), fmaxf(h0.z, h1.z), __int_as_float(cr));
-        p = parent_int[p];
+        p = up;
     }
 }
 
@@ -689,19 +817,21 @@ __global__ void __launch_bounds__(kTreeletBlock)
     }
     for (int level = 0; level < 128; ++level) {
         bool want = false;
+        int up = -1;
         TEntry c0{}, c1{};
         float area = 0.0f;
         if (walking) {
             if (p < 0 || p >= n - 1) {
                 walking = false;
             } else {
-                __threadfence();
-                if (atomicAdd(arrive + p, 1u) == 0u) {
+                // p's child words and its parent stay what they are until p is
+                // restructured, or an ancestor: read beside the arrival
+                const int32_t w0 = __float_as_int(__ldcg(&nodes[2 * (size_t)p].w));
+                const int32_t w1 = __float_as_int(__ldcg(&nodes[2 * (size_t)p + 1].w));
+                up = __ldcg(parent_int + p);
+                if (arrive_acq_rel(arrive + p) == 0u) {
                     walking = false;  // the other subtree is not final yet
                 } else {
-                    __threadfence();
-                    const int32_t w0 = __float_as_int(__ldcg(&nodes[2 * (size_t)p].w));
-                    const int32_t w1 = __float_as_int(__ldcg(&nodes[2 * (size_t)p + 1].w));
                     if (word_ok(w0, n) && word_ok(w1, n)) {
                         tentry_load(c0, nodes, leafbox, w0);
                         tentry_load(c1, nodes, leafbox, w1);
@@ -723,19 +853,20 @@ __global__ void __launch_bounds__(kTreeletBlock)
             const int32_t q = __shfl_sync(0xffffffffu, p, who);
             restructure_treelet_warp(q, n, who, c0, c1, area, nodes, parent_int, parent_leaf, leafbox, T);
         }
-        // the rewiring by the other lanes comes before this lane's fence and
+        // the rewiring by the other lanes comes before this lane's releasing
         // arrival at the parent
         __syncwarp();
-        if (walking) p = __ldcg(parent_int + p);
+        p = up;
         if (!__any_sync(0xffffffffu, walking)) break;
     }
 }
 
 // Slot-ordered sphere / material / meta records.  ids may alias meta (a
 // refit regathers from the meta words): each thread reads its slot's word
-// before writing it.
+// before writing it.  c (builds only): huge spheres become candidates for
+// hoisting (unordered, at most 64).
 __global__ void k_gather(const venu_sphere* __restrict__ s, const uint32_t* ids, uint32_t id_mask, uint32_t n,
-                         float4* __restrict__ sph, float4* __restrict__ mat, uint32_t* meta) {
+                         float4* __restrict__ sph, float4* __restrict__ mat, uint32_t* meta, LbvhCtl* c) {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     uint32_t id = ids[k] & id_mask;
@@ -745,6 +876,10 @@ __global__ void k_gather(const venu_sphere* __restrict__ s, const uint32_t* ids,
     float param = type == 1u ? sp.fuzz : (type == 2u ? sp.ir : 0.0f);
     mat[k] = make_float4(sp.albedo[0], sp.albedo[1], sp.albedo[2], param);
     meta[k] = id | (type << 30);
+    if (c && fabsf(sp.radius) > huge_threshold(c->b0)) {
+        const uint32_t i = atomicAdd(&c->hoist_cnt, 1u);
+        if (i < kHoistCandidates) c->hoist_buf[i] = k;
+    }
 }
 
 // Box of a leaf: the sphere's box rounded outwards (as k_refit makes it).
@@ -1093,6 +1228,10 @@ struct LbvhBuffers {
     float4* leafbox;
 };
 
+// Keys per lane of a sort tile (a warp's): short tiles while that still
+// spreads the keys over the SMs.
+uint32_t sort_rounds(uint32_t n) { return n <= 65536u ? 4u : n <= 262144u ? 8u : (uint32_t)kMaxTileKeys / 32u; }
+
 // Leaves a warp of k_treelets starts from: few while that still leaves warps
 // to spare (the nodes a warp serves in turn are then the chain that counts),
 // 32 once the whole GPU is busy.  Whole builds at 4 / 8 / 16 / 32: 485 spheres
@@ -1108,34 +1247,38 @@ uint32_t treelet_leaves_per_warp(uint32_t n) {
 // venu_lbvh_build_noalloc run exactly this sequence.
 cudaError_t launch_lbvh(const venu_sphere* s, uint32_t n, cudaStream_t st, const LbvhBuffers& B) {
     const uint32_t nint = n > 1 ? n - 1 : 1;
-    const uint32_t ntiles = cdiv(n, kTileKeys);
-    k_lbvh_init<<<1, 32, 0, st>>>(B.ctl);
-    cudaError_t e = cudaMemsetAsync(B.arrive, 0, sizeof(uint32_t) * nint, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(B.pint, 0xff, sizeof(int32_t) * nint, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(B.pleaf, 0xff, sizeof(int32_t) * n, st);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
     const uint32_t blocks = std::min(cdiv(n, 256), (uint32_t)(sm_count() * 8));
-    k_bounds<<<blocks, 256, 0, st>>>(s, n, B.ctl->b0);
-    k_morton<<<blocks, 256, 0, st>>>(s, n, B.ctl, B.keys, B.vals);
-    uint32_t *kin = B.keys, *kout = B.keys_alt, *vin = B.vals, *vout = B.vals_alt;
-    const uint32_t sblocks = cdiv(ntiles, kWarpsPerBlock);
-    for (int shift = 0; shift < 32; shift += kRadixBits) {
-        k_hist<<<sblocks, 32 * kWarpsPerBlock, 0, st>>>(kin, n, shift, ntiles, B.hist);
-        k_scan<<<1, 1024, 0, st>>>(B.hist, kBuckets * ntiles);
-        k_scatter<<<sblocks, 32 * kWarpsPerBlock, 0, st>>>(kin, vin, n, shift, ntiles, B.hist, kout, vout);
-        std::swap(kin, kout);
-        std::swap(vin, vout);
+    k_lbvh_init<<<blocks, 256, 0, st>>>(B.ctl, n, nint, B.arrive, B.pint, B.pleaf);
+    if (n <= kSmallScene) {
+        uint32_t n2 = 64;
+        while (n2 < n) n2 *= 2;
+        k_small_codes<<<1, std::min(n2 / 2, 1024u), 0, st>>>(s, n, n2, B.ctl, B.keys, B.vals);
+    } else {
+        const uint32_t few = std::min(cdiv(n, 256), (uint32_t)(sm_count() * 2));  // each block ends with atomics
+        k_bounds<<<few, 256, 0, st>>>(s, n, B.ctl->b0);
+        k_morton<<<few, 256, 0, st>>>(s, n, B.ctl, B.keys, B.vals);
+        uint32_t *kin = B.keys, *kout = B.keys_alt, *vin = B.vals, *vout = B.vals_alt;
+        const uint32_t rounds = sort_rounds(n), ntiles = cdiv(n, 32 * rounds);
+        const uint32_t sblocks = cdiv(ntiles, kWarpsPerBlock);
+        for (int pass = 0; pass < 4; ++pass) {
+            const int shift = pass * kRadixBits;
+            k_hist<<<sblocks, 32 * kWarpsPerBlock, 0, st>>>(kin, n, shift, ntiles, rounds, B.hist);
+            k_scan_rows<<<kBuckets, 256, 0, st>>>(B.hist, ntiles, B.ctl->totals + pass * kBuckets);
+            k_scatter<<<sblocks, 32 * kWarpsPerBlock, 0, st>>>(kin, vin, n, shift, ntiles, rounds, B.hist, kout, vout);
+            std::swap(kin, kout);
+            std::swap(vin, vout);
+        }
+        // four passes: the sorted codes / ids are back in B.keys / B.vals
     }
-    // four passes: the sorted codes / ids are back in B.keys / B.vals
     if (n > 1) {
         k_karras<<<cdiv(n - 1, 256), 256, 0, st>>>(B.keys, (int)n, B.nodes, B.pint, B.pleaf);
         const uint32_t per_warp = treelet_leaves_per_warp(n);
         k_treelets<<<cdiv(cdiv(n, per_warp), kTreeletBlock / 32), kTreeletBlock, 0, st>>>(
             s, B.vals, (int)n, (int)per_warp, B.nodes, B.pint, B.pleaf, B.leafbox, B.arrive);
     }
-    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, B.vals, 0xffffffffu, n, B.sph, B.mat, B.meta);
+    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, B.vals, 0xffffffffu, n, B.sph, B.mat, B.meta, n > 1 ? B.ctl : nullptr);
     if (n > 1) {
-        k_hoist_collect<<<cdiv(n, 256), 256, 0, st>>>(B.sph, n, B.ctl);
         k_hoist_finalize<<<1, 32, 0, st>>>(B.ctl, B.pleaf, B.nodes, n);
         if (B.trav) {
             e = launch_trav_layout(B.nodes, B.sph, n, B.trav, B.pint, B.pleaf, &B.ctl->hoisted, HoistList{},
@@ -1246,7 +1389,7 @@ venu_status build_scene(const venu_sphere* spheres_dev, uint32_t n, cudaStream_t
         set_error("venu_scene_create: more than 2^28 spheres");
         return VENU_ERR_TOO_LARGE;
     }
-    const uint32_t ntiles = cdiv(n, kTileKeys);
+    const uint32_t ntiles = cdiv(n, 32 * sort_rounds(n));
     const size_t hist_n = (size_t)kBuckets * ntiles;
     size_t bytes = 0;
     auto alloc = [&](void** p, size_t b) -> cudaError_t {
@@ -1294,7 +1437,7 @@ venu_status build_scene(const venu_sphere* spheres_dev, uint32_t n, cudaStream_t
     STEP(cudaEventRecord(e0, st));
     STEP(launch_lbvh(spheres_dev, n, st, B));
     STEP(cudaEventRecord(e1, st));
-    STEP(cudaMemcpyAsync(&hc, B.ctl, sizeof(LbvhCtl), cudaMemcpyDeviceToHost, st));
+    STEP(cudaMemcpyAsync(&hc, B.ctl, offsetof(LbvhCtl, totals), cudaMemcpyDeviceToHost, st));
     STEP(cudaStreamSynchronize(st));
     {
         float ms = 0.0f;
@@ -1349,7 +1492,8 @@ venu_status update_scene(venu_scene* S, const venu_sphere* s, cudaStream_t st) {
     // original index), then the boxes bottom-up over the kept parent links,
     // then the traversal records.  Topology, slot order and the hoisted set
     // stay those of the build.
-    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, S->meta, 0x3fffffffu, n, S->sph, S->mat, S->meta);
+    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, S->meta, 0x3fffffffu, n, S->sph, S->mat, S->meta,
+                                           nullptr);
     VENU_CUDA(cudaGetLastError());
     if (n == 1) return VENU_OK;
     float4* leafbox = nullptr;
@@ -1384,7 +1528,8 @@ namespace venu {
 namespace {
 
 constexpr uint32_t kNoAllocMaxSpheres = VENU_NOALLOC_MAX_SPHERES;
-constexpr uint32_t kNoAllocMaxTiles = (kNoAllocMaxSpheres + kTileKeys - 1) / kTileKeys;
+constexpr uint32_t kNoAllocMaxTiles = (kNoAllocMaxSpheres + 127) / 128;  // sort_rounds: 128 keys a tile
+static_assert(kNoAllocMaxSpheres <= 65536, "sort_rounds gives tiles of 128 keys up to 65536 spheres");
 constexpr size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr size_t kNA = kNoAllocMaxSpheres;
 constexpr size_t kOffCtl = 0;                                         // LbvhCtl
@@ -1396,7 +1541,7 @@ constexpr size_t kOffArrive = al256(kOffHist + 4 * (size_t)kBuckets * kNoAllocMa
 constexpr size_t kOffParentInt = al256(kOffArrive + 4 * kNA);
 constexpr size_t kOffParentLeaf = al256(kOffParentInt + 4 * kNA);
 constexpr size_t kOffLeafBox = al256(kOffParentLeaf + 4 * kNA);
-constexpr size_t kNoAllocScratchBytes = al256(kOffLeafBox + 32 * kNA);  // about 3.8 MB
+constexpr size_t kNoAllocScratchBytes = al256(kOffLeafBox + 32 * kNA);  // about 4.2 MB
 
 }  // namespace
 }  // namespace venu
