@@ -205,7 +205,7 @@ VENU_API venu_status venu_scene_destroy(venu_scene* scene);
  * venu_scene_create into buffers the caller owns, asynchronously on
  * `stream`, and calls no cudaMalloc, cudaFree or other allocating routine.
  *
- * Scratch lives in one fixed device array inside the library (about 4.2 MB
+ * Scratch lives in one fixed device array inside the library (about 2.1 MB
  * for VENU_NOALLOC_MAX_SPHERES spheres), which every GPU that loads the
  * library holds until the process exits.  n above VENU_NOALLOC_MAX_SPHERES
  * returns VENU_ERR_TOO_LARGE.  The first call on a device looks up that

@@ -356,9 +356,9 @@ extern "C" venu_status venu_image_write_pfm(const char* path, const float* rgba3
     return VENU_OK;
 }
 
-extern "C" venu_status venu_scene_create_device(const venu_sphere* spheres_dev, uint32_t n, void* stream,
-                                                venu_scene** out) {
-    if (!out || (!spheres_dev && n)) {
+namespace {
+venu_status create_scene(const venu_sphere* spheres, bool on_host, uint32_t n, void* stream, venu_scene** out) {
+    if (!out || (!spheres && n)) {
         set_error("venu_scene_create: NULL argument");
         return VENU_ERR_INVALID;
     }
@@ -366,7 +366,7 @@ extern "C" venu_status venu_scene_create_device(const venu_sphere* spheres_dev, 
     venu_status ds = require_device();
     if (ds != VENU_OK) return ds;
     venu_scene* s = new venu_scene();
-    venu_status rc = build_scene(spheres_dev, n, reinterpret_cast<cudaStream_t>(stream), s);
+    venu_status rc = build_scene(spheres, on_host, n, reinterpret_cast<cudaStream_t>(stream), s);
     if (rc != VENU_OK) {
         free_scene(s);
         delete s;
@@ -375,30 +375,16 @@ extern "C" venu_status venu_scene_create_device(const venu_sphere* spheres_dev, 
     *out = s;
     return VENU_OK;
 }
+}  // namespace
+
+extern "C" venu_status venu_scene_create_device(const venu_sphere* spheres_dev, uint32_t n, void* stream,
+                                                venu_scene** out) {
+    return create_scene(spheres_dev, false, n, stream, out);
+}
 
 extern "C" venu_status venu_scene_create(const venu_sphere* spheres_host, uint32_t n, void* stream,
                                          venu_scene** out) {
-    if (!out || (!spheres_host && n)) {
-        set_error("venu_scene_create: NULL argument");
-        return VENU_ERR_INVALID;
-    }
-    *out = nullptr;
-    venu_status ds = require_device();
-    if (ds != VENU_OK) return ds;
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    venu_sphere* d = nullptr;
-    if (n) {
-        VENU_CUDA(cudaMalloc(&d, sizeof(venu_sphere) * n));
-        cudaError_t e = cudaMemcpyAsync(d, spheres_host, sizeof(venu_sphere) * n, cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) {
-            cudaFree(d);
-            return cuda_fail(e, "venu_scene_create: upload");
-        }
-    }
-    venu_status rc = venu_scene_create_device(d, n, stream, out);
-    cudaStreamSynchronize(st);
-    cudaFree(d);
-    return rc;
+    return create_scene(spheres_host, true, n, stream, out);
 }
 
 extern "C" venu_status venu_scene_update_device(venu_scene* scene, const venu_sphere* spheres_dev, uint32_t n,
@@ -414,7 +400,7 @@ extern "C" venu_status venu_scene_update_device(venu_scene* scene, const venu_sp
     }
     venu_status ds = require_device();
     if (ds != VENU_OK) return ds;
-    return update_scene(scene, spheres_dev, reinterpret_cast<cudaStream_t>(stream));
+    return update_scene(scene, spheres_dev, false, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" venu_status venu_scene_update(venu_scene* scene, const venu_sphere* spheres_host, uint32_t n,
@@ -428,11 +414,7 @@ extern "C" venu_status venu_scene_update(venu_scene* scene, const venu_sphere* s
     if (ds != VENU_OK) return ds;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (n == 0) return VENU_OK;
-    venu_sphere* d = nullptr;
-    VENU_CUDA(cudaMallocAsync(&d, sizeof(venu_sphere) * n, st));
-    cudaError_t e = cudaMemcpyAsync(d, spheres_host, sizeof(venu_sphere) * n, cudaMemcpyHostToDevice, st);
-    venu_status rc = e == cudaSuccess ? update_scene(scene, d, st) : cuda_fail(e, "venu_scene_update: upload");
-    cudaFreeAsync(d, st);
+    venu_status rc = update_scene(scene, spheres_host, true, st);
     cudaError_t se = cudaStreamSynchronize(st);
     if (rc == VENU_OK && se != cudaSuccess) rc = cuda_fail(se, "venu_scene_update");
     return rc;

@@ -464,6 +464,7 @@ struct venu_batch {
     bool order_dirty = false;     // b->order changed since it was last uploaded (at the next run)
     uint32_t chunk = 0;  // rays traced per step (0: a whole iteration per step)
     uint64_t next_seq = 0;
+    DevPool mem;                      // job buffers
     uint32_t* h_interrupt = nullptr;  // mapped host word
     uint32_t* d_interrupt = nullptr;  // its device address
     venu_tuning tune = {2u, 8u, 256u, 0u, 256u, 0u, 1u};
@@ -536,6 +537,7 @@ venu_status build_graph(venu_batch* b) {
 void free_batch(venu_batch* b) {
     destroy_graph(b);
     for (auto& j : b->jobs) cudaFree(j.slots);  // seeds share the allocation
+    b->mem.destroy();
     for (int i = 0; i < 2; ++i) {
         cudaFree(b->q[i].o);
         cudaFree(b->q[i].d);
@@ -619,6 +621,8 @@ extern "C" venu_status venu_batch_create(uint32_t pool_paths, uint32_t max_jobs,
     if (e == cudaSuccess) e = cudaMalloc(&b->d_ctl, sizeof(LoopCtl));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_run, sizeof(RunCtl));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_collect, sizeof(CollectEntry) * max_jobs);
+    // kept between jobs: what a pool full of paths needs (16 + 4 bytes each), at most 512 MB
+    if (e == cudaSuccess) e = b->mem.create(std::min<uint64_t>((uint64_t)Q * 20u, 512ull << 20));
     if (e == cudaSuccess) e = cudaMemset(b->d_ctl, 0, sizeof(LoopCtl));
     if (e == cudaSuccess) e = cudaMemset(b->d_run, 0, sizeof(RunCtl));
     if (e == cudaSuccess) e = cudaMemset(b->d_jobs, 0, sizeof(DevJob) * max_jobs);
@@ -718,7 +722,7 @@ extern "C" venu_status venu_batch_submit_many(venu_batch* b, const venu_job_desc
         J = JobHost{};
         // one allocation: the sample slots, then the seed table
         void* buf = nullptr;
-        cudaError_t e = cudaMallocAsync(&buf, (sizeof(float4) + sizeof(uint32_t)) * total, st);
+        cudaError_t e = b->mem.alloc(&buf, (sizeof(float4) + sizeof(uint32_t)) * total, st);
         // a group holds kSeedGroup jobs and at most 2^31 pixels (one job has at most 2^30)
         if (e == cudaSuccess && (g.n == kSeedGroup || (uint64_t)g.pix_off[g.n] + npix > (1ull << 31)))
             e = launch_seed_group(b, g, st);

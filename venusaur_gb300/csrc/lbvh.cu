@@ -56,7 +56,6 @@ struct LbvhCtl {
     HoistList hoisted;    // n <= kMaxHoisted, 0 if more than kHoistCandidates
     uint32_t hoist_buf[64];
     uint32_t bad_words;   // child words k_trav_layout had to replace (never, for a sound build)
-    uint32_t totals[4 * kBuckets];  // digits of all codes, per radix pass
 };
 constexpr uint32_t kHoistCandidates = 64;
 
@@ -71,8 +70,9 @@ __device__ __forceinline__ float huge_threshold(const uint32_t* b0) {
 
 // What must start from a known value: the control block, the arrival counters
 // and the parent links.  One launch instead of four.
-__global__ void k_lbvh_init(LbvhCtl* c, uint32_t n, uint32_t nint, uint32_t* __restrict__ arrive,
-                            int32_t* __restrict__ pint, int32_t* __restrict__ pleaf) {
+__global__ void k_lbvh_init(LbvhCtl* c, uint32_t n, uint32_t nint, uint32_t* __restrict__ totals,
+                            uint32_t* __restrict__ arrive, int32_t* __restrict__ pint, int32_t* __restrict__ pleaf,
+                            uint32_t* __restrict__ trace_err) {
     const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
     if (i0 == 0) {
         for (int a = 0; a < 3; ++a) {
@@ -83,7 +83,10 @@ __global__ void k_lbvh_init(LbvhCtl* c, uint32_t n, uint32_t nint, uint32_t* __r
         c->hoisted.n = 0;
         c->bad_words = 0;
     }
-    for (uint32_t i = i0; i < 4u * kBuckets; i += step) c->totals[i] = 0u;
+    if (totals)
+        for (uint32_t i = i0; i < 4u * kBuckets; i += step) totals[i] = 0u;
+    if (trace_err)
+        for (uint32_t i = i0; i < kTraceWords; i += step) trace_err[i] = 0u;
     for (uint32_t i = i0; i < nint; i += step) {
         arrive[i] = 0u;
         pint[i] = -1;
@@ -144,7 +147,8 @@ __device__ __forceinline__ uint32_t quant10(float c, float lo, float ext) {
 // 18 % on 1 M spheres than per-axis scaling, equal on the RTIOW scene.)
 // Also counts the digits of each radix pass (the same for all orders).
 __global__ void __launch_bounds__(256) k_morton(const venu_sphere* __restrict__ s, uint32_t n, LbvhCtl* c,
-                                                uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+                                                uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                uint32_t* __restrict__ totals) {
     __shared__ uint32_t digits[4 * kBuckets];
     for (int i = threadIdx.x; i < 4 * kBuckets; i += blockDim.x) digits[i] = 0u;
     __syncthreads();
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(256) k_morton(const venu_sphere* __restrict__ 
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 4 * kBuckets; i += blockDim.x)
-        if (digits[i]) atomicAdd(&c->totals[i], digits[i]);
+        if (digits[i]) atomicAdd(totals + i, digits[i]);
 }
 
 // Bounds, codes and sort of a small scene in one block (in place of 15
@@ -431,28 +435,25 @@ __device__ __forceinline__ uint32_t arrive_acq_rel(uint32_t* counter) {
     return old;
 }
 
-// Leaf boxes + bottom-up refit of moved spheres.  The second thread to
-// arrive at a node computes its box; the arrivals publish the children's
-// boxes, which are read back through L2 (__ldcg).  The tree itself does not
-// change, so a node's child words and parent are read beside its arrival.
-// ids[k] & id_mask = original index of the sphere in slot k (the sorted
-// values during a build, the meta words during a refit of moved spheres).
-// Leaf words may carry the hoisted flag (refit after a build).
-__global__ void k_refit(const venu_sphere* __restrict__ s, const uint32_t* __restrict__ ids, uint32_t id_mask, int n,
-                        float4* nodes, const int32_t* __restrict__ parent_int,
-                        const int32_t* __restrict__ parent_leaf, float4* leafbox,
-                        uint32_t* __restrict__ arrive) {
+// Box of a leaf: the sphere's AABB with |radius|, rounded outwards.  An
+// exactly-zero difference rounds down to -0.0; "+ 0.0f" makes it +0.0 (still a
+// lower bound) so boxes never carry a signed zero.
+__device__ __forceinline__ void leaf_box(float4 s4, float4& lo, float4& hi) {
+    const float r = fabsf(s4.w);
+    lo = make_float4(__fsub_rd(s4.x, r) + 0.0f, __fsub_rd(s4.y, r) + 0.0f, __fsub_rd(s4.z, r) + 0.0f, 0.0f);
+    hi = make_float4(__fadd_ru(s4.x, r), __fadd_ru(s4.y, r), __fadd_ru(s4.z, r), 0.0f);
+}
+
+// Bottom-up refit of moved spheres (sph: slot order).  The second thread to
+// arrive at a node computes its box and leaves its counter at 0 for the next
+// refit; the arrivals publish the children's boxes, which are read back
+// through L2 (__ldcg).  The tree itself does not change, so a node's child
+// words and parent are read beside its arrival.  Leaf words may carry the
+// hoisted flag.
+__global__ void k_refit(const float4* __restrict__ sph, int n, float4* nodes, const int32_t* __restrict__ parent_int,
+                        const int32_t* __restrict__ parent_leaf, uint32_t* __restrict__ arrive) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const venu_sphere& sp = s[ids[k] & id_mask];
-    float r = fabsf(sp.radius);
-    // An exactly-zero difference rounds down to -0.0; "+ 0.0f" makes it +0.0
-    // (still a lower bound) so boxes never carry a signed zero.
-    float4 lo = make_float4(__fsub_rd(sp.center[0], r) + 0.0f, __fsub_rd(sp.center[1], r) + 0.0f,
-                            __fsub_rd(sp.center[2], r) + 0.0f, 0.0f);
-    float4 hi = make_float4(__fadd_ru(sp.center[0], r), __fadd_ru(sp.center[1], r), __fadd_ru(sp.center[2], r), 0.0f);
-    leafbox[2 * k] = lo;
-    leafbox[2 * k + 1] = hi;
     int p = parent_leaf[k];
     // A Karras tree over unique (code, index) keys is at most 63 levels deep;
     // the bound only guards against a corrupt parent chain.
@@ -461,13 +462,23 @@ __global__ void k_refit(const venu_sphere* __restrict__ s, const uint32_t* __res
         const int32_t cr = __float_as_int(__ldcg(&nodes[2 * p + 1].w));
         const int32_t up = parent_int[p];
         if (arrive_acq_rel(arrive + p) == 0u) return;
+        arrive[p] = 0u;
         const bool ok_l = (cl & kLeaf) ? (cl & kSlotMask) < n : cl < n - 1;
         const bool ok_r = (cr & kLeaf) ? (cr & kSlotMask) < n : cr < n - 1;
         if (!ok_l || !ok_r) return;
-        float4 l0 = (cl & kLeaf) ? __ldcg(leafbox + 2 * (cl & kSlotMask)) : __ldcg(nodes + 2 * cl);
-        float4 h0 = (cl & kLeaf) ? __ldcg(leafbox + 2 * (cl & kSlotMask) + 1) : __ldcg(nodes + 2 * cl + 1);
-        float4 l1 = (cr & kLeaf) ? __ldcg(leafbox + 2 * (cr & kSlotMask)) : __ldcg(nodes + 2 * cr);
-        float4 h1 = (cr & kLeaf) ? __ldcg(leafbox + 2 * (cr & kSlotMask) + 1) : __ldcg(nodes + 2 * cr + 1);
+        float4 l0, h0, l1, h1;
+        if (cl & kLeaf) {
+            leaf_box(sph[cl & kSlotMask], l0, h0);
+        } else {
+            l0 = __ldcg(nodes + 2 * cl);
+            h0 = __ldcg(nodes + 2 * cl + 1);
+        }
+        if (cr & kLeaf) {
+            leaf_box(sph[cr & kSlotMask], l1, h1);
+        } else {
+            l1 = __ldcg(nodes + 2 * cr);
+            h1 = __ldcg(nodes + 2 * cr + 1);
+        }
         nodes[2 * p] = make_float4(fminf(l0.x, l1.x), fminf(l0.y, l1.y), fminf(l0.z, l1.z), __int_as_float(cl));
         nodes[2 * p + 1] = make_float4(fmaxf(h0.x, h1.x), fmaxf(h0.y, h1.y), fmaxf(h0.z, h1.z), __int_as_float(cr));
         p = up;
@@ -543,9 +554,15 @@ struct TEntry {
     int32_t word, left, right;
 };
 
-__device__ __forceinline__ void tentry_load(TEntry& e, const float4* nodes, const float4* leafbox, int32_t word) {
-    const float4* src = (word & kLeaf) ? leafbox + 2 * (size_t)(word & kSlotMask) : nodes + 2 * (size_t)word;
-    const float4 lo = __ldcg(src), hi = __ldcg(src + 1);
+__device__ __forceinline__ void tentry_load(TEntry& e, const float4* nodes, const float4* __restrict__ sph,
+                                            int32_t word) {
+    float4 lo, hi;
+    if (word & kLeaf) {
+        leaf_box(sph[word & kSlotMask], lo, hi);
+    } else {
+        lo = __ldcg(nodes + 2 * (size_t)word);
+        hi = __ldcg(nodes + 2 * (size_t)word + 1);
+    }
     e.word = word;
     e.b.lo[0] = lo.x;
     e.b.lo[1] = lo.y;
@@ -597,7 +614,7 @@ __device__ __forceinline__ void solve_subset(TreeletSmem& T, int S) {
 // same N.
 __device__ void restructure_treelet_warp(int32_t N, int n, int who, const TEntry& c0, const TEntry& c1, float area_n,
                                          float4* nodes, int32_t* parent_int, int32_t* parent_leaf,
-                                         const float4* leafbox, TreeletSmem& T) {
+                                         const float4* __restrict__ sph, TreeletSmem& T) {
     constexpr uint32_t kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     // lane i < nl holds entry i, lane i < ni internal node i of the treelet
@@ -634,7 +651,7 @@ __device__ void restructure_treelet_warp(int32_t N, int n, int who, const TEntry
         if (lane == ni) my_int = c;
         ++ni;
         if (lane == bi || lane == nl) {
-            tentry_load(e, nodes, leafbox, lane == bi ? left : right);
+            tentry_load(e, nodes, sph, lane == bi ? left : right);
             area = (e.word & kLeaf) ? -1.0f : tbox_area(e.b);
         }
         ++nl;
@@ -796,25 +813,14 @@ __device__ void restructure_treelet_warp(int32_t N, int n, int who, const TEntry
 // to serve in turn (31 of them for 32 leaves) and more warps.
 constexpr int kTreeletBlock = 128;
 __global__ void __launch_bounds__(kTreeletBlock)
-    k_treelets(const venu_sphere* __restrict__ s, const uint32_t* __restrict__ ids, int n, int per_warp, float4* nodes,
-               int32_t* parent_int, int32_t* parent_leaf, float4* leafbox, uint32_t* __restrict__ arrive) {
+    k_treelets(const float4* __restrict__ sph, int n, int per_warp, float4* nodes, int32_t* parent_int,
+               int32_t* parent_leaf, uint32_t* __restrict__ arrive) {
     __shared__ TreeletSmem smem[kTreeletBlock / 32];
     TreeletSmem& T = smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const long long first = (long long)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp;
     bool walking = lane < per_warp && first + lane < n;
-    int p = -1;
-    if (walking) {
-        const int k = (int)first + lane;
-        const venu_sphere& sp = s[ids[k]];
-        const float r = fabsf(sp.radius);
-        // as in k_refit: outwards, never a signed zero
-        leafbox[2 * (size_t)k] = make_float4(__fsub_rd(sp.center[0], r) + 0.0f, __fsub_rd(sp.center[1], r) + 0.0f,
-                                             __fsub_rd(sp.center[2], r) + 0.0f, 0.0f);
-        leafbox[2 * (size_t)k + 1] = make_float4(__fadd_ru(sp.center[0], r), __fadd_ru(sp.center[1], r),
-                                                 __fadd_ru(sp.center[2], r), 0.0f);
-        p = parent_leaf[k];
-    }
+    int p = walking ? parent_leaf[(int)first + lane] : -1;
     for (int level = 0; level < 128; ++level) {
         bool want = false;
         int up = -1;
@@ -832,9 +838,10 @@ __global__ void __launch_bounds__(kTreeletBlock)
                 if (arrive_acq_rel(arrive + p) == 0u) {
                     walking = false;  // the other subtree is not final yet
                 } else {
+                    arrive[p] = 0u;  // as refits expect it
                     if (word_ok(w0, n) && word_ok(w1, n)) {
-                        tentry_load(c0, nodes, leafbox, w0);
-                        tentry_load(c1, nodes, leafbox, w1);
+                        tentry_load(c0, nodes, sph, w0);
+                        tentry_load(c1, nodes, sph, w1);
                         TBox u = c0.b;
                         tbox_add(u, c1.b);
                         nodes[2 * (size_t)p] = make_float4(u.lo[0], u.lo[1], u.lo[2], __int_as_float(w0));
@@ -851,7 +858,7 @@ __global__ void __launch_bounds__(kTreeletBlock)
         for (uint32_t m = __ballot_sync(0xffffffffu, want); m; m &= m - 1u) {
             const int who = __ffs(m) - 1;
             const int32_t q = __shfl_sync(0xffffffffu, p, who);
-            restructure_treelet_warp(q, n, who, c0, c1, area, nodes, parent_int, parent_leaf, leafbox, T);
+            restructure_treelet_warp(q, n, who, c0, c1, area, nodes, parent_int, parent_leaf, sph, T);
         }
         // the rewiring by the other lanes comes before this lane's releasing
         // arrival at the parent
@@ -880,13 +887,6 @@ __global__ void k_gather(const venu_sphere* __restrict__ s, const uint32_t* ids,
         const uint32_t i = atomicAdd(&c->hoist_cnt, 1u);
         if (i < kHoistCandidates) c->hoist_buf[i] = k;
     }
-}
-
-// Box of a leaf: the sphere's box rounded outwards (as k_refit makes it).
-__device__ __forceinline__ void leaf_box(float4 s4, float4& lo, float4& hi) {
-    const float r = fabsf(s4.w);
-    lo = make_float4(__fsub_rd(s4.x, r) + 0.0f, __fsub_rd(s4.y, r) + 0.0f, __fsub_rd(s4.z, r) + 0.0f, 0.0f);
-    hi = make_float4(__fadd_ru(s4.x, r), __fadd_ru(s4.y, r), __fadd_ru(s4.z, r), 0.0f);
 }
 
 // ---------------------------------------------------------------------------
@@ -1223,10 +1223,13 @@ struct LbvhBuffers {
     float4 *nodes, *trav, *sph, *mat;
     uint32_t *meta, *keys;
     LbvhCtl* ctl;
-    uint32_t *keys_alt, *vals, *vals_alt, *hist, *arrive;
+    uint32_t *keys_alt, *vals, *vals_alt, *hist, *totals, *arrive, *trace_err;
     int32_t *pint, *pleaf;
-    float4* leafbox;
 };
+
+// Bytes of the scratch that only the codes and their sort use (keys_alt,
+// vals, vals_alt, hist, totals; each 256-byte aligned).
+constexpr size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Keys per lane of a sort tile (a warp's): short tiles while that still
 // spreads the keys over the SMs.
@@ -1249,7 +1252,8 @@ cudaError_t launch_lbvh(const venu_sphere* s, uint32_t n, cudaStream_t st, const
     const uint32_t nint = n > 1 ? n - 1 : 1;
     cudaError_t e = cudaSuccess;
     const uint32_t blocks = std::min(cdiv(n, 256), (uint32_t)(sm_count() * 8));
-    k_lbvh_init<<<blocks, 256, 0, st>>>(B.ctl, n, nint, B.arrive, B.pint, B.pleaf);
+    k_lbvh_init<<<blocks, 256, 0, st>>>(B.ctl, n, nint, n > kSmallScene ? B.totals : nullptr, B.arrive, B.pint, B.pleaf,
+                                        B.trace_err);
     if (n <= kSmallScene) {
         uint32_t n2 = 64;
         while (n2 < n) n2 *= 2;
@@ -1257,27 +1261,29 @@ cudaError_t launch_lbvh(const venu_sphere* s, uint32_t n, cudaStream_t st, const
     } else {
         const uint32_t few = std::min(cdiv(n, 256), (uint32_t)(sm_count() * 2));  // each block ends with atomics
         k_bounds<<<few, 256, 0, st>>>(s, n, B.ctl->b0);
-        k_morton<<<few, 256, 0, st>>>(s, n, B.ctl, B.keys, B.vals);
+        k_morton<<<few, 256, 0, st>>>(s, n, B.ctl, B.keys, B.vals, B.totals);
         uint32_t *kin = B.keys, *kout = B.keys_alt, *vin = B.vals, *vout = B.vals_alt;
         const uint32_t rounds = sort_rounds(n), ntiles = cdiv(n, 32 * rounds);
         const uint32_t sblocks = cdiv(ntiles, kWarpsPerBlock);
         for (int pass = 0; pass < 4; ++pass) {
             const int shift = pass * kRadixBits;
             k_hist<<<sblocks, 32 * kWarpsPerBlock, 0, st>>>(kin, n, shift, ntiles, rounds, B.hist);
-            k_scan_rows<<<kBuckets, 256, 0, st>>>(B.hist, ntiles, B.ctl->totals + pass * kBuckets);
+            k_scan_rows<<<kBuckets, 256, 0, st>>>(B.hist, ntiles, B.totals + pass * kBuckets);
             k_scatter<<<sblocks, 32 * kWarpsPerBlock, 0, st>>>(kin, vin, n, shift, ntiles, rounds, B.hist, kout, vout);
             std::swap(kin, kout);
             std::swap(vin, vout);
         }
         // four passes: the sorted codes / ids are back in B.keys / B.vals
     }
+    // the gather is the last to read the spheres and the sort's buffers, which
+    // may lie where the nodes and the traversal records go
+    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, B.vals, 0xffffffffu, n, B.sph, B.mat, B.meta, n > 1 ? B.ctl : nullptr);
     if (n > 1) {
         k_karras<<<cdiv(n - 1, 256), 256, 0, st>>>(B.keys, (int)n, B.nodes, B.pint, B.pleaf);
         const uint32_t per_warp = treelet_leaves_per_warp(n);
         k_treelets<<<cdiv(cdiv(n, per_warp), kTreeletBlock / 32), kTreeletBlock, 0, st>>>(
-            s, B.vals, (int)n, (int)per_warp, B.nodes, B.pint, B.pleaf, B.leafbox, B.arrive);
+            B.sph, (int)n, (int)per_warp, B.nodes, B.pint, B.pleaf, B.arrive);
     }
-    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, B.vals, 0xffffffffu, n, B.sph, B.mat, B.meta, n > 1 ? B.ctl : nullptr);
     if (n > 1) {
         k_hoist_finalize<<<1, 32, 0, st>>>(B.ctl, B.pleaf, B.nodes, n);
         if (B.trav) {
@@ -1293,19 +1299,15 @@ cudaError_t launch_lbvh(const venu_sphere* s, uint32_t n, cudaStream_t st, const
 
 void free_scene(venu_scene* s) {
     if (!s) return;
-    cudaFree(s->nodes);
-    cudaFree(s->trav);
-    cudaFree(s->sph);
-    cudaFree(s->mat);
-    cudaFree(s->meta);
-    cudaFree(s->keys);
-    cudaFree(s->parents);
+    cudaFree(s->arena);
     cudaFree(s->wide);
     cudaFree(s->wide_src);
     s->wide = nullptr;
     s->wide_src = nullptr;
     s->nwide = 0;
+    s->arena = nullptr;
     s->parents = nullptr;
+    s->arrive = s->trace_err = nullptr;
     s->nodes = s->trav = nullptr;
     s->sph = s->mat = nullptr;
     s->meta = s->keys = nullptr;
@@ -1382,30 +1384,48 @@ wdone:
     return rc;
 }
 
-venu_status build_scene(const venu_sphere* spheres_dev, uint32_t n, cudaStream_t st, venu_scene* S) {
+// A scene's buffers are one allocation (cudaMalloc and cudaFree wait for the
+// device: 14 and 7 of them took longer than a small build), and the build's
+// scratch lies in it: the sort's buffers where the nodes go, uploaded spheres
+// where the traversal records go.
+venu_status build_scene(const venu_sphere* spheres, bool on_host, uint32_t n, cudaStream_t st, venu_scene* S) {
     S->n = n;
     if (n == 0) return VENU_OK;
     if (n > (1u << 28)) {
         set_error("venu_scene_create: more than 2^28 spheres");
         return VENU_ERR_TOO_LARGE;
     }
-    const uint32_t ntiles = cdiv(n, 32 * sort_rounds(n));
-    const size_t hist_n = (size_t)kBuckets * ntiles;
-    size_t bytes = 0;
-    auto alloc = [&](void** p, size_t b) -> cudaError_t {
-        bytes += b;
-        return cudaMalloc(p, b ? b : 16);
+    const size_t N = n, nint = n > 1 ? n - 1 : 1;
+    const bool general = n > kSmallScene;  // the radix sort, not the one-block path
+    const size_t hist_b = general ? al256(sizeof(uint32_t) * kBuckets * (size_t)cdiv(n, 32 * sort_rounds(n))) : 0;
+    const size_t words_b = al256(sizeof(uint32_t) * N);
+    const size_t sort_b = general ? 3 * words_b + hist_b + al256(sizeof(uint32_t) * 4 * kBuckets) : words_b;
+    const size_t nodes_b = al256(std::max(sizeof(float4) * 2 * nint, sort_b));
+    const size_t trav_b = al256(std::max(sizeof(float4) * (4 * nint + 2), sizeof(venu_sphere) * N));
+    const size_t sph_b = al256(sizeof(float4) * N), par_b = al256(sizeof(int32_t) * (nint + N));
+    const size_t arr_b = al256(sizeof(uint32_t) * nint), ctl_b = al256(sizeof(LbvhCtl));
+    const size_t err_b = al256(sizeof(uint32_t) * kTraceWords);
+    const size_t total = nodes_b + trav_b + 2 * sph_b + 2 * words_b + par_b + arr_b + ctl_b + err_b;
+    VENU_CUDA(cudaMalloc(&S->arena, total));
+    S->bytes = total;
+    unsigned char* at = static_cast<unsigned char*>(S->arena);
+    auto take = [&](size_t b) {
+        unsigned char* p = at;
+        at += b;
+        return p;
     };
-    const uint32_t nint = n > 1 ? n - 1 : 1;
-    VENU_CUDA(alloc((void**)&S->nodes, sizeof(float4) * 2 * nint));
-    VENU_CUDA(alloc((void**)&S->trav, sizeof(float4) * (4 * (size_t)nint + 2)));
-    VENU_CUDA(alloc((void**)&S->sph, sizeof(float4) * n));
-    VENU_CUDA(alloc((void**)&S->mat, sizeof(float4) * n));
-    VENU_CUDA(alloc((void**)&S->meta, sizeof(uint32_t) * n));
-    VENU_CUDA(alloc((void**)&S->keys, sizeof(uint32_t) * n));
-    VENU_CUDA(alloc((void**)&S->parents, sizeof(int32_t) * ((size_t)nint + n)));
-    S->bytes = bytes;
+    unsigned char* const scratch = take(nodes_b);
+    S->nodes = reinterpret_cast<float4*>(scratch);
+    S->trav = reinterpret_cast<float4*>(take(trav_b));
+    S->sph = reinterpret_cast<float4*>(take(sph_b));
+    S->mat = reinterpret_cast<float4*>(take(sph_b));
+    S->meta = reinterpret_cast<uint32_t*>(take(words_b));
+    S->keys = reinterpret_cast<uint32_t*>(take(words_b));
+    S->parents = reinterpret_cast<int32_t*>(take(par_b));
+    S->arrive = reinterpret_cast<uint32_t*>(take(arr_b));
     LbvhBuffers B{};
+    B.ctl = reinterpret_cast<LbvhCtl*>(take(ctl_b));
+    S->trace_err = reinterpret_cast<uint32_t*>(take(err_b));
     B.nodes = S->nodes;
     B.trav = S->trav;
     B.sph = S->sph;
@@ -1414,6 +1434,15 @@ venu_status build_scene(const venu_sphere* spheres_dev, uint32_t n, cudaStream_t
     B.keys = S->keys;
     B.pint = S->parents;
     B.pleaf = S->parents + nint;
+    B.arrive = S->arrive;
+    B.trace_err = S->trace_err;
+    B.vals = reinterpret_cast<uint32_t*>(scratch);
+    if (general) {
+        B.keys_alt = reinterpret_cast<uint32_t*>(scratch + words_b);
+        B.vals_alt = reinterpret_cast<uint32_t*>(scratch + 2 * words_b);
+        B.hist = reinterpret_cast<uint32_t*>(scratch + 3 * words_b);
+        B.totals = reinterpret_cast<uint32_t*>(scratch + 3 * words_b + hist_b);
+    }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     venu_status rc = VENU_OK;
     LbvhCtl hc;
@@ -1425,19 +1454,16 @@ venu_status build_scene(const venu_sphere* spheres_dev, uint32_t n, cudaStream_t
             goto done;                           \
         }                                        \
     } while (0)
-    STEP(cudaMalloc(&B.ctl, sizeof(LbvhCtl)));
-    STEP(cudaMalloc(&B.keys_alt, sizeof(uint32_t) * n));
-    STEP(cudaMalloc(&B.vals, sizeof(uint32_t) * n));
-    STEP(cudaMalloc(&B.vals_alt, sizeof(uint32_t) * n));
-    STEP(cudaMalloc(&B.hist, sizeof(uint32_t) * hist_n));
-    STEP(cudaMalloc(&B.arrive, sizeof(uint32_t) * nint));
-    STEP(cudaMalloc(&B.leafbox, sizeof(float4) * 2 * n));
+    if (on_host) {
+        STEP(cudaMemcpyAsync(S->trav, spheres, sizeof(venu_sphere) * N, cudaMemcpyHostToDevice, st));
+        spheres = reinterpret_cast<const venu_sphere*>(S->trav);
+    }
     STEP(cudaEventCreate(&e0));
     STEP(cudaEventCreate(&e1));
     STEP(cudaEventRecord(e0, st));
-    STEP(launch_lbvh(spheres_dev, n, st, B));
+    STEP(launch_lbvh(spheres, n, st, B));
     STEP(cudaEventRecord(e1, st));
-    STEP(cudaMemcpyAsync(&hc, B.ctl, offsetof(LbvhCtl, totals), cudaMemcpyDeviceToHost, st));
+    STEP(cudaMemcpyAsync(&hc, B.ctl, sizeof(LbvhCtl), cudaMemcpyDeviceToHost, st));
     STEP(cudaStreamSynchronize(st));
     {
         float ms = 0.0f;
@@ -1454,15 +1480,9 @@ venu_status build_scene(const venu_sphere* spheres_dev, uint32_t n, cudaStream_t
     }
 #undef STEP
 done:
-    cudaFree(B.ctl);
-    cudaFree(B.keys_alt);
-    cudaFree(B.vals);
-    cudaFree(B.vals_alt);
-    cudaFree(B.hist);
-    cudaFree(B.arrive);
-    cudaFree(B.leafbox);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
+    if (rc != VENU_OK) cudaStreamSynchronize(st);  // nothing may still write to what the caller frees
     return rc;
 }
 
@@ -1485,36 +1505,29 @@ venu_status ensure_wide(const venu_scene* S, cudaStream_t st) {
     return rc;
 }
 
-venu_status update_scene(venu_scene* S, const venu_sphere* s, cudaStream_t st) {
+venu_status update_scene(venu_scene* S, const venu_sphere* s, bool on_host, cudaStream_t st) {
     const uint32_t n = S->n;
     if (n == 0) return VENU_OK;
+    if (on_host) {  // by way of the traversal records, which are rewritten below
+        VENU_CUDA(cudaMemcpyAsync(S->trav, s, sizeof(venu_sphere) * n, cudaMemcpyHostToDevice, st));
+        s = reinterpret_cast<const venu_sphere*>(S->trav);
+    }
     // New sphere records into the same slots (meta holds each slot's
     // original index), then the boxes bottom-up over the kept parent links,
     // then the traversal records.  Topology, slot order and the hoisted set
-    // stay those of the build.
-    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, S->meta, 0x3fffffffu, n, S->sph, S->mat, S->meta,
-                                           nullptr);
+    // stay those of the build.  Nothing is allocated: the counters are the
+    // build's, back at 0 (two stream-ordered allocations took 180 us a call).
+    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, S->meta, 0x3fffffffu, n, S->sph, S->mat, S->meta, nullptr);
     VENU_CUDA(cudaGetLastError());
     if (n == 1) return VENU_OK;
-    float4* leafbox = nullptr;
-    uint32_t* arrive = nullptr;
-    VENU_CUDA(cudaMallocAsync(&leafbox, sizeof(float4) * 2 * n, st));
-    cudaError_t e = cudaMallocAsync(&arrive, sizeof(uint32_t) * (n - 1), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(arrive, 0, sizeof(uint32_t) * (n - 1), st);
-    if (e == cudaSuccess) {
-        k_refit<<<cdiv(n, 256), 256, 0, st>>>(s, S->meta, 0x3fffffffu, (int)n, S->nodes, S->parents,
-                                              S->parents + (n - 1), leafbox, arrive);
-        HoistList list{S->nhoist, {}};
-        for (int i = 0; i < kMaxHoisted; ++i) list.slot[i] = S->hoist[i];
-        e = launch_trav_layout(S->nodes, S->sph, n, S->trav, S->parents, S->parents + (n - 1), nullptr, list, nullptr,
-                               st);
-        if (e == cudaSuccess && S->nwide) k_wide_refit<<<cdiv(S->nwide, 128), 128, 0, st>>>(S->nodes, S->sph, S->nwide, S->wide_src,
-                                                                      S->wide);
-        if (e == cudaSuccess) e = cudaGetLastError();
-    }
-    cudaFreeAsync(leafbox, st);
-    if (arrive) cudaFreeAsync(arrive, st);
-    if (e != cudaSuccess) return cuda_fail(e, "venu_scene_update");
+    k_refit<<<cdiv(n, 256), 256, 0, st>>>(S->sph, (int)n, S->nodes, S->parents, S->parents + (n - 1), S->arrive);
+    HoistList list{S->nhoist, {}};
+    for (int i = 0; i < kMaxHoisted; ++i) list.slot[i] = S->hoist[i];
+    VENU_CUDA(launch_trav_layout(S->nodes, S->sph, n, S->trav, S->parents, S->parents + (n - 1), nullptr, list, nullptr,
+                                 st));
+    if (S->nwide)
+        k_wide_refit<<<cdiv(S->nwide, 128), 128, 0, st>>>(S->nodes, S->sph, S->nwide, S->wide_src, S->wide);
+    VENU_CUDA(cudaGetLastError());
     return VENU_OK;
 }
 
@@ -1530,18 +1543,17 @@ namespace {
 constexpr uint32_t kNoAllocMaxSpheres = VENU_NOALLOC_MAX_SPHERES;
 constexpr uint32_t kNoAllocMaxTiles = (kNoAllocMaxSpheres + 127) / 128;  // sort_rounds: 128 keys a tile
 static_assert(kNoAllocMaxSpheres <= 65536, "sort_rounds gives tiles of 128 keys up to 65536 spheres");
-constexpr size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr size_t kNA = kNoAllocMaxSpheres;
 constexpr size_t kOffCtl = 0;                                         // LbvhCtl
 constexpr size_t kOffKeysAlt = al256(kOffCtl + sizeof(LbvhCtl));
 constexpr size_t kOffVals = al256(kOffKeysAlt + 4 * kNA);
 constexpr size_t kOffValsAlt = al256(kOffVals + 4 * kNA);
 constexpr size_t kOffHist = al256(kOffValsAlt + 4 * kNA);
-constexpr size_t kOffArrive = al256(kOffHist + 4 * (size_t)kBuckets * kNoAllocMaxTiles);
+constexpr size_t kOffTotals = al256(kOffHist + 4 * (size_t)kBuckets * kNoAllocMaxTiles);
+constexpr size_t kOffArrive = al256(kOffTotals + 4 * 4 * (size_t)kBuckets);
 constexpr size_t kOffParentInt = al256(kOffArrive + 4 * kNA);
 constexpr size_t kOffParentLeaf = al256(kOffParentInt + 4 * kNA);
-constexpr size_t kOffLeafBox = al256(kOffParentLeaf + 4 * kNA);
-constexpr size_t kNoAllocScratchBytes = al256(kOffLeafBox + 32 * kNA);  // about 4.2 MB
+constexpr size_t kNoAllocScratchBytes = al256(kOffParentLeaf + 4 * kNA);  // about 2.1 MB
 
 }  // namespace
 }  // namespace venu
@@ -1621,7 +1633,7 @@ extern "C" venu_status venu_lbvh_build_noalloc(const venu_sphere* spheres_dev, u
     B.arrive = reinterpret_cast<uint32_t*>(base + kOffArrive);
     B.pint = reinterpret_cast<int32_t*>(base + kOffParentInt);
     B.pleaf = reinterpret_cast<int32_t*>(base + kOffParentLeaf);
-    B.leafbox = reinterpret_cast<float4*>(base + kOffLeafBox);
+    B.totals = reinterpret_cast<uint32_t*>(base + kOffTotals);
     // The scratch keeps the previous call's contents; launch_lbvh resets what
     // must start from a known value (bounds seeds, hoist counters, arrival
     // counters, parent links) before using it.

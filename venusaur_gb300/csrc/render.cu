@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 namespace venu {
@@ -1278,9 +1279,24 @@ extern "C" venu_status venu_trace(const venu_scene* scene, const float* rays_dev
     if (ds != VENU_OK) return ds;
     if (n == 0) return VENU_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    // an error word of the scene's (0 unless a call failed), so that a call
+    // neither allocates nor clears; one of its own for more calls at once than
+    // there are, and for a scene without spheres
     uint32_t* err = nullptr;
-    VENU_CUDA(cudaMalloc(&err, sizeof(uint32_t)));
-    cudaError_t e = cudaMemsetAsync(err, 0, sizeof(uint32_t), st);
+    int word = -1;
+    if (scene->trace_err) {
+        std::lock_guard<std::mutex> lock(scene->trace_mu);
+        for (uint32_t i = 0; i < kTraceWords && word < 0; ++i)
+            if (!(scene->trace_used >> i & 1u)) word = (int)i;
+        if (word >= 0) scene->trace_used |= 1ull << word;
+    }
+    cudaError_t e = cudaSuccess;
+    if (word >= 0) {
+        err = scene->trace_err + word;
+    } else {
+        VENU_CUDA(cudaMalloc(&err, sizeof(uint32_t)));
+        e = cudaMemsetAsync(err, 0, sizeof(uint32_t), st);
+    }
     const size_t tsm = traverse_smem(kTravBlock);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace_rays, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
     if (e == cudaSuccess) {
@@ -1291,7 +1307,16 @@ extern "C" venu_status venu_trace(const venu_scene* scene, const float* rays_dev
     uint32_t herr = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(err);
+    if (word >= 0) {
+        if (herr) {
+            cudaMemsetAsync(err, 0, sizeof(uint32_t), st);
+            cudaStreamSynchronize(st);
+        }
+        std::lock_guard<std::mutex> lock(scene->trace_mu);
+        scene->trace_used &= ~(1ull << word);
+    } else {
+        cudaFree(err);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "venu_trace");
     if (herr) {
         set_error("venu_trace: traversal stack overflow");

@@ -119,6 +119,7 @@ struct venu_server {
     venu_batch* batch = nullptr;    // bulk lane
     venu_batch* express = nullptr;  // express lane
     cudaStream_t st = nullptr;
+    venu::DevPool mem;              // accumulators and images
     std::unordered_map<uint64_t, SceneEntry> scenes;
     std::unordered_map<uint32_t, uint64_t> active[2];  // per lane: batch job id -> request id
     std::unordered_map<uint64_t, Session> sessions;
@@ -253,7 +254,7 @@ void admit(venu_server* s, Request& R) {
             S.accum = nullptr;
         }
         if (!S.accum) {
-            e = cudaMallocAsync(&S.accum, accum_bytes, s->st);
+            e = s->mem.alloc(&S.accum, accum_bytes, s->st);
             if (e == cudaSuccess) {
                 S.width = o.width;
                 S.height = o.height;
@@ -267,9 +268,9 @@ void admit(venu_server* s, Request& R) {
         R.session_accum = true;
         S.busy = e == cudaSuccess;
     } else {
-        e = cudaMallocAsync(&R.accum, accum_bytes, s->st);
+        e = s->mem.alloc(&R.accum, accum_bytes, s->st);
     }
-    if (e == cudaSuccess) e = cudaMallocAsync(&R.image8, npix * 4u, s->st);
+    if (e == cudaSuccess) e = s->mem.alloc(&R.image8, npix * 4u, s->st);
     if (e != cudaSuccess) {
         release_accum(s, R);
         release_scene(s, key);
@@ -538,7 +539,11 @@ extern "C" venu_status venu_server_create(uint64_t hbm_budget_bytes, uint32_t po
         return bs;
     }
     cudaError_t e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
+    // kept between requests: at most an eighth of the budget
+    if (e == cudaSuccess) e = s->mem.create(std::min<uint64_t>(hbm_budget_bytes / 8u, 256ull << 20));
     if (e != cudaSuccess) {
+        s->mem.destroy();
+        if (s->st) cudaStreamDestroy(s->st);
         venu_batch_destroy(s->express);
         venu_batch_destroy(s->batch);
         delete s;
@@ -728,6 +733,7 @@ extern "C" venu_status venu_server_destroy(venu_server* s) {
     if (s->th.joinable()) s->th.join();
     venu_batch_destroy(s->batch);
     venu_batch_destroy(s->express);
+    s->mem.destroy();
     if (s->st) cudaStreamDestroy(s->st);
     delete s;
     return VENU_OK;

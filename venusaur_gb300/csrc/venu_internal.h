@@ -43,8 +43,37 @@ cudaError_t prefer_l1(K kernel, int per_sm, size_t dyn) {
 
 }  // namespace venu
 
+namespace venu {
+constexpr uint32_t kTraceWords = 64;  // venu_trace calls of one scene that may run at once without allocating
+
+// Device memory handed out in stream order and kept for reuse up to `keep`
+// bytes (the default pool gives everything back at each synchronisation, and
+// mapping it again costs 100 us and more); destroyed with its owner.
+struct DevPool {
+    cudaMemPool_t pool = nullptr;
+    cudaError_t create(uint64_t keep) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        cudaError_t e = cudaGetDevice(&props.location.id);
+        if (e == cudaSuccess) e = cudaMemPoolCreate(&pool, &props);
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        return e;
+    }
+    template <typename T>
+    cudaError_t alloc(T** p, size_t bytes, cudaStream_t st) {
+        return cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, pool, st);
+    }
+    void destroy() {
+        if (pool) cudaMemPoolDestroy(pool);
+        pool = nullptr;
+    }
+};
+}  // namespace venu
+
 struct venu_scene {
     uint32_t n = 0;
+    void* arena = nullptr;     // the one allocation that holds the buffers below (but the wide tree)
     float4* nodes = nullptr;   // 2 per internal node
     float4* trav = nullptr;    // 4 per internal node: both children (traversal layout)
     float4* sph = nullptr;     // slot order
@@ -52,6 +81,10 @@ struct venu_scene {
     uint32_t* meta = nullptr;  // original id | material << 30
     uint32_t* keys = nullptr;  // sorted Morton codes
     int32_t* parents = nullptr;  // [n-1] parent of each internal node, then [n] of each leaf (for refits)
+    uint32_t* arrive = nullptr;  // [n-1] arrival counters of refits, 0 between them
+    uint32_t* trace_err = nullptr;         // [kTraceWords] error words of venu_trace calls, 0 unless one failed
+    mutable uint64_t trace_used = 0;       // those in use (a bit each)
+    mutable std::mutex trace_mu;
     // The 4-wide traversal tree (lbvh.cu), built on first use by a render
     // with traversal variant 4 or 5 (ensure_wide); a cache of the binary
     // tree, so it may be filled in through a const scene.
@@ -68,12 +101,13 @@ struct venu_scene {
 };
 
 namespace venu {
-// Builds the LBVH for `n` device spheres into `s` (allocates its buffers).
-venu_status build_scene(const venu_sphere* spheres_dev, uint32_t n, cudaStream_t stream, venu_scene* s);
+// Builds the LBVH for `n` spheres in device or host memory into `s` (allocates
+// its buffers).
+venu_status build_scene(const venu_sphere* spheres, bool on_host, uint32_t n, cudaStream_t stream, venu_scene* s);
 void free_scene(venu_scene* s);
-// Moves the scene's spheres to `spheres_dev` (same count, original order) and
+// Moves the scene's spheres to `spheres` (same count, original order) and
 // refits the boxes on `stream` (asynchronous).
-venu_status update_scene(venu_scene* s, const venu_sphere* spheres_dev, cudaStream_t stream);
+venu_status update_scene(venu_scene* s, const venu_sphere* spheres, bool on_host, cudaStream_t stream);
 // Builds the scene's 4-wide tree on `stream` unless it exists (blocking: the
 // collapse reads each level's size on the host).  Thread-safe.
 venu_status ensure_wide(const venu_scene* s, cudaStream_t stream);
