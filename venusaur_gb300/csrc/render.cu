@@ -22,18 +22,23 @@
 
 namespace venu {
 
-// The bounce loop of a wave run as one CUDA graph (fused variants): the
-// first bounce's kernel, then a while node over a body of two bounce kernels
-// (odd: queue 1 -> 0, even: queue 0 -> 1), each with its queues and
-// counters as fixed parameters.  The last block of each bounce launch
-// advances the loop: it clears the counters the next bounce writes to,
-// counts the bounce, and keeps the while node going only while the bounce
-// left rays to trace -- so a wave whose paths all finish early (in place, or
-// by depth) launches no empty bounces.
+// The bounce loop of a wave (fused variants), run as one CUDA graph or launched
+// from the host: the first bounce's kernel, then bounce kernels (odd: queue
+// 1 -> 0, even: queue 0 -> 1) while a bounce leaves more rays than the
+// finishing kernel takes, then that kernel, which runs the rest of the wave's
+// paths to their ends.  In the graph the bounces after the first are a while
+// node over a body of two.  The last block of each bounce launch advances the
+// loop: it clears the counters the next bounce writes to, counts the bounce,
+// and either keeps the loop going or hands what is left to the finishing
+// kernel; bounce launches that find no more rays than that do nothing.
 struct WaveCtl {
     uint32_t b;            // bounces of the wave traced so far
     uint32_t nb;           // at most this many (the maximum depth)
     uint32_t blocks_done;  // blocks of the running bounce launch that finished
+    uint32_t left;         // rays left to the finishing kernel ...
+    uint32_t left_q;       // ... in this queue ...
+    uint32_t left_first;   // ... or still to be made from the path seeds
+    uint32_t left_work;    // hand-out counter of the finishing kernel
     uint32_t pad;
 };
 
@@ -45,16 +50,18 @@ struct WaveCtl {
 __global__ void k_raygen(venu_camera cam, uint32_t W, uint32_t H, uint32_t p0, uint32_t P, uint32_t s0,
                          uint32_t k, uint32_t subframe, int max_depth, uint32_t* __restrict__ seeds,
                          Queue q, uint32_t* __restrict__ path_seeds, uint32_t* __restrict__ cnt,
-                         uint32_t* __restrict__ work, int nbounce, WaveCtl* __restrict__ ctl) {
+                         uint32_t* __restrict__ work, int nbounce, WaveCtl* __restrict__ ctl, uint32_t finish_max) {
     const uint32_t pl = blockIdx.x * blockDim.x + threadIdx.x;
     if (pl == 0) {
         cnt[0] = P * k;
         for (int b = 1; b <= nbounce; ++b) cnt[b] = 0;
         for (int b = 0; b <= nbounce; ++b) work[b] = 0;
-        if (ctl) {
-            ctl->b = 0u;
-            ctl->nb = (uint32_t)nbounce;
-        }
+        ctl->b = 0u;
+        ctl->nb = (uint32_t)nbounce;
+        ctl->left = P * k <= finish_max ? P * k : 0u;  // a small wave is all the finishing kernel's
+        ctl->left_q = 0u;
+        ctl->left_first = 1u;
+        ctl->left_work = 0u;
     }
     if (pl >= P) return;
     const DevCamera C = load_camera(cam);
@@ -230,33 +237,41 @@ __device__ __forceinline__ void trace_shade_loop(const SceneView& S, const Queue
     }
 }
 
-// The in-place launch (no more rays than the grid has threads): block b
-// takes rays [b * blockDim, (b + 1) * blockDim) and finishes them bounce by
-// bounce.  After bounces 1, 2, 4, 8, ... the block's surviving paths are
-// compacted to its first threads where that frees a warp (their state staged
-// through the unused output queue, at the block's own positions), so its
-// warps stay full while paths end at different bounces instead of idling
-// around the few long paths; in between each warp runs at its own pace.
-// This launch waits for its longest path (28-31 % of the issue slots used),
-// so a barrier at every bounce cost more than the fuller warps gave: against
-// that, 256x144 x 4 RTIOW 319 -> 303 us, 400x225 x 16 692 -> 679 us, larger
-// frames unchanged; after every 4th or 8th bounce only, 400x225 x 16 takes
-// 804 and 1073 us.  Each path goes through exactly the same arithmetic as in
-// the ordinary loop; only the thread that runs it changes.
+// The in-place launch (no more rays than the grid has threads): the blocks
+// take equal shares of the rays and finish them bounce by bounce.  After
+// bounces 1, 2, 4, 8, ... a block brings its surviving paths together (their
+// state staged through the unused output queue, at the block's own
+// positions); in between each warp runs at its own pace.  This launch waits
+// for its longest path (28-31 % of the issue slots used), so a barrier at
+// every bounce cost more than the fuller warps gave: against that, 256x144 x 4
+// RTIOW 319 -> 303 us, 400x225 x 16 692 -> 679 us; after every 4th or 8th
+// bounce only, 400x225 x 16 takes 804 and 1073 us.
+// While many paths live they are packed into few warps (issue is what they
+// share); from bounce 8 on they are dealt out to all warps of the block, as a
+// path runs faster the fewer others its warp takes with it: 256x144 x 4
+// 298 -> 275 us, 400x225 x 16 675 -> 651, 300k spheres 512x512 x 4 6.97 ->
+// 6.76 ms (from bounce 2: 290 / 666 / 6.74, from 16: 287 / 649 / 6.87).
+// Equal shares instead of full blocks first: 64x36 x 2 139 -> 107 us.
+// Each path goes through exactly the same arithmetic as in the ordinary loop;
+// only the thread that runs it changes.
+constexpr uint32_t kSpreadAfter = 8;
 template <bool COUNT, int KS, bool WIDE>
 __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Queue& qin, uint32_t n,
                                                      const Queue& qout, float4* __restrict__ slots,
-                                                     const PrimaryGen& gen, const DevCamera& cam, StackSmem sm,
-                                                     bool& overflow, TraceCounters& K, uint32_t& extra) {
+                                                     bool primary, const PrimaryGen& gen, const DevCamera& cam,
+                                                     StackSmem sm, bool& overflow, TraceCounters& K, uint32_t& extra) {
     __shared__ uint32_t warp_live[32];
     const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
-    const uint32_t base = blockIdx.x * blockDim.x;
-    const uint32_t i = base + t;  // this thread's state lives at i
-    bool live = i < n;
+    const uint32_t nw = blockDim.x >> 5;
+    const uint32_t per = (n + gridDim.x - 1u) / gridDim.x;  // rays of a block
+    uint32_t own = t;  // this thread holds the block's own-th state
+    const uint32_t base = blockIdx.x * per;
+    uint32_t i = base + own;  // this thread's state lives at i
+    bool live = own < per && i < n;
     float4 o4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d4 = o4;
     if (live) {
         uint32_t seed = 0;
-        if (gen.path_seeds) {
+        if (primary) {
             gen_primary(gen, cam, i, o4, d4, seed);
             qout.t[i] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(seed));
         } else {
@@ -270,8 +285,9 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
     for (;;) {
         const uint32_t cnt = (uint32_t)__syncthreads_count(live);
         if (cnt == 0) break;
-        if ((cnt + 31u) / 32u < (held + 31u) / 32u) {
-            // compaction: the live states to threads [0, cnt)
+        const bool spread = done >= kSpreadAfter;
+        if (spread ? cnt < held : (cnt + 31u) / 32u < (held + 31u) / 32u) {
+            // the live states become the block's states [0, cnt)
             const uint32_t m = __ballot_sync(0xffffffffu, live);
             if (lane == 0) warp_live[w] = (uint32_t)__popc(m);
             float4 t4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -285,7 +301,9 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
                 qout.t[base + pos] = t4;
             }
             __syncthreads();
-            live = t < cnt;
+            own = spread ? lane * nw + w : t;  // one to each warp in turn
+            i = base + own;
+            live = own < cnt;
             if (live) {
                 o4 = qout.o[i];
                 d4 = qout.d[i];
@@ -318,97 +336,66 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
 // The in-place launch with refills (in_place_factor > 1, its own kernel
 // instantiation, REFILL): a launch with at most in_place_factor rays per
 // thread of the grid finishes every path it takes bounce after bounce
-// instead of appending survivors to the next queue.  A block takes rays from the launch
-// with one atomic per refill (the same dynamic hand-out as the ordinary
-// loop), and at each bounce boundary compacts its surviving paths to its
-// first threads (their state staged through the unused output queue) and
-// gives the threads behind them fresh rays, so its warps stay full while
-// paths end at different bounces.  Each path goes through exactly the same
-// arithmetic as in the ordinary loop; only the thread that runs it changes.
-// A block's staging positions are those of the first rays it took, base0 +
-// [0, blockDim): it never holds more paths than that first chunk had rays
-// (a short first chunk is the launch's last), so they stay inside the queue.
-// The factor is a tuning field (venu_tuning.in_place_factor): finishing in
-// place keeps the warps of a block in step bounce by bounce, which pays on
-// scenes with long, divergent paths and costs on short ones.
+// instead of appending survivors to the next queue.  A warp takes fresh rays
+// from the launch (one atomic) between bounces as soon as kRefillLanes of its
+// lanes are idle, so its lanes stay busy while paths end at different
+// bounces; warps do not wait for one another.  Each path goes through exactly
+// the same arithmetic as in the ordinary loop; only the thread that runs it
+// changes.  A lane's throughput and seed stay at the position of the first ray
+// it took, in the unused output queue.
+// Against block-wide refills with a barrier a bounce: 400x225 x 16 RTIOW 757 ->
+// 744 us over the wide tree, 656 -> 624 over the binary one, 20k spheres
+// 256x256 x 8 838 -> 818 us (8 lanes: 747 / 624 / 812; 16: 756 / 634 / 811).
+// The factor is a tuning field (venu_tuning.in_place_factor).
+constexpr uint32_t kRefillLanes = 4;
 
 template <bool COUNT, int KS, bool WIDE>
 __device__ __forceinline__ void trace_shade_in_place_refill(const SceneView& S, const Queue& qin, uint32_t n,
                                                      uint32_t* __restrict__ work, const Queue& qout,
-                                                     float4* __restrict__ slots, const PrimaryGen& gen,
-                                                     const DevCamera& cam, StackSmem sm, bool& overflow,
-                                                     TraceCounters& K, uint32_t& extra) {
-    __shared__ uint32_t warp_live[32];
-    __shared__ uint32_t s_base;
-    const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
-    uint32_t base0 = 0xffffffffu;  // the block's staging positions start here (its first chunk)
-    uint32_t held = 0;             // threads [0, held) hold the block's paths
+                                                     float4* __restrict__ slots, bool primary,
+                                                     const PrimaryGen& gen, const DevCamera& cam, StackSmem sm,
+                                                     bool& overflow, TraceCounters& K, uint32_t& extra) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t own = 0xffffffffu;  // the first ray this lane took
     bool exhausted = false, live = false, first = false;
     float4 o4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d4 = o4;
     for (;;) {
-        const uint32_t cnt = (uint32_t)__syncthreads_count(live);
-        if (cnt == 0 && exhausted) break;
-        if (cnt < held || (!exhausted && cnt < blockDim.x)) {
-            const uint32_t i = base0 + t;
-            if (cnt < held) {  // the live states to threads [0, cnt)
-                const uint32_t m = __ballot_sync(0xffffffffu, live);
-                if (lane == 0) warp_live[w] = (uint32_t)__popc(m);
-                float4 t4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (live) t4 = qout.t[i];
-                __syncthreads();
-                uint32_t pos = (uint32_t)__popc(m & ((1u << lane) - 1u));
-                for (uint32_t v = 0; v < w; ++v) pos += warp_live[v];
-                if (live) {
-                    qout.o[base0 + pos] = o4;
-                    qout.d[base0 + pos] = d4;
-                    qout.t[base0 + pos] = t4;
-                }
-                __syncthreads();
-                if (t < cnt) {
-                    o4 = qout.o[i];
-                    d4 = qout.d[i];
-                }
-            }
-            uint32_t take = 0, base = 0;
-            if (!exhausted) {  // fresh rays for threads [cnt, blockDim)
-                const uint32_t need = blockDim.x - cnt;
-                if (t == 0) s_base = atomicAdd(work, need);
-                __syncthreads();
-                base = s_base;
-                take = base < n ? min(need, n - base) : 0u;
-                exhausted = take < need;
-                if (base0 == 0xffffffffu) base0 = base;  // the first chunk (cnt == 0 then)
-            }
-            live = t < cnt + take;
-            first = t >= cnt && live;
-            if (first) {
-                const uint32_t ray = base + (t - cnt);
-                const uint32_t j = base0 + t;
-                if (gen.path_seeds) {
+        const uint32_t idle = __ballot_sync(0xffffffffu, !live);
+        if (!exhausted && (uint32_t)__popc(idle) >= kRefillLanes) {
+            const uint32_t take = (uint32_t)__popc(idle);
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(work, take);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            exhausted = base + take >= n;
+            const uint32_t ray = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (!live && ray < n) {
+                live = first = true;
+                if (own == 0xffffffffu) own = ray;
+                if (primary) {
                     uint32_t seed = 0;
                     gen_primary(gen, cam, ray, o4, d4, seed);
-                    qout.t[j] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(seed));
+                    qout.t[own] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(seed));
                 } else {
                     o4 = qin.o[ray];
                     d4 = qin.d[ray];
-                    qout.t[j] = qin.t[ray];
+                    qout.t[own] = qin.t[ray];
                 }
             }
-            held = cnt + take;
         }
+        if (!__any_sync(0xffffffffu, live)) break;  // only once the launch has no rays left
         if (live) {
-            const uint32_t i = base0 + t;
             RayPre R = prep(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float th;
-            const int32_t k = trace_closest<COUNT, KS, WIDE>(S, R, 0.001f, 1e16f, th, sm, t, blockDim.x, overflow, K);
-            const ShadeOut r = shade_one<true>(S, o4, d4, qout.t[i], make_int2(__float_as_int(th), k));
+            const int32_t k = trace_closest<COUNT, KS, WIDE>(S, R, 0.001f, 1e16f, th, sm, threadIdx.x, blockDim.x,
+                                                           overflow, K);
+            const ShadeOut r = shade_one<true>(S, o4, d4, qout.t[own], make_int2(__float_as_int(th), k));
             if (!first) ++extra;
             first = false;
             if (r.cont) {
                 o4 = r.o;
                 d4 = r.d;
-                qout.t[i] = r.t;
+                qout.t[own] = r.t;
             } else {
                 slots[(uint32_t)__float_as_int(o4.w)] = r.result;
                 live = false;
@@ -417,15 +404,10 @@ __device__ __forceinline__ void trace_shade_in_place_refill(const SceneView& S, 
     }
 }
 
-// Traverse and shade in one pass: each warp takes 32 rays, traverses them,
-// then shades all 32 together once the warp has reconverged and appends the
-// continuing paths with one ballot and one atomic.  Saves the hit record
-// round trip, the second read of the rays and one launch per bounce.
-// WIDE: the 4-wide tree instead of the binary traversal layout (variant 4,
-// k_trace_shade_wide, with its own register cap).
-// The end of a bounce launch run inside the wave graph (see WaveCtl).
-__device__ __forceinline__ void wave_advance(WaveCtl* ctl, uint32_t* cnt_in, uint32_t* work,
-                                             const uint32_t* cnt_out, unsigned long long* stats,
+// The end of a bounce launch (see WaveCtl).  handle: the while node's
+// condition, 0 for a launch from the host.
+__device__ __forceinline__ void wave_advance(WaveCtl* ctl, uint32_t* cnt_in, uint32_t* work, const uint32_t* cnt_out,
+                                             uint32_t out_q, uint32_t finish_max, unsigned long long* stats,
                                              cudaGraphConditionalHandle handle) {
     __syncthreads();  // every thread of the block is done
     if (threadIdx.x != 0) return;
@@ -439,71 +421,117 @@ __device__ __forceinline__ void wave_advance(WaveCtl* ctl, uint32_t* cnt_in, uin
     *work = 0u;    // the hand-out counter of the bounce after it
     const uint32_t b = ctl->b + 1u;
     ctl->b = b;
-    atomicAdd(stats + 5, 1ull);  // bounce launches run
-    const uint32_t more = b < ctl->nb && *reinterpret_cast<const volatile uint32_t*>(cnt_out) > 0u;
-    cudaGraphSetConditional(handle, more);
+    const uint32_t next = *reinterpret_cast<const volatile uint32_t*>(cnt_out);
+    const bool more = b < ctl->nb && next > finish_max;
+    if (!more) {
+        ctl->left = next <= finish_max ? next : 0u;  // after the last bounce there are none
+        ctl->left_q = out_q;
+        ctl->left_first = 0u;
+    }
+    if (handle) {
+        atomicAdd(stats + 5, 1ull);  // bounce launches run
+        cudaGraphSetConditional(handle, more ? 1u : 0u);
+    }
 }
 
-template <bool COUNT, int KS, bool WIDE, bool REFILL>
+// Traverse and shade in one pass: each warp takes 32 rays, traverses them,
+// then shades all 32 together once the warp has reconverged and appends the
+// continuing paths with one ballot and one atomic.  Saves the hit record
+// round trip, the second read of the rays and one launch per bounce.
+// A launch with at most finish_max rays leaves them to k_finish.
+// WIDE: the 4-wide tree instead of the binary traversal records (variant 4,
+// k_trace_shade_wide, with its own register cap).
+template <bool COUNT, int KS, bool WIDE>
 __device__ __forceinline__ void trace_shade_body(const SceneView& S, const Queue& qin,
                                                  uint32_t* __restrict__ cnt_in, uint32_t* __restrict__ work,
                                                  const Queue& qout, uint32_t* __restrict__ cnt_out,
                                                  float4* __restrict__ slots, uint32_t* __restrict__ err,
                                                  unsigned long long* __restrict__ stats, const PrimaryGen& gen,
-                                                 WaveCtl* ctl, cudaGraphConditionalHandle handle) {
+                                                 WaveCtl* ctl, uint32_t out_q, uint32_t finish_max,
+                                                 cudaGraphConditionalHandle handle) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
     sm.e = reinterpret_cast<int2*>(smem);
     __shared__ DevCamera cam;  // the primary rays' camera basis, once per block
+    const uint32_t n = *cnt_in;
+    if (n <= finish_max) {
+        if (handle && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(handle, 0u);
+        return;
+    }
     if (gen.path_seeds) {      // a kernel parameter: the same in every thread
         if (threadIdx.x == 0) cam = load_camera(gen.cam);
         __syncthreads();
     }
-    const uint32_t n = *cnt_in;
-    const uint32_t lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats, (unsigned long long)n);
     TraceCounters K{0, 0};
     bool overflow = false;
-    uint32_t extra = 0;  // segments traced in place after a ray's first
-    if (n <= (REFILL ? gen.in_place_factor : 1u) * gridDim.x * blockDim.x) {
-        if (REFILL)
-            trace_shade_in_place_refill<COUNT, KS, WIDE>(S, qin, n, work, qout, slots, gen, cam, sm, overflow, K,
-                                                         extra);
-        else
-            trace_shade_in_place<COUNT, KS, WIDE>(S, qin, n, qout, slots, gen, cam, sm, overflow, K, extra);
-        for (int off = 16; off > 0; off >>= 1) extra += __shfl_xor_sync(0xffffffffu, extra, off);
-        if (lane == 0 && extra) atomicAdd(stats, (unsigned long long)extra);
-    } else {
-        trace_shade_loop<COUNT, KS, WIDE>(S, qin, n, work, qout, cnt_out, slots, gen, cam, sm, overflow, K);
-    }
+    trace_shade_loop<COUNT, KS, WIDE>(S, qin, n, work, qout, cnt_out, slots, gen, cam, sm, overflow, K);
     if (overflow) atomicOr(err, 1u);
     if (COUNT) flush_counters(K, stats);
-    if (ctl) wave_advance(ctl, cnt_in, work, cnt_out, stats, handle);
+    wave_advance(ctl, cnt_in, work, cnt_out, out_q, finish_max, stats, handle);
 }
 
-// REFILL: launches of up to in_place_factor rays per thread finish in place
-// with refills (a separate instantiation, so the ordinary kernel keeps its
-// registers).  ctl: the wave graph's loop control (nullptr for a launch
-// from the host's bounce loop).
-template <bool COUNT, int KS, bool REFILL = false>
+template <bool COUNT, int KS>
 __global__ void VENU_TRACE_BOUNDS k_trace_shade(SceneView S, Queue qin, uint32_t* __restrict__ cnt_in,
                                                 uint32_t* __restrict__ work, Queue qout,
                                                 uint32_t* __restrict__ cnt_out, float4* __restrict__ slots,
                                                 uint32_t* __restrict__ err, unsigned long long* __restrict__ stats,
-                                                PrimaryGen gen, WaveCtl* ctl, cudaGraphConditionalHandle handle) {
-    trace_shade_body<COUNT, KS, false, REFILL>(S, qin, cnt_in, work, qout, cnt_out, slots, err, stats, gen, ctl,
-                                               handle);
+                                                PrimaryGen gen, WaveCtl* ctl, uint32_t out_q, uint32_t finish_max,
+                                                cudaGraphConditionalHandle handle) {
+    trace_shade_body<COUNT, KS, false>(S, qin, cnt_in, work, qout, cnt_out, slots, err, stats, gen, ctl, out_q,
+                                       finish_max, handle);
 }
 
-template <bool COUNT, int KS, bool REFILL = false>
+template <bool COUNT, int KS>
 __global__ void VENU_WIDE_BOUNDS k_trace_shade_wide(SceneView S, Queue qin, uint32_t* __restrict__ cnt_in,
                                                     uint32_t* __restrict__ work, Queue qout,
                                                     uint32_t* __restrict__ cnt_out, float4* __restrict__ slots,
                                                     uint32_t* __restrict__ err,
                                                     unsigned long long* __restrict__ stats, PrimaryGen gen,
-                                                    WaveCtl* ctl, cudaGraphConditionalHandle handle) {
-    trace_shade_body<COUNT, KS, true, REFILL>(S, qin, cnt_in, work, qout, cnt_out, slots, err, stats, gen, ctl,
-                                              handle);
+                                                    WaveCtl* ctl, uint32_t out_q, uint32_t finish_max,
+                                                    cudaGraphConditionalHandle handle) {
+    trace_shade_body<COUNT, KS, true>(S, qin, cnt_in, work, qout, cnt_out, slots, err, stats, gen, ctl, out_q,
+                                      finish_max, handle);
+}
+
+// The finishing kernel: runs the paths that are left of a wave (WaveCtl) to
+// their ends.  A kernel of its own, so that the bounce kernels' code and
+// registers are not shaped by it (in one kernel with them, changes to this
+// part moved the bounce loop by up to 1.5 %; apart, the bounce kernel spills 12
+// bytes instead of 60): 1080p x 32 RTIOW 14.05 -> 13.95 ms, 256x144 x 4 278 ->
+// 260 us, 64x36 x 2 107 -> 90 us.  At 80 / 96 / 128 registers, with as many
+// fewer rays to take, the 256x144 frame takes 297 / 296 / 295 us.  REFILL
+// (in_place_factor > 1): with refills.
+template <bool COUNT, int KS, bool WIDE, bool REFILL>
+__global__ void VENU_TRACE_BOUNDS k_finish(SceneView S, Queue q0, Queue q1, float4* __restrict__ slots,
+                                           uint32_t* __restrict__ err, unsigned long long* __restrict__ stats,
+                                           PrimaryGen gen, WaveCtl* ctl) {
+    extern __shared__ unsigned char smem[];
+    StackSmem sm;
+    sm.e = reinterpret_cast<int2*>(smem);
+    __shared__ DevCamera cam;
+    const uint32_t n = ctl->left;
+    if (n == 0) return;
+    const bool primary = ctl->left_first != 0u;
+    const bool second = ctl->left_q != 0u;
+    const Queue qin = second ? q1 : q0, qout = second ? q0 : q1;
+    if (primary) {
+        if (threadIdx.x == 0) cam = load_camera(gen.cam);
+        __syncthreads();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats, (unsigned long long)n);
+    TraceCounters K{0, 0};
+    bool overflow = false;
+    uint32_t extra = 0;  // segments traced after a ray's first
+    if (REFILL)
+        trace_shade_in_place_refill<COUNT, KS, WIDE>(S, qin, n, &ctl->left_work, qout, slots, primary, gen, cam, sm,
+                                                     overflow, K, extra);
+    else
+        trace_shade_in_place<COUNT, KS, WIDE>(S, qin, n, qout, slots, primary, gen, cam, sm, overflow, K, extra);
+    extra = __reduce_add_sync(0xffffffffu, extra);
+    if ((threadIdx.x & 31u) == 0 && extra) atomicAdd(stats, (unsigned long long)extra);
+    if (overflow) atomicOr(err, 1u);
+    if (COUNT) flush_counters(K, stats);
 }
 
 __global__ void __launch_bounds__(512) k_shade(SceneView S, Queue qin, const int2* __restrict__ hits,
@@ -627,7 +655,8 @@ struct WaveGraphKey {
     unsigned long long* stats;
     WaveCtl* ctl;
     size_t fsm;
-    int grid, block;
+    int grid, block, finish_grid;
+    uint32_t finish_max;
     uint32_t kind;  // bits: 4-wide tree, shallow stack, counting build, in-place refills
 };
 
@@ -645,7 +674,7 @@ struct venu_renderer {
     uint32_t* err = nullptr;
     unsigned long long* stats = nullptr;  // segments, nodes, spheres, lane / warp steps, graph bounces
     venu_tuning tune = {2u, 32u, 128u, 0u, 128u, 0u, 1u};
-    int trav_blocks = 0, shade_blocks = 0, fused_blocks = 0;
+    int trav_blocks = 0, shade_blocks = 0, fused_blocks = 0, finish_blocks = 0;
     venu_render_stats last = {};
     uint32_t host_launches = 0;  // kernels the last render launched from the host
     bool graph_off = false;      // the wave graph could not be built: host bounce loops only
@@ -677,90 +706,74 @@ cudaError_t occupancy_grid(K kernel, int block, size_t smem, uint32_t per_sm_cap
 }
 
 template <typename K>
-cudaError_t set_smem_refill(K kernel, size_t smem) {
+cudaError_t set_smem(K kernel, size_t smem) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
+// The fused kernels' launch shape: one for the four instantiations of the
+// bounce kernel (the shallow-stack ones need less shared memory; same grid)
+// and one for those of the finishing kernel.
+template <bool WIDE, typename K8, typename K4, typename C8, typename C4>
+cudaError_t configure_fused(venu_renderer* r, K8 deep, K4 shallow, C8 count_deep, C4 count_shallow) {
+    const venu_tuning& t = r->tune;
+    const int tb = (int)t.traverse_block;
+    const size_t sm = traverse_smem(tb), ss = traverse_smem(tb, kSharedShallow);
+    cudaError_t e = occupancy_grid(deep, tb, sm, t.traverse_blocks_per_sm, r->fused_blocks);
+    if (e == cudaSuccess) e = set_smem(shallow, sm);
+    if (e == cudaSuccess) e = set_smem(count_deep, sm);
+    if (e == cudaSuccess) e = set_smem(count_shallow, sm);
+    if (e == cudaSuccess)
+        e = occupancy_grid(k_finish<false, kShared, WIDE, false>, tb, sm, t.traverse_blocks_per_sm, r->finish_blocks);
+    if (e == cudaSuccess) e = set_smem(k_finish<false, kSharedShallow, WIDE, false>, sm);
+    if (e == cudaSuccess) e = set_smem(k_finish<false, kShared, WIDE, true>, sm);
+    if (e == cudaSuccess) e = set_smem(k_finish<false, kSharedShallow, WIDE, true>, sm);
+    if (e == cudaSuccess) e = set_smem(k_finish<true, kShared, WIDE, false>, sm);
+    if (e == cudaSuccess) e = set_smem(k_finish<true, kSharedShallow, WIDE, false>, sm);
+    if (e == cudaSuccess) e = set_smem(k_finish<true, kShared, WIDE, true>, sm);
+    if (e == cudaSuccess) e = set_smem(k_finish<true, kSharedShallow, WIDE, true>, sm);
+    const int nsm = std::max(1, sm_count());
+    const int pb = std::max(1, r->fused_blocks / nsm), pf = std::max(1, r->finish_blocks / nsm);
+    if (e == cudaSuccess) e = prefer_l1(deep, pb, sm);
+    if (e == cudaSuccess) e = prefer_l1(shallow, pb, ss);
+    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kShared, WIDE, false>, pf, sm);
+    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kSharedShallow, WIDE, false>, pf, ss);
+    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kShared, WIDE, true>, pf, sm);
+    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kSharedShallow, WIDE, true>, pf, ss);
+    return e;
 }
 
 // Persistent grids: as many resident blocks as fit (or the tuned cap) on every SM.
 cudaError_t configure(venu_renderer* r) {
     const venu_tuning& t = r->tune;
-    const size_t sm = traverse_smem((int)t.traverse_block);
-    cudaError_t e;
+    const int tb = (int)t.traverse_block;
+    const size_t sm = traverse_smem(tb);
+    const int nsm = std::max(1, sm_count());
+    cudaError_t e = cudaSuccess;
     if (t.traverse_variant == 4) {  // the fused kernel over the 4-wide tree
-        e = occupancy_grid(k_trace_shade_wide<false, kShared>, (int)t.traverse_block, sm,
-                           t.traverse_blocks_per_sm, r->fused_blocks);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_trace_shade_wide<true, kShared>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sm);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_trace_shade_wide<false, kSharedShallow>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_trace_shade_wide<true, kSharedShallow>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e == cudaSuccess) e = set_smem_refill(k_trace_shade_wide<false, kShared, true>, sm);
-        if (e == cudaSuccess) e = set_smem_refill(k_trace_shade_wide<true, kShared, true>, sm);
-        if (e == cudaSuccess) e = set_smem_refill(k_trace_shade_wide<false, kSharedShallow, true>, sm);
-        if (e == cudaSuccess) e = set_smem_refill(k_trace_shade_wide<true, kSharedShallow, true>, sm);
-        if (e != cudaSuccess) return e;
+        e = configure_fused<true>(r, k_trace_shade_wide<false, kShared>, k_trace_shade_wide<false, kSharedShallow>,
+                                  k_trace_shade_wide<true, kShared>, k_trace_shade_wide<true, kSharedShallow>);
         r->trav_blocks = r->fused_blocks;
     } else if (t.traverse_variant >= 2) {  // the fused kernel: every bounce (2), the primary one (3, 5)
-        e = occupancy_grid(k_trace_shade<false, kShared>, (int)t.traverse_block, sm, t.traverse_blocks_per_sm,
-                           r->fused_blocks);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_trace_shade<true, kShared>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        // the shallow-tree instantiation needs less shared memory; same grid
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_trace_shade<false, kSharedShallow>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sm);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_trace_shade<true, kSharedShallow>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sm);
-        if (e == cudaSuccess) e = set_smem_refill(k_trace_shade<false, kShared, true>, sm);
-        if (e == cudaSuccess) e = set_smem_refill(k_trace_shade<true, kShared, true>, sm);
-        if (e == cudaSuccess) e = set_smem_refill(k_trace_shade<false, kSharedShallow, true>, sm);
-        if (e == cudaSuccess) e = set_smem_refill(k_trace_shade<true, kSharedShallow, true>, sm);
-        if (e != cudaSuccess) return e;
-    }
-    if (t.traverse_variant == 4) {
-    } else if (t.traverse_variant == 5) {  // later bounces: the separate traversal over the wide tree
-        e = occupancy_grid(k_traverse<false, true>, (int)t.traverse_block, sm, t.traverse_blocks_per_sm,
-                           r->trav_blocks);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_traverse<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    } else if (t.traverse_variant == 0 || t.traverse_variant == 3) {
-        e = occupancy_grid(k_traverse<false>, (int)t.traverse_block, sm, t.traverse_blocks_per_sm, r->trav_blocks);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_traverse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    } else if (t.traverse_variant == 2) {
+        e = configure_fused<false>(r, k_trace_shade<false, kShared>, k_trace_shade<false, kSharedShallow>,
+                                   k_trace_shade<true, kShared>, k_trace_shade<true, kSharedShallow>);
         r->trav_blocks = r->fused_blocks;
-    } else {
-        e = occupancy_grid(k_traverse_dyn<false>, (int)t.traverse_block, sm, t.traverse_blocks_per_sm, r->trav_blocks);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_traverse_dyn<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    }
+    if (e != cudaSuccess) return e;
+    if (t.traverse_variant == 5) {  // later bounces: the separate traversal over the wide tree
+        e = occupancy_grid(k_traverse<false, true>, tb, sm, t.traverse_blocks_per_sm, r->trav_blocks);
+        if (e == cudaSuccess) e = set_smem(k_traverse<true, true>, sm);
+        if (e == cudaSuccess) e = prefer_l1(k_traverse<false, true>, std::max(1, r->trav_blocks / nsm), sm);
+    } else if (t.traverse_variant == 0 || t.traverse_variant == 3) {
+        e = occupancy_grid(k_traverse<false>, tb, sm, t.traverse_blocks_per_sm, r->trav_blocks);
+        if (e == cudaSuccess) e = set_smem(k_traverse<true>, sm);
+        if (e == cudaSuccess) e = prefer_l1(k_traverse<false>, std::max(1, r->trav_blocks / nsm), sm);
+    } else if (t.traverse_variant == 1) {
+        e = occupancy_grid(k_traverse_dyn<false>, tb, sm, t.traverse_blocks_per_sm, r->trav_blocks);
+        if (e == cudaSuccess) e = set_smem(k_traverse_dyn<true>, sm);
+        if (e == cudaSuccess) e = prefer_l1(k_traverse_dyn<false>, std::max(1, r->trav_blocks / nsm), sm);
     }
     if (e == cudaSuccess) e = occupancy_grid(k_shade, (int)t.shade_block, 0, t.shade_blocks_per_sm, r->shade_blocks);
-    if (e != cudaSuccess) return e;
-    {
-        const int nsm = std::max(1, sm_count());
-        const int pf = std::max(1, r->fused_blocks / nsm), pt = std::max(1, r->trav_blocks / nsm);
-        const size_t shallow = traverse_smem((int)t.traverse_block, kSharedShallow);
-        if (t.traverse_variant == 4) {
-            if (e == cudaSuccess) e = prefer_l1(k_trace_shade_wide<false, kShared>, pf, sm);
-            if (e == cudaSuccess) e = prefer_l1(k_trace_shade_wide<false, kSharedShallow>, pf, shallow);
-            if (e == cudaSuccess) e = prefer_l1(k_trace_shade_wide<false, kShared, true>, pf, sm);
-            if (e == cudaSuccess) e = prefer_l1(k_trace_shade_wide<false, kSharedShallow, true>, pf, shallow);
-        } else if (t.traverse_variant >= 2) {
-            if (e == cudaSuccess) e = prefer_l1(k_trace_shade<false, kShared>, pf, sm);
-            if (e == cudaSuccess) e = prefer_l1(k_trace_shade<false, kSharedShallow>, pf, shallow);
-            if (e == cudaSuccess) e = prefer_l1(k_trace_shade<false, kShared, true>, pf, sm);
-            if (e == cudaSuccess) e = prefer_l1(k_trace_shade<false, kSharedShallow, true>, pf, shallow);
-        }
-        if (t.traverse_variant == 5 && e == cudaSuccess) e = prefer_l1(k_traverse<false, true>, pt, sm);
-        if ((t.traverse_variant == 0 || t.traverse_variant == 3) && e == cudaSuccess)
-            e = prefer_l1(k_traverse<false>, pt, sm);
-        if (t.traverse_variant == 1 && e == cudaSuccess) e = prefer_l1(k_traverse_dyn<false>, pt, sm);
-        if (e == cudaSuccess) e = prefer_l1(k_shade, std::max(1, r->shade_blocks / nsm), 0);
-    }
+    if (e == cudaSuccess) e = prefer_l1(k_shade, std::max(1, r->shade_blocks / nsm), 0);
     return e;
 }
 
@@ -814,47 +827,59 @@ cudaError_t alloc_queues(venu_renderer* r, uint32_t Q) {
 void destroy_wave_graph(venu_renderer* r);
 constexpr uint32_t kFusedWide = 1u, kFusedShallow = 2u, kFusedCount = 4u, kFusedRefill = 8u;
 
+#define VENU_FUSED_CS(LAUNCH, KERNEL)                            \
+    do {                                                         \
+        if (kind & kFusedCount) {                                \
+            if (kind & kFusedShallow) LAUNCH(KERNEL, true, kSharedShallow);  \
+            else LAUNCH(KERNEL, true, kShared);                  \
+        } else {                                                 \
+            if (kind & kFusedShallow) LAUNCH(KERNEL, false, kSharedShallow); \
+            else LAUNCH(KERNEL, false, kShared);                 \
+        }                                                        \
+    } while (0)
+
 // One bounce of the fused kernel (variant 2, or 4 over the 4-wide tree)
-// with the renderer's launch shape.  ctl / handle: the wave graph's loop
-// control, or nullptr / 0 for a launch from the host's bounce loop.
+// with the renderer's launch shape, into queue out_q.  h: the wave graph's
+// loop condition, or 0 for a launch from the host's bounce loop.
 cudaError_t launch_fused(const venu_renderer* r, cudaStream_t st, uint32_t kind, size_t fsm, const SceneView& S,
-                         const Queue& qi, uint32_t* cnt_in, uint32_t* work, const Queue& qo, uint32_t* cnt_out,
-                         const PrimaryGen& pg, WaveCtl* ctl, cudaGraphConditionalHandle h) {
+                         uint32_t* cnt_in, uint32_t* work, uint32_t out_q, uint32_t* cnt_out, const PrimaryGen& pg,
+                         uint32_t finish_max, cudaGraphConditionalHandle h) {
     const int grid = r->fused_blocks, tb = (int)r->tune.traverse_block;
-#define VENU_FUSED(KERNEL, C, KS, RF)                                                                       \
-    KERNEL<C, KS, RF><<<grid, tb, fsm, st>>>(S, qi, cnt_in, work, qo, cnt_out, r->slots, r->err, r->stats, pg, ctl, h)
-#define VENU_FUSED_RF(KERNEL, C, KS)                  \
-    do {                                              \
-        if (kind & kFusedRefill)                      \
-            VENU_FUSED(KERNEL, C, KS, true);          \
-        else                                          \
-            VENU_FUSED(KERNEL, C, KS, false);         \
-    } while (0)
-#define VENU_FUSED_CS(KERNEL, KS)                     \
-    do {                                              \
-        if (kind & kFusedCount)                       \
-            VENU_FUSED_RF(KERNEL, true, KS);          \
-        else                                          \
-            VENU_FUSED_RF(KERNEL, false, KS);         \
-    } while (0)
-    if (kind & kFusedWide) {
-        if (kind & kFusedShallow) VENU_FUSED_CS(k_trace_shade_wide, kSharedShallow);
-        else VENU_FUSED_CS(k_trace_shade_wide, kShared);
-    } else {
-        if (kind & kFusedShallow) VENU_FUSED_CS(k_trace_shade, kSharedShallow);
-        else VENU_FUSED_CS(k_trace_shade, kShared);
-    }
-#undef VENU_FUSED_CS
-#undef VENU_FUSED_RF
+    const Queue &qi = r->q[1u - out_q], &qo = r->q[out_q];
+#define VENU_FUSED(KERNEL, C, KS)                                                                              \
+    KERNEL<C, KS><<<grid, tb, fsm, st>>>(S, qi, cnt_in, work, qo, cnt_out, r->slots, r->err, r->stats, pg, r->ctl, \
+                                         out_q, finish_max, h)
+    if (kind & kFusedWide) VENU_FUSED_CS(VENU_FUSED, k_trace_shade_wide);
+    else VENU_FUSED_CS(VENU_FUSED, k_trace_shade);
 #undef VENU_FUSED
     return cudaGetLastError();
 }
 
+// What is left of a wave (see WaveCtl).
+cudaError_t launch_finish(const venu_renderer* r, cudaStream_t st, uint32_t kind, size_t fsm, const SceneView& S,
+                          const PrimaryGen& pg) {
+    const int grid = r->finish_blocks, tb = (int)r->tune.traverse_block;
+#define VENU_FINISH(WIDE, C, KS)                                                                                  \
+    do {                                                                                                          \
+        if (kind & kFusedRefill)                                                                                  \
+            k_finish<C, KS, WIDE, true>                                                                           \
+                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl);             \
+        else                                                                                                      \
+            k_finish<C, KS, WIDE, false>                                                                          \
+                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl);             \
+    } while (0)
+    if (kind & kFusedWide) VENU_FUSED_CS(VENU_FINISH, true);
+    else VENU_FUSED_CS(VENU_FINISH, false);
+#undef VENU_FINISH
+    return cudaGetLastError();
+}
+#undef VENU_FUSED_CS
+
 // Builds the wave graph for `key` (see WaveCtl): the first bounce (camera
-// rays from the per-path seeds, queue 0 -> 1), then while (rays left) {
-// queue 1 -> 0; queue 0 -> 1 }.  After an odd bounce that leaves no rays the
-// even one still starts and finds none, so a wave runs at most one empty
-// launch.
+// rays from the per-path seeds, queue 0 -> 1), while (more rays than the
+// finishing kernel takes) { queue 1 -> 0; queue 0 -> 1 }, the finishing
+// kernel.  After an odd bounce that ends the loop the even one still starts
+// and finds nothing to do.
 venu_status build_wave_graph(venu_renderer* r, const WaveGraphKey& key) {
     destroy_wave_graph(r);
     if (!r->cap) VENU_CUDA(cudaStreamCreateWithFlags(&r->cap, cudaStreamNonBlocking));
@@ -865,8 +890,8 @@ venu_status build_wave_graph(venu_renderer* r, const WaveGraphKey& key) {
     PrimaryGen later = key.pg;
     later.path_seeds = nullptr;  // bounces after the first read their rays from the queue
     VENU_CUDA(cudaStreamBeginCaptureToGraph(r->cap, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    cudaError_t le = launch_fused(r, r->cap, key.kind, key.fsm, key.S, key.q0, key.cnt, key.work, key.q1,
-                                  key.cnt + 1, key.pg, key.ctl, h);
+    cudaError_t le = launch_fused(r, r->cap, key.kind, key.fsm, key.S, key.cnt, key.work, 1u, key.cnt + 1, key.pg,
+                                  key.finish_max, h);
     cudaGraph_t captured = nullptr;
     cudaError_t ee = cudaStreamEndCapture(r->cap, &captured);
     if (le != cudaSuccess) return cuda_fail(le, "venu_render: capture of the first bounce");
@@ -887,13 +912,18 @@ venu_status build_wave_graph(venu_renderer* r, const WaveGraphKey& key) {
     VENU_CUDA(cudaGraphAddNode(&loop, g, &first, nullptr, 1, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     VENU_CUDA(cudaStreamBeginCaptureToGraph(r->cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    le = launch_fused(r, r->cap, key.kind, key.fsm, key.S, key.q1, key.cnt + 1, key.work + 1, key.q0, key.cnt,
-                      later, key.ctl, h);
+    le = launch_fused(r, r->cap, key.kind, key.fsm, key.S, key.cnt + 1, key.work + 1, 0u, key.cnt, later,
+                      key.finish_max, h);
     if (le == cudaSuccess)
-        le = launch_fused(r, r->cap, key.kind, key.fsm, key.S, key.q0, key.cnt, key.work, key.q1, key.cnt + 1,
-                          later, key.ctl, h);
+        le = launch_fused(r, r->cap, key.kind, key.fsm, key.S, key.cnt, key.work, 1u, key.cnt + 1, later,
+                          key.finish_max, h);
     ee = cudaStreamEndCapture(r->cap, &captured);
     if (le != cudaSuccess) return cuda_fail(le, "venu_render: capture of the bounce loop");
+    if (ee != cudaSuccess) return cuda_fail(ee, "venu_render: cudaStreamEndCapture");
+    VENU_CUDA(cudaStreamBeginCaptureToGraph(r->cap, g, &loop, nullptr, 1, cudaStreamCaptureModeRelaxed));
+    le = launch_finish(r, r->cap, key.kind, key.fsm, key.S, key.pg);
+    ee = cudaStreamEndCapture(r->cap, &captured);
+    if (le != cudaSuccess) return cuda_fail(le, "venu_render: capture of the finishing kernel");
     if (ee != cudaSuccess) return cuda_fail(ee, "venu_render: cudaStreamEndCapture");
     VENU_CUDA(cudaGraphInstantiate(&r->wexec, g, 0));
     r->wkey = key;
@@ -1099,9 +1129,16 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
         pg.depth = (int)maxd - 1;
         pg.div_P = make_fastdiv(PP);
         pg.div_W = make_fastdiv(W);
-        pg.in_place_factor = tu.in_place_factor ? tu.in_place_factor : 1u;
         return pg;
     };
+    // waves and bounces of at most this many rays are the finishing kernel's
+    // (a thread takes one, or in_place_factor with refills); the separate
+    // traversals after a fused first bounce (variants 3, 5) only leave it whole waves
+    const uint64_t factor = tu.in_place_factor ? tu.in_place_factor : 1u;
+    const uint32_t finish_max =
+        gen0 ? (uint32_t)std::min<uint64_t>(factor * r->finish_blocks * (uint64_t)tb, 0xffffffffu) : 0u;
+    const uint32_t bounce_max = fused ? finish_max : 0u;
+    use_graph = use_graph && (uint64_t)npix * k > finish_max;
     if (use_graph) {
         WaveGraphKey key;
         std::memset(&key, 0, sizeof key);
@@ -1118,6 +1155,8 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
         key.ctl = r->ctl;
         key.fsm = fsm;
         key.grid = r->fused_blocks;
+        key.finish_grid = r->finish_blocks;
+        key.finish_max = finish_max;
         key.block = tb;
         key.kind = kind;
         if (!r->wexec || std::memcmp(&key, &r->wkey, sizeof key) != 0) {
@@ -1136,17 +1175,29 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
             const uint32_t PP = std::min(P, npix - p0);
             k_raygen<<<(PP + 255) / 256, 256, 0, st>>>(*camera, W, H, p0, PP, s0, kk, opts->subframe_index,
                                                        (int)maxd, r->seeds, r->q[0], path_seeds, r->cnt, r->work,
-                                                       nb, use_graph ? r->ctl : nullptr);
+                                                       nb, r->ctl, finish_max);
             PrimaryGen pg = primary_gen(p0, PP);
+            pg.path_seeds = path_seeds;
+            const bool small = (uint64_t)PP * kk <= finish_max;
             ++launches;
-            if (use_graph) {  // the bounce loop of this wave: one graph launch
-                VENU_CUDA(cudaGraphLaunch(r->wexec, st));
-                k_accumulate<<<(PP + 255) / 256, 256, 0, st>>>(r->slots, p0, PP, kk, accum);
+            if (small) {
+                if (prof) {
+                    for (int i = 0; i < 2; ++i) {
+                        cudaEvent_t a, z;
+                        VENU_CUDA(next_events(r, a, z));
+                        VENU_CUDA(cudaEventRecord(a, st));
+                        if (i == 0) VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg));
+                        VENU_CUDA(cudaEventRecord(z, st));
+                    }
+                } else {
+                    VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg));
+                }
                 ++launches;
-                ++waves;
-                continue;
+            } else if (use_graph) {  // the bounce loop of this wave: one graph launch
+                VENU_CUDA(cudaGraphLaunch(r->wexec, st));
+                ++launches;  // the finishing kernel; the bounces count themselves
             }
-            for (int b = 0; b < nb; ++b) {
+            for (int b = 0; b < nb && !small && !use_graph; ++b) {
                 const Queue& qi = r->q[b & 1];
                 const Queue& qo = r->q[(b + 1) & 1];
                 cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr, e3 = nullptr;
@@ -1167,18 +1218,14 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
                 }
                 if (v == 2 || v == 4) {
                     pg.path_seeds = (b == 0) ? path_seeds : nullptr;
-                    VENU_CUDA(launch_fused(r, st, kind, fsm, S, qi, r->cnt + b, r->work + b, qo, r->cnt + b + 1,
-                                           pg, nullptr, 0));
+                    VENU_CUDA(launch_fused(r, st, kind, fsm, S, r->cnt + b, r->work + b, (uint32_t)((b + 1) & 1),
+                                           r->cnt + b + 1, pg, bounce_max, 0));
                     if (prof) {
                         VENU_CUDA(cudaEventRecord(e1, st));
                         VENU_CUDA(cudaEventRecord(e2, st));
                         VENU_CUDA(cudaEventRecord(e3, st));
                     }
                     launches += 1;
-                    // a first bounce that the fused kernel finishes in place
-                    // finishes every path: no later bounce has rays
-                    if (b == 0 && (uint64_t)PP * kk <= (uint64_t)pg.in_place_factor * r->fused_blocks * (uint64_t)tb)
-                        break;
                     continue;
                 }
                 if (v == 0) {
@@ -1210,6 +1257,20 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
                 k_shade<<<r->shade_blocks, sb, 0, st>>>(S, qi, r->hits, r->cnt + b, qo, r->cnt + b + 1, r->slots);
                 if (prof) VENU_CUDA(cudaEventRecord(e3, st));
                 launches += 2;
+            }
+            if (fused && !small && !use_graph) {  // what the bounces left
+                if (prof) {
+                    for (int i = 0; i < 2; ++i) {
+                        cudaEvent_t a, z;
+                        VENU_CUDA(next_events(r, a, z));
+                        VENU_CUDA(cudaEventRecord(a, st));
+                        if (i == 0) VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg));
+                        VENU_CUDA(cudaEventRecord(z, st));
+                    }
+                } else {
+                    VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg));
+                }
+                ++launches;
             }
             k_accumulate<<<(PP + 255) / 256, 256, 0, st>>>(r->slots, p0, PP, kk, accum);
             ++launches;
