@@ -9,8 +9,8 @@
 //                        with __ballot_sync + a warp prefix, finished paths
 //                        write their radiance to their sample slot);
 //   accumulate one thread per pixel, Kahan-adds the wave's samples in
-//              sample order.
-// A resolve pass writes the running mean (RGBA32F) and sRGB RGBA8.
+//              sample order; the last wave's also writes the running mean
+//              (RGBA32F) and sRGB RGBA8.
 // Queue counts live on the device; the host never waits inside a render.
 #include "render_kernels.cuh"
 #include "venu_internal.h"
@@ -50,12 +50,15 @@ struct WaveCtl {
 __global__ void k_raygen(venu_camera cam, uint32_t W, uint32_t H, uint32_t p0, uint32_t P, uint32_t s0,
                          uint32_t k, uint32_t subframe, int max_depth, uint32_t* __restrict__ seeds,
                          Queue q, uint32_t* __restrict__ path_seeds, uint32_t* __restrict__ cnt,
-                         uint32_t* __restrict__ work, int nbounce, WaveCtl* __restrict__ ctl, uint32_t finish_max) {
+                         uint32_t* __restrict__ work, int nbounce, WaveCtl* __restrict__ ctl, uint32_t finish_max,
+                         unsigned long long* __restrict__ stats) {
     const uint32_t pl = blockIdx.x * blockDim.x + threadIdx.x;
     if (pl == 0) {
         cnt[0] = P * k;
         for (int b = 1; b <= nbounce; ++b) cnt[b] = 0;
         for (int b = 0; b <= nbounce; ++b) work[b] = 0;
+        if (s0 == 0 && p0 == 0)  // the render's first wave
+            for (int i = 0; i < 6; ++i) stats[i] = 0ull;
         ctl->b = 0u;
         ctl->nb = (uint32_t)nbounce;
         ctl->left = P * k <= finish_max ? P * k : 0u;  // a small wave is all the finishing kernel's
@@ -563,25 +566,29 @@ __global__ void __launch_bounds__(512) k_shade(SceneView S, Queue qin, const int
 }
 
 // Kahan-adds samples [0, k) of pixels [p0, p0+P) from their slots, in order.
+// HBM traffic is all it costs, so a render's first wave starts from zero
+// (reset) instead of reading a cleared accumulator back, and its last one
+// resolves the pixel (the running mean, RGBA32F and sRGB RGBA8) while it holds
+// the sums, in place of a clear and a resolve launch.
 __global__ void k_accumulate(const float4* __restrict__ slots, uint32_t p0, uint32_t P, uint32_t k,
-                             float4* __restrict__ accum) {
+                             float4* __restrict__ accum, bool reset, float4* __restrict__ image_f,
+                             uchar4* __restrict__ image8) {
     const uint32_t pl = blockIdx.x * blockDim.x + threadIdx.x;
     if (pl >= P) return;
     const uint32_t pix = p0 + pl;
-    float4 a0 = accum[2 * (size_t)pix], a1 = accum[2 * (size_t)pix + 1];
+    float4 a0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), a1 = a0;
+    if (!reset) {
+        a0 = accum[2 * (size_t)pix];
+        a1 = accum[2 * (size_t)pix + 1];
+    }
     for (uint32_t s = 0; s < k; ++s) kahan_add(a0, a1, __ldcs(slots + (size_t)s * P + pl));
     accum[2 * (size_t)pix] = a0;
     accum[2 * (size_t)pix + 1] = a1;
-}
-
-__global__ void k_resolve(const float4* __restrict__ accum, uint32_t npix, float4* __restrict__ image_f,
-                          uchar4* __restrict__ image8) {
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pix >= npix) return;
-    float4 a0 = accum[2 * (size_t)pix];
-    f3 mean = mk(a0.x / a0.w, a0.y / a0.w, a0.z / a0.w);
-    if (image_f) image_f[pix] = make_float4(mean.x, mean.y, mean.z, 1.0f);
-    if (image8) image8[pix] = make_color(mean);
+    if (image_f || image8) {
+        const f3 mean = mk(a0.x / a0.w, a0.y / a0.w, a0.z / a0.w);
+        if (image_f) image_f[pix] = make_float4(mean.x, mean.y, mean.z, 1.0f);
+        if (image8) image8[pix] = make_color(mean);
+    }
 }
 
 // Arbitrary rays -> closest hit (t, original id, front face).
@@ -1057,9 +1064,7 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
         VENU_CUDA(cudaMalloc(&r->seeds, sizeof(uint32_t) * npix));
         r->seeds_cap = npix;
     }
-    if (opts->flags & VENU_FLAG_RESET_ACCUM)
-        VENU_CUDA(cudaMemsetAsync(accum_dev, 0, sizeof(float) * VENU_ACCUM_FLOATS_PER_PIXEL * npix64, st));
-    VENU_CUDA(cudaMemsetAsync(r->stats, 0, sizeof(unsigned long long) * 6, st));
+    const bool reset = (opts->flags & VENU_FLAG_RESET_ACCUM) != 0;
     if (r->tune.traverse_variant == 4u || r->tune.traverse_variant == 5u) {
         const venu_status ws = ensure_wide(scene, st);  // the first such render builds it
         if (ws != VENU_OK) return ws;
@@ -1175,7 +1180,7 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
             const uint32_t PP = std::min(P, npix - p0);
             k_raygen<<<(PP + 255) / 256, 256, 0, st>>>(*camera, W, H, p0, PP, s0, kk, opts->subframe_index,
                                                        (int)maxd, r->seeds, r->q[0], path_seeds, r->cnt, r->work,
-                                                       nb, r->ctl, finish_max);
+                                                       nb, r->ctl, finish_max, r->stats);
             PrimaryGen pg = primary_gen(p0, PP);
             pg.path_seeds = path_seeds;
             const bool small = (uint64_t)PP * kk <= finish_max;
@@ -1272,15 +1277,13 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
                 }
                 ++launches;
             }
-            k_accumulate<<<(PP + 255) / 256, 256, 0, st>>>(r->slots, p0, PP, kk, accum);
+            const bool last = s0 + kk == spp;  // of these pixels
+            k_accumulate<<<(PP + 255) / 256, 256, 0, st>>>(
+                r->slots, p0, PP, kk, accum, reset && s0 == 0, last ? reinterpret_cast<float4*>(image_f_dev) : nullptr,
+                last ? reinterpret_cast<uchar4*>(image8_dev) : nullptr);
             ++launches;
             ++waves;
         }
-    }
-    if (image_f_dev || image8_dev) {
-        k_resolve<<<(npix + 255) / 256, 256, 0, st>>>(accum, npix, reinterpret_cast<float4*>(image_f_dev),
-                                                      reinterpret_cast<uchar4*>(image8_dev));
-        ++launches;
     }
     VENU_CUDA(cudaGetLastError());
     r->last = venu_render_stats{};
