@@ -324,7 +324,7 @@ __device__ __forceinline__ void trace_shade_multi_loop(const DevJob* __restrict_
             }
             job = __float_as_uint(d4.w) >> 8;
             for (bool first = true;; first = false) {
-                RayPre R = prep(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+                RayPre R = prep_for<COUNT>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
                 R.from = from;
                 float t;
                 int32_t k;

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const ui
         const uint32_t i = base + lane;
         if (i < n) {
             float4 o4 = __ldcs(q.o + i), d4 = __ldcs(q.d + i);
-            RayPre R = prep(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<COUNT, WIDE>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float t;
             int32_t k = trace_closest<COUNT, kShared, WIDE>(S, R, 0.001f, 1e16f, t, sm, threadIdx.x, blockDim.x,
@@ -155,13 +155,15 @@ __global__ void __launch_bounds__(256) k_traverse_dyn(SceneView S, Queue q, cons
                 if (my < n) {
                     ray = my;
                     const float4 o4 = __ldcs(q.o + my), d4 = __ldcs(q.d + my);
-                    RayPre R = prep(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+                    RayPre R = prep_for<COUNT>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
                     R.from = packed_from(d4.w);
                     const float m = COUNT ? 0.0f : ray_margin(S, R);
                     if (COUNT ? R.axis : !(m <= kFarMarginMax)) {
                         // a ray that needs per-axis margins (rare): traced to the
                         // end now with the canonical loop, on this lane's free
                         // stack; the lane stays idle
+                        R = prep<false>(R.o, R.d);
+                        R.from = packed_from(d4.w);
                         axis_margins(R);
                         float t;
                         const int32_t kk = trace_with<Tracer<COUNT, true, true>>(
@@ -221,7 +223,7 @@ __device__ __forceinline__ void trace_shade_loop(const SceneView& S, const Queue
                 d4 = qin.d[i];
             }
             slot = (uint32_t)__float_as_int(o4.w);
-            RayPre R = prep(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<COUNT, WIDE>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float t;
             const int32_t k =
@@ -317,7 +319,7 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
         const uint32_t until = done ? 2u * done : 1u;
         for (; done < until && __any_sync(0xffffffffu, live); ++done) {
             if (!live) continue;
-            RayPre R = prep(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<COUNT, WIDE>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float th;
             const int32_t k = trace_closest<COUNT, KS, WIDE>(S, R, 0.001f, 1e16f, th, sm, t, blockDim.x, overflow, K);
@@ -387,7 +389,7 @@ __device__ __forceinline__ void trace_shade_in_place_refill(const SceneView& S, 
         }
         if (!__any_sync(0xffffffffu, live)) break;  // only once the launch has no rays left
         if (live) {
-            RayPre R = prep(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<COUNT, WIDE>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float th;
             const int32_t k = trace_closest<COUNT, KS, WIDE>(S, R, 0.001f, 1e16f, th, sm, threadIdx.x, blockDim.x,
@@ -603,7 +605,7 @@ __global__ void __launch_bounds__(128) k_trace_rays(SceneView S, const float* __
     if (i >= n) return;
     f3 o = mk(rays[6 * (size_t)i], rays[6 * (size_t)i + 1], rays[6 * (size_t)i + 2]);
     f3 d = mk(rays[6 * (size_t)i + 3], rays[6 * (size_t)i + 4], rays[6 * (size_t)i + 5]);
-    RayPre R = prep(o, d);
+    RayPre R = prep_for<false>(o, d);
     TraceCounters K{0, 0};
     bool overflow = false;
     float t;

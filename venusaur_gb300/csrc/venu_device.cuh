@@ -97,7 +97,12 @@ __device__ __forceinline__ float rnd(uint32_t& s) {
 // kept): an acceptance rate of 52% (sphere) / 79% (disk) makes that bound
 // unreachable in practice, and it guarantees termination on the GPU.
 constexpr int kMaxTries = 4096;
-__device__ __forceinline__ float rnd_pm1(uint32_t& s) { return -1.0f + (1.0f - -1.0f) * rnd(s); }
+// -1 + 2 rnd(s): both products are by powers of two and the sum is a multiple
+// of 2^-23 in [-1, 1), so one fmaf of the 24-bit integer gives the same float.
+__device__ __forceinline__ float rnd_pm1(uint32_t& s) {
+    s = 1664525u * s + 1013904223u;
+    return fmaf((float)(s & 0x00FFFFFFu), 1.1920928955078125e-07f, -1.0f);  // 2^-23
+}
 __device__ __forceinline__ f3 random_in_unit_sphere(uint32_t& s) {  // :117-125
     f3 p;
     for (int i = 0; i < kMaxTries; ++i) {
@@ -280,6 +285,16 @@ __device__ __forceinline__ void axis_margins(RayPre& R) {
     R.axis = true;
 }
 
+// 1/x by the hardware approximation (one ulp), for x not subnormal.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// APPROX: 1/d good to an ulp, which is all the fast walk asks of it (it serves
+// the slab tests alone; 1/a below enters the hits and stays correctly rounded).
+template <bool APPROX>
 __device__ __forceinline__ RayPre prep(f3 o, f3 d) {
     RayPre R;
     R.from = -1;
@@ -288,7 +303,7 @@ __device__ __forceinline__ RayPre prep(f3 o, f3 d) {
     float dx = fabsf(d.x) < 1e-20f ? copysignf(1e-20f, d.x) : d.x;
     float dy = fabsf(d.y) < 1e-20f ? copysignf(1e-20f, d.y) : d.y;
     float dz = fabsf(d.z) < 1e-20f ? copysignf(1e-20f, d.z) : d.z;
-    R.inv = mk(1.0f / dx, 1.0f / dy, 1.0f / dz);
+    R.inv = APPROX ? mk(rcp_approx(dx), rcp_approx(dy), rcp_approx(dz)) : mk(1.0f / dx, 1.0f / dy, 1.0f / dz);
     const float px = o.x * R.inv.x, py = o.y * R.inv.y, pz = o.z * R.inv.z;
     const float mx = fabsf(px) * 4.76837158203125e-07f;  // 2^-21
     const float my = fabsf(py) * 4.76837158203125e-07f;
@@ -546,17 +561,18 @@ __device__ __forceinline__ void up_front(T& W, const SceneView& S, TraceCounters
 // them at once in the node's step the 1080p RTIOW frame gains 4 %, a batch of
 // small renders 9 %.
 //
-// Nothing is lost by it: '// the records' half extents are widened by
+// Nothing is lost by it: the records' half extents are widened by
 // e = 1.5 2^-19 E, where E is the largest |C| + |r| of the leaves.
 // sphere_test may accept a point that lies off the sphere by up to
 // 12 2^-24 (|h| + r) (h = o - C; roundings of h, of h.d, of the products with
 // d and of the root), and the slab parameters above are off by at most
-// 4 2^-24 (|o| + E) |1/d|: together 16 2^-24 (|o| + E) in units of length,
-// which is 2^-19 E for |o| = E.  For origins further out the rest, at most
-// 2 2^-20 (|o| - E) max|1/d|, is added to the exit parameter with a factor of
-// two (m); where that exceeds kFarMarginMax the ray takes the canonical walk
-// with margins per axis.  A sphere that is not finite is not part of E; its
-// box is NaN or infinite, and such a box is always met.
+// 5 2^-24 (|o| + E) |1/d| (1/d an ulp off): together 17 2^-24 (|o| + E) in units
+// of length, 34 2^-24 E for |o| = E against e = 48 2^-24 E.  For origins further
+// out the rest, at most 34 2^-24 (|o| - E) max|1/d| over entry and exit, is
+// added to the exit parameter as 64 2^-24 (m); where that exceeds kFarMarginMax
+// the ray takes the canonical walk with margins per axis.  A sphere that is not
+// finite is not part of E; its box is NaN or infinite, and such a box is always
+// met.
 // ---------------------------------------------------------------------------
 constexpr float kFarMarginMax = 1.0f;
 
@@ -976,6 +992,11 @@ struct WideTracer {
     }
 };
 
+template <bool COUNT, bool WIDE = false>
+__device__ __forceinline__ RayPre prep_for(f3 o, f3 d) {
+    return prep<!COUNT && !WIDE>(o, d);
+}
+
 template <class T>
 __device__ __forceinline__ int32_t trace_with(const SceneView& S, const RayPre& R, float m, float tmin, float tmax,
                                               float& t_out, StackSmem sm, uint32_t tid, uint32_t bdim,
@@ -988,7 +1009,7 @@ __device__ __forceinline__ int32_t trace_with(const SceneView& S, const RayPre& 
     return W.result(t_out);
 }
 
-// Closest hit of one ray (R from prep).  The binary tree: the fast walk,
+// Closest hit of one ray (R from prep_for<COUNT, WIDE>).  The binary tree: the fast walk,
 // unless the ray starts far outside the scene (rare) or the build counts;
 // those, and the wide tree, take the shared-margin loop, or the per-axis one
 // for the rare near-axis-parallel ray.  KS: shared-memory stack entries per
@@ -1008,7 +1029,8 @@ __device__ __forceinline__ int32_t trace_closest(const SceneView& S, const RayPr
     }
     const float m = COUNT ? 0.0f : ray_margin(S, R);
     if (COUNT ? R.axis : !(m <= kFarMarginMax)) {
-        RayPre A = R;
+        RayPre A = prep<false>(R.o, R.d);
+        A.from = R.from;
         axis_margins(A);
         return trace_with<Tracer<COUNT, true, true, KS>>(S, A, 0.0f, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
     }
