@@ -1071,17 +1071,15 @@ cudaError_t launch_trav_layout(const float4* nodes, const float4* sph, uint32_t 
 // depend on it: the closest hit is the same for any conservative traversal
 // (minimum t, ties to the smaller slot).
 //
-// Node layout (kWideF4 float4s: 128 bytes for 4 children, 256 for 8), with
-// H = kWideW / 4 float4s per plane:
-//   [0, 6H)   child boxes, structure of arrays: lo.x, hi.x, lo.y, hi.y,
-//             lo.z, hi.z, each H float4s of four children
-//   [6H, 7H)  child words: an internal child's wide index, or a leaf's
-//             0x80000000 | slot (an unused entry or a hoisted leaf:
-//             0x80000000 | 0x40000000, never tested)
-//   [7H]      {valid mask | leaf mask << 8 (int bits), 0, 0, 0}
-// wide_src[kWideW w + c] keeps the binary word of child c (internal node
-// index or leaf word), so a refit of moved spheres can recompute the boxes
-// in place.
+// Node layout (kWideF4 float4s, 128 bytes), structure of arrays over the four
+// children:
+//   [2a], [2a + 1]  centres and half extents of the child boxes on axis a
+//   [6]             child words: an internal child's wide index, or a leaf's
+//                   0x80000000 | slot (flags kept)
+// The boxes are those of the binary traversal records (widened, hoisted leaves
+// taken out); an unused entry's is empty (half extents -inf).
+// wide_src[kWideW w + c] is the record of child c, 2 p + side for binary node
+// p (or kNoRecord), from which a refit of moved spheres copies the box again.
 // ---------------------------------------------------------------------------
 constexpr int kWideChildren = kWideW;
 
@@ -1090,9 +1088,15 @@ __device__ __forceinline__ float box_area(float4 lo, float4 hi) {
     return dx * dy + dy * dz + dz * dx;
 }
 
-__device__ int wide_collapse(const float4* __restrict__ nodes, int32_t r, int32_t w[kWideChildren]) {
+constexpr int32_t kNoRecord = -1;
+
+// w: the entries' words, rec: the traversal records they come from.
+__device__ int wide_collapse(const float4* __restrict__ nodes, int32_t r, int32_t w[kWideChildren],
+                             int32_t rec[kWideChildren]) {
     w[0] = __float_as_int(nodes[2 * r].w);
     w[1] = __float_as_int(nodes[2 * r + 1].w);
+    rec[0] = 2 * r;
+    rec[1] = 2 * r + 1;
     int cnt = 2;
     while (cnt < kWideChildren) {
         int best = -1;
@@ -1108,6 +1112,8 @@ __device__ int wide_collapse(const float4* __restrict__ nodes, int32_t r, int32_
         if (best < 0) break;
         const int32_t q = w[best];
         w[best] = __float_as_int(nodes[2 * q].w);
+        rec[best] = 2 * q;
+        rec[cnt] = 2 * q + 1;
         w[cnt++] = __float_as_int(nodes[2 * q + 1].w);
     }
     return cnt;
@@ -1119,8 +1125,8 @@ __global__ void k_wide_frontier(const float4* __restrict__ nodes, const int32_t*
                                 int32_t* __restrict__ fout, uint32_t* __restrict__ nout, uint32_t* __restrict__ flag) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nin) return;
-    int32_t w[kWideChildren];
-    const int c = wide_collapse(nodes, fin[i], w);
+    int32_t w[kWideChildren], rec[kWideChildren];
+    const int c = wide_collapse(nodes, fin[i], w, rec);
     for (int j = 0; j < c; ++j) {
         if (w[j] & kLeaf) continue;
         flag[w[j]] = 1u;
@@ -1128,91 +1134,58 @@ __global__ void k_wide_frontier(const float4* __restrict__ nodes, const int32_t*
     }
 }
 
-// Writes wide node w from the binary words of its children (src[0..7];
-// kLeaf | kHoisted for an unused entry).  idx maps a binary internal node to
-// its wide index.
-__device__ void wide_write_node(const float4* __restrict__ nodes, const float4* __restrict__ sph,
-                                const uint32_t* __restrict__ idx, const int32_t* src, float4* __restrict__ W) {
-    float lo[3][kWideChildren], hi[3][kWideChildren];
-    int32_t word[kWideChildren];
-    uint32_t valid = 0, leafm = 0;
-    for (int c = 0; c < kWideChildren; ++c) {
-        const int32_t b = src[c];
-        float4 l = make_float4(0.0f, 0.0f, 0.0f, 0.0f), h = l;
-        if (b & kLeaf) {
-            word[c] = b;
-            if (!(b & kHoisted)) {
-                leaf_box(sph[b & kSlotMask], l, h);
-                valid |= 1u << c;
-                leafm |= 1u << c;
-            }
-        } else {
-            l = nodes[2 * b];
-            h = nodes[2 * b + 1];
-            word[c] = (int32_t)idx[b];
-            valid |= 1u << c;
+// The boxes of a wide node from its children's traversal records.
+__device__ void wide_boxes(const float4* __restrict__ trav, const int32_t rec[kWideChildren], float4* __restrict__ W) {
+    float c[3][kWideChildren], h[3][kWideChildren];
+    for (int j = 0; j < kWideChildren; ++j) {
+        float4 a = make_float4(0.0f, 0.0f, -INFINITY, -INFINITY), b = make_float4(0.0f, -INFINITY, 0.0f, 0.0f);
+        if (rec[j] != kNoRecord) {
+            a = trav[2 * (size_t)rec[j]];
+            b = trav[2 * (size_t)rec[j] + 1];
         }
-        lo[0][c] = l.x; lo[1][c] = l.y; lo[2][c] = l.z;
-        hi[0][c] = h.x; hi[1][c] = h.y; hi[2][c] = h.z;
+        c[0][j] = a.x; c[1][j] = a.y; c[2][j] = b.x;
+        h[0][j] = a.z; h[1][j] = a.w; h[2][j] = b.y;
     }
     for (int a = 0; a < 3; ++a) {
-        for (int half = 0; half < kWideH; ++half) {
-            const int c = 4 * half;
-            W[2 * a * kWideH + half] = make_float4(lo[a][c], lo[a][c + 1], lo[a][c + 2], lo[a][c + 3]);
-            W[(2 * a + 1) * kWideH + half] = make_float4(hi[a][c], hi[a][c + 1], hi[a][c + 2], hi[a][c + 3]);
-        }
+        W[2 * a] = make_float4(c[a][0], c[a][1], c[a][2], c[a][3]);
+        W[2 * a + 1] = make_float4(h[a][0], h[a][1], h[a][2], h[a][3]);
     }
-    for (int half = 0; half < kWideH; ++half) {
-        const int c = 4 * half;
-        W[6 * kWideH + half] = make_float4(__int_as_float(word[c]), __int_as_float(word[c + 1]),
-                                           __int_as_float(word[c + 2]), __int_as_float(word[c + 3]));
-    }
-    W[7 * kWideH] = make_float4(__int_as_float((int)(valid | (leafm << 8))), 0.0f, 0.0f, 0.0f);
-    if (kWideH == 2) W[15] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
 // One thread per binary internal node; the flagged ones write their wide node.
-__global__ void k_wide_write(const float4* __restrict__ nodes, const float4* __restrict__ sph, uint32_t n,
+// idx maps a binary internal node to its wide index.
+__global__ void k_wide_write(const float4* __restrict__ nodes, const float4* __restrict__ trav, uint32_t n,
                              const uint32_t* __restrict__ flag, const uint32_t* __restrict__ idx,
                              float4* __restrict__ wide, int32_t* __restrict__ wide_src) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n - 1 || !flag[r]) return;
-    int32_t w[kWideChildren];
-    const int c = wide_collapse(nodes, (int32_t)r, w);
-    for (int j = c; j < kWideChildren; ++j) w[j] = kLeaf | kHoisted;
+    int32_t w[kWideChildren], rec[kWideChildren];
+    const int c = wide_collapse(nodes, (int32_t)r, w, rec);
+    for (int j = 0; j < kWideChildren; ++j) {
+        if (j >= c) {
+            w[j] = kLeaf | kHoisted;
+            rec[j] = kNoRecord;
+        } else if (!(w[j] & kLeaf)) {
+            w[j] = (int32_t)idx[w[j]];
+        }
+    }
     const uint32_t k = idx[r];
-    for (int j = 0; j < kWideChildren; ++j) wide_src[(size_t)kWideChildren * k + j] = w[j];
-    wide_write_node(nodes, sph, idx, w, wide + kWideF4 * (size_t)k);
+    for (int j = 0; j < kWideChildren; ++j) wide_src[(size_t)kWideChildren * k + j] = rec[j];
+    float4* W = wide + kWideF4 * (size_t)k;
+    wide_boxes(trav, rec, W);
+    W[6] = make_float4(__int_as_float(w[0]), __int_as_float(w[1]), __int_as_float(w[2]), __int_as_float(w[3]));
+    W[7] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
-// Refit of moved spheres: the same topology, boxes recomputed from the
-// refit binary nodes and the new spheres.  idx is not needed: the child
-// words of internal children stay as they are.
-__global__ void k_wide_refit(const float4* __restrict__ nodes, const float4* __restrict__ sph, uint32_t nwide,
-                             const int32_t* __restrict__ wide_src, float4* __restrict__ wide) {
+// Refit of moved spheres: the same topology and words, the boxes from the
+// refit traversal records.
+__global__ void k_wide_refit(const float4* __restrict__ trav, uint32_t nwide, const int32_t* __restrict__ wide_src,
+                             float4* __restrict__ wide) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nwide) return;
-    float4* W = wide + kWideF4 * (size_t)k;
-    float lo[3][kWideChildren], hi[3][kWideChildren];
-    for (int c = 0; c < kWideChildren; ++c) {
-        const int32_t b = wide_src[(size_t)kWideChildren * k + c];
-        float4 l = make_float4(0.0f, 0.0f, 0.0f, 0.0f), h = l;
-        if (b & kLeaf) {
-            if (!(b & kHoisted)) leaf_box(sph[b & kSlotMask], l, h);
-        } else {
-            l = nodes[2 * b];
-            h = nodes[2 * b + 1];
-        }
-        lo[0][c] = l.x; lo[1][c] = l.y; lo[2][c] = l.z;
-        hi[0][c] = h.x; hi[1][c] = h.y; hi[2][c] = h.z;
-    }
-    for (int a = 0; a < 3; ++a) {
-        for (int half = 0; half < kWideH; ++half) {
-            const int c = 4 * half;
-            W[2 * a * kWideH + half] = make_float4(lo[a][c], lo[a][c + 1], lo[a][c + 2], lo[a][c + 3]);
-            W[(2 * a + 1) * kWideH + half] = make_float4(hi[a][c], hi[a][c + 1], hi[a][c + 2], hi[a][c + 3]);
-        }
-    }
+    int32_t rec[kWideChildren];
+    for (int j = 0; j < kWideChildren; ++j) rec[j] = wide_src[(size_t)kWideChildren * k + j];
+    wide_boxes(trav, rec, wide + kWideF4 * (size_t)k);
 }
 
 inline uint32_t cdiv(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
@@ -1371,7 +1344,7 @@ venu_status build_wide(const venu_scene* S, cudaStream_t st) {
     WSTEP(cudaMalloc(&S->wide_src, sizeof(int32_t) * kWideChildren * (size_t)nwide));
     S->nwide = nwide;
     S->bytes += sizeof(float4) * kWideF4 * (size_t)nwide + sizeof(int32_t) * kWideChildren * (size_t)nwide;
-    k_wide_write<<<cdiv(nint, 128), 128, 0, st>>>(S->nodes, S->sph, n, flag, idx, S->wide, S->wide_src);
+    k_wide_write<<<cdiv(nint, 128), 128, 0, st>>>(S->nodes, S->trav, n, flag, idx, S->wide, S->wide_src);
     WSTEP(cudaGetLastError());
     WSTEP(cudaStreamSynchronize(st));
 #undef WSTEP
@@ -1526,7 +1499,7 @@ venu_status update_scene(venu_scene* S, const venu_sphere* s, bool on_host, cuda
     VENU_CUDA(launch_trav_layout(S->nodes, S->sph, n, S->trav, S->parents, S->parents + (n - 1), nullptr, list, nullptr,
                                  st));
     if (S->nwide)
-        k_wide_refit<<<cdiv(S->nwide, 128), 128, 0, st>>>(S->nodes, S->sph, S->nwide, S->wide_src, S->wide);
+        k_wide_refit<<<cdiv(S->nwide, 128), 128, 0, st>>>(S->trav, S->nwide, S->wide_src, S->wide);
     VENU_CUDA(cudaGetLastError());
     return VENU_OK;
 }

@@ -221,18 +221,11 @@ constexpr int32_t kSlotMask = 0x3fffffff;
 constexpr int32_t kNone = 0x7fffffff;
 constexpr int kMaxHoisted = 4;
 
-// Children per node of the wide traversal tree (4; 8 measured slower on
-// every workload here) and its node layout in float4s: per axis a
-// the lo planes of the children at 2a*H + h and the hi planes at
-// (2a+1)*H + h (h = 0..H-1, four children per float4), then the child words
-// at 6H + h and the masks at 7H.
-#ifndef VENU_WIDE_CHILDREN
-#define VENU_WIDE_CHILDREN 4
-#endif
-constexpr int kWideW = VENU_WIDE_CHILDREN;
-constexpr int kWideH = kWideW / 4;
-constexpr int kWideF4 = 8 * kWideH;
-static_assert(kWideW == 4 || kWideW == 8, "the wide tree has 4 or 8 children per node");
+// Children per node of the wide traversal tree (4; 8 measured slower on every
+// workload here) and its float4s: centres and half extents of the four
+// children's boxes per axis at 2a and 2a + 1, then the child words at 6.
+constexpr int kWideW = 4;
+constexpr int kWideF4 = 8;
 
 struct SceneView {
     const float4* __restrict__ nodes;  // 2 float4 per internal node: {lo, left} {hi, right}
@@ -791,53 +784,32 @@ struct Tracer {
 // Closest-hit traversal of the wide tree (node layout in lbvh.cu).
 //
 // A step loads one node and tests all of its child boxes with the same
-// instructions in every lane (structure-of-arrays loads, four children per
-// float4), pushes the hit internal children but the nearest farthest first
+// instructions in every lane (the fast walk's boxes and margins, with the same
+// bounds: three FMAs a slab and no minimum or maximum, which run at half
+// rate), pushes the hit internal children but the nearest farthest first
 // onto the same shared-memory / local-memory stack as the binary traversal
 // (ordered by a sorting network on keys of entry distance and child number
 // when more than two are hit), tests the spheres of the leaf children whose
 // boxes were hit, then descends to the nearest child unless a sphere hit now
 // culls it, else pops (popped entries are culled against the closest hit).
 // ---------------------------------------------------------------------------
-template <bool AXIS>
-__device__ __forceinline__ bool box_test_s(const RayPre& R, float lx, float ly, float lz, float hx, float hy,
-                                           float hz, float tmin, float tcap, float& tnear) {
-    const f3 nh = AXIS ? R.n1 : R.n0;
-    float t0x = fmaf(lx, R.inv.x, R.n0.x), t1x = fmaf(hx, R.inv.x, nh.x);
-    float t0y = fmaf(ly, R.inv.y, R.n0.y), t1y = fmaf(hy, R.inv.y, nh.y);
-    float t0z = fmaf(lz, R.inv.z, R.n0.z), t1z = fmaf(hz, R.inv.z, nh.z);
-    float tn = fmax3(fminf(t0x, t1x), fminf(t0y, t1y), fmaxf(fminf(t0z, t1z), tmin));
-    float tf = fmin3(fmaxf(t0x, t1x), fmaxf(t0y, t1y), fminf(fmaxf(t0z, t1z), tcap));
-    tnear = tn;
-    return AXIS ? tn <= tf * 1.00000095367431640625f : tn <= fmaf(tf, 1.00000095367431640625f, R.n1.x);
-}
-
 __device__ __forceinline__ void cswap(uint32_t& a, uint32_t& b) {
     const uint32_t lo = min(a, b), hi = max(a, b);
     a = lo;
     b = hi;
 }
 
-// Batcher's odd-even merge sort of 8 keys, ascending (19 comparators).
+// Batcher's odd-even merge sort of 4 keys, ascending.
 __device__ __forceinline__ void sort4(uint32_t k[4]) {
     cswap(k[0], k[1]); cswap(k[2], k[3]);
     cswap(k[0], k[2]); cswap(k[1], k[3]);
     cswap(k[1], k[2]);
 }
 
-__device__ __forceinline__ void sort8(uint32_t k[8]) {
-    cswap(k[0], k[1]); cswap(k[2], k[3]); cswap(k[4], k[5]); cswap(k[6], k[7]);
-    cswap(k[0], k[2]); cswap(k[1], k[3]); cswap(k[4], k[6]); cswap(k[5], k[7]);
-    cswap(k[1], k[2]); cswap(k[5], k[6]);
-    cswap(k[0], k[4]); cswap(k[1], k[5]); cswap(k[2], k[6]); cswap(k[3], k[7]);
-    cswap(k[2], k[4]); cswap(k[3], k[5]);
-    cswap(k[1], k[2]); cswap(k[3], k[4]); cswap(k[5], k[6]);
-}
-
-template <bool COUNT, bool AXIS = false, int KS = kShared>
+template <bool COUNT, int KS = kShared>
 struct WideTracer {
     RayPre R;
-    float tmin, tmax, best_t;
+    float tmin, tmax, best_t, m;
     int32_t best, cur;
     int sp;
     uint32_t guard;
@@ -850,9 +822,20 @@ struct WideTracer {
         }
     }
 
-    __device__ __forceinline__ bool begin(const SceneView& S, const RayPre& R_, float, float tmin_, float tmax_,
+    // Entry (clipped to tmin) and exit of a box.
+    __device__ __forceinline__ void interval(float cx, float hx, float cy, float hy, float cz, float hz, float& tn,
+                                             float& tf) const {
+        const float tx = fmaf(cx, R.inv.x, R.n0.x), ty = fmaf(cy, R.inv.y, R.n0.y), tz = fmaf(cz, R.inv.z, R.n0.z);
+        const float ax = fabsf(R.inv.x), ay = fabsf(R.inv.y), az = fabsf(R.inv.z);
+        tn = fmaxf(fmax3(fmaf(hx, -ax, tx), fmaf(hy, -ay, ty), fmaf(hz, -az, tz)), tmin);
+        tf = fmin3(fmaf(hx, ax, tx), fmaf(hy, ay, ty), fmaf(hz, az, tz));
+    }
+    __device__ __forceinline__ bool meets(float tn, float tf) const { return tn <= fminf(tf, best_t) + m; }
+
+    __device__ __forceinline__ bool begin(const SceneView& S, const RayPre& R_, float m_, float tmin_, float tmax_,
                                           TraceCounters& K) {
         R = R_;
+        m = m_;
         tmin = tmin_;
         tmax = tmax_;
         best_t = tmax_;
@@ -862,10 +845,11 @@ struct WideTracer {
         if (n == 0) return false;
         up_front(*this, S, K);
         if (n == 1) return false;
-        float tn;
-        float4 rlo = __ldg(S.nodes + 0), rhi = __ldg(S.nodes + 1);
+        const float4 r0 = __ldg(root_record(S)), r1 = __ldg(root_record(S) + 1);
+        float tn, tf;
+        interval(r0.x, r0.z, r0.y, r0.w, r1.x, r1.y, tn, tf);
         if (COUNT) ++K.nodes;
-        if (!box_test<AXIS>(R, rlo, rhi, tmin, best_t, tn)) return false;
+        if (!meets(tn, tf)) return false;
         cur = 0;
         // every wide node is expanded at most once per ray, and there are
         // fewer than n of them: the guard turns a cyclic tree into an error
@@ -900,35 +884,43 @@ struct WideTracer {
             if ((tid & 31u) == (uint32_t)(__ffs(am) - 1)) ++K.warp_steps;
         }
         const float4* N = S.wide + kWideF4 * (size_t)cur;
-        const uint32_t masks = __float_as_uint(__ldg(N + 7 * kWideH).x);
-        const uint32_t leafm = (masks >> 8) & 0xffu, intm = masks & ~leafm & 0xffu;
         // key of child c: its entry distance's bits with c in the low three
         // bits (distances are >= tmin > 0, so the bits order like the
         // values; the cut makes a key's distance a lower bound), all ones
-        // unless it is a hit internal child
+        // unless it is a hit internal child.  Unused entries and hoisted
+        // leaves have empty boxes.
         uint32_t key[kWideW];
         uint32_t lhit = 0;
-#pragma unroll
-        for (int h = 0; h < kWideH; ++h) {
-            const float4 lx = __ldg(N + h), hx = __ldg(N + kWideH + h);
-            const float4 ly = __ldg(N + 2 * kWideH + h), hy = __ldg(N + 3 * kWideH + h);
-            const float4 lz = __ldg(N + 4 * kWideH + h), hz = __ldg(N + 5 * kWideH + h);
-            float t;
-#define VENU_WIDE_CHILD(J, C)                                                                       \
-    {                                                                                               \
-        const bool ok = box_test_s<AXIS>(R, lx.C, ly.C, lz.C, hx.C, hy.C, hz.C, tmin, best_t, t); \
-        lhit |= (uint32_t)ok << (J);                                                                \
-        key[J] = (ok && ((intm >> (J)) & 1u)) ? ((__float_as_uint(t) & ~7u) | (uint32_t)(J)) : 0xffffffffu; \
+        const int32_t* words = reinterpret_cast<const int32_t*>(N + 6);
+        {
+            const int4 w4 = __ldg(reinterpret_cast<const int4*>(words));
+            if (COUNT) K.nodes += (w4.x >= 0) + (w4.y >= 0) + (w4.z >= 0) + (w4.w >= 0);
+            f2 cx01, cx23, hx01, hx23, cy01, cy23, hy01, hy23, cz01, cz23, hz01, hz23;
+            ldg32(N, cx01, cx23, hx01, hx23);
+            ldg32(N + 2, cy01, cy23, hy01, hy23);
+            ldg32(N + 4, cz01, cz23, hz01, hz23);
+#define VENU_WIDE_PAIR(P, I, W0, W1)                                                                  \
+    {                                                                                                 \
+        float cxa, cxb, hxa, hxb, cya, cyb, hya, hyb, cza, czb, hza, hzb, tn, tf;                     \
+        unpack2(cx##P, cxa, cxb);                                                                     \
+        unpack2(hx##P, hxa, hxb);                                                                     \
+        unpack2(cy##P, cya, cyb);                                                                     \
+        unpack2(hy##P, hya, hyb);                                                                     \
+        unpack2(cz##P, cza, czb);                                                                     \
+        unpack2(hz##P, hza, hzb);                                                                     \
+        interval(cxa, hxa, cya, hya, cza, hza, tn, tf);                                               \
+        bool ok = meets(tn, tf);                                                                      \
+        lhit |= (uint32_t)(ok && (W0) < 0) << (I);                                                    \
+        key[I] = ok && (W0) >= 0 ? (__float_as_uint(tn) & ~7u) | (uint32_t)(I) : 0xffffffffu;         \
+        interval(cxb, hxb, cyb, hyb, czb, hzb, tn, tf);                                               \
+        ok = meets(tn, tf);                                                                           \
+        lhit |= (uint32_t)(ok && (W1) < 0) << ((I) + 1);                                              \
+        key[(I) + 1] = ok && (W1) >= 0 ? (__float_as_uint(tn) & ~7u) | (uint32_t)((I) + 1) : 0xffffffffu; \
     }
-            VENU_WIDE_CHILD(4 * h + 0, x)
-            VENU_WIDE_CHILD(4 * h + 1, y)
-            VENU_WIDE_CHILD(4 * h + 2, z)
-            VENU_WIDE_CHILD(4 * h + 3, w)
-#undef VENU_WIDE_CHILD
+            VENU_WIDE_PAIR(01, 0, w4.x, w4.y)
+            VENU_WIDE_PAIR(23, 2, w4.z, w4.w)
+#undef VENU_WIDE_PAIR
         }
-        lhit &= leafm;
-        if (COUNT) K.nodes += (uint32_t)__popc(masks & 0xffu);
-        const int32_t* words = reinterpret_cast<const int32_t*>(N + 6 * kWideH);
         // the hit internal children but the nearest onto the stack, farthest
         // first (one or two hits without sorting); the nearest is descended
         // unless the leaf tests below cull it
@@ -946,7 +938,7 @@ struct WideTracer {
                 push(sm, tid, bdim, spill, overflow, __ldg(words + (kmax & 7u)),
                      __uint_as_float(kmax & ~7u));
             } else if (nhit > 2u) {
-                if (kWideW == 8) sort8(key); else sort4(key);
+                sort4(key);
 #pragma unroll
                 for (int i = kWideW - 1; i >= 1; --i) {
                     if (key[i] != 0xffffffffu)
@@ -965,7 +957,7 @@ struct WideTracer {
                 leaf(k, __ldg(S.sph + k));
             }
         }
-        if (kmin != 0xffffffffu && __uint_as_float(kmin & ~7u) <= best_t) {
+        if (kmin != 0xffffffffu && __uint_as_float(kmin & ~7u) <= best_t + m) {
             cur = __ldg(words + (kmin & 7u));
             return true;
         }
@@ -974,7 +966,7 @@ struct WideTracer {
             int2* const p = sm.e + ((uint32_t)(sp & (KS - 1)) * bdim + tid);
             const int2 e = *p;
             if (sp >= KS) *p = spill[sp - KS];
-            if (__int_as_float(e.y) <= best_t) {
+            if (__int_as_float(e.y) <= best_t + m) {
                 cur = e.x;
                 return true;
             }
@@ -994,7 +986,7 @@ struct WideTracer {
 
 template <bool COUNT, bool WIDE = false>
 __device__ __forceinline__ RayPre prep_for(f3 o, f3 d) {
-    return prep<!COUNT && !WIDE>(o, d);
+    return prep<!COUNT || WIDE>(o, d);
 }
 
 template <class T>
@@ -1009,31 +1001,26 @@ __device__ __forceinline__ int32_t trace_with(const SceneView& S, const RayPre& 
     return W.result(t_out);
 }
 
-// Closest hit of one ray (R from prep_for<COUNT, WIDE>).  The binary tree: the fast walk,
-// unless the ray starts far outside the scene (rare) or the build counts;
-// those, and the wide tree, take the shared-margin loop, or the per-axis one
-// for the rare near-axis-parallel ray.  KS: shared-memory stack entries per
-// thread (the kernel's StackSmem holds KS of them).
+// Closest hit of one ray (R from prep_for<COUNT, WIDE>): the fast walk, over
+// the binary or the wide tree.  Rays that start far outside the scene (rare)
+// take the canonical walk with per-axis margins; counting builds of the binary
+// tree the canonical walk with one margin, or per axis for the rare
+// near-axis-parallel ray.  KS: shared-memory stack entries per thread (the
+// kernel's StackSmem holds KS of them).
 template <bool COUNT, int KS = kShared, bool WIDE = false>
 __device__ __forceinline__ int32_t trace_closest(const SceneView& S, const RayPre& R, float tmin,
                                                  float tmax, float& t_out, StackSmem sm,
                                                  uint32_t tid, uint32_t bdim, bool& overflow,
                                                  TraceCounters& K) {
-    if (WIDE) {
-        if (R.axis) {
-            RayPre A = R;
-            axis_margins(A);
-            return trace_with<WideTracer<COUNT, true, KS>>(S, A, 0.0f, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
-        }
-        return trace_with<WideTracer<COUNT, false, KS>>(S, R, 0.0f, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
-    }
-    const float m = COUNT ? 0.0f : ray_margin(S, R);
-    if (COUNT ? R.axis : !(m <= kFarMarginMax)) {
+    const float m = COUNT && !WIDE ? 0.0f : ray_margin(S, R);
+    if (COUNT && !WIDE ? R.axis : !(m <= kFarMarginMax)) {
         RayPre A = prep<false>(R.o, R.d);
         A.from = R.from;
         axis_margins(A);
         return trace_with<Tracer<COUNT, true, true, KS>>(S, A, 0.0f, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
     }
+    if (WIDE)
+        return trace_with<WideTracer<COUNT, KS>>(S, R, m, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
     return trace_with<Tracer<COUNT, COUNT, false, KS>>(S, R, m, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
 }
 
