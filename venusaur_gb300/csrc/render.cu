@@ -81,17 +81,35 @@ __global__ void k_raygen(venu_camera cam, uint32_t W, uint32_t H, uint32_t p0, u
     seeds[pix] = seed;
 }
 
-// WIDE: over the 4-wide tree (variant 5's later bounces).
-// The separate traversal and shading kernels read each queue entry and hit
-// record once: they load and store them evict-first (ld/st.global.cs), which
-// leaves more of L1 and L2 to the node set (1M spheres, variant 3: +0.5 %).
-// The fused kernel keeps plain accesses: the same hints measured -0.45 % on
-// the RTIOW scene there.
+// The separate traversal.  WIDE: over the 4-wide tree (variant 5's later
+// bounces).  The separate traversal and shading kernels read each queue entry
+// and hit record once: they load and store them evict-first
+// (ld/st.global.cs), which leaves more of L1 and L2 to the node set (1M
+// spheres, variant 3: +0.5 %).  The fused kernel keeps plain accesses: the
+// same hints measured -0.45 % on the RTIOW scene there.
+//
+// A bounce of at least walk_min rays is split over two kernels: this one only
+// tests each ray against the sphere it leaves and the hoisted ones, a whole
+// warp at a time, and leaves its closest hit so far in the hit record; k_walk
+// walks the tree from there with lanes that take a new ray when theirs is
+// done.  On large scenes a warp has 12 of 32 lanes in its walk on average
+// (its rays take 20 to 400 steps) and waits for L2 most of the time; the
+// refills bring that to 24.  They only pay because a refill is cheap -- the
+// up-front tests with their long refined branch are done -- and because lanes
+// vote every kWalkSteps steps only and walk on by themselves in between (a
+// vote a step costs more than the lanes it fills).  Then the L1 data pipe is
+// the bound (85 % of its wavefronts: two 32-byte loads a step and lane).
+// Bounces of few rays end with their longest walk either way.
+constexpr int32_t kHitDone = 0x40000000;  // in a hit record: nothing left to walk
+constexpr int32_t kMissDone = kHitDone | 0x3fffffff;
+constexpr int kWalkSteps = 16;
+constexpr uint32_t kWalkRefill = 8;  // idle lanes of a warp that fetch together
+
 template <bool COUNT, bool WIDE = false>
 __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const uint32_t* __restrict__ cnt,
                                                   uint32_t* __restrict__ work, int2* __restrict__ hits,
                                                   uint32_t* __restrict__ err,
-                                                  unsigned long long* __restrict__ stats) {
+                                                  unsigned long long* __restrict__ stats, uint32_t walk_min) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
     sm.e = reinterpret_cast<int2*>(smem);
@@ -100,6 +118,31 @@ __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const ui
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats, (unsigned long long)n);
     TraceCounters K{0, 0};
     bool overflow = false;
+    if (!COUNT && !WIDE && n >= walk_min) {
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            const float4 o4 = __ldcs(q.o + i), d4 = __ldcs(q.d + i);
+            RayPre R = prep_for<false>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            R.from = packed_from(d4.w);
+            float t;
+            int32_t k;
+            if (!(ray_margin(S, R) <= kFarMarginMax)) {  // rare: traced to the end now
+                R = prep<false>(R.o, R.d);
+                R.from = packed_from(d4.w);
+                axis_margins(R);
+                k = trace_with<Tracer<false, true, true>>(S, R, 0.0f, 0.001f, 1e16f, t, sm, threadIdx.x, blockDim.x,
+                                                          overflow, K);
+                k = k < 0 ? kMissDone : k | kHitDone;
+            } else {
+                Tracer<false> T;
+                T.open(R, 0.0f, 0.001f, 1e16f, 1e16f, kNone);
+                up_front(T, S, K);
+                k = T.result(t);
+            }
+            hits[i] = make_int2(__float_as_int(t), k);
+        }
+        if (overflow) atomicOr(err, 1u);
+        return;
+    }
     for (;;) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(work, 32u);
@@ -118,6 +161,63 @@ __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const ui
     }
     if (overflow) atomicOr(err, 1u);
     if (COUNT) flush_counters(K, stats);
+}
+
+__global__ void VENU_TRACE_BOUNDS k_walk(SceneView S, Queue q, const uint32_t* __restrict__ cnt,
+                                         uint32_t* __restrict__ work, int2* __restrict__ hits,
+                                         uint32_t* __restrict__ err, uint32_t walk_min) {
+    extern __shared__ unsigned char smem[];
+    StackSmem sm;
+    sm.e = reinterpret_cast<int2*>(smem);
+    const uint32_t n = *cnt;
+    if (n < walk_min) return;  // k_traverse did it
+    const uint32_t lane = threadIdx.x & 31;
+    TraceCounters K{0, 0};
+    bool overflow = false;
+    Tracer<false> T;
+    int2 spill[kSpill];
+    uint32_t ray = 0;
+    bool active = false;
+    for (uint32_t idle = 0xffffffffu;;) {
+        // the idle lanes take the next rays
+        const uint32_t take = (uint32_t)__popc(idle);
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(work, take);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const bool exhausted = base >= n || n - base <= take;
+        if (!active && base < n) {
+            ray = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (ray < n) {
+                const int2 h = hits[ray];
+                if (h.y >= kHitDone) {
+                    hits[ray].y = h.y == kMissDone ? -1 : h.y & (kHitDone - 1);
+                } else {
+                    const float4 o4 = __ldcs(q.o + ray), d4 = __ldcs(q.d + ray);
+                    RayPre R = prep_for<false>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+                    R.from = packed_from(d4.w);
+                    T.open(R, ray_margin(S, R), 0.001f, 1e16f, __int_as_float(h.x), h.y < 0 ? kNone : h.y);
+                    active = T.enter(S, K);  // else the record stands as it is
+                }
+            }
+        }
+        // walk until enough lanes are idle, at the end until all are
+        const uint32_t enough = exhausted ? 32u : kWalkRefill;
+        for (;;) {
+            idle = __ballot_sync(0xffffffffu, !active);
+            if ((uint32_t)__popc(idle) >= enough) break;
+            if (active) {
+                for (int i = 0; i < kWalkSteps && active; ++i)
+                    active = T.step(S, sm, threadIdx.x, blockDim.x, spill, overflow, K);
+                if (!active) {
+                    float t;
+                    const int32_t k = T.result(t);
+                    __stcs(hits + ray, make_int2(__float_as_int(t), k));
+                }
+            }
+        }
+        if (exhausted) break;
+    }
+    if (overflow) atomicOr(err, 1u);
 }
 
 // Persistent lanes: a lane whose ray is finished takes a new one as soon as
@@ -683,7 +783,7 @@ struct venu_renderer {
     uint32_t* err = nullptr;
     unsigned long long* stats = nullptr;  // segments, nodes, spheres, lane / warp steps, graph bounces
     venu_tuning tune = {2u, 32u, 128u, 0u, 128u, 0u, 1u};
-    int trav_blocks = 0, shade_blocks = 0, fused_blocks = 0, finish_blocks = 0;
+    int trav_blocks = 0, shade_blocks = 0, fused_blocks = 0, finish_blocks = 0, walk_blocks = 0;
     venu_render_stats last = {};
     uint32_t host_launches = 0;  // kernels the last render launched from the host
     bool graph_off = false;      // the wave graph could not be built: host bounce loops only
@@ -701,6 +801,14 @@ struct venu_renderer {
 namespace {
 constexpr int kTravBlock = 128;  // venu_trace
 constexpr uint32_t kMaxDepth = 64;
+// Where k_traverse is split (variants 0 and 3; ms without -> with, from 1M rays
+// up).  By scene, 1080p x 8: 485 spheres 4.96 -> 5.43, 2k 5.00 -> 5.24, 7k 8.73
+// -> 8.79, 20k 14.45 -> 14.01, 100k 33.4 -> 30.7, 300k 60.9 -> 54.0, 1M 153.3 ->
+// 133.1 (short walks do not need the refills).  By rays: split from 512k up,
+// 640x360 x 4 on 300k spheres takes 8.80 instead of 8.48; from 2M up, 1280x720
+// x 8 on 1M spheres 65.1 instead of 64.4.
+constexpr uint32_t kWalkSpheres = 16384, kWalkRays = 1u << 20;
+
 
 template <typename K>
 cudaError_t occupancy_grid(K kernel, int block, size_t smem, uint32_t per_sm_cap, int& grid) {
@@ -776,6 +884,8 @@ cudaError_t configure(venu_renderer* r) {
         e = occupancy_grid(k_traverse<false>, tb, sm, t.traverse_blocks_per_sm, r->trav_blocks);
         if (e == cudaSuccess) e = set_smem(k_traverse<true>, sm);
         if (e == cudaSuccess) e = prefer_l1(k_traverse<false>, std::max(1, r->trav_blocks / nsm), sm);
+        if (e == cudaSuccess) e = occupancy_grid(k_walk, tb, sm, t.traverse_blocks_per_sm, r->walk_blocks);
+        if (e == cudaSuccess) e = prefer_l1(k_walk, std::max(1, r->walk_blocks / nsm), sm);
     } else if (t.traverse_variant == 1) {
         e = occupancy_grid(k_traverse_dyn<false>, tb, sm, t.traverse_blocks_per_sm, r->trav_blocks);
         if (e == cudaSuccess) e = set_smem(k_traverse_dyn<true>, sm);
@@ -1111,6 +1221,9 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
     // the SM's memory to L1 (measured: RTIOW +0.5 %; 1M spheres -4.5 %)
     const bool shallow = scene->n <= 4096u;
     uint32_t* const path_seeds = gen0 ? reinterpret_cast<uint32_t*>(r->q[0].t) : nullptr;
+    // bounces that k_walk takes (see k_traverse): counting builds never split
+    const uint32_t walk_min =
+        !count && scene->n >= kWalkSpheres && (uint64_t)npix * k >= kWalkRays ? kWalkRays : ~0u;
     // the fused variants run each wave's bounce loop as one graph launch
     // (WaveCtl) when every wave covers all pixels, so that the graph's
     // parameters are the same for every wave; the profiling build times
@@ -1238,17 +1351,22 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
                 if (v == 0) {
                     if (count)
                         k_traverse<true><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b, r->hits,
-                                                                         r->err, r->stats);
+                                                                         r->err, r->stats, ~0u);
                     else
                         k_traverse<false><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b, r->hits,
-                                                                          r->err, r->stats);
+                                                                          r->err, r->stats, walk_min);
+                    if (walk_min != ~0u) {
+                        k_walk<<<r->walk_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b, r->hits, r->err,
+                                                                walk_min);
+                        ++launches;
+                    }
                 } else if (v == 5) {
                     if (count)
                         k_traverse<true, true><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b,
-                                                                               r->hits, r->err, r->stats);
+                                                                               r->hits, r->err, r->stats, ~0u);
                     else
                         k_traverse<false, true><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b,
-                                                                                r->hits, r->err, r->stats);
+                                                                                r->hits, r->err, r->stats, ~0u);
                 } else {
                     if (count)
                         k_traverse_dyn<true><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b, r->hits,
