@@ -693,24 +693,16 @@ __global__ void k_accumulate(const float4* __restrict__ slots, uint32_t p0, uint
     }
 }
 
-// Arbitrary rays -> closest hit (t, original id, front face).
-__global__ void __launch_bounds__(128) k_trace_rays(SceneView S, const float* __restrict__ rays, uint32_t n,
-                                                    float tmin, float tmax, float* __restrict__ t_out,
-                                                    int32_t* __restrict__ id_out, uint32_t* __restrict__ front_out,
-                                                    uint32_t* __restrict__ err) {
-    extern __shared__ unsigned char smem[];
-    StackSmem sm;
-    sm.e = reinterpret_cast<int2*>(smem);
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    f3 o = mk(rays[6 * (size_t)i], rays[6 * (size_t)i + 1], rays[6 * (size_t)i + 2]);
-    f3 d = mk(rays[6 * (size_t)i + 3], rays[6 * (size_t)i + 4], rays[6 * (size_t)i + 5]);
-    RayPre R = prep_for<false>(o, d);
-    TraceCounters K{0, 0};
-    bool overflow = false;
-    float t;
-    int32_t k = trace_closest<false>(S, R, tmin, tmax, t, sm, threadIdx.x, blockDim.x, overflow, K);
-    if (overflow) atomicOr(err, 1u);
+__device__ __forceinline__ void load_ray(const float* __restrict__ rays, uint32_t i, f3& o, f3& d) {
+    const float* r = rays + 6 * (size_t)i;
+    o = mk(r[0], r[1], r[2]);
+    d = mk(r[3], r[4], r[5]);
+}
+
+// The caller's record of ray i: slot k at distance t, or a miss (k < 0).
+__device__ __forceinline__ void store_trace(const SceneView& S, f3 o, f3 d, uint32_t i, float t, int32_t k,
+                                            float* __restrict__ t_out, int32_t* __restrict__ id_out,
+                                            uint32_t* __restrict__ front_out) {
     if (t_out) t_out[i] = t;
     uint32_t front = 0;
     int32_t id = -1;
@@ -723,6 +715,108 @@ __global__ void __launch_bounds__(128) k_trace_rays(SceneView S, const float* __
     }
     if (id_out) id_out[i] = id;
     if (front_out) front_out[i] = front;
+}
+
+// Arbitrary rays -> closest hit (t, original id, front face), `per_warp` rays a
+// warp: 32, or fewer where there are not enough rays for a warp on every
+// scheduler (a warp is as slow as all the different walks of its rays
+// together): 1001 rays on 20k spheres 137 -> 105 us the whole call, 10k 138 ->
+// 120, 1001 on RTIOW 50 -> 45.
+// UP_FRONT: only the up-front tests, the closest hit so far left in t_out and
+// id_out (a slot, or kNone) for k_trace_walk.
+template <bool UP_FRONT>
+__global__ void __launch_bounds__(128) k_trace_rays(SceneView S, const float* __restrict__ rays, uint32_t n,
+                                                    uint32_t per_warp, float tmin, float tmax,
+                                                    float* __restrict__ t_out, int32_t* __restrict__ id_out,
+                                                    uint32_t* __restrict__ front_out, uint32_t* __restrict__ err,
+                                                    uint32_t* __restrict__ work) {
+    extern __shared__ unsigned char smem[];
+    StackSmem sm;
+    sm.e = reinterpret_cast<int2*>(smem);
+    const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    if (UP_FRONT && gt == 0) *work = 0u;
+    const uint32_t i = (gt >> 5) * per_warp + lane;
+    if (lane >= per_warp || i >= n) return;
+    f3 o, d;
+    load_ray(rays, i, o, d);
+    RayPre R = prep_for<false>(o, d);
+    TraceCounters K{0, 0};
+    bool overflow = false;
+    float t;
+    if (UP_FRONT) {
+        Tracer<false> T;
+        T.open(R, 0.0f, tmin, tmax, tmax, kNone);
+        up_front(T, S, K);
+        t_out[i] = T.best_t;
+        id_out[i] = T.best;
+        return;
+    }
+    const int32_t k = trace_closest<false>(S, R, tmin, tmax, t, sm, threadIdx.x, blockDim.x, overflow, K);
+    if (overflow) atomicOr(err, 1u);
+    store_trace(S, o, d, i, t, k, t_out, id_out, front_out);
+}
+
+// The walks of many rays, as k_walk.
+__global__ void __launch_bounds__(128, 8) k_trace_walk(SceneView S, const float* __restrict__ rays, uint32_t n, float tmin,
+                                                       float tmax, float* __restrict__ t_out,
+                                                       int32_t* __restrict__ id_out, uint32_t* __restrict__ front_out,
+                                                       uint32_t* __restrict__ err, uint32_t* __restrict__ work) {
+    extern __shared__ unsigned char smem[];
+    StackSmem sm;
+    sm.e = reinterpret_cast<int2*>(smem);
+    const uint32_t lane = threadIdx.x & 31;
+    TraceCounters K{0, 0};
+    bool overflow = false;
+    Tracer<false> T;
+    int2 spill[kSpill];
+    uint32_t ray = 0;
+    bool active = false;
+    for (uint32_t idle = 0xffffffffu;;) {
+        const uint32_t take = (uint32_t)__popc(idle);
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(work, take);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const bool exhausted = base >= n || n - base <= take;
+        if (!active && base < n) {
+            ray = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (ray < n) {
+                f3 o, d;
+                load_ray(rays, ray, o, d);
+                RayPre R = prep_for<false>(o, d);
+                const float m = ray_margin(S, R), t0 = t_out[ray];
+                const int32_t k0 = id_out[ray];
+                float t;
+                int32_t k;
+                if (!(m <= kFarMarginMax)) {  // rare: traced to the end now, on this lane's free stack
+                    R = prep<false>(o, d);
+                    axis_margins(R);
+                    k = trace_with<Tracer<false, true, true>>(S, R, 0.0f, tmin, tmax, t, sm, threadIdx.x, blockDim.x,
+                                                              overflow, K);
+                } else {
+                    T.open(R, m, tmin, tmax, t0, k0);
+                    active = T.enter(S, K);
+                    k = T.result(t);
+                }
+                if (!active) store_trace(S, o, d, ray, t, k, t_out, id_out, front_out);
+            }
+        }
+        const uint32_t enough = exhausted ? 32u : kWalkRefill;
+        for (;;) {
+            idle = __ballot_sync(0xffffffffu, !active);
+            if ((uint32_t)__popc(idle) >= enough) break;
+            if (active) {
+                for (int i = 0; i < kWalkSteps && active; ++i)
+                    active = T.step(S, sm, threadIdx.x, blockDim.x, spill, overflow, K);
+                if (!active) {
+                    float t;
+                    const int32_t k = T.result(t);
+                    store_trace(S, T.R.o, T.R.d, ray, t, k, t_out, id_out, front_out);
+                }
+            }
+        }
+        if (exhausted) break;
+    }
+    if (overflow) atomicOr(err, 1u);
 }
 
 SceneView view_of(const venu_scene* s) {
@@ -808,6 +902,10 @@ constexpr uint32_t kMaxDepth = 64;
 // 640x360 x 4 on 300k spheres takes 8.80 instead of 8.48; from 2M up, 1280x720
 // x 8 on 1M spheres 65.1 instead of 64.4.
 constexpr uint32_t kWalkSpheres = 16384, kWalkRays = 1u << 20;
+// Where a caller's rays are split the same way (us without -> with): 1M rays on
+// 20k spheres 636 -> 719, 2M on 50k 1472 -> 1512, 2M on 100k 1656 -> 1536, 2M on
+// 200k 1740 -> 1508, 500k on 100k 589 -> 549, 250k on 200k 359 -> 360.
+constexpr uint32_t kTraceWalkSpheres = 65536, kTraceWalkRays = 1u << 18;
 
 
 template <typename K>
@@ -1470,22 +1568,35 @@ extern "C" venu_status venu_trace(const venu_scene* scene, const float* rays_dev
     int word = -1;
     if (scene->trace_err) {
         std::lock_guard<std::mutex> lock(scene->trace_mu);
-        for (uint32_t i = 0; i < kTraceWords && word < 0; ++i)
+        for (uint32_t i = 0; i < kTraceWords / 2 && word < 0; ++i)
             if (!(scene->trace_used >> i & 1u)) word = (int)i;
         if (word >= 0) scene->trace_used |= 1ull << word;
     }
     cudaError_t e = cudaSuccess;
     if (word >= 0) {
-        err = scene->trace_err + word;
+        err = scene->trace_err + 2 * word;
     } else {
-        VENU_CUDA(cudaMalloc(&err, sizeof(uint32_t)));
-        e = cudaMemsetAsync(err, 0, sizeof(uint32_t), st);
+        VENU_CUDA(cudaMalloc(&err, 2 * sizeof(uint32_t)));
+        e = cudaMemsetAsync(err, 0, 2 * sizeof(uint32_t), st);
     }
-    const size_t tsm = traverse_smem(kTravBlock);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace_rays, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
+    const size_t tsm = traverse_smem(kTravBlock);  // 8 KB: below the size that needs an attribute
     if (e == cudaSuccess) {
-        k_trace_rays<<<(n + kTravBlock - 1) / kTravBlock, kTravBlock, tsm, st>>>(view_of(scene), rays_dev, n, tmin,
-                                                                               tmax, t_dev, id_dev, front_dev, err);
+        const SceneView S = view_of(scene);
+        // split as k_traverse (the hits so far travel in the caller's outputs)
+        const bool walk = t_dev && id_dev && scene->n >= kTraceWalkSpheres && n >= kTraceWalkRays;
+        const uint32_t warps = kTravBlock / 32u;
+        const uint32_t fill = (uint32_t)sm_count() * 4u * warps;  // a warp or more on every scheduler
+        const uint32_t per_warp = walk ? 32u : std::min(32u, (n + fill - 1u) / fill);
+        const uint32_t grid = (n + warps * per_warp - 1u) / (warps * per_warp);
+        if (walk) {
+            k_trace_rays<true><<<grid, kTravBlock, tsm, st>>>(S, rays_dev, n, per_warp, tmin, tmax, t_dev, id_dev,
+                                                             front_dev, err, err + 1);
+            k_trace_walk<<<sm_count() * 8, kTravBlock, tsm, st>>>(S, rays_dev, n, tmin, tmax, t_dev, id_dev, front_dev,
+                                                                err, err + 1);
+        } else {
+            k_trace_rays<false><<<grid, kTravBlock, tsm, st>>>(S, rays_dev, n, per_warp, tmin, tmax, t_dev, id_dev,
+                                                              front_dev, err, nullptr);
+        }
         e = cudaGetLastError();
     }
     uint32_t herr = 0;

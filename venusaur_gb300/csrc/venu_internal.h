@@ -44,7 +44,7 @@ cudaError_t prefer_l1(K kernel, int per_sm, size_t dyn) {
 }  // namespace venu
 
 namespace venu {
-constexpr uint32_t kTraceWords = 64;  // venu_trace calls of one scene that may run at once without allocating
+constexpr uint32_t kTraceWords = 64;  // two for each venu_trace call of a scene that may run without allocating
 
 // Device memory handed out in stream order and kept for reuse up to `keep`
 // bytes (the default pool gives everything back at each synchronisation, and
@@ -82,8 +82,9 @@ struct venu_scene {
     uint32_t* keys = nullptr;  // sorted Morton codes
     int32_t* parents = nullptr;  // [n-1] parent of each internal node, then [n] of each leaf (for refits)
     uint32_t* arrive = nullptr;  // [n-1] arrival counters of refits, 0 between them
-    uint32_t* trace_err = nullptr;         // [kTraceWords] error words of venu_trace calls, 0 unless one failed
-    mutable uint64_t trace_used = 0;       // those in use (a bit each)
+    uint32_t* trace_err = nullptr;         // [kTraceWords] error word (0 unless one failed) and hand-out counter
+                                           // of each venu_trace call
+    mutable uint64_t trace_used = 0;       // the pairs in use (a bit each)
     mutable std::mutex trace_mu;
     // The 4-wide traversal tree (lbvh.cu), built on first use by a render
     // with traversal variant 4 or 5 (ensure_wide); a cache of the binary
