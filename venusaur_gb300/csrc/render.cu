@@ -438,10 +438,9 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
     }
 }
 
-// The in-place launch with refills (in_place_factor > 1, its own kernel
-// instantiation, REFILL): a launch with at most in_place_factor rays per
-// thread of the grid finishes every path it takes bounce after bounce
-// instead of appending survivors to the next queue.  A warp takes fresh rays
+// The in-place launch with refills (its own kernel instantiation, REFILL), for
+// up to 16 rays per thread of the grid: it finishes every path it takes bounce
+// after bounce instead of appending survivors to the next queue.  A warp takes fresh rays
 // from the launch (one atomic) between bounces as soon as kRefillLanes of its
 // lanes are idle, so its lanes stay busy while paths end at different
 // bounces; warps do not wait for one another.  Each path goes through exactly
@@ -451,7 +450,6 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
 // Against block-wide refills with a barrier a bounce: 400x225 x 16 RTIOW 757 ->
 // 744 us over the wide tree, 656 -> 624 over the binary one, 20k spheres
 // 256x256 x 8 838 -> 818 us (8 lanes: 747 / 624 / 812; 16: 756 / 634 / 811).
-// The factor is a tuning field (venu_tuning.in_place_factor).
 constexpr uint32_t kRefillLanes = 4;
 
 template <bool COUNT, int KS, bool WIDE>
@@ -512,7 +510,7 @@ __device__ __forceinline__ void trace_shade_in_place_refill(const SceneView& S, 
 // The end of a bounce launch (see WaveCtl).  handle: the while node's
 // condition, 0 for a launch from the host.
 __device__ __forceinline__ void wave_advance(WaveCtl* ctl, uint32_t* cnt_in, uint32_t* work, const uint32_t* cnt_out,
-                                             uint32_t out_q, uint32_t finish_max, unsigned long long* stats,
+                                             uint32_t out_q, uint32_t next_max, unsigned long long* stats,
                                              cudaGraphConditionalHandle handle) {
     __syncthreads();  // every thread of the block is done
     if (threadIdx.x != 0) return;
@@ -527,9 +525,9 @@ __device__ __forceinline__ void wave_advance(WaveCtl* ctl, uint32_t* cnt_in, uin
     const uint32_t b = ctl->b + 1u;
     ctl->b = b;
     const uint32_t next = *reinterpret_cast<const volatile uint32_t*>(cnt_out);
-    const bool more = b < ctl->nb && next > finish_max;
+    const bool more = b < ctl->nb && next > next_max;
     if (!more) {
-        ctl->left = next <= finish_max ? next : 0u;  // after the last bounce there are none
+        ctl->left = next <= next_max ? next : 0u;  // after the last bounce there are none
         ctl->left_q = out_q;
         ctl->left_first = 0u;
     }
@@ -543,7 +541,8 @@ __device__ __forceinline__ void wave_advance(WaveCtl* ctl, uint32_t* cnt_in, uin
 // then shades all 32 together once the warp has reconverged and appends the
 // continuing paths with one ballot and one atomic.  Saves the hit record
 // round trip, the second read of the rays and one launch per bounce.
-// A launch with at most finish_max rays leaves them to k_finish.
+// A launch with at most finish_max rays leaves them to k_finish, as it leaves
+// up to next_max continuing rays.
 // WIDE: the 4-wide tree instead of the binary traversal records (variant 4,
 // k_trace_shade_wide, with its own register cap).
 template <bool COUNT, int KS, bool WIDE>
@@ -553,7 +552,7 @@ __device__ __forceinline__ void trace_shade_body(const SceneView& S, const Queue
                                                  float4* __restrict__ slots, uint32_t* __restrict__ err,
                                                  unsigned long long* __restrict__ stats, const PrimaryGen& gen,
                                                  WaveCtl* ctl, uint32_t out_q, uint32_t finish_max,
-                                                 cudaGraphConditionalHandle handle) {
+                                                 uint32_t next_max, cudaGraphConditionalHandle handle) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
     sm.e = reinterpret_cast<int2*>(smem);
@@ -573,7 +572,7 @@ __device__ __forceinline__ void trace_shade_body(const SceneView& S, const Queue
     trace_shade_loop<COUNT, KS, WIDE>(S, qin, n, work, qout, cnt_out, slots, gen, cam, sm, overflow, K);
     if (overflow) atomicOr(err, 1u);
     if (COUNT) flush_counters(K, stats);
-    wave_advance(ctl, cnt_in, work, cnt_out, out_q, finish_max, stats, handle);
+    wave_advance(ctl, cnt_in, work, cnt_out, out_q, next_max, stats, handle);
 }
 
 template <bool COUNT, int KS>
@@ -582,9 +581,9 @@ __global__ void VENU_TRACE_BOUNDS k_trace_shade(SceneView S, Queue qin, uint32_t
                                                 uint32_t* __restrict__ cnt_out, float4* __restrict__ slots,
                                                 uint32_t* __restrict__ err, unsigned long long* __restrict__ stats,
                                                 PrimaryGen gen, WaveCtl* ctl, uint32_t out_q, uint32_t finish_max,
-                                                cudaGraphConditionalHandle handle) {
+                                                uint32_t next_max, cudaGraphConditionalHandle handle) {
     trace_shade_body<COUNT, KS, false>(S, qin, cnt_in, work, qout, cnt_out, slots, err, stats, gen, ctl, out_q,
-                                       finish_max, handle);
+                                       finish_max, next_max, handle);
 }
 
 template <bool COUNT, int KS>
@@ -594,9 +593,9 @@ __global__ void VENU_WIDE_BOUNDS k_trace_shade_wide(SceneView S, Queue qin, uint
                                                     uint32_t* __restrict__ err,
                                                     unsigned long long* __restrict__ stats, PrimaryGen gen,
                                                     WaveCtl* ctl, uint32_t out_q, uint32_t finish_max,
-                                                    cudaGraphConditionalHandle handle) {
+                                                    uint32_t next_max, cudaGraphConditionalHandle handle) {
     trace_shade_body<COUNT, KS, true>(S, qin, cnt_in, work, qout, cnt_out, slots, err, stats, gen, ctl, out_q,
-                                      finish_max, handle);
+                                      finish_max, next_max, handle);
 }
 
 // The finishing kernel: runs the paths that are left of a wave (WaveCtl) to
@@ -605,18 +604,19 @@ __global__ void VENU_WIDE_BOUNDS k_trace_shade_wide(SceneView S, Queue qin, uint
 // part moved the bounce loop by up to 1.5 %; apart, the bounce kernel spills 12
 // bytes instead of 60): 1080p x 32 RTIOW 14.05 -> 13.95 ms, 256x144 x 4 278 ->
 // 260 us, 64x36 x 2 107 -> 90 us.  At 80 / 96 / 128 registers, with as many
-// fewer rays to take, the 256x144 frame takes 297 / 296 / 295 us.  REFILL
-// (in_place_factor > 1): with refills.
+// fewer rays to take, the 256x144 frame takes 297 / 296 / 295 us.  REFILL:
+// with refills, for more than spread_max rays (a thread each of the grid); the
+// other instantiation takes no more than that.
 template <bool COUNT, int KS, bool WIDE, bool REFILL>
 __global__ void VENU_TRACE_BOUNDS k_finish(SceneView S, Queue q0, Queue q1, float4* __restrict__ slots,
                                            uint32_t* __restrict__ err, unsigned long long* __restrict__ stats,
-                                           PrimaryGen gen, WaveCtl* ctl) {
+                                           PrimaryGen gen, WaveCtl* ctl, uint32_t spread_max) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
     sm.e = reinterpret_cast<int2*>(smem);
     __shared__ DevCamera cam;
     const uint32_t n = ctl->left;
-    if (n == 0) return;
+    if (n == 0 || (n > spread_max) != REFILL) return;
     const bool primary = ctl->left_first != 0u;
     const bool second = ctl->left_q != 0u;
     const Queue qin = second ? q1 : q0, qout = second ? q0 : q1;
@@ -859,7 +859,7 @@ struct WaveGraphKey {
     WaveCtl* ctl;
     size_t fsm;
     int grid, block, finish_grid;
-    uint32_t finish_max;
+    uint32_t first_max, finish_max;
     uint32_t kind;  // bits: 4-wide tree, shallow stack, counting build, in-place refills
 };
 
@@ -1042,7 +1042,7 @@ cudaError_t alloc_queues(venu_renderer* r, uint32_t Q) {
 }
 
 void destroy_wave_graph(venu_renderer* r);
-constexpr uint32_t kFusedWide = 1u, kFusedShallow = 2u, kFusedCount = 4u, kFusedRefill = 8u;
+constexpr uint32_t kFusedWide = 1u, kFusedShallow = 2u, kFusedCount = 4u;
 
 #define VENU_FUSED_CS(LAUNCH, KERNEL)                            \
     do {                                                         \
@@ -1060,30 +1060,33 @@ constexpr uint32_t kFusedWide = 1u, kFusedShallow = 2u, kFusedCount = 4u, kFused
 // loop condition, or 0 for a launch from the host's bounce loop.
 cudaError_t launch_fused(const venu_renderer* r, cudaStream_t st, uint32_t kind, size_t fsm, const SceneView& S,
                          uint32_t* cnt_in, uint32_t* work, uint32_t out_q, uint32_t* cnt_out, const PrimaryGen& pg,
-                         uint32_t finish_max, cudaGraphConditionalHandle h) {
+                         uint32_t finish_max, uint32_t next_max, cudaGraphConditionalHandle h) {
     const int grid = r->fused_blocks, tb = (int)r->tune.traverse_block;
     const Queue &qi = r->q[1u - out_q], &qo = r->q[out_q];
 #define VENU_FUSED(KERNEL, C, KS)                                                                              \
     KERNEL<C, KS><<<grid, tb, fsm, st>>>(S, qi, cnt_in, work, qo, cnt_out, r->slots, r->err, r->stats, pg, r->ctl, \
-                                         out_q, finish_max, h)
+                                         out_q, finish_max, next_max, h)
     if (kind & kFusedWide) VENU_FUSED_CS(VENU_FUSED, k_trace_shade_wide);
     else VENU_FUSED_CS(VENU_FUSED, k_trace_shade);
 #undef VENU_FUSED
     return cudaGetLastError();
 }
 
-// What is left of a wave (see WaveCtl).
+// What is left of a wave (see WaveCtl): by the refilling kernel, by the
+// spreading one, or by whichever finds its number of rays.
+constexpr uint32_t kFinishRefill = 1u, kFinishSpread = 2u;
 cudaError_t launch_finish(const venu_renderer* r, cudaStream_t st, uint32_t kind, size_t fsm, const SceneView& S,
-                          const PrimaryGen& pg) {
+                          const PrimaryGen& pg, uint32_t which) {
     const int grid = r->finish_blocks, tb = (int)r->tune.traverse_block;
+    const uint32_t spread_max = (uint32_t)grid * (uint32_t)tb;
 #define VENU_FINISH(WIDE, C, KS)                                                                                  \
     do {                                                                                                          \
-        if (kind & kFusedRefill)                                                                                  \
+        if (which & kFinishRefill)                                                                                \
             k_finish<C, KS, WIDE, true>                                                                           \
-                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl);             \
-        else                                                                                                      \
+                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, spread_max); \
+        if (which & kFinishSpread)                                                                                \
             k_finish<C, KS, WIDE, false>                                                                          \
-                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl);             \
+                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, spread_max); \
     } while (0)
     if (kind & kFusedWide) VENU_FUSED_CS(VENU_FINISH, true);
     else VENU_FUSED_CS(VENU_FINISH, false);
@@ -1108,7 +1111,7 @@ venu_status build_wave_graph(venu_renderer* r, const WaveGraphKey& key) {
     later.path_seeds = nullptr;  // bounces after the first read their rays from the queue
     VENU_CUDA(cudaStreamBeginCaptureToGraph(r->cap, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     cudaError_t le = launch_fused(r, r->cap, key.kind, key.fsm, key.S, key.cnt, key.work, 1u, key.cnt + 1, key.pg,
-                                  key.finish_max, h);
+                                  key.first_max, key.finish_max, h);
     cudaGraph_t captured = nullptr;
     cudaError_t ee = cudaStreamEndCapture(r->cap, &captured);
     if (le != cudaSuccess) return cuda_fail(le, "venu_render: capture of the first bounce");
@@ -1130,15 +1133,15 @@ venu_status build_wave_graph(venu_renderer* r, const WaveGraphKey& key) {
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     VENU_CUDA(cudaStreamBeginCaptureToGraph(r->cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     le = launch_fused(r, r->cap, key.kind, key.fsm, key.S, key.cnt + 1, key.work + 1, 0u, key.cnt, later,
-                      key.finish_max, h);
+                      key.finish_max, key.finish_max, h);
     if (le == cudaSuccess)
         le = launch_fused(r, r->cap, key.kind, key.fsm, key.S, key.cnt, key.work, 1u, key.cnt + 1, later,
-                          key.finish_max, h);
+                          key.finish_max, key.finish_max, h);
     ee = cudaStreamEndCapture(r->cap, &captured);
     if (le != cudaSuccess) return cuda_fail(le, "venu_render: capture of the bounce loop");
     if (ee != cudaSuccess) return cuda_fail(ee, "venu_render: cudaStreamEndCapture");
     VENU_CUDA(cudaStreamBeginCaptureToGraph(r->cap, g, &loop, nullptr, 1, cudaStreamCaptureModeRelaxed));
-    le = launch_finish(r, r->cap, key.kind, key.fsm, key.S, key.pg);
+    le = launch_finish(r, r->cap, key.kind, key.fsm, key.S, key.pg, kFinishRefill | kFinishSpread);
     ee = cudaStreamEndCapture(r->cap, &captured);
     if (le != cudaSuccess) return cuda_fail(le, "venu_render: capture of the finishing kernel");
     if (ee != cudaSuccess) return cuda_fail(ee, "venu_render: cudaStreamEndCapture");
@@ -1333,7 +1336,7 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
     VENU_CUDA(cudaStreamIsCapturing(st, &cap_status));
     bool use_graph = fused && !prof && P == npix && !r->graph_off && cap_status == cudaStreamCaptureStatusNone;
     const uint32_t kind = (tu.traverse_variant == 4u ? kFusedWide : 0u) | (shallow ? kFusedShallow : 0u) |
-                          (count ? kFusedCount : 0u) | (tu.in_place_factor > 1u ? kFusedRefill : 0u);
+                          (count ? kFusedCount : 0u);
     const size_t fsm = shallow ? traverse_smem(tb, kSharedShallow) : tsm;
     // the camera-ray generator of the wave of pixels [p0, p0 + PP)
     auto primary_gen = [&](uint32_t p0, uint32_t PP) {
@@ -1349,14 +1352,22 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
         pg.div_W = make_fastdiv(W);
         return pg;
     };
-    // waves and bounces of at most this many rays are the finishing kernel's
-    // (a thread takes one, or in_place_factor with refills); the separate
-    // traversals after a fused first bounce (variants 3, 5) only leave it whole waves
-    const uint64_t factor = tu.in_place_factor ? tu.in_place_factor : 1u;
-    const uint32_t finish_max =
-        gen0 ? (uint32_t)std::min<uint64_t>(factor * r->finish_blocks * (uint64_t)tb, 0xffffffffu) : 0u;
+    // The finishing kernels take whole waves of at most first_max rays and, of the
+    // fused variants, what a bounce leaves when that is at most finish_max.  An
+    // in_place_factor above 1 asks for that many rays per thread of their grid.
+    // Otherwise: up to 16, but whole waves only of small scenes, where camera
+    // rays lose little by sharing warps with later bounces; of large ones a ray
+    // per thread (ms at 1 / 8 / 16 for both): RTIOW 400x225 x 16 0.625 / 0.572 /
+    // 0.558, 1280x720 x 1 at depth 4 0.495 / 0.431 / 0.430, 300k spheres 512x512 x
+    // 4 with its build 6.73 / 5.89 / 5.90; but 100k 1080p x 1, whose 2.1M camera
+    // rays only 16 takes, 4.99 / 4.46 / 5.16.
+    const uint64_t threads = (uint64_t)r->finish_blocks * (uint64_t)tb;
+    const uint64_t asked = tu.in_place_factor > 1u ? tu.in_place_factor : 16u;
+    const uint32_t finish_max = gen0 ? (uint32_t)std::min<uint64_t>(asked * threads, 0xffffffffu) : 0u;
+    const uint32_t first_max =
+        gen0 ? (uint32_t)(tu.in_place_factor > 1u || shallow ? finish_max : threads) : 0u;
     const uint32_t bounce_max = fused ? finish_max : 0u;
-    use_graph = use_graph && (uint64_t)npix * k > finish_max;
+    use_graph = use_graph && (uint64_t)npix * k > first_max;
     if (use_graph) {
         WaveGraphKey key;
         std::memset(&key, 0, sizeof key);
@@ -1374,6 +1385,7 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
         key.fsm = fsm;
         key.grid = r->fused_blocks;
         key.finish_grid = r->finish_blocks;
+        key.first_max = first_max;
         key.finish_max = finish_max;
         key.block = tb;
         key.kind = kind;
@@ -1393,10 +1405,14 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
             const uint32_t PP = std::min(P, npix - p0);
             k_raygen<<<(PP + 255) / 256, 256, 0, st>>>(*camera, W, H, p0, PP, s0, kk, opts->subframe_index,
                                                        (int)maxd, r->seeds, r->q[0], path_seeds, r->cnt, r->work,
-                                                       nb, r->ctl, finish_max, r->stats);
+                                                       nb, r->ctl, first_max, r->stats);
             PrimaryGen pg = primary_gen(p0, PP);
             pg.path_seeds = path_seeds;
-            const bool small = (uint64_t)PP * kk <= finish_max;
+            const bool small = (uint64_t)PP * kk <= first_max;
+            const uint32_t which = !small                               ? kFinishRefill | kFinishSpread
+                                   : (uint64_t)PP * kk > threads ? kFinishRefill
+                                                                        : kFinishSpread;
+            const uint32_t finishes = small ? 1u : 2u;
             ++launches;
             if (small) {
                 if (prof) {
@@ -1404,16 +1420,16 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
                         cudaEvent_t a, z;
                         VENU_CUDA(next_events(r, a, z));
                         VENU_CUDA(cudaEventRecord(a, st));
-                        if (i == 0) VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg));
+                        if (i == 0) VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg, which));
                         VENU_CUDA(cudaEventRecord(z, st));
                     }
                 } else {
-                    VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg));
+                    VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg, which));
                 }
-                ++launches;
+                launches += finishes;
             } else if (use_graph) {  // the bounce loop of this wave: one graph launch
                 VENU_CUDA(cudaGraphLaunch(r->wexec, st));
-                ++launches;  // the finishing kernel; the bounces count themselves
+                launches += finishes;  // the bounces count themselves
             }
             for (int b = 0; b < nb && !small && !use_graph; ++b) {
                 const Queue& qi = r->q[b & 1];
@@ -1437,7 +1453,7 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
                 if (v == 2 || v == 4) {
                     pg.path_seeds = (b == 0) ? path_seeds : nullptr;
                     VENU_CUDA(launch_fused(r, st, kind, fsm, S, r->cnt + b, r->work + b, (uint32_t)((b + 1) & 1),
-                                           r->cnt + b + 1, pg, bounce_max, 0));
+                                           r->cnt + b + 1, pg, b == 0 ? 0u : bounce_max, bounce_max, 0));
                     if (prof) {
                         VENU_CUDA(cudaEventRecord(e1, st));
                         VENU_CUDA(cudaEventRecord(e2, st));
@@ -1487,13 +1503,13 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
                         cudaEvent_t a, z;
                         VENU_CUDA(next_events(r, a, z));
                         VENU_CUDA(cudaEventRecord(a, st));
-                        if (i == 0) VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg));
+                        if (i == 0) VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg, which));
                         VENU_CUDA(cudaEventRecord(z, st));
                     }
                 } else {
-                    VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg));
+                    VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg, which));
                 }
-                ++launches;
+                launches += finishes;
             }
             const bool last = s0 + kk == spp;  // of these pixels
             k_accumulate<<<(PP + 255) / 256, 256, 0, st>>>(
