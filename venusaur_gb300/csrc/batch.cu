@@ -55,6 +55,8 @@ struct LoopCtl {  // device-owned loop state
     uint32_t parity;        // the queue traced in this iteration; flipped by k_plan
     uint32_t chunk_end;     // this step traces input rays [chunk_start, chunk_end)
     uint32_t chunk_start;
+    uint32_t pending;       // paths are left that no plan has handed out yet
+    uint32_t pad;
     unsigned long long segments, paths_done, iterations;
 };
 
@@ -187,6 +189,7 @@ __device__ uint32_t plan_iteration(const DevJob* __restrict__ jobs, unsigned lon
         ctl->chunk_start = 0u;
         ctl->chunk_end = min(chunk, survivors + off);
         ctl->parity = (uint32_t)out;
+        ctl->pending = more ? 1u : 0u;
     }
     return (survivors + off > 0u || more) ? 1u : 0u;
 }
@@ -274,32 +277,73 @@ __device__ __forceinline__ void gen_primary(const DevJob* __restrict__ jobs, con
     d4 = make_float4(d.x, d.y, d.z, __uint_as_float((j << 8) | ((uint32_t)((int)J.max_depth - 1) & kDepthMask)));
 }
 
-// A pointer read that the compiler may not merge with an earlier read of the
-// same field (so the value is not kept live in a register meanwhile).
-template <typename T>
-__device__ __forceinline__ T ld_volatile_ptr(const T* p) {
-    return *reinterpret_cast<const volatile T*>(p);
+// Up to this many rays per thread of its grid, a step that no more new paths
+// follow runs its paths to their ends (k_finish_multi); with new paths to come,
+// or in chunked steps, whose caller wants the loop back soon, one.  At 1 / 2 / 8
+// rays a thread, 96 uneven jobs take 6.90 / 6.78 / 6.65 ms, 8 small ones 0.80 /
+// 0.73 / 0.54.
+constexpr uint32_t kFinishFactor = 8;
+__device__ __forceinline__ bool finish_step(const LoopCtl* ctl, const RunCtl* run, uint32_t threads) {
+    const uint32_t m = ctl->chunk_end - ctl->chunk_start;
+    return m <= (run->chunk || ctl->pending ? 1u : kFinishFactor) * threads;
 }
 
-// One warp-batch loop of the batch kernel.  IN_PLACE (a step with no more
-// rays than the grid has threads): each path is finished in place, bounce
-// after bounce (the step leaves no survivors); the output queue is unused
-// then, and its throughput slot i carries ray i's state between bounces.
-// (Chunked steps: survivors of earlier chunks of the iteration sit below
-// chunk_start, which no scratch index reaches.)  A separate instantiation,
-// so the ordinary loop keeps its registers.
-template <bool COUNT, bool IN_PLACE>
-__device__ __forceinline__ void trace_shade_multi_loop(const DevJob* __restrict__ jobs,
-                                                       unsigned long long* __restrict__ job_done, LoopCtl* ctl,
-                                                       const uint32_t* __restrict__ plan_job,
-                                                       const unsigned long long* __restrict__ plan_start,
-                                                       const uint32_t* __restrict__ plan_off, const Queue& qin,
-                                                       const Queue& qout, int in, int out, StackSmem sm,
-                                                       bool& overflow, TraceCounters& K, uint32_t& finished,
-                                                       uint32_t& traced) {
+// One segment of a path: its closest hit, then its shading.
+template <bool COUNT>
+__device__ __forceinline__ ShadeOut trace_shade_job(const DevJob* __restrict__ jobs, uint32_t job, int32_t from,
+                                                    float4 o4, float4 d4, const float4* t_src, float4 t_fresh,
+                                                    StackSmem sm, bool& overflow, TraceCounters& K) {
+    RayPre R = prep_for<COUNT>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+    R.from = from;
+    float t;
+    const SceneView* G = &jobs[job].scene;
+    const JobScene S{G->trav, G};
+    const int32_t k = trace_closest<COUNT>(S, R, 0.001f, 1e16f, t, sm, threadIdx.x, blockDim.x, overflow, K);
+    // the shading pointers are read here instead of being kept in registers
+    // through the traversal (the job table is L1/L2-resident)
+    SceneView S2;
+    S2.sph = G->sph;
+    S2.mat = G->mat;
+    S2.meta = G->meta;
+    const float4 t4 = t_src ? *t_src : t_fresh;
+    const ShadeOut r = shade_one<false>(S2, o4, d4, t4, make_int2(__float_as_int(t), k));
+    if (!r.cont) jobs[job].slots[(uint32_t)__float_as_int(o4.w)] = r.result;
+    return r;
+}
+
+// Finished paths per job: one atomic per distinct job in the warp (the result
+// is not read: a fire-and-forget reduction; k_plan notices finished jobs).
+__device__ __forceinline__ void count_finished(unsigned long long* __restrict__ job_done, bool fin, uint32_t job,
+                                               uint32_t& finished) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t key = fin ? job : 0xFFFFFFFFu;
+    const uint32_t peers = __match_any_sync(0xffffffffu, key);
+    if (fin && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&job_done[job], (unsigned long long)__popc(peers));
+    finished += __popc(__ballot_sync(0xffffffffu, fin));
+}
+
+// One iteration's input (or a chunk of it): each warp takes 32 rays, traces and
+// shades them, and appends the continuing paths to the other queue.
+template <bool COUNT>
+__global__ void VENU_TRACE_MULTI_BOUNDS k_trace_shade_multi(const DevJob* __restrict__ jobs,
+                                                           unsigned long long* __restrict__ job_done, LoopCtl* ctl,
+                                                           const RunCtl* __restrict__ run,
+                                                           const uint32_t* __restrict__ plan_job,
+                                                           const unsigned long long* __restrict__ plan_start,
+                                                           const uint32_t* __restrict__ plan_off,
+                                                           Queue q0, Queue q1, uint32_t finish_threads) {
+    extern __shared__ unsigned char smem[];
+    StackSmem sm;
+    sm.e = reinterpret_cast<int2*>(smem);
+    if (finish_step(ctl, run, finish_threads)) return;
+    const int in = (int)(ctl->parity & 1u), out = 1 - in;
+    const Queue qin = in ? q1 : q0, qout = in ? q0 : q1;
     const uint32_t n = ctl->chunk_end;  // this step: input rays [chunk_start, chunk_end)
     const uint32_t gen_base = ctl->gen_base, np = ctl->plan_n;  // new paths from gen_base on
     const uint32_t lane = threadIdx.x & 31;
+    TraceCounters K{0, 0};
+    bool overflow = false;
+    uint32_t finished = 0, traced = 0;
     for (;;) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(&ctl->work[in], 32u);
@@ -323,35 +367,9 @@ __device__ __forceinline__ void trace_shade_multi_loop(const DevJob* __restrict_
                 from = qin.from[i];
             }
             job = __float_as_uint(d4.w) >> 8;
-            for (bool first = true;; first = false) {
-                RayPre R = prep_for<COUNT>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
-                R.from = from;
-                float t;
-                int32_t k;
-                {
-                    const SceneView S = jobs[job].scene;
-                    k = trace_closest<COUNT>(S, R, 0.001f, 1e16f, t, sm, threadIdx.x, blockDim.x, overflow, K);
-                }
-                ++traced;  // per lane: one segment
-                // the shading pointers are read again here instead of being kept in
-                // registers through the traversal (the job table is L1/L2-resident)
-                SceneView S2;
-                const SceneView* G = &jobs[job].scene;
-                S2.sph = ld_volatile_ptr(&G->sph);
-                S2.mat = ld_volatile_ptr(&G->mat);
-                S2.meta = ld_volatile_ptr(&G->meta);
-                const float4 t4 = (IN_PLACE && !first) ? qout.t[i]
-                                  : fresh                ? make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(seed))
-                                                         : qin.t[i];
-                const float4 ow = o4;  // .w: the path's slot
-                r = shade_one<false>(S2, o4, d4, t4, make_int2(__float_as_int(t), k));
-                if (!r.cont) jobs[job].slots[(uint32_t)__float_as_int(ow.w)] = r.result;
-                if (!IN_PLACE || !r.cont) break;
-                o4 = r.o;
-                d4 = r.d;
-                from = r.from;
-                qout.t[i] = r.t;
-            }
+            r = trace_shade_job<COUNT>(jobs, job, from, o4, d4, fresh ? nullptr : qin.t + i,
+                                       make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(seed)), sm, overflow, K);
+            ++traced;  // per lane: one segment
         }
         const uint32_t pos = warp_append(r.cont, &ctl->cnt[out]);
         if (r.cont) {
@@ -360,45 +378,94 @@ __device__ __forceinline__ void trace_shade_multi_loop(const DevJob* __restrict_
             qout.t[pos] = r.t;
             qout.from[pos] = r.from;
         }
-        // finished paths per job: one atomic per distinct job in the warp
-        const bool fin = valid && !r.cont;
-        const uint32_t key = fin ? job : 0xFFFFFFFFu;
-        const uint32_t peers = __match_any_sync(0xffffffffu, key);
-        // (the result is not read: a fire-and-forget reduction; k_plan
-        // notices finished jobs)
-        if (fin && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&job_done[job], (unsigned long long)__popc(peers));
-        finished += __popc(__ballot_sync(0xffffffffu, fin));
+        count_finished(job_done, valid && !r.cont, job, finished);
     }
-}
-
-template <bool COUNT>
-__global__ void VENU_TRACE_MULTI_BOUNDS k_trace_shade_multi(const DevJob* __restrict__ jobs,
-                                                           unsigned long long* __restrict__ job_done, LoopCtl* ctl,
-                                                           const uint32_t* __restrict__ plan_job,
-                                                           const unsigned long long* __restrict__ plan_start,
-                                                           const uint32_t* __restrict__ plan_off,
-                                                           Queue q0, Queue q1) {
-    extern __shared__ unsigned char smem[];
-    StackSmem sm;
-    sm.e = reinterpret_cast<int2*>(smem);
-    const int in = (int)(ctl->parity & 1u), out = 1 - in;
-    const Queue qin = in ? q1 : q0, qout = in ? q0 : q1;
-    const uint32_t lane = threadIdx.x & 31;
-    TraceCounters K{0, 0};
-    bool overflow = false;
-    uint32_t finished = 0, traced = 0;
-    if (ctl->chunk_end - ctl->chunk_start <= gridDim.x * blockDim.x)
-        trace_shade_multi_loop<COUNT, true>(jobs, job_done, ctl, plan_job, plan_start, plan_off, qin, qout, in, out,
-                                            sm, overflow, K, finished, traced);
-    else
-        trace_shade_multi_loop<COUNT, false>(jobs, job_done, ctl, plan_job, plan_start, plan_off, qin, qout, in, out,
-                                             sm, overflow, K, finished, traced);
-    for (int off = 16; off > 0; off >>= 1) traced += __shfl_xor_sync(0xffffffffu, traced, off);
+    traced = __reduce_add_sync(0xffffffffu, traced);
     if (lane == 0 && finished) atomicAdd(&ctl->paths_done, (unsigned long long)finished);
     if (lane == 0 && traced) atomicAdd(&ctl->segments, (unsigned long long)traced);
     if (overflow) atomicOr(&ctl->err, 1u);
 }
 
+// A step of few rays (finish_step): every path is run to its end, bounce after
+// bounce, the step leaves no survivors; a warp takes new rays as soon as
+// kRefillLanes of its lanes are idle, as the renderer's finishing kernel.  The
+// output queue is unused then, and its throughput slot of the first ray a lane
+// took carries that lane's state between bounces.  (Chunked steps: survivors of
+// earlier chunks of the iteration sit below chunk_start, which no scratch index
+// reaches.)  A kernel of its own, so that the ordinary loop keeps its registers.
+template <bool COUNT>
+__global__ void VENU_TRACE_MULTI_BOUNDS k_finish_multi(const DevJob* __restrict__ jobs,
+                                                      unsigned long long* __restrict__ job_done, LoopCtl* ctl,
+                                                      const RunCtl* __restrict__ run,
+                                                      const uint32_t* __restrict__ plan_job,
+                                                      const unsigned long long* __restrict__ plan_start,
+                                                      const uint32_t* __restrict__ plan_off,
+                                                      Queue q0, Queue q1) {
+    extern __shared__ unsigned char smem[];
+    StackSmem sm;
+    sm.e = reinterpret_cast<int2*>(smem);
+    if (ctl->chunk_end == ctl->chunk_start || !finish_step(ctl, run, gridDim.x * blockDim.x)) return;
+    const int in = (int)(ctl->parity & 1u);
+    const Queue qin = in ? q1 : q0, qout = in ? q0 : q1;
+    const uint32_t n = ctl->chunk_end;
+    const uint32_t gen_base = ctl->gen_base, np = ctl->plan_n;
+    const uint32_t lane = threadIdx.x & 31;
+    TraceCounters K{0, 0};
+    bool overflow = false;
+    uint32_t finished = 0, traced = 0;
+    uint32_t own = 0xffffffffu;  // the first ray this lane took
+    uint32_t job = 0xFFFFFFFFu;
+    int32_t from = -1;
+    bool exhausted = false, live = false;
+    float4 o4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d4 = o4;
+    for (;;) {
+        const uint32_t idle = __ballot_sync(0xffffffffu, !live);
+        if (!exhausted && (uint32_t)__popc(idle) >= kRefillLanes) {
+            const uint32_t take = (uint32_t)__popc(idle);
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&ctl->work[in], take);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            exhausted = base >= n || n - base <= take;
+            const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (!live && base < n && i < n) {
+                live = true;
+                if (own == 0xffffffffu) own = i;
+                if (i >= gen_base) {
+                    uint32_t seed = 0;
+                    gen_primary(jobs, plan_job, plan_start, plan_off, np, i - gen_base, o4, d4, seed);
+                    from = -1;
+                    qout.t[own] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(seed));
+                } else {
+                    o4 = qin.o[i];
+                    d4 = qin.d[i];
+                    from = qin.from[i];
+                    qout.t[own] = qin.t[i];
+                }
+                job = __float_as_uint(d4.w) >> 8;
+            }
+        }
+        if (!__any_sync(0xffffffffu, live)) break;  // only once the step has no rays left
+        bool fin = false;
+        if (live) {
+            const ShadeOut r = trace_shade_job<COUNT>(jobs, job, from, o4, d4, qout.t + own, o4, sm, overflow, K);
+            ++traced;
+            if (r.cont) {
+                o4 = r.o;
+                d4 = r.d;
+                from = r.from;
+                qout.t[own] = r.t;
+            } else {
+                live = false;
+                fin = true;
+            }
+        }
+        count_finished(job_done, fin, job, finished);
+    }
+    traced = __reduce_add_sync(0xffffffffu, traced);
+    if (lane == 0 && finished) atomicAdd(&ctl->paths_done, (unsigned long long)finished);
+    if (lane == 0 && traced) atomicAdd(&ctl->segments, (unsigned long long)traced);
+    if (overflow) atomicOr(&ctl->err, 1u);
+}
 
 // Accumulate (Kahan, sample order) and resolve finished jobs: one thread per
 // pixel of the listed jobs.
@@ -468,7 +535,7 @@ struct venu_batch {
     uint32_t* h_interrupt = nullptr;  // mapped host word
     uint32_t* d_interrupt = nullptr;  // its device address
     venu_tuning tune = {2u, 8u, 256u, 0u, 256u, 0u, 1u};
-    int trav_blocks = 0;
+    int trav_blocks = 0, finish_blocks = 0;
     cudaStream_t cap = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -478,26 +545,35 @@ struct venu_batch {
 
 namespace {
 
-cudaError_t batch_configure(venu_batch* b) {
+template <typename K>
+cudaError_t batch_grid(const venu_batch* b, K kernel, int& blocks) {
     const size_t sm = traverse_smem((int)b->tune.traverse_block);
-    cudaError_t e = cudaFuncSetAttribute(k_trace_shade_multi<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     int per_sm = 0;
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_shade_multi<false>,
-                                                          (int)b->tune.traverse_block, sm);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)b->tune.traverse_block, sm);
     if (e != cudaSuccess) return e;
     per_sm = std::max(1, per_sm);
     if (b->tune.traverse_blocks_per_sm) per_sm = std::min(per_sm, (int)b->tune.traverse_blocks_per_sm);
-    b->trav_blocks = per_sm * sm_count();
-    return prefer_l1(k_trace_shade_multi<false>, per_sm, sm);
+    blocks = per_sm * sm_count();
+    return prefer_l1(kernel, per_sm, sm);
+}
+
+cudaError_t batch_configure(venu_batch* b) {
+    const cudaError_t e = batch_grid(b, k_trace_shade_multi<false>, b->trav_blocks);
+    return e == cudaSuccess ? batch_grid(b, k_finish_multi<false>, b->finish_blocks) : e;
 }
 
 // One iteration of the path loop: trace the parity queue and the planned new
 // paths, then plan (which also sets the loop condition and flips the parity).
 cudaError_t launch_body(venu_batch* b, cudaStream_t st, bool use_handle) {
     const size_t sm = traverse_smem((int)b->tune.traverse_block);
-    k_trace_shade_multi<false><<<b->trav_blocks, b->tune.traverse_block, sm, st>>>(
-        b->d_jobs, b->d_done, b->d_ctl, b->d_plan_job, b->d_plan_start, b->d_plan_off, b->q[0], b->q[1]);
+    const uint32_t tb = b->tune.traverse_block;
+    k_trace_shade_multi<false><<<b->trav_blocks, tb, sm, st>>>(b->d_jobs, b->d_done, b->d_ctl, b->d_run, b->d_plan_job,
+                                                              b->d_plan_start, b->d_plan_off, b->q[0], b->q[1],
+                                                              (uint32_t)b->finish_blocks * tb);
+    k_finish_multi<false><<<b->finish_blocks, tb, sm, st>>>(b->d_jobs, b->d_done, b->d_ctl, b->d_run, b->d_plan_job,
+                                                           b->d_plan_start, b->d_plan_off, b->q[0], b->q[1]);
     k_plan<<<1, 32, 0, st>>>(b->d_jobs, b->d_next, b->d_done, b->d_seen, b->d_order, b->d_run, b->d_ctl, b->d_plan_job,
                              b->d_plan_start, b->d_plan_off, b->Q, b->d_interrupt, b->handle, use_handle ? 1 : 0);
     return cudaGetLastError();

@@ -450,7 +450,6 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
 // Against block-wide refills with a barrier a bounce: 400x225 x 16 RTIOW 757 ->
 // 744 us over the wide tree, 656 -> 624 over the binary one, 20k spheres
 // 256x256 x 8 838 -> 818 us (8 lanes: 747 / 624 / 812; 16: 756 / 634 / 811).
-constexpr uint32_t kRefillLanes = 4;
 
 template <bool COUNT, int KS, bool WIDE>
 __device__ __forceinline__ void trace_shade_in_place_refill(const SceneView& S, const Queue& qin, uint32_t n,

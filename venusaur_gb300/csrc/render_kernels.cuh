@@ -166,6 +166,9 @@ __device__ __forceinline__ ShadeOut shade_one(const SceneView& S, float4 o4, flo
     return out;
 }
 
+// Idle lanes of a warp that take new rays together in the finishing kernels.
+constexpr uint32_t kRefillLanes = 4;
+
 // Warp-aggregated append: one atomic per warp, positions from the ballot.
 __device__ __forceinline__ uint32_t warp_append(bool pred, uint32_t* counter) {
     const uint32_t lane = threadIdx.x & 31;

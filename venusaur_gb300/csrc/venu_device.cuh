@@ -239,6 +239,25 @@ struct SceneView {
     int32_t hoist[kMaxHoisted];        // their slots (ascending)
 };
 
+// A scene by its entry in a job table (the batch engine): only the record
+// pointer is held in registers through a walk, the rest is read where it is
+// needed, through L1 (96 uneven jobs 6.65 -> 6.55 ms against a whole SceneView a
+// lane; with volatile reads, which pass L1 by, 7.86).
+struct JobScene {
+    const float4* __restrict__ trav;
+    const SceneView* g;
+};
+__device__ __forceinline__ const float4* sv_sph(const SceneView& S) { return S.sph; }
+__device__ __forceinline__ const float4* sv_sph(const JobScene& S) { return S.g->sph; }
+__device__ __forceinline__ const float4* sv_nodes(const SceneView& S) { return S.nodes; }
+__device__ __forceinline__ const float4* sv_nodes(const JobScene& S) { return S.g->nodes; }
+__device__ __forceinline__ uint32_t sv_n(const SceneView& S) { return S.n; }
+__device__ __forceinline__ uint32_t sv_n(const JobScene& S) { return S.g->n; }
+__device__ __forceinline__ uint32_t sv_nhoist(const SceneView& S) { return S.nhoist; }
+__device__ __forceinline__ uint32_t sv_nhoist(const JobScene& S) { return S.g->nhoist; }
+__device__ __forceinline__ int32_t sv_hoist(const SceneView& S, int h) { return S.hoist[h]; }
+__device__ __forceinline__ int32_t sv_hoist(const JobScene& S, int h) { return S.g->hoist[h]; }
+
 // Slab test: a box's entry / exit parameter on axis k is
 // fma(lo_k or hi_k, inv_k, offset).  The offset -(o_k inv_k) is rounded, which
 // a margin of |o_k inv_k| 2^-21 covers (several times that rounding).
@@ -522,14 +541,15 @@ __device__ __forceinline__ void flush_counters(const TraceCounters& K, unsigned 
 // their hit distances already cull boxes behind them.  The closest hit
 // does not depend on the order of the tests.  (A scene of one sphere has
 // it hoisted, see view_of.)  One copy of the test for all of them.
-template <typename T>
-__device__ __forceinline__ void up_front(T& W, const SceneView& S, TraceCounters& K) {
+template <typename T, class SV>
+__device__ __forceinline__ void up_front(T& W, const SV& S, TraceCounters& K) {
+    const int nh = (int)sv_nhoist(S);
 #pragma unroll 1
-    for (int h = W.R.from >= 0 ? -1 : 0; h < (int)S.nhoist; ++h) {
-        const int32_t k = h < 0 ? W.R.from : S.hoist[h];
+    for (int h = W.R.from >= 0 ? -1 : 0; h < nh; ++h) {
+        const int32_t k = h < 0 ? W.R.from : sv_hoist(S, h);
         if (h >= 0 && k == W.R.from) continue;
         ++K.spheres;
-        W.leaf(k, __ldg(S.sph + k));
+        W.leaf(k, __ldg(sv_sph(S) + k));
     }
 }
 
@@ -576,10 +596,14 @@ __device__ __forceinline__ float far_margin(f3 o, f3 inv, float E) {
 
 // The root's record behind the n - 1 node records: {c.x, c.y, h.x, h.y},
 // {c.z, h.z, E, 0}.
-__device__ __forceinline__ const float4* root_record(const SceneView& S) { return S.trav + 4 * (size_t)(S.n - 1u); }
+template <class SV>
+__device__ __forceinline__ const float4* root_record(const SV& S) {
+    return S.trav + 4 * (size_t)(sv_n(S) - 1u);
+}
 
-__device__ __forceinline__ float ray_margin(const SceneView& S, const RayPre& R) {
-    return S.n > 1u ? far_margin(R.o, R.inv, __ldg(&root_record(S)[1].z)) : 0.0f;
+template <class SV>
+__device__ __forceinline__ float ray_margin(const SV& S, const RayPre& R) {
+    return sv_n(S) > 1u ? far_margin(R.o, R.inv, __ldg(&root_record(S)[1].z)) : 0.0f;
 }
 
 // Per-lane traversal state.  begin() prepares a ray and tests the root;
@@ -619,10 +643,11 @@ struct Tracer {
     __device__ __forceinline__ bool meets(float tn, float tf) const { return tn <= fminf(tf, best_t) + m; }
 
     // R_ from prep(); AXIS: with per-axis margins.  m_: far_margin (fast walk).
-    __device__ __forceinline__ bool begin(const SceneView& S, const RayPre& R_, float m_, float tmin_, float tmax_,
+    template <class SV>
+    __device__ __forceinline__ bool begin(const SV& S, const RayPre& R_, float m_, float tmin_, float tmax_,
                                           TraceCounters& K) {
         open(R_, m_, tmin_, tmax_, tmax_, kNone);
-        if (S.n == 0) return false;
+        if (sv_n(S) == 0) return false;
         up_front(*this, S, K);
         return enter(S, K);
     }
@@ -639,12 +664,13 @@ struct Tracer {
     }
 
     // Tests the root; false: no node to walk.
-    __device__ __forceinline__ bool enter(const SceneView& S, TraceCounters& K) {
-        const uint32_t n = S.n;
+    template <class SV>
+    __device__ __forceinline__ bool enter(const SV& S, TraceCounters& K) {
+        const uint32_t n = sv_n(S);
         if (n <= 1) return false;
         float tn;
         if (CANON) {
-            float4 rlo = __ldg(S.nodes + 0), rhi = __ldg(S.nodes + 1);
+            float4 rlo = __ldg(sv_nodes(S) + 0), rhi = __ldg(sv_nodes(S) + 1);
             if (COUNT) ++K.nodes;
             if (!box_test<AXIS>(R, rlo, rhi, tmin, best_t, tn)) return false;
         } else {
@@ -667,7 +693,8 @@ struct Tracer {
 
     // spill: this thread's local-memory stack entries beyond the KS in shared
     // memory.
-    __device__ __forceinline__ bool step(const SceneView& S, StackSmem sm, uint32_t tid, uint32_t bdim,
+    template <class SV>
+    __device__ __forceinline__ bool step(const SV& S, StackSmem sm, uint32_t tid, uint32_t bdim,
                                          int2* spill, bool& overflow, TraceCounters& K) {
         // Every word of the traversal records is in range (checked when the
         // records are written), so only termination needs guarding here.
@@ -697,11 +724,11 @@ struct Tracer {
                     const int32_t k = w & kSlotMask;
                     if (!(w & kHoisted) && k != R.from) {
                         if (COUNT) ++K.spheres;
-                        leaf(k, __ldg(S.sph + k));
+                        leaf(k, __ldg(sv_sph(S) + k));
                     }
                 } else {
                     if (COUNT) ++K.nodes;
-                    h = box_test<AXIS>(R, __ldg(S.nodes + 2 * (size_t)w), __ldg(S.nodes + 2 * (size_t)w + 1), tmin,
+                    h = box_test<AXIS>(R, __ldg(sv_nodes(S) + 2 * (size_t)w), __ldg(sv_nodes(S) + 2 * (size_t)w + 1), tmin,
                                        best_t, tn);
                 }
                 if (c) {
@@ -749,7 +776,7 @@ struct Tracer {
         if (!have && !pop(sm, tid, bdim, spill)) return false;
         while (!CANON && cur < 0) {
             const int32_t k = cur & kSlotMask;
-            if (k != R.from) leaf(k, __ldg(S.sph + k));
+            if (k != R.from) leaf(k, __ldg(sv_sph(S) + k));
             if (!pop(sm, tid, bdim, spill)) return false;
         }
         return true;
@@ -989,8 +1016,8 @@ __device__ __forceinline__ RayPre prep_for(f3 o, f3 d) {
     return prep<!COUNT || WIDE>(o, d);
 }
 
-template <class T>
-__device__ __forceinline__ int32_t trace_with(const SceneView& S, const RayPre& R, float m, float tmin, float tmax,
+template <class T, class SV>
+__device__ __forceinline__ int32_t trace_with(const SV& S, const RayPre& R, float m, float tmin, float tmax,
                                               float& t_out, StackSmem sm, uint32_t tid, uint32_t bdim,
                                               bool& overflow, TraceCounters& K) {
     T W;
@@ -1007,8 +1034,8 @@ __device__ __forceinline__ int32_t trace_with(const SceneView& S, const RayPre& 
 // tree the canonical walk with one margin, or per axis for the rare
 // near-axis-parallel ray.  KS: shared-memory stack entries per thread (the
 // kernel's StackSmem holds KS of them).
-template <bool COUNT, int KS = kShared, bool WIDE = false>
-__device__ __forceinline__ int32_t trace_closest(const SceneView& S, const RayPre& R, float tmin,
+template <bool COUNT, int KS = kShared, bool WIDE = false, class SV>
+__device__ __forceinline__ int32_t trace_closest(const SV& S, const RayPre& R, float tmin,
                                                  float tmax, float& t_out, StackSmem sm,
                                                  uint32_t tid, uint32_t bdim, bool& overflow,
                                                  TraceCounters& K) {
@@ -1019,7 +1046,7 @@ __device__ __forceinline__ int32_t trace_closest(const SceneView& S, const RayPr
         axis_margins(A);
         return trace_with<Tracer<COUNT, true, true, KS>>(S, A, 0.0f, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
     }
-    if (WIDE)
+    if constexpr (WIDE)
         return trace_with<WideTracer<COUNT, KS>>(S, R, m, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
     return trace_with<Tracer<COUNT, COUNT, false, KS>>(S, R, m, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
 }
