@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const ui
     if (COUNT) flush_counters(K, stats);
 }
 
-__global__ void VENU_TRACE_BOUNDS k_walk(SceneView S, Queue q, const uint32_t* __restrict__ cnt,
+__global__ void VENU_WALK_BOUNDS k_walk(SceneView S, Queue q, const uint32_t* __restrict__ cnt,
                                          uint32_t* __restrict__ work, int2* __restrict__ hits,
                                          uint32_t* __restrict__ err, uint32_t walk_min) {
     extern __shared__ unsigned char smem[];
@@ -607,7 +607,7 @@ __global__ void VENU_WIDE_BOUNDS k_trace_shade_wide(SceneView S, Queue qin, uint
 // with refills, for more than spread_max rays (a thread each of the grid); the
 // other instantiation takes no more than that.
 template <bool COUNT, int KS, bool WIDE, bool REFILL>
-__global__ void VENU_TRACE_BOUNDS k_finish(SceneView S, Queue q0, Queue q1, float4* __restrict__ slots,
+__global__ void VENU_FINISH_BOUNDS k_finish(SceneView S, Queue q0, Queue q1, float4* __restrict__ slots,
                                            uint32_t* __restrict__ err, unsigned long long* __restrict__ stats,
                                            PrimaryGen gen, WaveCtl* ctl, uint32_t spread_max) {
     extern __shared__ unsigned char smem[];

@@ -18,15 +18,24 @@
 #ifndef VENU_MINMAX3
 #define VENU_MINMAX3 1
 #endif
-// Register cap of the fused traverse+shade kernels.  64 registers let 8
-// blocks of 128 threads (32 warps) stay resident per SM instead of 6 at the
-// 80 the compiler picks on its own, at the cost of a few spilled bytes;
-// measured on GB300: +8 % segments/s on the RTIOW scene, +6 % on 1M spheres
-// (72: +5 %, 56: +7 %, 48: slower).
+// Register caps of the binary tree's kernels.  The bounce kernel: at 56 nine
+// blocks of 128 threads (36 warps) stay resident per SM (1080p x 32 RTIOW at 48 /
+// 56 / 64 / 72: 13.53 / 13.23 / 13.36 / 14.28 ms).  The finishing kernel: 64 (400x225
+// x 16 at 48 / 56 / 64: 588 / 562 / 559 us; 300k spheres gain 1.6 % at 56, the
+// 4-wide tree loses 4 %).  The walk of large bounces: 64 (1M spheres 1080p x 4 at
+// 56 / 64 / 72: 72.1 / 71.2 / 79.2 ms).
 #ifndef VENU_TRACE_MAXREG
-#define VENU_TRACE_MAXREG 64
+#define VENU_TRACE_MAXREG 56
 #endif
 #define VENU_TRACE_BOUNDS __maxnreg__(VENU_TRACE_MAXREG)
+#ifndef VENU_FINISH_MAXREG
+#define VENU_FINISH_MAXREG 64
+#endif
+#define VENU_FINISH_BOUNDS __maxnreg__(VENU_FINISH_MAXREG)
+#ifndef VENU_WALK_MAXREG
+#define VENU_WALK_MAXREG 64
+#endif
+#define VENU_WALK_BOUNDS __maxnreg__(VENU_WALK_MAXREG)
 // Register cap of the fused kernel over the wide tree.  With 4 children per
 // node, 64 registers (8 resident 128-thread blocks per SM, a few spilled
 // bytes) beat 72 and 80 (6 and 5 blocks) on RTIOW (+5 %) and 1M spheres
@@ -35,7 +44,7 @@
 #define VENU_WIDE_MAXREG 64
 #endif
 #define VENU_WIDE_BOUNDS __maxnreg__(VENU_WIDE_MAXREG)
-// The multi-job kernel of the batch engine keeps a per-ray scene view.
+// The batch engine's kernels (96 uneven jobs at 56 / 64 / 72: 6.66 / 6.54 / 7.16 ms).
 #ifndef VENU_TRACE_MULTI_MAXREG
 #define VENU_TRACE_MULTI_MAXREG 64
 #endif
