@@ -109,11 +109,13 @@ template <bool COUNT, bool WIDE = false>
 __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const uint32_t* __restrict__ cnt,
                                                   uint32_t* __restrict__ work, int2* __restrict__ hits,
                                                   uint32_t* __restrict__ err,
-                                                  unsigned long long* __restrict__ stats, uint32_t walk_min) {
+                                                  unsigned long long* __restrict__ stats, uint32_t walk_min,
+                                                  uint32_t leave_max) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
     sm.e = reinterpret_cast<int2*>(smem);
     const uint32_t n = *cnt;
+    if (n <= leave_max) return;  // the finishing kernel's
     const uint32_t lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats, (unsigned long long)n);
     TraceCounters K{0, 0};
@@ -165,12 +167,12 @@ __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const ui
 
 __global__ void VENU_WALK_BOUNDS k_walk(SceneView S, Queue q, const uint32_t* __restrict__ cnt,
                                          uint32_t* __restrict__ work, int2* __restrict__ hits,
-                                         uint32_t* __restrict__ err, uint32_t walk_min) {
+                                         uint32_t* __restrict__ err, uint32_t walk_min, uint32_t leave_max) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
     sm.e = reinterpret_cast<int2*>(smem);
     const uint32_t n = *cnt;
-    if (n < walk_min) return;  // k_traverse did it
+    if (n < walk_min || n <= leave_max) return;  // k_traverse did it, or k_finish will
     const uint32_t lane = threadIdx.x & 31;
     TraceCounters K{0, 0};
     bool overflow = false;
@@ -597,6 +599,36 @@ __global__ void VENU_WIDE_BOUNDS k_trace_shade_wide(SceneView S, Queue qin, uint
                                       finish_max, next_max, handle);
 }
 
+// What the finishing kernels take: what the bounce kernels noted in WaveCtl, or
+// (cnt not null) what the separate traversals left, the first bounce b >= 1 of
+// at most leave_max rays.
+struct LeftOf {
+    const uint32_t* cnt;
+    uint32_t nb, leave_max;
+};
+__device__ __forceinline__ void find_left(const WaveCtl* ctl, LeftOf src, uint32_t& n, bool& primary, bool& second) {
+    if (!src.cnt) {
+        n = ctl->left;
+        primary = ctl->left_first != 0u;
+        second = ctl->left_q != 0u;
+        return;
+    }
+    n = 0;
+    primary = second = false;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t b0 = 1; b0 < src.nb; b0 += 32u) {
+        const uint32_t b = b0 + lane;
+        const uint32_t c = b < src.nb ? src.cnt[b] : 0xffffffffu;
+        const uint32_t m = __ballot_sync(0xffffffffu, c <= src.leave_max);
+        if (m) {
+            const int first = __ffs(m) - 1;
+            n = __shfl_sync(0xffffffffu, c, first);
+            second = ((b0 + (uint32_t)first) & 1u) != 0u;
+            return;
+        }
+    }
+}
+
 // The finishing kernel: runs the paths that are left of a wave (WaveCtl) to
 // their ends.  A kernel of its own, so that the bounce kernels' code and
 // registers are not shaped by it (in one kernel with them, changes to this
@@ -609,15 +641,15 @@ __global__ void VENU_WIDE_BOUNDS k_trace_shade_wide(SceneView S, Queue qin, uint
 template <bool COUNT, int KS, bool WIDE, bool REFILL>
 __global__ void VENU_FINISH_BOUNDS k_finish(SceneView S, Queue q0, Queue q1, float4* __restrict__ slots,
                                            uint32_t* __restrict__ err, unsigned long long* __restrict__ stats,
-                                           PrimaryGen gen, WaveCtl* ctl, uint32_t spread_max) {
+                                           PrimaryGen gen, WaveCtl* ctl, uint32_t spread_max, LeftOf src) {
     extern __shared__ unsigned char smem[];
     StackSmem sm;
     sm.e = reinterpret_cast<int2*>(smem);
     __shared__ DevCamera cam;
-    const uint32_t n = ctl->left;
+    uint32_t n;
+    bool primary, second;
+    find_left(ctl, src, n, primary, second);
     if (n == 0 || (n > spread_max) != REFILL) return;
-    const bool primary = ctl->left_first != 0u;
-    const bool second = ctl->left_q != 0u;
     const Queue qin = second ? q1 : q0, qout = second ? q0 : q1;
     if (primary) {
         if (threadIdx.x == 0) cam = load_camera(gen.cam);
@@ -638,10 +670,128 @@ __global__ void VENU_FINISH_BOUNDS k_finish(SceneView S, Queue q0, Queue q1, flo
     if (COUNT) flush_counters(K, stats);
 }
 
+// k_finish for large scenes, whose walks are long and uneven (20 to 400 steps): a
+// lane whose walk is done does not wait for the other 31.  Once half of a
+// warp's paths are through their walks, those are shaded together, start their
+// next segments (or new paths) and walk on; the lanes vote every kWalkSteps
+// steps, as in k_walk.  Shading and the up-front tests then run for half a warp
+// at a time, which long walks pay for and short ones do not.
+// Against k_finish, from 7168 spheres up (ms): 8k spheres 1080p x 8 8.28 -> 8.13,
+// 100k 1080p x 1 4.37 -> 3.95, 300k 512x512 x 4 with its build 5.72 -> 5.28, 1M
+// 1080p x 1 20.8 -> 18.6; 5k 640x480 x 4 0.780 -> 0.797.  Serving at half of the
+// paths (an eighth: 19.0 on the last), votes every 16 steps (8: 28.3, 64: 19.3).
+template <int KS>
+__global__ void VENU_WALK_BOUNDS k_finish_walk(SceneView S, Queue q0, Queue q1, float4* __restrict__ slots,
+                                               uint32_t* __restrict__ err, unsigned long long* __restrict__ stats,
+                                               PrimaryGen gen, WaveCtl* ctl, uint32_t spread_max, LeftOf src) {
+    extern __shared__ unsigned char smem[];
+    StackSmem sm;
+    sm.e = reinterpret_cast<int2*>(smem);
+    __shared__ DevCamera cam;
+    uint32_t n;
+    bool primary, second;
+    find_left(ctl, src, n, primary, second);
+    if (n == 0 || n <= spread_max) return;
+    const Queue qin = second ? q1 : q0, qout = second ? q0 : q1;
+    if (primary) {
+        if (threadIdx.x == 0) cam = load_camera(gen.cam);
+        __syncthreads();
+    }
+    const uint32_t lane = threadIdx.x & 31u;
+    TraceCounters K{0, 0};
+    bool overflow = false;
+    Tracer<false, false, false, KS> T;
+    int2 spill[kSpill];
+    uint32_t own = 0xffffffffu;  // the first ray this lane took
+    uint32_t traced = 0, slot = 0, dbits = 0;
+    bool has = false, walking = false, exhausted = false;
+    for (;;) {
+        float4 o4, d4;
+        bool start = false;
+        if (has && !walking) {
+            float t;
+            const int32_t k = T.result(t);
+            const ShadeOut r = shade_one<true>(
+                S, make_float4(T.R.o.x, T.R.o.y, T.R.o.z, __int_as_float((int)slot)),
+                make_float4(T.R.d.x, T.R.d.y, T.R.d.z, __uint_as_float(dbits)), qout.t[own], make_int2(__float_as_int(t), k));
+            if (r.cont) {
+                o4 = r.o;
+                d4 = r.d;
+                qout.t[own] = r.t;
+                start = true;
+            } else {
+                slots[slot] = r.result;
+                has = false;
+            }
+        }
+        if (!exhausted) {
+            const uint32_t empty = __ballot_sync(0xffffffffu, !has);
+            const uint32_t take = (uint32_t)__popc(empty);
+            if (take) {
+                uint32_t base = 0;
+                if (lane == 0) base = atomicAdd(&ctl->left_work, take);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                exhausted = base >= n || n - base <= take;
+                const uint32_t ray = base + (uint32_t)__popc(empty & ((1u << lane) - 1u));
+                if (!has && base < n && ray < n) {
+                    has = start = true;
+                    if (own == 0xffffffffu) own = ray;
+                    if (primary) {
+                        uint32_t seed = 0;
+                        gen_primary(gen, cam, ray, o4, d4, seed);
+                        qout.t[own] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(seed));
+                    } else {
+                        o4 = qin.o[ray];
+                        d4 = qin.d[ray];
+                        qout.t[own] = qin.t[ray];
+                    }
+                    slot = (uint32_t)__float_as_int(o4.w);
+                }
+            }
+        }
+        if (start) {
+            ++traced;
+            dbits = __float_as_uint(d4.w);
+            RayPre R = prep_for<false>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            R.from = packed_from(d4.w);
+            const float m = ray_margin(S, R);
+            T.open(R, m, 0.001f, 1e16f, 1e16f, kNone);
+            if (!(m <= kFarMarginMax)) {  // rare: traced to the end now
+                R = prep<false>(R.o, R.d);
+                R.from = packed_from(d4.w);
+                axis_margins(R);
+                float t;
+                const int32_t k = trace_with<Tracer<false, true, true, KS>>(S, R, 0.0f, 0.001f, 1e16f, t, sm, threadIdx.x,
+                                                                           blockDim.x, overflow, K);
+                T.best_t = t;
+                T.best = k < 0 ? kNone : k;
+            } else {
+                up_front(T, S, K);
+                walking = T.enter(S, K);
+            }
+        }
+        const uint32_t paths = (uint32_t)__popc(__ballot_sync(0xffffffffu, has));
+        if (paths == 0u) break;  // only once there are no rays left
+        const uint32_t enough = max(1u, paths >> 1);
+        for (;;) {
+            const uint32_t w = __ballot_sync(0xffffffffu, walking);
+            if (paths - (uint32_t)__popc(w) >= enough) break;
+            if (walking)
+                for (int i = 0; i < kWalkSteps && walking; ++i)
+                    walking = T.step(S, sm, threadIdx.x, blockDim.x, spill, overflow, K);
+        }
+    }
+    traced = __reduce_add_sync(0xffffffffu, traced);
+    if (lane == 0 && traced) atomicAdd(stats, (unsigned long long)traced);
+    if (overflow) atomicOr(err, 1u);
+}
+
 __global__ void __launch_bounds__(512) k_shade(SceneView S, Queue qin, const int2* __restrict__ hits,
                                                const uint32_t* __restrict__ cnt_in, Queue qout,
-                                               uint32_t* __restrict__ cnt_out, float4* __restrict__ slots) {
+                                               uint32_t* __restrict__ cnt_out, float4* __restrict__ slots,
+                                               uint32_t leave_max) {
     const uint32_t n = *cnt_in;
+    if (n <= leave_max) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
@@ -901,6 +1051,7 @@ constexpr uint32_t kMaxDepth = 64;
 // 640x360 x 4 on 300k spheres takes 8.80 instead of 8.48; from 2M up, 1280x720
 // x 8 on 1M spheres 65.1 instead of 64.4.
 constexpr uint32_t kWalkSpheres = 16384, kWalkRays = 1u << 20;
+constexpr uint32_t kFinishWalkSpheres = 7168;  // see k_finish_walk
 // Where a caller's rays are split the same way (us without -> with): 1M rays on
 // 20k spheres 636 -> 719, 2M on 50k 1472 -> 1512, 2M on 100k 1656 -> 1536, 2M on
 // 200k 1740 -> 1508, 500k on 100k 589 -> 549, 250k on 200k 359 -> 360.
@@ -945,6 +1096,9 @@ cudaError_t configure_fused(venu_renderer* r, K8 deep, K4 shallow, C8 count_deep
     if (e == cudaSuccess) e = set_smem(k_finish<true, kSharedShallow, WIDE, false>, sm);
     if (e == cudaSuccess) e = set_smem(k_finish<true, kShared, WIDE, true>, sm);
     if (e == cudaSuccess) e = set_smem(k_finish<true, kSharedShallow, WIDE, true>, sm);
+    if (!WIDE && e == cudaSuccess) e = set_smem(k_finish_walk<kShared>, sm);
+    if (!WIDE && e == cudaSuccess) e = set_smem(k_finish_walk<kSharedShallow>, sm);
+    if (!WIDE && e == cudaSuccess) e = prefer_l1(k_finish_walk<kShared>, std::max(1, r->finish_blocks / std::max(1, sm_count())), sm);
     const int nsm = std::max(1, sm_count());
     const int pb = std::max(1, r->fused_blocks / nsm), pf = std::max(1, r->finish_blocks / nsm);
     if (e == cudaSuccess) e = prefer_l1(deep, pb, sm);
@@ -1075,17 +1229,21 @@ cudaError_t launch_fused(const venu_renderer* r, cudaStream_t st, uint32_t kind,
 // spreading one, or by whichever finds its number of rays.
 constexpr uint32_t kFinishRefill = 1u, kFinishSpread = 2u;
 cudaError_t launch_finish(const venu_renderer* r, cudaStream_t st, uint32_t kind, size_t fsm, const SceneView& S,
-                          const PrimaryGen& pg, uint32_t which) {
+                          const PrimaryGen& pg, uint32_t which, LeftOf src = LeftOf{nullptr, 0u, 0u}) {
     const int grid = r->finish_blocks, tb = (int)r->tune.traverse_block;
     const uint32_t spread_max = (uint32_t)grid * (uint32_t)tb;
+    const bool walk = S.n >= kFinishWalkSpheres && !(kind & (kFusedWide | kFusedCount));
 #define VENU_FINISH(WIDE, C, KS)                                                                                  \
     do {                                                                                                          \
-        if (which & kFinishRefill)                                                                                \
+        if (walk && (which & kFinishRefill))                                                                      \
+            k_finish_walk<KS><<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, \
+                                                     spread_max, src);                                            \
+        else if (which & kFinishRefill)                                                                           \
             k_finish<C, KS, WIDE, true>                                                                           \
-                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, spread_max); \
+                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, spread_max, src); \
         if (which & kFinishSpread)                                                                                \
             k_finish<C, KS, WIDE, false>                                                                          \
-                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, spread_max); \
+                <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, spread_max, src); \
     } while (0)
     if (kind & kFusedWide) VENU_FUSED_CS(VENU_FINISH, true);
     else VENU_FUSED_CS(VENU_FINISH, false);
@@ -1361,11 +1519,17 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
     // 4 with its build 6.73 / 5.89 / 5.90; but 100k 1080p x 1, whose 2.1M camera
     // rays only 16 takes, 4.99 / 4.46 / 5.16.
     const uint64_t threads = (uint64_t)r->finish_blocks * (uint64_t)tb;
-    const uint64_t asked = tu.in_place_factor > 1u ? tu.in_place_factor : 16u;
+        // Scenes that k_finish_walk serves are its own after the first bounce (at 16 /
+    // 64 / any number of rays a thread, 1080p x 8 on 20k spheres takes 12.9 / 12.9 /
+    // 12.5 ms, on 300k 54.7 / 52.0 / 50.5; RTIOW at any number 15.0 instead of 13.3
+    // over its bounces), but not of the separate traversals.
+    const bool walks = scene->n >= kFinishWalkSpheres && tu.traverse_variant == 2u && !count;
+    const uint64_t asked = tu.in_place_factor > 1u ? tu.in_place_factor : walks ? 1u << 20 : 16u;
     const uint32_t finish_max = gen0 ? (uint32_t)std::min<uint64_t>(asked * threads, 0xffffffffu) : 0u;
     const uint32_t first_max =
         gen0 ? (uint32_t)(tu.in_place_factor > 1u || shallow ? finish_max : threads) : 0u;
     const uint32_t bounce_max = fused ? finish_max : 0u;
+    const uint32_t leave_max = gen0 && !fused ? finish_max : 0u;
     use_graph = use_graph && (uint64_t)npix * k > first_max;
     if (use_graph) {
         WaveGraphKey key;
@@ -1464,22 +1628,22 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
                 if (v == 0) {
                     if (count)
                         k_traverse<true><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b, r->hits,
-                                                                         r->err, r->stats, ~0u);
+                                                                         r->err, r->stats, ~0u, leave_max);
                     else
                         k_traverse<false><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b, r->hits,
-                                                                          r->err, r->stats, walk_min);
+                                                                          r->err, r->stats, walk_min, leave_max);
                     if (walk_min != ~0u) {
                         k_walk<<<r->walk_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b, r->hits, r->err,
-                                                                walk_min);
+                                                                walk_min, leave_max);
                         ++launches;
                     }
                 } else if (v == 5) {
                     if (count)
                         k_traverse<true, true><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b,
-                                                                               r->hits, r->err, r->stats, ~0u);
+                                                                               r->hits, r->err, r->stats, ~0u, leave_max);
                     else
                         k_traverse<false, true><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b,
-                                                                                r->hits, r->err, r->stats, ~0u);
+                                                                                r->hits, r->err, r->stats, ~0u, leave_max);
                 } else {
                     if (count)
                         k_traverse_dyn<true><<<r->trav_blocks, tb, tsm, st>>>(S, qi, r->cnt + b, r->work + b, r->hits,
@@ -1492,21 +1656,23 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
                     VENU_CUDA(cudaEventRecord(e1, st));
                     VENU_CUDA(cudaEventRecord(e2, st));
                 }
-                k_shade<<<r->shade_blocks, sb, 0, st>>>(S, qi, r->hits, r->cnt + b, qo, r->cnt + b + 1, r->slots);
+                k_shade<<<r->shade_blocks, sb, 0, st>>>(S, qi, r->hits, r->cnt + b, qo, r->cnt + b + 1, r->slots,
+                                                        leave_max);
                 if (prof) VENU_CUDA(cudaEventRecord(e3, st));
                 launches += 2;
             }
-            if (fused && !small && !use_graph) {  // what the bounces left
+            if (gen0 && !small && !use_graph) {  // what the bounces left
+                const LeftOf src = fused ? LeftOf{nullptr, 0u, 0u} : LeftOf{r->cnt, (uint32_t)nb, leave_max};
                 if (prof) {
                     for (int i = 0; i < 2; ++i) {
                         cudaEvent_t a, z;
                         VENU_CUDA(next_events(r, a, z));
                         VENU_CUDA(cudaEventRecord(a, st));
-                        if (i == 0) VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg, which));
+                        if (i == 0) VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg, which, src));
                         VENU_CUDA(cudaEventRecord(z, st));
                     }
                 } else {
-                    VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg, which));
+                    VENU_CUDA(launch_finish(r, st, kind, fsm, S, pg, which, src));
                 }
                 launches += finishes;
             }
