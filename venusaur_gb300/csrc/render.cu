@@ -1096,9 +1096,9 @@ cudaError_t configure_fused(venu_renderer* r, K8 deep, K4 shallow, C8 count_deep
     if (e == cudaSuccess) e = set_smem(k_finish<true, kSharedShallow, WIDE, false>, sm);
     if (e == cudaSuccess) e = set_smem(k_finish<true, kShared, WIDE, true>, sm);
     if (e == cudaSuccess) e = set_smem(k_finish<true, kSharedShallow, WIDE, true>, sm);
-    if (!WIDE && e == cudaSuccess) e = set_smem(k_finish_walk<kShared>, sm);
-    if (!WIDE && e == cudaSuccess) e = set_smem(k_finish_walk<kSharedShallow>, sm);
-    if (!WIDE && e == cudaSuccess) e = prefer_l1(k_finish_walk<kShared>, std::max(1, r->finish_blocks / std::max(1, sm_count())), sm);
+    if (e == cudaSuccess) e = set_smem(k_finish_walk<kShared>, sm);
+    if (e == cudaSuccess) e = set_smem(k_finish_walk<kSharedShallow>, sm);
+    if (e == cudaSuccess) e = prefer_l1(k_finish_walk<kShared>, std::max(1, r->finish_blocks / std::max(1, sm_count())), sm);
     const int nsm = std::max(1, sm_count());
     const int pb = std::max(1, r->fused_blocks / nsm), pf = std::max(1, r->finish_blocks / nsm);
     if (e == cudaSuccess) e = prefer_l1(deep, pb, sm);
@@ -1232,7 +1232,7 @@ cudaError_t launch_finish(const venu_renderer* r, cudaStream_t st, uint32_t kind
                           const PrimaryGen& pg, uint32_t which, LeftOf src = LeftOf{nullptr, 0u, 0u}) {
     const int grid = r->finish_blocks, tb = (int)r->tune.traverse_block;
     const uint32_t spread_max = (uint32_t)grid * (uint32_t)tb;
-    const bool walk = S.n >= kFinishWalkSpheres && !(kind & (kFusedWide | kFusedCount));
+    const bool walk = S.n >= kFinishWalkSpheres && !(kind & kFusedCount);  // over the binary tree always
 #define VENU_FINISH(WIDE, C, KS)                                                                                  \
     do {                                                                                                          \
         if (walk && (which & kFinishRefill))                                                                      \
@@ -1522,9 +1522,10 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
         // Scenes that k_finish_walk serves are its own after the first bounce (at 16 /
     // 64 / any number of rays a thread, 1080p x 8 on 20k spheres takes 12.9 / 12.9 /
     // 12.5 ms, on 300k 54.7 / 52.0 / 50.5; RTIOW at any number 15.0 instead of 13.3
-    // over its bounces), but not of the separate traversals.
-    const bool walks = scene->n >= kFinishWalkSpheres && tu.traverse_variant == 2u && !count;
-    const uint64_t asked = tu.in_place_factor > 1u ? tu.in_place_factor : walks ? 1u << 20 : 16u;
+    // over its bounces); after the separate traversals it takes up to 32 (1M 1919x1079
+    // x 8 at 8 / 16 / 32 / 64: 131.0 / 129.6 / 129.2 / 130.3 ms).
+    const bool walks = scene->n >= kFinishWalkSpheres && !count;
+    const uint64_t asked = tu.in_place_factor > 1u ? tu.in_place_factor : !walks ? 16u : fused ? 1u << 20 : 32u;
     const uint32_t finish_max = gen0 ? (uint32_t)std::min<uint64_t>(asked * threads, 0xffffffffu) : 0u;
     const uint32_t first_max =
         gen0 ? (uint32_t)(tu.in_place_factor > 1u || shallow ? finish_max : threads) : 0u;
