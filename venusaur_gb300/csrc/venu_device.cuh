@@ -542,6 +542,21 @@ __device__ __forceinline__ void flush_counters(const TraceCounters& K, unsigned 
     }
 }
 
+// Whether the ray surely does not hit the sphere it leaves again: it heads
+// outwards (hb > 0), so both roots but c/q are negative, and c/q, which is at
+// most -c / hb, lies below tmin > 0.  The refined c (sphere_test) differs from
+// the plain one by at most (5 |h|^2 + r^2 + |c|) 2^-24, here 4 2^-24 of
+// |h|^2 + r^2, and hb by at most 2^-24 |h| |d|, which is 2^-9 of it where the
+// cosine is above 2^-15.  Anything not finite takes the test.
+__device__ __forceinline__ bool left_behind(const RayPre& R, float4 s4, float tmin) {
+    const float hx = R.o.x - s4.x, hy = R.o.y - s4.y, hz = R.o.z - s4.z;
+    const float hb = fmaf(hx, R.d.x, fmaf(hy, R.d.y, hz * R.d.z));
+    const float hh = fmaf(hx, hx, fmaf(hy, hy, hz * hz));
+    const float r2 = s4.w * s4.w;
+    return hb > 1e-15f && hb * hb > hh * R.a * 9.31322574615478515625e-10f &&      // 2^-30
+           fmaf(hh + r2, -2.384185791015625e-07f, hh - r2) > hb * tmin * -0.99f;  // 2^-22
+}
+
 // Tested up front, with the whole warp converged: first the sphere the
 // ray leaves (R.from; its origin lies within r/16 of that surface, so its
 // test takes sphere_test's long refined branch, which in the walk would
@@ -550,13 +565,23 @@ __device__ __forceinline__ void flush_counters(const TraceCounters& K, unsigned 
 // their hit distances already cull boxes behind them.  The closest hit
 // does not depend on the order of the tests.  (A scene of one sphere has
 // it hoisted, see view_of.)  One copy of the test for all of them.
+// Most rays leave their sphere behind; those test the ground while the others
+// test the sphere they came from, and a warp without rays inside glass takes
+// one round of the test instead of two (RTIOW 1920x1080 x 32 13.24 -> 13.04 ms,
+// 256x144 x 4 240 -> 228 us).
 template <typename T, class SV>
 __device__ __forceinline__ void up_front(T& W, const SV& S, TraceCounters& K) {
     const int nh = (int)sv_nhoist(S);
+    const int32_t from = W.R.from;
+    int h = 0;
+    if (from >= 0) {
+        if (left_behind(W.R, __ldg(sv_sph(S) + from), W.tmin)) ++K.spheres;
+        else h = -1;
+    }
 #pragma unroll 1
-    for (int h = W.R.from >= 0 ? -1 : 0; h < nh; ++h) {
-        const int32_t k = h < 0 ? W.R.from : sv_hoist(S, h);
-        if (h >= 0 && k == W.R.from) continue;
+    for (; h < nh; ++h) {
+        const int32_t k = h < 0 ? from : sv_hoist(S, h);
+        if (h >= 0 && k == from) continue;
         ++K.spheres;
         W.leaf(k, __ldg(sv_sph(S) + k));
     }
