@@ -402,6 +402,18 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
     return r;
 }
 
+// Packed sum and product; fma2(b, neg1, a) is a - b (one rounding).
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // 32 bytes with one instruction (32-byte aligned, read-only data).
 __device__ __forceinline__ void ldg32(const void* p, f2& a, f2& b, f2& c, f2& d) {
     asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
@@ -414,8 +426,10 @@ __device__ __forceinline__ void ldg32(const void* p, f2& a, f2& b, f2& c, f2& d)
 // roots come from q = -(b + sign(b) sqrt(disc)) as q/a and c/q (no
 // cancellation).  When the origin is close to the surface relative to the
 // radius (|c| < (|h|^2 + r^2)/16), c = |o-C|^2 - r^2 and h are refined with
-// TwoDiff/TwoProduct/TwoSum error terms, so the near root c/q keeps full
-// relative accuracy even for the r = 1000 ground sphere.  Root selection
+// TwoDiff/TwoProduct/TwoSum error terms (x and y packed; packing the second half
+// of the branch as well loses again what this gains: RTIOW 1920x1080 x 32 13.10
+// -> 12.95 ms, 13.07 with both), so the near root c/q keeps full relative accuracy
+// even for the r = 1000 ground sphere.  Root selection
 // follows Core/RayTracer.cu:248-253: the smaller root in [tmin, tmax], else
 // the larger.
 __device__ __forceinline__ bool sphere_test(const RayPre& R, float4 S, float tmin, float tmax,
@@ -430,15 +444,24 @@ __device__ __forceinline__ bool sphere_test(const RayPre& R, float4 S, float tmi
     // the centre (h.d > 0): both roots are negative, no hit.
     if (hb > 0.0f && c > (hh + r2) * 9.5367431640625e-07f) return false;  // 2^-20
     float discp;
+    const f2 neg1 = pack2(-1.0f, -1.0f);
     if (fabsf(c) < (hh + r2) * 0.0625f) {
         // exact residuals of h = o - C (TwoDiff)
-        float bvx = R.o.x - hx, bvy = R.o.y - hy, bvz = R.o.z - hz;
-        float ex = (R.o.x - (hx + bvx)) + (bvx - S.x);
-        float ey = (R.o.y - (hy + bvy)) + (bvy - S.y);
+        const f2 O = pack2(R.o.x, R.o.y), Cn = pack2(-S.x, -S.y), H = pack2(hx, hy);
+        const f2 Bv = fma2(H, neg1, O);
+        const f2 E2 = add2(fma2(add2(H, Bv), neg1, O), add2(Bv, Cn));
+        float bvz = R.o.z - hz;
+        float ex, ey;
+        unpack2(E2, ex, ey);
         float ez = (R.o.z - (hz + bvz)) + (bvz - S.z);
         // c = |h + e|^2 - r^2 from exact squares and compensated sums
-        float px = hx * hx, py = hy * hy, pz = hz * hz;
-        float qx = fmaf(hx, hx, -px), qy = fmaf(hy, hy, -py), qz = fmaf(hz, hz, -pz);
+        const f2 P2 = mul2(H, H);
+        const f2 Q2 = fma2(H, H, mul2(P2, neg1));
+        float px, py, qx, qy;
+        unpack2(P2, px, py);
+        unpack2(Q2, qx, qy);
+        float pz = hz * hz;
+        float qz = fmaf(hz, hz, -pz);
         float qr = fmaf(r, r, -r2);
         float s1, e1, s2, e2, s3, e3;
         two_sum(px, py, s1, e1);
