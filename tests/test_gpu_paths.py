@@ -185,6 +185,24 @@ def test_finishing_shares(venu, oracle, cuda, W, H, spp, variant, factor):
     assert wf.stats()["segments"] == want["segments"]
 
 
+# scenes of 7168 spheres and more finish over the binary tree with refilled walks
+@pytest.mark.parametrize("n", [7167, 7168])
+@pytest.mark.parametrize("variant,factor", [(0, 1), (1, 1), (2, 1), (2, 16), (3, 1), (4, 1), (4, 16), (5, 1)])
+def test_finishing_walks(venu, oracle, cuda, n, variant, factor):
+    W, H, spp, depth = 311, 101, 2, 30
+    sp = oracle.scene_random(n, 21, (-40, 0, -40), (40, 12, 40))
+    cam = oracle.camera((30, 10, 30), (0, 4, 0), 40.0, W / H, 0.05, 30.0)
+    want = oracle.render(sp, cam, W, H, spp, subframe=1, max_depth=depth, mode=pyoracle.MODE_GB300)
+    ds = venu.DeviceScene(sp)
+    wf = venu.Wavefront(0)
+    wf.set_tuning(traverse_variant=variant, in_place_factor=factor)
+    acc = venu.new_accum(W, H)
+    wf.render(ds, cam, W, H, spp, acc, subframe=1, max_depth=depth, reset=True)
+    cuda.cuda.synchronize()
+    assert np.array_equal(acc.cpu().numpy().view(np.uint32), want["accum"].view(np.uint32))
+    assert wf.stats()["segments"] == want["segments"]
+
+
 def test_waves_accumulate_and_resolve_once(venu, oracle, cuda):
     """Several waves of part of the pixels and of part of the samples: each pixel
     starts from zero (or from what is there) once and is resolved once."""
