@@ -203,6 +203,24 @@ def test_finishing_walks(venu, oracle, cuda, n, variant, factor):
     assert wf.stats()["segments"] == want["segments"]
 
 
+# the block's survivors are placed by a sum over its 2 to 16 warps
+@pytest.mark.parametrize("shade_block", [64, 96, 480, 512])
+@pytest.mark.parametrize("variant", [0, 3])
+def test_separate_shading_blocks(venu, oracle, cuda, variant, shade_block):
+    W, H, spp, depth = 641, 487, 2, 6  # twice what one 128-thread block an SM leaves to the finishing kernel
+    sp = oracle.scene_random(500, 31, (-10, 0, -10), (10, 3, 10))
+    cam = oracle.camera((13, 2, 3), (0, 1, 0), 30.0, W / H, 0.1, 10.0)
+    want = oracle.render(sp, cam, W, H, spp, subframe=1, max_depth=depth, mode=pyoracle.MODE_GB300)
+    ds = venu.DeviceScene(sp)
+    wf = venu.Wavefront(0)
+    wf.set_tuning(traverse_variant=variant, traverse_block=128, traverse_blocks_per_sm=1, shade_block=shade_block)
+    acc = venu.new_accum(W, H)
+    wf.render(ds, cam, W, H, spp, acc, subframe=1, max_depth=depth, reset=True)
+    cuda.cuda.synchronize()
+    assert np.array_equal(acc.cpu().numpy().view(np.uint32), want["accum"].view(np.uint32))
+    assert wf.stats()["segments"] == want["segments"]
+
+
 def test_waves_accumulate_and_resolve_once(venu, oracle, cuda):
     """Several waves of part of the pixels and of part of the samples: each pixel
     starts from zero (or from what is there) once and is resolved once."""
