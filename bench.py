@@ -80,23 +80,26 @@ KERNEL_SOURCES = ("venusaur_gb300/csrc/venu_device.cuh", "venusaur_gb300/csrc/re
 # segments; lanes_per_inst = smsp__thread_inst_executed_per_inst_executed.ratio
 # (active lanes per issued instruction, all instructions).  `sha` is
 # kernel_sources_sha() of the captured build.  Each figure is summed over the
-# k_trace_shade (and, for variant 3, k_traverse) launches of two renders of
+# launches of the fused bounce, separate traversal, walk, shading and finishing
+# kernels of two renders of
 # `bench.py --config <c> --spp <s> --profile-render --tuning <variant>`
-# (c2: 4 spp, c3: 2 spp, c1: its own 16 spp; "/f8": in_place_factor 8;
-# traverse_block 256 for c2/v2, c3/v2 and c3/v3, 128 for the others)
+# (c2: 4 spp, c3: 16 spp, c1: its own 16 spp; traverse_block 128;
+# "/f8": in_place_factor 8)
 # under ncu --metrics
 # dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum,
 # smsp__inst_executed.sum,smsp__thread_inst_executed.sum.
-NCU_FIGURES = {"sha": "7ec4d38e57e4d468", "commit": "4264606", "figures": {
-    "c2/v2": {"dram_b_per_seg": 62.6, "lanes_per_inst": 15.87, "warp_inst_per_seg": 82.1},
-    "c2/v4": {"dram_b_per_seg": 63.86, "lanes_per_inst": 17.82, "warp_inst_per_seg": 84.3},
-    "c1/v2": {"dram_b_per_seg": 38.26, "lanes_per_inst": 14.14, "warp_inst_per_seg": 104.0},
-    "c1/v2/f8": {"dram_b_per_seg": 25.28, "lanes_per_inst": 14.96, "warp_inst_per_seg": 108.5},
-    "c1/v4": {"dram_b_per_seg": 41.31, "lanes_per_inst": 16.01, "warp_inst_per_seg": 104.6},
-    "c1/v4/f8": {"dram_b_per_seg": 26.64, "lanes_per_inst": 16.92, "warp_inst_per_seg": 110.1},
-    "c3/v3": {"dram_b_per_seg": 62.21, "lanes_per_inst": 6.58, "warp_inst_per_seg": 657.5},
-    "c3/v2": {"dram_b_per_seg": 127.3, "lanes_per_inst": 6.41, "warp_inst_per_seg": 721.7},
-    "c3/v5": {"dram_b_per_seg": 60.63, "lanes_per_inst": 8.48, "warp_inst_per_seg": 630.0},
+NCU_FIGURES = {"sha": "3907a01b4837d234", "commit": "9b77301", "figures": {
+    "c2/v2": {"dram_b_per_seg": 57.43, "lanes_per_inst": 14.71, "warp_inst_per_seg": 71.5},
+    "c2/v2/f8": {"dram_b_per_seg": 60.82, "lanes_per_inst": 14.65, "warp_inst_per_seg": 71.9},
+    "c2/v4": {"dram_b_per_seg": 57.67, "lanes_per_inst": 16.04, "warp_inst_per_seg": 81.3},
+    "c1/v2": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.97, "warp_inst_per_seg": 94.2},
+    "c1/v2/f8": {"dram_b_per_seg": 24.84, "lanes_per_inst": 12.06, "warp_inst_per_seg": 92.9},
+    "c1/v3": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.98, "warp_inst_per_seg": 94.1},
+    "c1/v4": {"dram_b_per_seg": 2.4, "lanes_per_inst": 11.97, "warp_inst_per_seg": 107.7},
+    "c1/v4/f8": {"dram_b_per_seg": 25.79, "lanes_per_inst": 12.95, "warp_inst_per_seg": 105.5},
+    "c3/v3": {"dram_b_per_seg": 75.6, "lanes_per_inst": 10.67, "warp_inst_per_seg": 397.8},
+    "c3/v2": {"dram_b_per_seg": 13.86, "lanes_per_inst": 9.38, "warp_inst_per_seg": 479.7},
+    "c3/v5": {"dram_b_per_seg": 39.6, "lanes_per_inst": 8.4, "warp_inst_per_seg": 548.0},
 }}
 
 
@@ -771,10 +774,11 @@ def measure_plain(venu, torch, rep, name, cfg, args, steps, warmup, headline):
     # write after the bounce).
     trav_bytes = nodes * 32 + sph * 16
     if fused:
-        kernel = "k_trace_shade" if variant == 2 else "k_trace_shade_wide"
+        kernel = ("k_trace_shade" if variant == 2 else "k_trace_shade_wide") + ", k_finish"
         kbytes = trav_bytes + paths_c * 32 + (segs_c - paths_c) * 112
     elif variant in (3, 5):  # fused primary bounce, separate traversal after it
-        kernel = "k_trace_shade (primary) + k_traverse" + (" (4-wide tree)" if variant == 5 else "")
+        kernel = ("k_trace_shade (primary), k_traverse" + (" (4-wide tree)" if variant == 5 else ", k_walk")
+                  + ", k_finish")
         kbytes = trav_bytes + paths_c * 32 + (segs_c - paths_c) * 40
     else:
         kernel = "k_traverse"
