@@ -637,7 +637,11 @@ __device__ __forceinline__ void find_left(const WaveCtl* ctl, LeftOf src, uint32
 // 260 us, 64x36 x 2 107 -> 90 us.  At 80 / 96 / 128 registers, with as many
 // fewer rays to take, the 256x144 frame takes 297 / 296 / 295 us.  REFILL:
 // with refills, for more than spread_max rays (a thread each of the grid); the
-// other instantiation takes no more than that.
+// other instantiation takes no more than that.  WIDE: counting builds of variant 4
+// alone.  The others finish over the binary tree after either bounce kernel: a
+// warp with few active lanes waits for every instruction of a wide step (RTIOW
+// 400x225 x 16 654 -> 579 us with variant 4, 256x144 x 4 250 -> 227, 5k random
+// spheres 640x360 x 4 655 -> 593, 1280x720 x 8 3.74 -> 3.69 ms).
 template <bool COUNT, int KS, bool WIDE, bool REFILL>
 __global__ void VENU_FINISH_BOUNDS k_finish(SceneView S, Queue q0, Queue q1, float4* __restrict__ slots,
                                            uint32_t* __restrict__ err, unsigned long long* __restrict__ stats,
@@ -1111,10 +1115,10 @@ cudaError_t configure_fused(venu_renderer* r, K8 deep, K4 shallow, C8 count_deep
     if (e == cudaSuccess) e = set_smem(count_deep, sm);
     if (e == cudaSuccess) e = set_smem(count_shallow, sm);
     if (e == cudaSuccess)
-        e = occupancy_grid(k_finish<false, kShared, WIDE, false>, tb, sm, t.traverse_blocks_per_sm, r->finish_blocks);
-    if (e == cudaSuccess) e = set_smem(k_finish<false, kSharedShallow, WIDE, false>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish<false, kShared, WIDE, true>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish<false, kSharedShallow, WIDE, true>, sm);
+        e = occupancy_grid(k_finish<false, kShared, false, false>, tb, sm, t.traverse_blocks_per_sm, r->finish_blocks);
+    if (e == cudaSuccess) e = set_smem(k_finish<false, kSharedShallow, false, false>, sm);
+    if (e == cudaSuccess) e = set_smem(k_finish<false, kShared, false, true>, sm);
+    if (e == cudaSuccess) e = set_smem(k_finish<false, kSharedShallow, false, true>, sm);
     if (e == cudaSuccess) e = set_smem(k_finish<true, kShared, WIDE, false>, sm);
     if (e == cudaSuccess) e = set_smem(k_finish<true, kSharedShallow, WIDE, false>, sm);
     if (e == cudaSuccess) e = set_smem(k_finish<true, kShared, WIDE, true>, sm);
@@ -1126,10 +1130,10 @@ cudaError_t configure_fused(venu_renderer* r, K8 deep, K4 shallow, C8 count_deep
     const int pb = std::max(1, r->fused_blocks / nsm), pf = std::max(1, r->finish_blocks / nsm);
     if (e == cudaSuccess) e = prefer_l1(deep, pb, sm);
     if (e == cudaSuccess) e = prefer_l1(shallow, pb, ss);
-    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kShared, WIDE, false>, pf, sm);
-    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kSharedShallow, WIDE, false>, pf, ss);
-    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kShared, WIDE, true>, pf, sm);
-    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kSharedShallow, WIDE, true>, pf, ss);
+    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kShared, false, false>, pf, sm);
+    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kSharedShallow, false, false>, pf, ss);
+    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kShared, false, true>, pf, sm);
+    if (e == cudaSuccess) e = prefer_l1(k_finish<false, kSharedShallow, false, true>, pf, ss);
     return e;
 }
 
@@ -1255,17 +1259,17 @@ cudaError_t launch_finish(const venu_renderer* r, cudaStream_t st, uint32_t kind
                           const PrimaryGen& pg, uint32_t which, LeftOf src = LeftOf{nullptr, 0u, 0u}) {
     const int grid = r->finish_blocks, tb = (int)r->tune.traverse_block;
     const uint32_t spread_max = (uint32_t)grid * (uint32_t)tb;
-    const bool walk = S.n >= kFinishWalkSpheres && !(kind & kFusedCount);  // over the binary tree always
+    const bool walk = S.n >= kFinishWalkSpheres && !(kind & kFusedCount);
 #define VENU_FINISH(WIDE, C, KS)                                                                                  \
     do {                                                                                                          \
         if (walk && (which & kFinishRefill))                                                                      \
             k_finish_walk<KS><<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, \
                                                      spread_max, src);                                            \
         else if (which & kFinishRefill)                                                                           \
-            k_finish<C, KS, WIDE, true>                                                                           \
+            k_finish<C, KS, C && WIDE, true>                                                                           \
                 <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, spread_max, src); \
         if (which & kFinishSpread)                                                                                \
-            k_finish<C, KS, WIDE, false>                                                                          \
+            k_finish<C, KS, C && WIDE, false>                                                                          \
                 <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, spread_max, src); \
     } while (0)
     if (kind & kFusedWide) VENU_FUSED_CS(VENU_FINISH, true);
