@@ -88,15 +88,15 @@ KERNEL_SOURCES = ("venusaur_gb300/csrc/venu_device.cuh", "venusaur_gb300/csrc/re
 # under ncu --metrics
 # dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum,
 # smsp__inst_executed.sum,smsp__thread_inst_executed.sum.
-NCU_FIGURES = {"sha": "3907a01b4837d234", "commit": "9b77301", "figures": {
+NCU_FIGURES = {"sha": "aec54f6529d487da", "commit": "47604f3", "figures": {
     "c2/v2": {"dram_b_per_seg": 57.43, "lanes_per_inst": 14.71, "warp_inst_per_seg": 71.5},
     "c2/v2/f8": {"dram_b_per_seg": 60.82, "lanes_per_inst": 14.65, "warp_inst_per_seg": 71.9},
-    "c2/v4": {"dram_b_per_seg": 57.67, "lanes_per_inst": 16.04, "warp_inst_per_seg": 81.3},
+    "c2/v4": {"dram_b_per_seg": 57.4, "lanes_per_inst": 15.87, "warp_inst_per_seg": 79.0},
     "c1/v2": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.97, "warp_inst_per_seg": 94.2},
     "c1/v2/f8": {"dram_b_per_seg": 24.84, "lanes_per_inst": 12.06, "warp_inst_per_seg": 92.9},
     "c1/v3": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.98, "warp_inst_per_seg": 94.1},
-    "c1/v4": {"dram_b_per_seg": 2.4, "lanes_per_inst": 11.97, "warp_inst_per_seg": 107.7},
-    "c1/v4/f8": {"dram_b_per_seg": 25.79, "lanes_per_inst": 12.95, "warp_inst_per_seg": 105.5},
+    "c1/v4": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.97, "warp_inst_per_seg": 94.2},
+    "c1/v4/f8": {"dram_b_per_seg": 24.64, "lanes_per_inst": 12.6, "warp_inst_per_seg": 95.4},
     "c3/v3": {"dram_b_per_seg": 75.6, "lanes_per_inst": 10.67, "warp_inst_per_seg": 397.8},
     "c3/v2": {"dram_b_per_seg": 13.86, "lanes_per_inst": 9.38, "warp_inst_per_seg": 479.7},
     "c3/v5": {"dram_b_per_seg": 39.6, "lanes_per_inst": 8.4, "warp_inst_per_seg": 548.0},
