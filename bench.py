@@ -96,6 +96,7 @@ NCU_FIGURES = {"sha": "aec54f6529d487da", "commit": "47604f3", "figures": {
     "c1/v2/f8": {"dram_b_per_seg": 24.84, "lanes_per_inst": 12.06, "warp_inst_per_seg": 92.9},
     "c1/v3": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.98, "warp_inst_per_seg": 94.1},
     "c1/v4": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.97, "warp_inst_per_seg": 94.2},
+    "c1/v5": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.97, "warp_inst_per_seg": 94.2},
     "c1/v4/f8": {"dram_b_per_seg": 24.64, "lanes_per_inst": 12.6, "warp_inst_per_seg": 95.4},
     "c3/v3": {"dram_b_per_seg": 75.6, "lanes_per_inst": 10.67, "warp_inst_per_seg": 397.8},
     "c3/v2": {"dram_b_per_seg": 13.86, "lanes_per_inst": 9.38, "warp_inst_per_seg": 479.7},
