@@ -414,6 +414,7 @@ extern "C" venu_status venu_scene_update(venu_scene* scene, const venu_sphere* s
     if (ds != VENU_OK) return ds;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (n == 0) return VENU_OK;
+    std::lock_guard<std::mutex> lock(scene->update_mu);  // the upload's memory is free again after the wait below
     venu_status rc = update_scene(scene, spheres_host, true, st);
     cudaError_t se = cudaStreamSynchronize(st);
     if (rc == VENU_OK && se != cudaSuccess) rc = cuda_fail(se, "venu_scene_update");

@@ -1275,8 +1275,10 @@ void free_scene(venu_scene* s) {
     cudaFree(s->arena);
     cudaFree(s->wide);
     cudaFree(s->wide_src);
+    cudaFree(s->upload);
     s->wide = nullptr;
     s->wide_src = nullptr;
+    s->upload = nullptr;
     s->nwide = 0;
     s->arena = nullptr;
     s->parents = nullptr;
@@ -1481,15 +1483,20 @@ venu_status ensure_wide(const venu_scene* S, cudaStream_t st) {
 venu_status update_scene(venu_scene* S, const venu_sphere* s, bool on_host, cudaStream_t st) {
     const uint32_t n = S->n;
     if (n == 0) return VENU_OK;
-    if (on_host) {  // by way of the traversal records, which are rewritten below
-        VENU_CUDA(cudaMemcpyAsync(S->trav, s, sizeof(venu_sphere) * n, cudaMemcpyHostToDevice, st));
-        s = reinterpret_cast<const venu_sphere*>(S->trav);
+    if (on_host) {  // a failed upload leaves the scene as it was
+        const size_t bytes = sizeof(venu_sphere) * (size_t)n;
+        if (!S->upload) {
+            VENU_CUDA(cudaMalloc(&S->upload, bytes));
+            S->bytes += bytes;
+        }
+        VENU_CUDA(cudaMemcpyAsync(S->upload, s, bytes, cudaMemcpyHostToDevice, st));
+        s = S->upload;
     }
     // New sphere records into the same slots (meta holds each slot's
     // original index), then the boxes bottom-up over the kept parent links,
     // then the traversal records.  Topology, slot order and the hoisted set
-    // stay those of the build.  Nothing is allocated: the counters are the
-    // build's, back at 0 (two stream-ordered allocations took 180 us a call).
+    // stay those of the build.  The counters are the build's, back at 0 (two
+    // stream-ordered allocations took 180 us a call).
     k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, S->meta, 0x3fffffffu, n, S->sph, S->mat, S->meta, nullptr);
     VENU_CUDA(cudaGetLastError());
     if (n == 1) return VENU_OK;

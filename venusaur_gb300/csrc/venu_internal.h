@@ -94,6 +94,11 @@ struct venu_scene {
     mutable uint32_t nwide = 0;
     mutable float wide_ms = 0.0f;        // wall time of the wide tree's collapse
     mutable std::mutex wide_mu;          // serialises that first build
+    // venu_scene_update's spheres on their way in: memory that no walk reads, so
+    // that renders in flight on other streams never meet anything but records
+    // in the traversal records.  Allocated by the first such update.
+    venu_sphere* upload = nullptr;
+    std::mutex update_mu;         // one upload at a time
     float bounds[6] = {0, 0, 0, 0, 0, 0};
     uint32_t nhoist = 0;          // huge spheres tested before traversal
     int32_t hoist[4] = {0, 0, 0, 0};
