@@ -180,7 +180,9 @@ VENU_API venu_status venu_scene_create_device(const venu_sphere* spheres_dev, ui
  * distances aside).  Quality degrades as spheres move far from where the
  * tree was built: rebuild with venu_scene_create then.  The host variant
  * uploads and returns when done; the device variant is asynchronous on
- * `stream` and `spheres_dev` must stay valid until it completes. */
+ * `stream` and `spheres_dev` must stay valid until it completes.  Updates of
+ * one scene run one after another in call order, whatever their streams; a
+ * captured one is ordered by its graph alone. */
 VENU_API venu_status venu_scene_update(venu_scene* scene, const venu_sphere* spheres_host, uint32_t n, void* stream);
 VENU_API venu_status venu_scene_update_device(venu_scene* scene, const venu_sphere* spheres_dev, uint32_t n,
                                               void* stream);

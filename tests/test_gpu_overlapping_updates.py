@@ -76,3 +76,56 @@ def test_host_updates_from_threads(venu, oracle, cuda):
         th.join()
     assert not failed
     assert np.array_equal(ds.export_bvh()["nodes"].view(np.uint32), oracle.lbvh_refit(sp, to).view(np.uint32))
+
+
+def test_overlapping_refits_leave_no_trace(venu, oracle, cuda):
+    """Refits of one scene from two streams at once, all to the same pose: the scene
+    has that pose afterwards, and a later refit is exact."""
+    torch = cuda
+    n = 60_000
+    sp = oracle.scene_random(n, 71)
+    a, b = _moved(sp, 1, 0.5), _moved(sp, 2, 0.5)
+    want_a, want_b = oracle.lbvh_refit(sp, a), oracle.lbvh_refit(sp, b)
+    ds = venu.DeviceScene(sp)
+    dev_a = torch.from_numpy(a.view(np.uint8).copy()).cuda()
+    dev_b = torch.from_numpy(b.view(np.uint8).copy()).cuda()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for _ in range(30):
+        for s in streams:
+            for _ in range(4):
+                ds.update_device(dev_a, n, stream=s)
+    torch.cuda.synchronize()
+    assert np.array_equal(ds.export_bvh()["nodes"].view(np.uint32), want_a.view(np.uint32))
+    ds.update_device(dev_b, n)
+    torch.cuda.synchronize()
+    assert np.array_equal(ds.export_bvh()["nodes"].view(np.uint32), want_b.view(np.uint32))
+
+
+def test_captured_refit(venu, oracle, cuda):
+    """A refit captured into a graph replays beside refits that are launched, and
+    alone."""
+    torch = cuda
+    n = 60_000
+    sp = oracle.scene_random(n, 74)
+    a, b = _moved(sp, 1, 0.5), _moved(sp, 2, 0.5)
+    want_a, want_b = oracle.lbvh_refit(sp, a), oracle.lbvh_refit(sp, b)
+    ds = venu.DeviceScene(sp)
+    dev = torch.from_numpy(a.view(np.uint8).copy()).cuda()
+    dev_b = torch.from_numpy(b.view(np.uint8).copy()).cuda()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ds.update_device(dev, n)
+    side = torch.cuda.Stream()
+    for _ in range(20):
+        graph.replay()
+        ds.update_device(dev, n, stream=side)
+    torch.cuda.synchronize()
+    assert np.array_equal(ds.export_bvh()["nodes"].view(np.uint32), want_a.view(np.uint32))
+    ds.update_device(dev_b, n)
+    torch.cuda.synchronize()
+    assert np.array_equal(ds.export_bvh()["nodes"].view(np.uint32), want_b.view(np.uint32))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(ds.export_bvh()["nodes"].view(np.uint32), want_a.view(np.uint32))

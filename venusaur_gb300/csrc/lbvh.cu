@@ -445,9 +445,9 @@ __device__ __forceinline__ void leaf_box(float4 s4, float4& lo, float4& hi) {
 }
 
 // Bottom-up refit of moved spheres (sph: slot order).  The second thread to
-// arrive at a node computes its box and leaves its counter at 0 for the next
-// refit; the arrivals publish the children's boxes, which are read back
-// through L2 (__ldcg).  The tree itself does not change, so a node's child
+// arrive at a node (counters from 0, see k_gather) computes its box; the
+// arrivals publish the children's boxes, which are read back through L2
+// (__ldcg).  The tree itself does not change, so a node's child
 // words and parent are read beside its arrival.  Leaf words may carry the
 // hoisted flag.
 __global__ void k_refit(const float4* __restrict__ sph, int n, float4* nodes, const int32_t* __restrict__ parent_int,
@@ -462,7 +462,6 @@ __global__ void k_refit(const float4* __restrict__ sph, int n, float4* nodes, co
         const int32_t cr = __float_as_int(__ldcg(&nodes[2 * p + 1].w));
         const int32_t up = parent_int[p];
         if (arrive_acq_rel(arrive + p) == 0u) return;
-        arrive[p] = 0u;
         const bool ok_l = (cl & kLeaf) ? (cl & kSlotMask) < n : cl < n - 1;
         const bool ok_r = (cr & kLeaf) ? (cr & kSlotMask) < n : cr < n - 1;
         if (!ok_l || !ok_r) return;
@@ -838,7 +837,6 @@ __global__ void __launch_bounds__(kTreeletBlock)
                 if (arrive_acq_rel(arrive + p) == 0u) {
                     walking = false;  // the other subtree is not final yet
                 } else {
-                    arrive[p] = 0u;  // as refits expect it
                     if (word_ok(w0, n) && word_ok(w1, n)) {
                         tentry_load(c0, nodes, sph, w0);
                         tentry_load(c1, nodes, sph, w1);
@@ -871,11 +869,14 @@ __global__ void __launch_bounds__(kTreeletBlock)
 // Slot-ordered sphere / material / meta records.  ids may alias meta (a
 // refit regathers from the meta words): each thread reads its slot's word
 // before writing it.  c (builds only): huge spheres become candidates for
-// hoisting (unordered, at most 64).
+// hoisting (unordered, at most 64).  arrive (refits only): the n - 1 arrival
+// counters, cleared for the refit that follows.
 __global__ void k_gather(const venu_sphere* __restrict__ s, const uint32_t* ids, uint32_t id_mask, uint32_t n,
-                         float4* __restrict__ sph, float4* __restrict__ mat, uint32_t* meta, LbvhCtl* c) {
+                         float4* __restrict__ sph, float4* __restrict__ mat, uint32_t* meta, LbvhCtl* c,
+                         uint32_t* __restrict__ arrive) {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
+    if (arrive && k < n - 1u) arrive[k] = 0u;
     uint32_t id = ids[k] & id_mask;
     const venu_sphere& sp = s[id];
     uint32_t type = sp.material > 2u ? 2u : sp.material;
@@ -1250,7 +1251,8 @@ cudaError_t launch_lbvh(const venu_sphere* s, uint32_t n, cudaStream_t st, const
     }
     // the gather is the last to read the spheres and the sort's buffers, which
     // may lie where the nodes and the traversal records go
-    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, B.vals, 0xffffffffu, n, B.sph, B.mat, B.meta, n > 1 ? B.ctl : nullptr);
+    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, B.vals, 0xffffffffu, n, B.sph, B.mat, B.meta, n > 1 ? B.ctl : nullptr,
+                                         nullptr);
     if (n > 1) {
         k_karras<<<cdiv(n - 1, 256), 256, 0, st>>>(B.keys, (int)n, B.nodes, B.pint, B.pleaf);
         const uint32_t per_warp = treelet_leaves_per_warp(n);
@@ -1276,6 +1278,8 @@ void free_scene(venu_scene* s) {
     cudaFree(s->wide);
     cudaFree(s->wide_src);
     cudaFree(s->upload);
+    if (s->refit_done) cudaEventDestroy(s->refit_done);
+    s->refit_done = nullptr;
     s->wide = nullptr;
     s->wide_src = nullptr;
     s->upload = nullptr;
@@ -1480,9 +1484,44 @@ venu_status ensure_wide(const venu_scene* S, cudaStream_t st) {
     return rc;
 }
 
+namespace {
+// The refit's launches, with its n - 1 arrival counters.
+cudaError_t launch_refit(venu_scene* S, const venu_sphere* s, uint32_t* arrive, cudaStream_t st) {
+    const uint32_t n = S->n;
+    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, S->meta, 0x3fffffffu, n, S->sph, S->mat, S->meta, nullptr, arrive);
+    if (n == 1) return cudaGetLastError();
+    k_refit<<<cdiv(n, 256), 256, 0, st>>>(S->sph, (int)n, S->nodes, S->parents, S->parents + (n - 1), arrive);
+    HoistList list{S->nhoist, {}};
+    for (int i = 0; i < kMaxHoisted; ++i) list.slot[i] = S->hoist[i];
+    const cudaError_t e = launch_trav_layout(S->nodes, S->sph, n, S->trav, S->parents, S->parents + (n - 1), nullptr, list,
+                                             nullptr, st);
+    if (e != cudaSuccess) return e;
+    if (S->nwide) k_wide_refit<<<cdiv(S->nwide, 128), 128, 0, st>>>(S->trav, S->nwide, S->wide_src, S->wide);
+    return cudaGetLastError();
+}
+}  // namespace
+
+// New sphere records into the same slots (meta holds each slot's original
+// index), then the boxes bottom-up over the kept parent links, then the
+// traversal records.  Topology, slot order and the hoisted set stay those of the
+// build.
+//
+// The arrival counters are the build's (two stream-ordered allocations took
+// 180 us a call), cleared by each refit, and refits of one scene run one after
+// another: two that overlapped would count each other's arrivals and make boxes
+// from children that are not there yet.  A captured refit, which can replay
+// beside any other, brings counters of its own into the graph.
 venu_status update_scene(venu_scene* S, const venu_sphere* s, bool on_host, cudaStream_t st) {
     const uint32_t n = S->n;
     if (n == 0) return VENU_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    VENU_CUDA(cudaStreamIsCapturing(st, &capture));
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    std::lock_guard<std::mutex> lock(S->refit_mu);
+    if (!captured) {
+        if (S->refit_done) VENU_CUDA(cudaStreamWaitEvent(st, S->refit_done, 0));
+        else VENU_CUDA(cudaEventCreateWithFlags(&S->refit_done, cudaEventDisableTiming));
+    }
     if (on_host) {  // a failed upload leaves the scene as it was
         const size_t bytes = sizeof(venu_sphere) * (size_t)n;
         if (!S->upload) {
@@ -1492,23 +1531,12 @@ venu_status update_scene(venu_scene* S, const venu_sphere* s, bool on_host, cuda
         VENU_CUDA(cudaMemcpyAsync(S->upload, s, bytes, cudaMemcpyHostToDevice, st));
         s = S->upload;
     }
-    // New sphere records into the same slots (meta holds each slot's
-    // original index), then the boxes bottom-up over the kept parent links,
-    // then the traversal records.  Topology, slot order and the hoisted set
-    // stay those of the build.  The counters are the build's, back at 0 (two
-    // stream-ordered allocations took 180 us a call).
-    k_gather<<<cdiv(n, 256), 256, 0, st>>>(s, S->meta, 0x3fffffffu, n, S->sph, S->mat, S->meta, nullptr);
-    VENU_CUDA(cudaGetLastError());
-    if (n == 1) return VENU_OK;
-    k_refit<<<cdiv(n, 256), 256, 0, st>>>(S->sph, (int)n, S->nodes, S->parents, S->parents + (n - 1), S->arrive);
-    HoistList list{S->nhoist, {}};
-    for (int i = 0; i < kMaxHoisted; ++i) list.slot[i] = S->hoist[i];
-    VENU_CUDA(launch_trav_layout(S->nodes, S->sph, n, S->trav, S->parents, S->parents + (n - 1), nullptr, list, nullptr,
-                                 st));
-    if (S->nwide)
-        k_wide_refit<<<cdiv(S->nwide, 128), 128, 0, st>>>(S->trav, S->nwide, S->wide_src, S->wide);
-    VENU_CUDA(cudaGetLastError());
-    return VENU_OK;
+    uint32_t* arrive = S->arrive;
+    if (captured && n > 1) VENU_CUDA(cudaMallocAsync(&arrive, sizeof(uint32_t) * (n - 1), st));
+    cudaError_t e = launch_refit(S, s, arrive, st);
+    const cudaError_t end = !captured ? cudaEventRecord(S->refit_done, st) : n > 1 ? cudaFreeAsync(arrive, st) : cudaSuccess;
+    if (e == cudaSuccess) e = end;
+    return e == cudaSuccess ? VENU_OK : cuda_fail(e, "venu_scene_update");
 }
 
 }  // namespace venu

@@ -81,7 +81,7 @@ struct venu_scene {
     uint32_t* meta = nullptr;  // original id | material << 30
     uint32_t* keys = nullptr;  // sorted Morton codes
     int32_t* parents = nullptr;  // [n-1] parent of each internal node, then [n] of each leaf (for refits)
-    uint32_t* arrive = nullptr;  // [n-1] arrival counters of refits, 0 between them
+    uint32_t* arrive = nullptr;  // [n-1] arrival counters of the build and of refits
     uint32_t* trace_err = nullptr;         // [kTraceWords] error word (0 unless one failed) and hand-out counter
                                            // of each venu_trace call
     mutable uint64_t trace_used = 0;       // the pairs in use (a bit each)
@@ -99,6 +99,10 @@ struct venu_scene {
     // in the traversal records.  Allocated by the first such update.
     venu_sphere* upload = nullptr;
     std::mutex update_mu;         // one upload at a time
+    // Refits share the counters, so each waits on the device for the one before
+    // it, on whatever stream that ran (refit_done, recorded by the first).
+    cudaEvent_t refit_done = nullptr;
+    std::mutex refit_mu;
     float bounds[6] = {0, 0, 0, 0, 0, 0};
     uint32_t nhoist = 0;          // huge spheres tested before traversal
     int32_t hoist[4] = {0, 0, 0, 0};
