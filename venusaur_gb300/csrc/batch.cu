@@ -548,10 +548,9 @@ namespace {
 template <typename K>
 cudaError_t batch_grid(const venu_batch* b, K kernel, int& blocks) {
     const size_t sm = traverse_smem((int)b->tune.traverse_block);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     int per_sm = 0;
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)b->tune.traverse_block, sm);
+    const cudaError_t e =
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)b->tune.traverse_block, sm);
     if (e != cudaSuccess) return e;
     per_sm = std::max(1, per_sm);
     if (b->tune.traverse_blocks_per_sm) per_sm = std::min(per_sm, (int)b->tune.traverse_blocks_per_sm);

@@ -1013,6 +1013,11 @@ SceneView view_of(const venu_scene* s) {
     return v;
 }
 
+// At most 16 KB (256 threads).  No kernel sets cudaFuncAttributeMaxDynamicSharedMemorySize:
+// up to 48 KB needs no attribute, and one that a renderer set would be every other
+// renderer's limit too (the attribute is the kernel's on the device), so that setting
+// up small blocks made the launches of larger ones fail.
+static_assert(256 * kShared * sizeof(int2) <= 32 * 1024, "the stacks fit without the attribute");
 size_t traverse_smem(int block, int entries) { return (size_t)block * entries * sizeof(int2); }
 size_t traverse_smem(int block) { return traverse_smem(block, kShared); }
 
@@ -1087,9 +1092,8 @@ constexpr uint32_t kTraceWalkSpheres = 65536, kTraceWalkRays = 1u << 18;
 
 template <typename K>
 cudaError_t occupancy_grid(K kernel, int block, size_t smem, uint32_t per_sm_cap, int& grid) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per_sm = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
     if (e != cudaSuccess) return e;
     per_sm = std::max(1, per_sm);
     if (per_sm_cap) per_sm = std::min(per_sm, (int)per_sm_cap);
@@ -1097,34 +1101,17 @@ cudaError_t occupancy_grid(K kernel, int block, size_t smem, uint32_t per_sm_cap
     return cudaSuccess;
 }
 
-template <typename K>
-cudaError_t set_smem(K kernel, size_t smem) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-}
-
-// The fused kernels' launch shape: one for the four instantiations of the
-// bounce kernel (the shallow-stack ones need less shared memory; same grid)
-// and one for those of the finishing kernel.
-template <bool WIDE, typename K8, typename K4, typename C8, typename C4>
-cudaError_t configure_fused(venu_renderer* r, K8 deep, K4 shallow, C8 count_deep, C4 count_shallow) {
+// The fused kernels' launch shape: one for all instantiations of the bounce
+// kernel (the shallow-stack ones need less shared memory; same grid) and one for
+// those of the finishing kernel.
+template <typename K8, typename K4>
+cudaError_t configure_fused(venu_renderer* r, K8 deep, K4 shallow) {
     const venu_tuning& t = r->tune;
     const int tb = (int)t.traverse_block;
     const size_t sm = traverse_smem(tb), ss = traverse_smem(tb, kSharedShallow);
     cudaError_t e = occupancy_grid(deep, tb, sm, t.traverse_blocks_per_sm, r->fused_blocks);
-    if (e == cudaSuccess) e = set_smem(shallow, sm);
-    if (e == cudaSuccess) e = set_smem(count_deep, sm);
-    if (e == cudaSuccess) e = set_smem(count_shallow, sm);
     if (e == cudaSuccess)
         e = occupancy_grid(k_finish<false, kShared, false, false>, tb, sm, t.traverse_blocks_per_sm, r->finish_blocks);
-    if (e == cudaSuccess) e = set_smem(k_finish<false, kSharedShallow, false, false>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish<false, kShared, false, true>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish<false, kSharedShallow, false, true>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish<true, kShared, WIDE, false>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish<true, kSharedShallow, WIDE, false>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish<true, kShared, WIDE, true>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish<true, kSharedShallow, WIDE, true>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish_walk<kShared>, sm);
-    if (e == cudaSuccess) e = set_smem(k_finish_walk<kSharedShallow>, sm);
     if (e == cudaSuccess) e = prefer_l1(k_finish_walk<kShared>, std::max(1, r->finish_blocks / std::max(1, sm_count())), sm);
     const int nsm = std::max(1, sm_count());
     const int pb = std::max(1, r->fused_blocks / nsm), pf = std::max(1, r->finish_blocks / nsm);
@@ -1145,28 +1132,23 @@ cudaError_t configure(venu_renderer* r) {
     const int nsm = std::max(1, sm_count());
     cudaError_t e = cudaSuccess;
     if (t.traverse_variant == 4) {  // the fused kernel over the 4-wide tree
-        e = configure_fused<true>(r, k_trace_shade_wide<false, kShared>, k_trace_shade_wide<false, kSharedShallow>,
-                                  k_trace_shade_wide<true, kShared>, k_trace_shade_wide<true, kSharedShallow>);
+        e = configure_fused(r, k_trace_shade_wide<false, kShared>, k_trace_shade_wide<false, kSharedShallow>);
         r->trav_blocks = r->fused_blocks;
     } else if (t.traverse_variant >= 2) {  // the fused kernel: every bounce (2), the primary one (3, 5)
-        e = configure_fused<false>(r, k_trace_shade<false, kShared>, k_trace_shade<false, kSharedShallow>,
-                                   k_trace_shade<true, kShared>, k_trace_shade<true, kSharedShallow>);
+        e = configure_fused(r, k_trace_shade<false, kShared>, k_trace_shade<false, kSharedShallow>);
         r->trav_blocks = r->fused_blocks;
     }
     if (e != cudaSuccess) return e;
     if (t.traverse_variant == 5) {  // later bounces: the separate traversal over the wide tree
         e = occupancy_grid(k_traverse<false, true>, tb, sm, t.traverse_blocks_per_sm, r->trav_blocks);
-        if (e == cudaSuccess) e = set_smem(k_traverse<true, true>, sm);
         if (e == cudaSuccess) e = prefer_l1(k_traverse<false, true>, std::max(1, r->trav_blocks / nsm), sm);
     } else if (t.traverse_variant == 0 || t.traverse_variant == 3) {
         e = occupancy_grid(k_traverse<false>, tb, sm, t.traverse_blocks_per_sm, r->trav_blocks);
-        if (e == cudaSuccess) e = set_smem(k_traverse<true>, sm);
         if (e == cudaSuccess) e = prefer_l1(k_traverse<false>, std::max(1, r->trav_blocks / nsm), sm);
         if (e == cudaSuccess) e = occupancy_grid(k_walk, tb, sm, t.traverse_blocks_per_sm, r->walk_blocks);
         if (e == cudaSuccess) e = prefer_l1(k_walk, std::max(1, r->walk_blocks / nsm), sm);
     } else if (t.traverse_variant == 1) {
         e = occupancy_grid(k_traverse_dyn<false>, tb, sm, t.traverse_blocks_per_sm, r->trav_blocks);
-        if (e == cudaSuccess) e = set_smem(k_traverse_dyn<true>, sm);
         if (e == cudaSuccess) e = prefer_l1(k_traverse_dyn<false>, std::max(1, r->trav_blocks / nsm), sm);
     }
     if (e == cudaSuccess) e = occupancy_grid(k_shade, (int)t.shade_block, 0, t.shade_blocks_per_sm, r->shade_blocks);
