@@ -419,7 +419,9 @@ VENU_API venu_status venu_batch_destroy(venu_batch* b);
  * time from any thread; the server admits them first-come first-served
  * while the device memory they need fits the HBM budget, keeps scene BVHs
  * resident across requests that share a scene_key (evicting unused ones,
- * least recently used first, when the budget needs room), advances every
+ * least recently used first, when the budget needs room), keeps some of the
+ * finished jobs' memory for the next ones while the budget has room for it
+ * (given back before a scene is evicted), advances every
  * admitted job together in the shared path pool a few iterations at a time,
  * and retires finished jobs: image copied to host memory, buffers freed,
  * latency recorded.  A request that can never fit the budget fails with
@@ -466,7 +468,8 @@ typedef struct venu_server_stats {
     double busy_seconds;        /* wall time with at least one admitted job */
     uint64_t evictions;         /* resident scenes evicted to make room under the budget */
     uint64_t admission_waits;   /* server steps at which the next request waited for room */
-    uint64_t peak_resident_bytes; /* most device bytes held at once (scenes, jobs, sessions) */
+    uint64_t peak_resident_bytes; /* most device bytes held at once (scenes, jobs, sessions, and
+                                     finished jobs' memory kept for the next ones) */
 } venu_server_stats;
 
 /* Test hooks: make the next admission fail as if its allocation failed

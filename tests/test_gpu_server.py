@@ -180,3 +180,28 @@ def test_server_lru_eviction_counted(venu, oracle, cuda):
     assert r["status"] == 0 and np.array_equal(r["image"], want0["image8"].reshape(r["image"].shape))
     assert srv.stats()["evictions"] >= 2
     srv.close()
+
+
+def test_server_kept_memory_counts(venu, oracle, cuda):
+    """A finished large job's buffers are kept for the next one only while the
+    budget has room for them: once a large scene takes most of it, the device
+    memory held since the server's start stays within the budget (and the
+    granularity of the allocators)."""
+    torch = cuda
+    budget = 320 << 20
+    cam = oracle.camera((60, 15, 60), (0, 0, 0), 20.0, 1.0, 0.1, 10.0)
+    small, large = oracle.scene_random(2000, 1), oracle.scene_random(1_200_000, 2)
+    srv = venu.Server(hbm_budget_bytes=budget, pool_paths=16 << 20, max_jobs=4)
+    # kernels, graphs and their local memory first
+    assert srv.wait(srv.submit(cam, 64, 64, 1, spheres=small, max_depth=4))["status"] == 0
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    # 10.5 M paths: 210 MB of job buffers and 37 MB of accumulator and image
+    assert srv.wait(srv.submit(cam, 1024, 1024, 10, spheres=small, max_depth=4))["status"] == 0
+    # 1.2 M spheres: 289 MB by the server's estimate
+    assert srv.wait(srv.submit(cam, 64, 64, 1, spheres=large, scene_key=9, max_depth=4))["status"] == 0
+    held = free0 - torch.cuda.mem_get_info()[0]
+    st = srv.stats()
+    assert st["failed"] == 0 and st["peak_resident_bytes"] <= budget
+    assert held <= budget + (32 << 20)
+    srv.close()

@@ -543,6 +543,8 @@ struct venu_batch {
     uint64_t graph_launches = 0, resident = 0;
 };
 
+venu::DevPool* venu::batch_pool(venu_batch* b) { return &b->mem; }
+
 namespace {
 
 template <typename K>
@@ -803,10 +805,10 @@ extern "C" venu_status venu_batch_submit_many(venu_batch* b, const venu_job_desc
             e = launch_seed_group(b, g, st);
         if (e != cudaSuccess) {
             // nothing of this call is admitted: free what it allocated
-            if (buf) cudaFreeAsync(buf, st);
+            if (buf) b->mem.free(buf, (sizeof(float4) + sizeof(uint32_t)) * total, st);
             for (uint32_t m = 0; m < k; ++m) {
                 JobHost& P = b->jobs[slots[m]];
-                cudaFreeAsync(P.slots, st);
+                b->mem.free(P.slots, P.bytes, st);
                 P = JobHost{};
             }
             b->jobs[slot] = JobHost{};
@@ -950,7 +952,7 @@ extern "C" venu_status venu_batch_collect(venu_batch* b, void* stream, uint32_t*
     if (!fin.empty()) {
         for (uint32_t slot : fin) {
             JobHost& J = b->jobs[slot];
-            VENU_CUDA(cudaFreeAsync(J.slots, st));  // seeds share the allocation
+            VENU_CUDA(b->mem.free(J.slots, J.bytes, st));  // seeds share the allocation
             b->resident -= J.bytes;
             J = JobHost{};
         }

@@ -83,9 +83,10 @@ constexpr uint32_t kBulkChunk = 4u << 20;      // bulk rays per step while the e
 // node of 128 + 16 bytes per two spheres).  Once built, the
 // scene's own byte count replaces the estimate.
 uint64_t scene_estimate(uint32_t n) { return (uint64_t)n * 240u + 4096u; }
-uint64_t image_bytes(const venu_render_opts& o) {
-    return (uint64_t)o.width * o.height * (sizeof(float) * VENU_ACCUM_FLOATS_PER_PIXEL + 4u);
+uint64_t accum_bytes(const venu_render_opts& o) {
+    return (uint64_t)o.width * o.height * sizeof(float) * VENU_ACCUM_FLOATS_PER_PIXEL;
 }
+uint64_t image_bytes(const venu_render_opts& o) { return accum_bytes(o) + (uint64_t)o.width * o.height * 4u; }
 
 }  // namespace
 
@@ -178,6 +179,21 @@ void evict_for(venu_server* s, uint64_t need) {
     }
 }
 
+// What the pools of the server and of its two batches keep: it counts towards
+// the budget, and goes before a scene does when admission needs the room.
+uint64_t kept_bound(const venu_server* s) {
+    return s->mem.kept_bound() + venu::batch_pool(s->batch)->kept_bound() + venu::batch_pool(s->express)->kept_bound();
+}
+uint64_t kept(const venu_server* s) {
+    return s->mem.kept() + venu::batch_pool(s->batch)->kept() + venu::batch_pool(s->express)->kept();
+}
+void trim_pools(venu_server* s) {
+    cudaStreamSynchronize(s->st);  // the frees of the last step
+    s->mem.trim();
+    venu::batch_pool(s->batch)->trim();
+    venu::batch_pool(s->express)->trim();
+}
+
 // The request's accumulator: freed if it is the request's own; a session's
 // stays (and the session is free for its next request).
 void release_accum(venu_server* s, Request& R) {
@@ -186,13 +202,13 @@ void release_accum(venu_server* s, Request& R) {
         if (it != s->sessions.end()) {
             it->second.busy = false;
             if (it->second.end_pending) {
-                if (it->second.accum) cudaFreeAsync(it->second.accum, s->st);
+                if (it->second.accum) s->mem.free(it->second.accum, it->second.bytes, s->st);
                 s->resident -= it->second.bytes;
                 s->sessions.erase(it);
             }
         }
     } else if (R.accum) {
-        cudaFreeAsync(R.accum, s->st);
+        s->mem.free(R.accum, accum_bytes(R.req.opts), s->st);
     }
     R.accum = nullptr;
 }
@@ -241,7 +257,7 @@ void admit(venu_server* s, Request& R) {
     it->second.refs += 1;
     it->second.last_use = ++s->use_clock;
     const uint64_t npix = (uint64_t)o.width * o.height;
-    const uint64_t accum_bytes = npix * sizeof(float) * VENU_ACCUM_FLOATS_PER_PIXEL;
+    const uint64_t acc_bytes = accum_bytes(o);
     bool reset = true;
     cudaError_t e = cudaSuccess;
     if (R.req.session) {
@@ -249,17 +265,17 @@ void admit(venu_server* s, Request& R) {
         Session& S = s->sessions[R.req.session];
         reset = !S.accum || S.width != o.width || S.height != o.height || (o.flags & VENU_FLAG_RESET_ACCUM);
         if (S.accum && (S.width != o.width || S.height != o.height)) {
-            cudaFreeAsync(S.accum, s->st);
+            s->mem.free(S.accum, S.bytes, s->st);
             s->resident -= S.bytes;
             S.accum = nullptr;
         }
         if (!S.accum) {
-            e = s->mem.alloc(&S.accum, accum_bytes, s->st);
+            e = s->mem.alloc(&S.accum, acc_bytes, s->st);
             if (e == cudaSuccess) {
                 S.width = o.width;
                 S.height = o.height;
-                S.bytes = accum_bytes;
-                s->resident += accum_bytes;
+                S.bytes = acc_bytes;
+                s->resident += acc_bytes;
             } else {
                 S.accum = nullptr;
             }
@@ -268,7 +284,7 @@ void admit(venu_server* s, Request& R) {
         R.session_accum = true;
         S.busy = e == cudaSuccess;
     } else {
-        e = s->mem.alloc(&R.accum, accum_bytes, s->st);
+        e = s->mem.alloc(&R.accum, acc_bytes, s->st);
     }
     if (e == cudaSuccess) e = s->mem.alloc(&R.image8, npix * 4u, s->st);
     if (e != cudaSuccess) {
@@ -292,7 +308,7 @@ void admit(venu_server* s, Request& R) {
     venu_status bs = venu_batch_submit(s->lane(R.lane), &d, s->st, &jid);
     if (bs != VENU_OK) {
         release_accum(s, R);
-        cudaFreeAsync(R.image8, s->st);
+        s->mem.free(R.image8, npix * 4u, s->st);
         R.image8 = nullptr;
         release_scene(s, key);
         complete(s, R, bs);
@@ -300,7 +316,7 @@ void admit(venu_server* s, Request& R) {
     }
     R.scene_key = key;
     R.job_bytes = venu_batch_job_bytes(o.width, o.height, o.samples_per_pixel) + image_bytes(o) -
-                  (R.session_accum ? accum_bytes : 0u);  // a session's accumulator is counted with the session
+                  (R.session_accum ? acc_bytes : 0u);  // a session's accumulator is counted with the session
     s->resident += R.job_bytes;
     s->active[R.lane][jid] = R.id;
     std::lock_guard<std::mutex> lock(s->mu);
@@ -308,7 +324,7 @@ void admit(venu_server* s, Request& R) {
 }
 
 void free_session(venu_server* s, std::unordered_map<uint64_t, Session>::iterator it) {
-    if (it->second.accum) cudaFreeAsync(it->second.accum, s->st);
+    if (it->second.accum) s->mem.free(it->second.accum, it->second.bytes, s->st);
     s->resident -= it->second.bytes;
     s->sessions.erase(it);
 }
@@ -363,7 +379,7 @@ venu_status run_lane(venu_server* s, int l, uint32_t max_iter, std::vector<uint3
     cudaError_t ce = cudaStreamSynchronize(s->st);
     for (Request* R : done) {
         release_accum(s, *R);
-        cudaFreeAsync(R->image8, s->st);
+        s->mem.free(R->image8, (uint64_t)R->req.opts.width * R->req.opts.height * 4u, s->st);
         R->image8 = nullptr;
         s->resident -= R->job_bytes;
         release_scene(s, R->scene_key);
@@ -433,6 +449,7 @@ void server_loop(venu_server* s) {
                 complete(s, *R, VENU_ERR_OOM);
                 continue;
             }
+            if (s->resident + kept_bound(s) + need > s->budget) trim_pools(s);
             if (s->resident + need > s->budget) evict_for(s, need);
             if (s->resident + need > s->budget || s->n_active_all() >= s->max_jobs) {  // wait for room
                 std::lock_guard<std::mutex> lock(s->mu);
@@ -449,7 +466,7 @@ void server_loop(venu_server* s) {
             std::lock_guard<std::mutex> lock(s->mu);
             s->n_active = (uint32_t)s->n_active_all();
             s->resident_shared = s->resident;
-            s->peak_resident = std::max(s->peak_resident, s->resident);
+            s->peak_resident = std::max(s->peak_resident, s->resident + kept(s));
         }
         if (s->n_active_all() == 0) {
             std::unique_lock<std::mutex> lock(s->mu);
@@ -539,7 +556,7 @@ extern "C" venu_status venu_server_create(uint64_t hbm_budget_bytes, uint32_t po
         return bs;
     }
     cudaError_t e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
-    // kept between requests: at most an eighth of the budget
+    // kept between requests, beside what the batches keep (see kept_bound)
     if (e == cudaSuccess) e = s->mem.create(std::min<uint64_t>(hbm_budget_bytes / 8u, 256ull << 20));
     if (e != cudaSuccess) {
         s->mem.destroy();

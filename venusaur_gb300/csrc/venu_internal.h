@@ -48,10 +48,13 @@ constexpr uint32_t kTraceWords = 64;  // two for each venu_trace call of a scene
 
 // Device memory handed out in stream order and kept for reuse up to `keep`
 // bytes (the default pool gives everything back at each synchronisation, and
-// mapping it again costs 100 us and more); destroyed with its owner.
+// mapping it again costs 100 us and more); destroyed with its owner.  What it
+// keeps is at most what was freed since the last trim.
 struct DevPool {
     cudaMemPool_t pool = nullptr;
-    cudaError_t create(uint64_t keep) {
+    uint64_t keep = 0, freed = 0;
+    cudaError_t create(uint64_t keep_bytes) {
+        keep = keep_bytes;
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -63,6 +66,23 @@ struct DevPool {
     template <typename T>
     cudaError_t alloc(T** p, size_t bytes, cudaStream_t st) {
         return cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, pool, st);
+    }
+    cudaError_t free(void* p, uint64_t bytes, cudaStream_t st) {
+        freed += bytes;
+        return cudaFreeAsync(p, st);
+    }
+    uint64_t kept_bound() const { return freed < keep ? freed : keep; }
+    uint64_t kept() const {  // the bound, or the unused part of the pool where that is less
+        uint64_t reserved = 0, used = 0;
+        if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess || used > reserved)
+            return kept_bound();
+        return reserved - used < kept_bound() ? reserved - used : kept_bound();
+    }
+    // Gives the unused memory back; the frees must have completed.
+    cudaError_t trim() {
+        freed = 0;
+        return cudaMemPoolTrimTo(pool, 0);
     }
     void destroy() {
         if (pool) cudaMemPoolDestroy(pool);
@@ -121,4 +141,5 @@ venu_status update_scene(venu_scene* s, const venu_sphere* spheres, bool on_host
 // Builds the scene's 4-wide tree on `stream` unless it exists (blocking: the
 // collapse reads each level's size on the host).  Thread-safe.
 venu_status ensure_wide(const venu_scene* s, cudaStream_t stream);
+DevPool* batch_pool(venu_batch* b);  // its job buffers
 }  // namespace venu
