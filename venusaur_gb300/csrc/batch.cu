@@ -293,11 +293,11 @@ template <bool COUNT>
 __device__ __forceinline__ ShadeOut trace_shade_job(const DevJob* __restrict__ jobs, uint32_t job, int32_t from,
                                                     float4 o4, float4 d4, const float4* t_src, float4 t_fresh,
                                                     StackSmem sm, bool& overflow, TraceCounters& K) {
-    RayPre R = prep_for<COUNT>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
-    R.from = from;
-    float t;
     const SceneView* G = &jobs[job].scene;
     const JobScene S{G->trav, G};
+    RayPre R = prep_for<COUNT>(S, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+    R.from = from;
+    float t;
     const int32_t k = trace_closest<COUNT>(S, R, 0.001f, 1e16f, t, sm, threadIdx.x, blockDim.x, overflow, K);
     // the shading pointers are read here instead of being kept in registers
     // through the traversal (the job table is L1/L2-resident)

@@ -904,7 +904,7 @@ __global__ void k_gather(const venu_sphere* __restrict__ s, const uint32_t* ids,
 // array stays the exported form.
 //
 // Behind the n - 1 records stands the root's: {c.x, c.y, h.x, h.y},
-// {c.z, h.z, E, 0}.
+// {c.z, h.z, 0, 0}, {G, -2^-18 E}.  All boxes are relative to G.
 //
 // A hoisted leaf is tested before the walk, so its box is empty here
 // (h = -inf is never met), and k_hoist_clean takes it out of the boxes above
@@ -916,14 +916,12 @@ __global__ void k_gather(const venu_sphere* __restrict__ s, const uint32_t* ids,
 // index checks: a word that is not (which a sound build never produces) is
 // replaced by a skipped leaf and counted in *bad.
 // ---------------------------------------------------------------------------
-// |C| + |r| of a sphere, 0 unless finite: the bits of non-negative floats
-// order like the values.
-__device__ __forceinline__ uint32_t extent_bits(float4 s4) {
-    const float e = sqrtf(s4.x * s4.x + s4.y * s4.y + s4.z * s4.z) * 1.000001f + fabsf(s4.w);
-    return e <= 3.0e38f ? __float_as_uint(e) : 0u;
+// How far the box of a record is widened: 24 2^-24 (Q + E), Q the sum of its
+// farthest corner's coordinates (an upper bound of the corner's distance).
+__device__ __forceinline__ float widen_of(float3 lo, float3 hi, float E) {
+    const float Q = (fmaxf(fabsf(lo.x), fabsf(hi.x)) + fmaxf(fabsf(lo.y), fabsf(hi.y))) + fmaxf(fabsf(lo.z), fabsf(hi.z));
+    return (Q + E) * 1.430511474609375e-06f;  // 1.5 2^-20
 }
-
-__device__ __forceinline__ float widen_of(float E) { return E * 2.86102294921875e-06f; }  // 1.5 2^-19
 
 __device__ __forceinline__ void centre_half(float lo, float hi, float e, float& c, float& h) {
     c = 0.5f * lo + 0.5f * hi;
@@ -931,32 +929,83 @@ __device__ __forceinline__ void centre_half(float lo, float hi, float e, float& 
     if (!(lo <= hi)) h = __int_as_float(0x7fc00000);  // a NaN box is always met
 }
 
-__device__ __forceinline__ void write_child(float4* rec, float4 lo, float4 hi, float e, int32_t w) {
-    float cx, cy, cz, hx, hy, hz;
-    centre_half(lo.x, hi.x, e, cx, hx);
-    centre_half(lo.y, hi.y, e, cy, hy);
-    centre_half(lo.z, hi.z, e, cz, hz);
-    if ((w & kLeaf) && (w & kHoisted)) {
-        cx = cy = cz = 0.0f;
-        hx = hy = hz = -INFINITY;
-    }
-    rec[0] = make_float4(cx, cy, hx, hy);
-    rec[1] = make_float4(cz, hz, __int_as_float(w), 0.0f);
+// A box relative to G (rounded outwards), widened, as centres and half extents.
+// frame: the third of the root's float4s.
+__device__ __forceinline__ void frame_box(float4 lo4, float4 hi4, float4 frame, float3& c, float3& h) {
+    const float3 lo = make_float3(__fsub_rd(lo4.x, frame.x), __fsub_rd(lo4.y, frame.y), __fsub_rd(lo4.z, frame.z));
+    const float3 hi = make_float3(__fsub_ru(hi4.x, frame.x), __fsub_ru(hi4.y, frame.y), __fsub_ru(hi4.z, frame.z));
+    const float e = widen_of(lo, hi, frame.w * -262144.0f);
+    centre_half(lo.x, hi.x, e, c.x, h.x);
+    centre_half(lo.y, hi.y, e, c.y, h.y);
+    centre_half(lo.z, hi.z, e, c.z, h.z);
 }
 
-// E into the root's record (zeroed before): over all leaves but the listed
-// slots.
-__global__ void k_extent(const float4* __restrict__ sph, uint32_t n, const HoistList* __restrict__ ctl_list,
-                         HoistList list, uint32_t* __restrict__ extent) {
-    const HoistList H = ctl_list ? *ctl_list : list;
-    uint32_t ext = 0;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        bool hoisted = false;
-        for (uint32_t i = 0; i < H.n; ++i) hoisted = hoisted || H.slot[i] == (int32_t)k;
-        if (!hoisted) ext = max(ext, extent_bits(sph[k]));
+__device__ __forceinline__ void write_child(float4* rec, float4 lo, float4 hi, float4 frame, int32_t w) {
+    float3 c, h;
+    frame_box(lo, hi, frame, c, h);
+    if ((w & kLeaf) && (w & kHoisted)) {
+        c = make_float3(0.0f, 0.0f, 0.0f);
+        h = make_float3(-INFINITY, -INFINITY, -INFINITY);
     }
-    ext = __reduce_max_sync(0xffffffffu, ext);
-    if ((threadIdx.x & 31u) == 0 && ext) atomicMax(extent, ext);
+    rec[0] = make_float4(c.x, c.y, h.x, h.y);
+    rec[1] = make_float4(c.z, h.z, __int_as_float(w), 0.0f);
+}
+
+// The value that is left of a warp's samples (two a lane) at the low end, or the
+// high one, when `trim` have been taken away there.  At least one is valid.
+__device__ float trimmed_end(float a, bool va, float b, bool vb, uint32_t trim, bool high) {
+    const uint32_t flip = high ? 0xffffffffu : 0u;
+    uint32_t x = va ? f2u(a) ^ flip : 0xffffffffu, y = vb ? f2u(b) ^ flip : 0xffffffffu;
+    for (;; --trim) {
+        const uint32_t m = __reduce_min_sync(0xffffffffu, min(x, y));
+        if (trim == 0u) return u2f(m ^ flip);
+        const uint32_t has = __ballot_sync(0xffffffffu, min(x, y) == m);
+        if ((threadIdx.x & 31u) == (uint32_t)__ffs(has) - 1u) {
+            if (x == m) x = 0xffffffffu;
+            else y = 0xffffffffu;
+        }
+    }
+}
+
+// G and E of the records (one warp): 64 spheres evenly spaced in slot order, the
+// hoisted and those that are not finite left out.  G is the middle of their
+// centres' box and E twice the largest |C - G| + |r|, each once the four outermost
+// samples at an end are dropped, so that a few far spheres do not decide.  The
+// walk is right with any G and E (venu_device.cuh); they settle how much boxes are
+// widened and which rays need a margin.  Twice the radius, because the margin
+// takes |p| as the sum of its coordinates, and an origin in a corner of the scene
+// should need none: a nearly axis-parallel ray with a margin goes the slow way and
+// its warp waits for it (at once the radius: 1M ray queries on 20k spheres 667 ->
+// 918 us, 96 uneven jobs 6.88 -> 7.19 ms, 100k moving spheres 2.10 -> 2.23 ms).
+__global__ void k_frame(const float4* __restrict__ sph, uint32_t n, const HoistList* __restrict__ ctl_list,
+                        HoistList list, float4* __restrict__ frame) {
+    const HoistList H = ctl_list ? *ctl_list : list;
+    float4 s[2];
+    bool ok[2];
+    for (int j = 0; j < 2; ++j) {
+        const uint32_t k = (uint32_t)((unsigned long long)(2u * threadIdx.x + (uint32_t)j) * n / 64u);
+        s[j] = sph[k];
+        ok[j] = isfinite(s[j].x) && isfinite(s[j].y) && isfinite(s[j].z) && isfinite(s[j].w);
+        for (uint32_t i = 0; i < H.n; ++i) ok[j] = ok[j] && H.slot[i] != (int32_t)k;
+    }
+    const uint32_t valid = __reduce_add_sync(0xffffffffu, (uint32_t)ok[0] + (uint32_t)ok[1]);
+    float4 F = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (valid) {
+        const uint32_t trim = min(4u, valid / 4u);
+        F.x = 0.5f * trimmed_end(s[0].x, ok[0], s[1].x, ok[1], trim, false) +
+              0.5f * trimmed_end(s[0].x, ok[0], s[1].x, ok[1], trim, true);
+        F.y = 0.5f * trimmed_end(s[0].y, ok[0], s[1].y, ok[1], trim, false) +
+              0.5f * trimmed_end(s[0].y, ok[0], s[1].y, ok[1], trim, true);
+        F.z = 0.5f * trimmed_end(s[0].z, ok[0], s[1].z, ok[1], trim, false) +
+              0.5f * trimmed_end(s[0].z, ok[0], s[1].z, ok[1], trim, true);
+        float q[2];
+        for (int j = 0; j < 2; ++j) {
+            const float x = s[j].x - F.x, y = s[j].y - F.y, z = s[j].z - F.z;
+            q[j] = fminf(sqrtf(x * x + y * y + z * z) + fabsf(s[j].w), 1e30f);
+        }
+        F.w = -7.62939453125e-06f * trimmed_end(q[0], ok[0], q[1], ok[1], trim, true);  // -2 2^-18
+    }
+    if (threadIdx.x == 0) *frame = F;
 }
 
 __global__ void k_trav_layout(const float4* __restrict__ nodes, const float4* __restrict__ sph, uint32_t n,
@@ -964,16 +1013,12 @@ __global__ void k_trav_layout(const float4* __restrict__ nodes, const float4* __
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2u * (n - 1u)) return;
     float4* const root = trav + 4 * (size_t)(n - 1u);
-    const float e = widen_of(root[1].z);
+    const float4 frame = root[2];
     if (i == 0) {
-        float4 c;
-        const float4 lo = nodes[0], hi = nodes[1];
-        float cz, hz;
-        centre_half(lo.x, hi.x, e, c.x, c.z);
-        centre_half(lo.y, hi.y, e, c.y, c.w);
-        centre_half(lo.z, hi.z, e, cz, hz);
-        root[0] = c;
-        reinterpret_cast<float2*>(root + 1)[0] = make_float2(cz, hz);  // E beside it stays
+        float3 c, h;
+        frame_box(nodes[0], nodes[1], frame, c, h);
+        root[0] = make_float4(c.x, c.y, h.x, h.y);
+        root[1] = make_float4(c.z, h.z, 0.0f, 0.0f);
     }
     const uint32_t p = i >> 1, c = i & 1u;
     int32_t w = __float_as_int(nodes[2 * p + c].w);
@@ -990,7 +1035,7 @@ __global__ void k_trav_layout(const float4* __restrict__ nodes, const float4* __
         lo = nodes[2 * w];
         hi = nodes[2 * w + 1];
     }
-    write_child(trav + 4 * (size_t)p + 2 * c, lo, hi, e, w);
+    write_child(trav + 4 * (size_t)p + 2 * c, lo, hi, frame, w);
 }
 
 // Takes the hoisted leaves out of the boxes of the nodes above them, in the
@@ -998,8 +1043,9 @@ __global__ void k_trav_layout(const float4* __restrict__ nodes, const float4* __
 // node's box becomes the union of its record's two children (rounded
 // outwards), written into its parent's record, or the root's.  Walks of
 // several leaves run one after another, so a node above two of them is
-// written last by the later walk, with both taken out.  The widening is in
-// the children already.
+// written last by the later walk, with both taken out.  The children's boxes
+// are widened for their own coordinates; the union's, which may be larger, take
+// 8 2^-24 of their sum more (the slab parameters' 4 2^-24 Q).
 __global__ void k_hoist_clean(float4* trav, const int32_t* __restrict__ pint, const int32_t* __restrict__ pleaf,
                               uint32_t n, const HoistList* __restrict__ ctl_list, HoistList list) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
@@ -1012,7 +1058,12 @@ __global__ void k_hoist_clean(float4* trav, const int32_t* __restrict__ pint, co
             const int32_t q = pint[p];
             const float c0[3] = {a0.x, a0.y, b0.x}, h0[3] = {a0.z, a0.w, b0.y};
             const float c1[3] = {a1.x, a1.y, b1.x}, h1[3] = {a1.z, a1.w, b1.y};
-            float c[3], h[3];
+            float c[3], h[3], far = 0.0f;
+            for (int ax = 0; ax < 3; ++ax) {
+                if (h0[ax] != -INFINITY && h1[ax] != -INFINITY)
+                    far += fmaxf(fabsf(c0[ax]) + h0[ax], fabsf(c1[ax]) + h1[ax]);
+            }
+            const float e = far * 4.76837158203125e-07f;  // 8 2^-24
             for (int ax = 0; ax < 3; ++ax) {
                 const bool e0 = h0[ax] == -INFINITY, e1 = h1[ax] == -INFINITY;
                 if (e0) {
@@ -1024,7 +1075,7 @@ __global__ void k_hoist_clean(float4* trav, const int32_t* __restrict__ pint, co
                 } else {
                     const float l0 = __fsub_rd(c0[ax], h0[ax]), u0 = __fadd_ru(c0[ax], h0[ax]);
                     const float l1 = __fsub_rd(c1[ax], h1[ax]), u1 = __fadd_ru(c1[ax], h1[ax]);
-                    centre_half(fminf(l0, l1), fmaxf(u0, u1), 0.0f, c[ax], h[ax]);
+                    centre_half(fminf(l0, l1), fmaxf(u0, u1), e, c[ax], h[ax]);
                     // a NaN box is always met, and so is every box above it
                     if (!(l0 <= u0) || !(l1 <= u1)) h[ax] = __int_as_float(0x7fc00000);
                 }
@@ -1050,11 +1101,7 @@ __global__ void k_hoist_clean(float4* trav, const int32_t* __restrict__ pint, co
 cudaError_t launch_trav_layout(const float4* nodes, const float4* sph, uint32_t n, float4* trav, const int32_t* pint,
                                const int32_t* pleaf, const HoistList* ctl_list, HoistList list, uint32_t* bad,
                                cudaStream_t st) {
-    float4* const root = trav + 4 * (size_t)(n - 1);
-    const cudaError_t e = cudaMemsetAsync(root, 0, 2 * sizeof(float4), st);
-    if (e != cudaSuccess) return e;
-    k_extent<<<std::min((n + 255) / 256, (uint32_t)(sm_count() * 4)), 256, 0, st>>>(
-        sph, n, ctl_list, list, reinterpret_cast<uint32_t*>(&root[1].z));
+    k_frame<<<1, 32, 0, st>>>(sph, n, ctl_list, list, trav + 4 * (size_t)(n - 1) + 2);
     k_trav_layout<<<(2 * (n - 1) + 255) / 256, 256, 0, st>>>(nodes, sph, n, trav, bad);
     if (ctl_list || list.n) k_hoist_clean<<<1, 32, 0, st>>>(trav, pint, pleaf, n, ctl_list, list);
     return cudaGetLastError();
@@ -1380,7 +1427,7 @@ venu_status build_scene(const venu_sphere* spheres, bool on_host, uint32_t n, cu
     const size_t words_b = al256(sizeof(uint32_t) * N);
     const size_t sort_b = general ? 3 * words_b + hist_b + al256(sizeof(uint32_t) * 4 * kBuckets) : words_b;
     const size_t nodes_b = al256(std::max(sizeof(float4) * 2 * nint, sort_b));
-    const size_t trav_b = al256(std::max(sizeof(float4) * (4 * nint + 2), sizeof(venu_sphere) * N));
+    const size_t trav_b = al256(std::max(sizeof(float4) * (4 * nint + 3), sizeof(venu_sphere) * N));
     const size_t sph_b = al256(sizeof(float4) * N), par_b = al256(sizeof(int32_t) * (nint + N));
     const size_t arr_b = al256(sizeof(uint32_t) * nint), ctl_b = al256(sizeof(LbvhCtl));
     const size_t err_b = al256(sizeof(uint32_t) * kTraceWords);

@@ -123,11 +123,11 @@ __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const ui
     if (!COUNT && !WIDE && n >= walk_min) {
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
             const float4 o4 = __ldcs(q.o + i), d4 = __ldcs(q.d + i);
-            RayPre R = prep_for<false>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<false>(S, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float t;
             int32_t k;
-            if (!(ray_margin(S, R) <= kFarMarginMax)) {  // rare: traced to the end now
+            if (!(R.m <= kFarMarginMax)) {  // rare: traced to the end now
                 R = prep<false>(R.o, R.d);
                 R.from = packed_from(d4.w);
                 axis_margins(R);
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) k_traverse(SceneView S, Queue q, const ui
         const uint32_t i = base + lane;
         if (i < n) {
             float4 o4 = __ldcs(q.o + i), d4 = __ldcs(q.d + i);
-            RayPre R = prep_for<COUNT, WIDE>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<COUNT, WIDE>(S, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float t;
             int32_t k = trace_closest<COUNT, kShared, WIDE>(S, R, 0.001f, 1e16f, t, sm, threadIdx.x, blockDim.x,
@@ -195,9 +195,9 @@ __global__ void VENU_WALK_BOUNDS k_walk(SceneView S, Queue q, const uint32_t* __
                     hits[ray].y = h.y == kMissDone ? -1 : h.y & (kHitDone - 1);
                 } else {
                     const float4 o4 = __ldcs(q.o + ray), d4 = __ldcs(q.d + ray);
-                    RayPre R = prep_for<false>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+                    RayPre R = prep_for<false>(S, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
                     R.from = packed_from(d4.w);
-                    T.open(R, ray_margin(S, R), 0.001f, 1e16f, __int_as_float(h.x), h.y < 0 ? kNone : h.y);
+                    T.open(R, R.m, 0.001f, 1e16f, __int_as_float(h.x), h.y < 0 ? kNone : h.y);
                     active = T.enter(S, K);  // else the record stands as it is
                 }
             }
@@ -257,9 +257,9 @@ __global__ void __launch_bounds__(256) k_traverse_dyn(SceneView S, Queue q, cons
                 if (my < n) {
                     ray = my;
                     const float4 o4 = __ldcs(q.o + my), d4 = __ldcs(q.d + my);
-                    RayPre R = prep_for<COUNT>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+                    RayPre R = prep_for<COUNT>(S, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
                     R.from = packed_from(d4.w);
-                    const float m = COUNT ? 0.0f : ray_margin(S, R);
+                    const float m = R.m;  // 0 in counting builds
                     if (COUNT ? R.axis : !(m <= kFarMarginMax)) {
                         // a ray that needs per-axis margins (rare): traced to the
                         // end now with the canonical loop, on this lane's free
@@ -325,7 +325,7 @@ __device__ __forceinline__ void trace_shade_loop(const SceneView& S, const Queue
                 d4 = qin.d[i];
             }
             slot = (uint32_t)__float_as_int(o4.w);
-            RayPre R = prep_for<COUNT, WIDE>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<COUNT, WIDE>(S, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float t;
             const int32_t k =
@@ -421,7 +421,7 @@ __device__ __forceinline__ void trace_shade_in_place(const SceneView& S, const Q
         const uint32_t until = done ? 2u * done : 1u;
         for (; done < until && __any_sync(0xffffffffu, live); ++done) {
             if (!live) continue;
-            RayPre R = prep_for<COUNT, WIDE>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<COUNT, WIDE>(S, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float th;
             const int32_t k = trace_closest<COUNT, KS, WIDE>(S, R, 0.001f, 1e16f, th, sm, t, blockDim.x, overflow, K);
@@ -488,7 +488,7 @@ __device__ __forceinline__ void trace_shade_in_place_refill(const SceneView& S, 
         }
         if (!__any_sync(0xffffffffu, live)) break;  // only once the launch has no rays left
         if (live) {
-            RayPre R = prep_for<COUNT, WIDE>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<COUNT, WIDE>(S, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
             float th;
             const int32_t k = trace_closest<COUNT, KS, WIDE>(S, R, 0.001f, 1e16f, th, sm, threadIdx.x, blockDim.x,
@@ -756,9 +756,9 @@ __global__ void VENU_WALK_BOUNDS k_finish_walk(SceneView S, Queue q0, Queue q1, 
         if (start) {
             ++traced;
             dbits = __float_as_uint(d4.w);
-            RayPre R = prep_for<false>(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
+            RayPre R = prep_for<false>(S, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z));
             R.from = packed_from(d4.w);
-            const float m = ray_margin(S, R);
+            const float m = R.m;
             T.open(R, m, 0.001f, 1e16f, 1e16f, kNone);
             if (!(m <= kFarMarginMax)) {  // rare: traced to the end now
                 R = prep<false>(R.o, R.d);
@@ -915,7 +915,7 @@ __global__ void __launch_bounds__(128) k_trace_rays(SceneView S, const float* __
     if (lane >= per_warp || i >= n) return;
     f3 o, d;
     load_ray(rays, i, o, d);
-    RayPre R = prep_for<false>(o, d);
+    RayPre R = prep_for<false>(S, o, d);
     TraceCounters K{0, 0};
     bool overflow = false;
     float t;
@@ -958,8 +958,8 @@ __global__ void __launch_bounds__(128, 8) k_trace_walk(SceneView S, const float*
             if (ray < n) {
                 f3 o, d;
                 load_ray(rays, ray, o, d);
-                RayPre R = prep_for<false>(o, d);
-                const float m = ray_margin(S, R), t0 = t_out[ray];
+                RayPre R = prep_for<false>(S, o, d);
+                const float m = R.m, t0 = t_out[ray];
                 const int32_t k0 = id_out[ray];
                 float t;
                 int32_t k;

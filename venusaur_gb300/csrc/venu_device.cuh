@@ -283,9 +283,10 @@ __device__ __forceinline__ int32_t sv_hoist(const JobScene& S, int h) { return S
 //   the others) and traverse with their own instantiation of the loop.
 //   from: slot of the sphere the ray leaves (its origin lies on that
 //   sphere's surface), or -1 (camera rays, rays from the caller).
+//   m: what the fast walk adds to exit parameters (far_margin).
 struct RayPre {
     f3 o, d, inv, n0, n1;
-    float a, inv_a;
+    float a, inv_a, m;
     bool axis;
     int32_t from;
 };
@@ -319,6 +320,7 @@ template <bool APPROX>
 __device__ __forceinline__ RayPre prep(f3 o, f3 d) {
     RayPre R;
     R.from = -1;
+    R.m = 0.0f;
     R.o = o;
     R.d = d;
     float dx = fabsf(d.x) < 1e-20f ? copysignf(1e-20f, d.x) : d.x;
@@ -620,7 +622,7 @@ __device__ __forceinline__ void up_front(T& W, const SV& S, TraceCounters& K) {
 //
 // Every other ray takes the fast walk over the traversal records (lbvh.cu):
 // a box is kept as centre c and half extent h per axis, so its entry and exit
-// are fma(h, -|1/d|, tc) and fma(h, |1/d|, tc) with tc = fma(c, 1/d, -o/d)
+// are fma(h, -|1/d|, tc) and fma(h, |1/d|, tc) with tc = fma(c, 1/d, -p/d)
 // and need no minimum and maximum per slab.  What bounds a step is issue and
 // the ALU pipe (minima, maxima, compares and selects run at half the rate of
 // the FMAs), and whatever one lane of a warp needs all of them pay for; so
@@ -631,36 +633,55 @@ __device__ __forceinline__ void up_front(T& W, const SV& S, TraceCounters& K) {
 // them at once in the node's step the 1080p RTIOW frame gains 4 %, a batch of
 // small renders 9 %.
 //
-// Nothing is lost by it: the records' half extents are widened by
-// e = 1.5 2^-19 E, where E is the largest |C| + |r| of the leaves.
-// sphere_test may accept a point that lies off the sphere by up to
-// 12 2^-24 (|h| + r) (h = o - C; roundings of h, of h.d, of the products with
-// d and of the root), and the slab parameters above are off by at most
-// 5 2^-24 (|o| + E) |1/d| (1/d an ulp off): together 17 2^-24 (|o| + E) in units
-// of length, 34 2^-24 E for |o| = E against e = 48 2^-24 E.  For origins further
-// out the rest, at most 34 2^-24 (|o| - E) max|1/d| over entry and exit, is
-// added to the exit parameter as 64 2^-24 (m); where that exceeds kFarMarginMax
-// the ray takes the canonical walk with margins per axis.  A sphere that is not
-// finite is not part of E; its box is NaN or infinite, and such a box is always
-// met.
+// Nothing is lost by it.  The records hold the boxes relative to a point G in
+// the middle of the scene, and so does the ray: p = o - G.  sphere_test may
+// accept a point that lies off the sphere by up to 12 2^-24 (|h| + r) (h = o - C;
+// roundings of h, of h.d, of the products with d and of the root), |h| + r is at
+// most |p| + Q with Q the distance from G of the farthest corner of the sphere's
+// box or of any box around it, and the slab parameters above are off by at most
+// 2^-24 (4 Q + 6 |p|) |1/d| (1/d an ulp off, p and p/d rounded): together
+// 2^-24 (16 Q + 18 |p|) in units of length.  The half extents are widened by
+// 24 2^-24 (Q + E), E twice the radius around G of nearly all spheres (k_frame),
+// which covers origins with |p| <= E.  For origins further out the
+// rest, at most 36 2^-24 (|p| - E) max|1/d| over entry and exit, is added to the
+// exit parameter as 64 2^-24 (m); where that exceeds kFarMarginMax the ray takes
+// the canonical walk with margins per axis.  So neither a scene's offset nor a
+// few spheres far from the others widen boxes by more than the rounding there
+// asks for: with one widening for all, 1.5 2^-19 of the largest |C| + r, RTIOW
+// moved by 1e6 took 67 box and 58 sphere tests a segment instead of 16 and 2.
+// A box that is not finite is always met.
 // ---------------------------------------------------------------------------
 constexpr float kFarMarginMax = 1.0f;
 
-__device__ __forceinline__ float far_margin(f3 o, f3 inv, float E) {
-    const float out = fmaxf((fabsf(o.x) + fabsf(o.y) + fabsf(o.z)) - E, 0.0f);
-    return out * fmax3(fabsf(inv.x), fabsf(inv.y), fabsf(inv.z)) * 3.814697265625e-06f;  // 2^-18
+// w: -2^-18 E
+__device__ __forceinline__ float far_margin(f3 p, f3 inv, float w) {
+    const float out = fmaxf(fmaf(fabsf(p.x) + fabsf(p.y) + fabsf(p.z), 3.814697265625e-06f, w), 0.0f);  // 2^-18
+    return out * fmax3(fabsf(inv.x), fabsf(inv.y), fabsf(inv.z));
 }
 
 // The root's record behind the n - 1 node records: {c.x, c.y, h.x, h.y},
-// {c.z, h.z, E, 0}.
+// {c.z, h.z, 0, 0}, {G, -2^-18 E}.
 template <class SV>
 __device__ __forceinline__ const float4* root_record(const SV& S) {
     return S.trav + 4 * (size_t)(sv_n(S) - 1u);
 }
 
+// A ray for the records of S.  G and E are read first, so that they are there
+// when the reciprocals are.
 template <class SV>
-__device__ __forceinline__ float ray_margin(const SV& S, const RayPre& R) {
-    return sv_n(S) > 1u ? far_margin(R.o, R.inv, __ldg(&root_record(S)[1].z)) : 0.0f;
+__device__ __forceinline__ RayPre prep_frame(const SV& S, f3 o, f3 d) {
+    const bool tree = sv_n(S) > 1u;
+    const float4 F = tree ? __ldg(root_record(S) + 2) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    RayPre R = prep<true>(o, d);
+    // -p, x and y packed
+    const f2 p_xy = fma2(pack2(R.o.x, R.o.y), pack2(-1.0f, -1.0f), pack2(F.x, F.y));
+    f3 p;
+    unpack2(p_xy, p.x, p.y);
+    p.z = F.z - R.o.z;
+    unpack2(mul2(p_xy, pack2(R.inv.x, R.inv.y)), R.n0.x, R.n0.y);
+    R.n0.z = p.z * R.inv.z;
+    R.m = tree ? far_margin(p, R.inv, F.w) : 0.0f;
+    return R;
 }
 
 // Per-lane traversal state.  begin() prepares a ray and tests the root;
@@ -699,7 +720,8 @@ struct Tracer {
     }
     __device__ __forceinline__ bool meets(float tn, float tf) const { return tn <= fminf(tf, best_t) + m; }
 
-    // R_ from prep(); AXIS: with per-axis margins.  m_: far_margin (fast walk).
+    // R_ from prep(), for the fast walk from prep_frame(); AXIS: with per-axis
+    // margins.
     template <class SV>
     __device__ __forceinline__ bool begin(const SV& S, const RayPre& R_, float m_, float tmin_, float tmax_,
                                           TraceCounters& K) {
@@ -1068,9 +1090,10 @@ struct WideTracer {
     }
 };
 
-template <bool COUNT, bool WIDE = false>
-__device__ __forceinline__ RayPre prep_for(f3 o, f3 d) {
-    return prep<!COUNT || WIDE>(o, d);
+template <bool COUNT, bool WIDE = false, class SV>
+__device__ __forceinline__ RayPre prep_for(const SV& S, f3 o, f3 d) {
+    if constexpr (COUNT && !WIDE) return prep<false>(o, d);
+    else return prep_frame(S, o, d);
 }
 
 template <class T, class SV>
@@ -1096,16 +1119,15 @@ __device__ __forceinline__ int32_t trace_closest(const SV& S, const RayPre& R, f
                                                  float tmax, float& t_out, StackSmem sm,
                                                  uint32_t tid, uint32_t bdim, bool& overflow,
                                                  TraceCounters& K) {
-    const float m = COUNT && !WIDE ? 0.0f : ray_margin(S, R);
-    if (COUNT && !WIDE ? R.axis : !(m <= kFarMarginMax)) {
+    if (COUNT && !WIDE ? R.axis : !(R.m <= kFarMarginMax)) {
         RayPre A = prep<false>(R.o, R.d);
         A.from = R.from;
         axis_margins(A);
         return trace_with<Tracer<COUNT, true, true, KS>>(S, A, 0.0f, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
     }
     if constexpr (WIDE)
-        return trace_with<WideTracer<COUNT, KS>>(S, R, m, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
-    return trace_with<Tracer<COUNT, COUNT, false, KS>>(S, R, m, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
+        return trace_with<WideTracer<COUNT, KS>>(S, R, R.m, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
+    return trace_with<Tracer<COUNT, COUNT, false, KS>>(S, R, R.m, tmin, tmax, t_out, sm, tid, bdim, overflow, K);
 }
 
 // ---------------------------------------------------------------------------
