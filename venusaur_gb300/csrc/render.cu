@@ -1074,7 +1074,6 @@ struct venu_renderer {
 };
 
 namespace {
-constexpr int kTravBlock = 128;  // venu_trace
 constexpr uint32_t kMaxDepth = 64;
 // Where k_traverse is split (variants 0 and 3; ms without -> with, from 1M rays
 // up).  By scene, 1080p x 8: 485 spheres 4.96 -> 5.43, 2k 5.00 -> 5.24, 7k 8.73
@@ -1084,12 +1083,6 @@ constexpr uint32_t kMaxDepth = 64;
 // x 8 on 1M spheres 65.1 instead of 64.4.
 constexpr uint32_t kWalkSpheres = 16384, kWalkRays = 1u << 20;
 constexpr uint32_t kFinishWalkSpheres = 7168;  // see k_finish_walk
-// Where a caller's rays are split the same way (us without -> with): 1M rays on
-// 20k spheres 636 -> 719, 2M on 50k 1472 -> 1512, 2M on 100k 1656 -> 1536, 2M on
-// 200k 1740 -> 1508, 500k on 100k 589 -> 549, 250k on 200k 359 -> 360.
-constexpr uint32_t kTraceWalkSpheres = 65536, kTraceWalkRays = 1u << 18;
-
-
 template <typename K>
 cudaError_t occupancy_grid(K kernel, int block, size_t smem, uint32_t per_sm_cap, int& grid) {
     int per_sm = 0;
@@ -1770,23 +1763,18 @@ extern "C" venu_status venu_trace(const venu_scene* scene, const float* rays_dev
         VENU_CUDA(cudaMalloc(&err, 2 * sizeof(uint32_t)));
         e = cudaMemsetAsync(err, 0, 2 * sizeof(uint32_t), st);
     }
-    const size_t tsm = traverse_smem(kTravBlock);  // 8 KB: below the size that needs an attribute
+    const size_t tsm = traverse_smem((int)kTraceBlock);
     if (e == cudaSuccess) {
         const SceneView S = view_of(scene);
-        // split as k_traverse (the hits so far travel in the caller's outputs)
-        const bool walk = t_dev && id_dev && scene->n >= kTraceWalkSpheres && n >= kTraceWalkRays;
-        const uint32_t warps = kTravBlock / 32u;
-        const uint32_t fill = (uint32_t)sm_count() * 4u * warps;  // a warp or more on every scheduler
-        const uint32_t per_warp = walk ? 32u : std::min(32u, (n + fill - 1u) / fill);
-        const uint32_t grid = (n + warps * per_warp - 1u) / (warps * per_warp);
-        if (walk) {
-            k_trace_rays<true><<<grid, kTravBlock, tsm, st>>>(S, rays_dev, n, per_warp, tmin, tmax, t_dev, id_dev,
-                                                             front_dev, err, err + 1);
-            k_trace_walk<<<sm_count() * 8, kTravBlock, tsm, st>>>(S, rays_dev, n, tmin, tmax, t_dev, id_dev, front_dev,
-                                                                err, err + 1);
+        const TracePlan P = trace_plan(scene->n, n, t_dev && id_dev, (uint32_t)sm_count());
+        if (P.walk) {
+            k_trace_rays<true><<<P.grid, kTraceBlock, tsm, st>>>(S, rays_dev, n, P.per_warp, tmin, tmax, t_dev, id_dev,
+                                                                front_dev, err, err + 1);
+            k_trace_walk<<<sm_count() * 8, kTraceBlock, tsm, st>>>(S, rays_dev, n, tmin, tmax, t_dev, id_dev, front_dev,
+                                                                 err, err + 1);
         } else {
-            k_trace_rays<false><<<grid, kTravBlock, tsm, st>>>(S, rays_dev, n, per_warp, tmin, tmax, t_dev, id_dev,
-                                                              front_dev, err, nullptr);
+            k_trace_rays<false><<<P.grid, kTraceBlock, tsm, st>>>(S, rays_dev, n, P.per_warp, tmin, tmax, t_dev, id_dev,
+                                                                 front_dev, err, nullptr);
         }
         e = cudaGetLastError();
     }

@@ -46,6 +46,30 @@ cudaError_t prefer_l1(K kernel, int per_sm, size_t dyn) {
 namespace venu {
 constexpr uint32_t kTraceWords = 64;  // two for each venu_trace call of a scene that may run without allocating
 
+// How venu_trace runs n rays: blocks of kTraceBlock threads, per_warp rays a warp
+// (fewer than 32 while that puts a warp or more on every scheduler); walk: split
+// as the renderer's k_traverse, the hits so far in the caller's outputs (both).
+// Where the split pays (us without -> with): 1M rays on 20k spheres 636 -> 719, 2M
+// on 50k 1472 -> 1512, 2M on 100k 1656 -> 1536, 2M on 200k 1740 -> 1508, 500k on
+// 100k 589 -> 549, 250k on 200k 359 -> 360; and its hand-out counter, which each
+// warp takes past n once, must not wrap.  64 bits: n + a grid may not fit 32.
+constexpr uint32_t kTraceBlock = 128;
+constexpr uint32_t kTraceWalkSpheres = 65536, kTraceWalkRays = 1u << 18, kTraceWalkMost = 1u << 31;
+struct TracePlan {
+    uint32_t per_warp, grid;
+    bool walk;
+};
+inline TracePlan trace_plan(uint32_t spheres, uint32_t n, bool both_outputs, uint32_t sms) {
+    TracePlan p;
+    p.walk = both_outputs && spheres >= kTraceWalkSpheres && n >= kTraceWalkRays && n <= kTraceWalkMost;
+    const uint32_t warps = kTraceBlock / 32u;
+    const uint64_t fill = (uint64_t)sms * 4u * warps;
+    const uint64_t share = ((uint64_t)n + fill - 1u) / fill;
+    p.per_warp = p.walk || share > 32u ? 32u : (uint32_t)share;
+    p.grid = (uint32_t)(((uint64_t)n + warps * p.per_warp - 1u) / (warps * p.per_warp));
+    return p;
+}
+
 // Device memory handed out in stream order and kept for reuse up to `keep`
 // bytes (the default pool gives everything back at each synchronisation, and
 // mapping it again costs 100 us and more); destroyed with its owner.  What it
