@@ -70,7 +70,7 @@ def test_hit_spheres_are_met(oracle, r, at):
     assert hit.sum() > m // 4
     d0 = np.where(np.abs(d) < F(1e-20), np.copysign(F(1e-20), d), d)
     inv = F(1.0) / d0
-    inv = np.where(rng.random(inv.shape) < 0.5, inv, np.nextafter(inv, inv * F(2)))
+    inv = np.choose(rng.integers(0, 3, inv.shape), [inv, np.nextafter(inv, inv * F(2)), np.nextafter(inv, F(0))])
     # its own box; one that another sphere nearby extends; one that a far one does
     R = F(r)
     lo = np.repeat(_down(C.astype(np.float64) - float(R))[None], m, 0)
