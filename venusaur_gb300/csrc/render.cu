@@ -684,7 +684,6 @@ __global__ void VENU_FINISH_BOUNDS k_finish(SceneView S, Queue q0, Queue q1, flo
 // 100k 1080p x 1 4.37 -> 3.95, 300k 512x512 x 4 with its build 5.72 -> 5.28, 1M
 // 1080p x 1 20.8 -> 18.6; 5k 640x480 x 4 0.780 -> 0.797.  Serving at half of the
 // paths (an eighth: 19.0 on the last), votes every 16 steps (8: 28.3, 64: 19.3).
-template <int KS>
 __global__ void VENU_WALK_BOUNDS k_finish_walk(SceneView S, Queue q0, Queue q1, float4* __restrict__ slots,
                                                uint32_t* __restrict__ err, unsigned long long* __restrict__ stats,
                                                PrimaryGen gen, WaveCtl* ctl, uint32_t spread_max, LeftOf src) {
@@ -704,7 +703,7 @@ __global__ void VENU_WALK_BOUNDS k_finish_walk(SceneView S, Queue q0, Queue q1, 
     const uint32_t lane = threadIdx.x & 31u;
     TraceCounters K{0, 0};
     bool overflow = false;
-    Tracer<false, false, false, KS> T;
+    Tracer<false> T;
     int2 spill[kSpill];
     uint32_t own = 0xffffffffu;  // the first ray this lane took
     uint32_t traced = 0, slot = 0, dbits = 0;
@@ -765,8 +764,8 @@ __global__ void VENU_WALK_BOUNDS k_finish_walk(SceneView S, Queue q0, Queue q1, 
                 R.from = packed_from(d4.w);
                 axis_margins(R);
                 float t;
-                const int32_t k = trace_with<Tracer<false, true, true, KS>>(S, R, 0.0f, 0.001f, 1e16f, t, sm, threadIdx.x,
-                                                                           blockDim.x, overflow, K);
+                const int32_t k = trace_with<Tracer<false, true, true>>(S, R, 0.0f, 0.001f, 1e16f, t, sm, threadIdx.x,
+                                                                       blockDim.x, overflow, K);
                 T.best_t = t;
                 T.best = k < 0 ? kNone : k;
             } else {
@@ -1082,7 +1081,9 @@ constexpr uint32_t kMaxDepth = 64;
 // 640x360 x 4 on 300k spheres takes 8.80 instead of 8.48; from 2M up, 1280x720
 // x 8 on 1M spheres 65.1 instead of 64.4.
 constexpr uint32_t kWalkSpheres = 16384, kWalkRays = 1u << 20;
+constexpr uint32_t kShallowSpheres = 4096;      // kSharedShallow stack entries serve up to here
 constexpr uint32_t kFinishWalkSpheres = 7168;  // see k_finish_walk
+static_assert(kFinishWalkSpheres > kShallowSpheres, "k_finish_walk has the deep stack alone");
 template <typename K>
 cudaError_t occupancy_grid(K kernel, int block, size_t smem, uint32_t per_sm_cap, int& grid) {
     int per_sm = 0;
@@ -1105,7 +1106,7 @@ cudaError_t configure_fused(venu_renderer* r, K8 deep, K4 shallow) {
     cudaError_t e = occupancy_grid(deep, tb, sm, t.traverse_blocks_per_sm, r->fused_blocks);
     if (e == cudaSuccess)
         e = occupancy_grid(k_finish<false, kShared, false, false>, tb, sm, t.traverse_blocks_per_sm, r->finish_blocks);
-    if (e == cudaSuccess) e = prefer_l1(k_finish_walk<kShared>, std::max(1, r->finish_blocks / std::max(1, sm_count())), sm);
+    if (e == cudaSuccess) e = prefer_l1(k_finish_walk, std::max(1, r->finish_blocks / std::max(1, sm_count())), sm);
     const int nsm = std::max(1, sm_count());
     const int pb = std::max(1, r->fused_blocks / nsm), pf = std::max(1, r->finish_blocks / nsm);
     if (e == cudaSuccess) e = prefer_l1(deep, pb, sm);
@@ -1238,8 +1239,8 @@ cudaError_t launch_finish(const venu_renderer* r, cudaStream_t st, uint32_t kind
 #define VENU_FINISH(WIDE, C, KS)                                                                                  \
     do {                                                                                                          \
         if (walk && (which & kFinishRefill))                                                                      \
-            k_finish_walk<KS><<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, \
-                                                     spread_max, src);                                            \
+            k_finish_walk<<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl,     \
+                                                 spread_max, src);                                                \
         else if (which & kFinishRefill)                                                                           \
             k_finish<C, KS, C && WIDE, true>                                                                           \
                 <<<grid, tb, fsm, st>>>(S, r->q[0], r->q[1], r->slots, r->err, r->stats, pg, r->ctl, spread_max, src); \
@@ -1479,7 +1480,7 @@ extern "C" venu_status venu_render(venu_renderer* r, const venu_scene* scene, co
     const bool gen0 = tu.traverse_variant >= 2u;
     // small scenes have shallow trees: a 4-entry shared stack leaves more of
     // the SM's memory to L1 (measured: RTIOW +0.5 %; 1M spheres -4.5 %)
-    const bool shallow = scene->n <= 4096u;
+    const bool shallow = scene->n <= kShallowSpheres;
     uint32_t* const path_seeds = gen0 ? reinterpret_cast<uint32_t*>(r->q[0].t) : nullptr;
     // bounces that k_walk takes (see k_traverse): counting builds never split
     const uint32_t walk_min =
