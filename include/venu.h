@@ -316,10 +316,10 @@ typedef struct venu_tuning {
     uint32_t traverse_blocks_per_sm; /* 0 = as many as fit */
     uint32_t shade_block;            /* threads per shade block: 64..512, multiple of 32 */
     uint32_t shade_blocks_per_sm;    /* 0 = as many as fit */
-    uint32_t in_place_factor;        /* fused variants: once at most this many rays per thread of the
+    uint32_t in_place_factor;        /* variants 2 to 5: once at most this many rays per thread of the
                                         finishing kernel's grid are left, it runs them to their ends,
                                         refilling finished threads (2..16; 0 or 1: the renderer
-                                        chooses; the batch engine ignores it) */
+                                        chooses; variants 0 and 1 and the batch engine ignore it) */
 } venu_tuning;
 VENU_API venu_status venu_renderer_set_tuning(venu_renderer* r, const venu_tuning* t);
 VENU_API venu_status venu_renderer_get_tuning(const venu_renderer* r, venu_tuning* t);
@@ -357,7 +357,9 @@ typedef struct venu_batch_stats {
 
 #define VENU_BATCH_NO_GRAPH 1u /* run the path loop from the host (one launch per stage) */
 
-/* pool_paths: paths in flight (0 = 64 Mi, about 7 GB); max_jobs: concurrently admitted jobs (<= 4096). */
+/* pool_paths: paths in flight (0 = 64 Mi, about 7 GB); max_jobs: concurrently admitted jobs (<= 4096).
+ * Collected jobs' buffers are kept for the next jobs, up to 20 bytes per path of the pool and
+ * 512 MB, until the batch is destroyed. */
 VENU_API venu_status venu_batch_create(uint32_t pool_paths, uint32_t max_jobs, uint32_t flags, venu_batch** out);
 VENU_API venu_status venu_batch_set_tuning(venu_batch* b, const venu_tuning* t);
 /* Bytes venu_batch_submit allocates for a job of this size (seed table + slots). */
@@ -374,7 +376,9 @@ VENU_API venu_status venu_batch_submit_many(venu_batch* b, const venu_job_desc* 
 /* Runs the shared path loop for at most max_iterations steps (0 = until
  * every admitted job has finished) as one graph launch on `stream`; a step
  * is one iteration (every queued ray traced once) unless venu_batch_set_chunk
- * splits iterations.  With VENU_RUN_STOP_ON_FINISH the loop also ends after
+ * splits iterations, and a step of few rays (up to one per thread of the finishing
+ * kernel's grid, about 156 thousand, or 8 per thread once no path is left to
+ * hand out and steps are not chunked) runs all of its paths to their ends.  With VENU_RUN_STOP_ON_FINISH the loop also ends after
  * the step in which a job's last path finished, so a server can hand results
  * out at once. */
 #define VENU_RUN_STOP_ON_FINISH 1u

@@ -12,7 +12,9 @@
 //                new paths the last plan handed out: those camera rays are
 //                made in the kernel, from each job's precomputed raygen
 //                seed table, and never pass through memory;
-//   plan         one thread hands the free pool slots to the admitted jobs
+//   finish       instead of that, when few rays are left and no new paths
+//                follow (finish_step): each path to its end;
+//   plan         one warp hands the free pool slots to the admitted jobs
 //                in plan order (submission order, or shortest first);
 //
 // repeated under a device-side while condition, so the whole loop is one

@@ -94,7 +94,8 @@ __global__ void k_raygen(venu_camera cam, uint32_t W, uint32_t H, uint32_t p0, u
 // walks the tree from there with lanes that take a new ray when theirs is
 // done.  On large scenes a warp has 12 of 32 lanes in its walk on average
 // (its rays take 20 to 400 steps) and waits for L2 most of the time; the
-// refills bring that to 24.  They only pay because a refill is cheap -- the
+// refills bring that to 24 (10 per instruction: in most steps one or two of them
+// test a leaf's sphere while the others wait).  They only pay because a refill is cheap -- the
 // up-front tests with their long refined branch are done -- and because lanes
 // vote every kWalkSteps steps only and walk on by themselves in between (a
 // vote a step costs more than the lanes it fills).  Then the L1 data pipe is
@@ -632,8 +633,7 @@ __device__ __forceinline__ void find_left(const WaveCtl* ctl, LeftOf src, uint32
 // The finishing kernel: runs the paths that are left of a wave (WaveCtl) to
 // their ends.  A kernel of its own, so that the bounce kernels' code and
 // registers are not shaped by it (in one kernel with them, changes to this
-// part moved the bounce loop by up to 1.5 %; apart, the bounce kernel spills 12
-// bytes instead of 60): 1080p x 32 RTIOW 14.05 -> 13.95 ms, 256x144 x 4 278 ->
+// part moved the bounce loop by up to 1.5 %): 1080p x 32 RTIOW 14.05 -> 13.95 ms, 256x144 x 4 278 ->
 // 260 us, 64x36 x 2 107 -> 90 us.  At 80 / 96 / 128 registers, with as many
 // fewer rays to take, the 256x144 frame takes 297 / 296 / 295 us.  REFILL:
 // with refills, for more than spread_max rays (a thread each of the grid); the
@@ -1040,7 +1040,7 @@ struct WaveGraphKey {
     size_t fsm;
     int grid, block, finish_grid;
     uint32_t first_max, finish_max;
-    uint32_t kind;  // bits: 4-wide tree, shallow stack, counting build, in-place refills
+    uint32_t kind;  // bits: 4-wide tree, shallow stack, counting build
 };
 
 struct venu_renderer {

@@ -314,8 +314,11 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return r;
 }
 
-// APPROX: 1/d good to an ulp, which is all the fast walk asks of it (it serves
-// the slab tests alone; 1/a below enters the hits and stays correctly rounded).
+// APPROX: 1/d good to an ulp, which is all the fast walk asks of it: it serves
+// the slab tests alone, whose margins count the ulp, and no hit depends on it (1/a
+// below enters the hits and stays correctly rounded).  Correctly rounded: RTIOW
+// 1920x1080 x 256 +0.8 %, 1200x800 x 16 +1.6 %, 96 uneven jobs +0.7 %, images the
+// same.
 template <bool APPROX>
 __device__ __forceinline__ RayPre prep(f3 o, f3 d) {
     RayPre R;
@@ -525,17 +528,17 @@ __device__ __forceinline__ bool sphere_test(const RayPre& R, float4 S, float tmi
 // Closest-hit traversal of the binary LBVH.
 //
 // Children are tested at their parent, from the parent's 64-byte record in
-// the traversal layout (one contiguous 4 x float4 load): internal children by
-// their box, leaf children directly by their sphere, stored inline.  The
-// nearer hit child is descended; the farther one's index and entry distance
-// go on a per-thread stack whose top kShared entries live in shared
-// memory (ring buffer, layout [entry][thread] so a warp touches 32 distinct
-// banks) and whose older entries spill to local memory.  Ties on t go to the
-// smaller slot, so the result does not depend on traversal order.
+// the traversal layout (two 32-byte loads), leaves by their boxes as internal
+// nodes are.  The nearer hit child is descended; the farther one's word and entry
+// distance go on a per-thread stack whose first kShared entries live in shared
+// memory (layout [entry][thread] so a warp touches 32 distinct banks) and the
+// deeper ones in local memory.  (The walk of the wide tree below keeps its top
+// entries in shared memory instead, as a ring.)  Ties on t go to the smaller slot,
+// so the result does not depend on traversal order.
 // ---------------------------------------------------------------------------
 constexpr int kShared = 8;   // shared-memory entries per thread (power of two)
 constexpr int kSharedShallow = 4;  // the fused kernel's choice for shallow trees (small scenes)
-constexpr int kSpill = 72;   // local-memory entries beyond those
+constexpr int kSpill = 72;   // local-memory entries beside those
 
 struct StackSmem {
     int2* e;     // [kShared][block]: {node, entry distance}

@@ -29,8 +29,10 @@ def candidates(space=None):
                                              space["traverse_block"], space["shade_block"],
                                              space["in_place_factor"]):
         # the refill threshold matters to the dynamic-fetch variant only, the
-        # shade block to the variants with a separate shade kernel only, the
-        # in-place factor to the variants that are fused on every bounce only
+        # shade block to the variants with a separate shade kernel only; the
+        # in-place factor is tried with the variants that are fused on every
+        # bounce (3 and 5 obey it as well, but leave it little to do: 1M spheres
+        # 1919x1079 x 8 at 8 / 16 / 32 rays a thread 131.0 / 129.6 / 129.2 ms)
         key = (v, r if v == 1 else 32, tb, sb if v not in (2, 4) else 256, f if v in (2, 4) else 1)
         if key in seen:
             continue
