@@ -80,27 +80,28 @@ KERNEL_SOURCES = ("venusaur_gb300/csrc/venu_device.cuh", "venusaur_gb300/csrc/re
 # segments; lanes_per_inst = smsp__thread_inst_executed_per_inst_executed.ratio
 # (active lanes per issued instruction, all instructions).  `sha` is
 # kernel_sources_sha() of the captured build.  Each figure is summed over the
-# launches of the fused bounce, separate traversal, walk, shading and finishing
-# kernels of two renders of
+# launches of the fused bounce, separate traversal, walk and finishing kernels
+# (not k_shade, which walks nothing) of two renders of
 # `bench.py --config <c> --spp <s> --profile-render --tuning <variant>`
 # (c2: 4 spp, c3: 16 spp, c1: its own 16 spp; traverse_block 128;
-# "/f8": in_place_factor 8)
+# "/f8": in_place_factor 8; c1/v5, whose wave is the finishing kernel's as
+# c1/v4's, takes that one's figures)
 # under ncu --metrics
 # dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum,
 # smsp__inst_executed.sum,smsp__thread_inst_executed.sum.
-NCU_FIGURES = {"sha": "aec54f6529d487da", "commit": "47604f3", "figures": {
-    "c2/v2": {"dram_b_per_seg": 57.43, "lanes_per_inst": 14.71, "warp_inst_per_seg": 71.5},
-    "c2/v2/f8": {"dram_b_per_seg": 60.82, "lanes_per_inst": 14.65, "warp_inst_per_seg": 71.9},
-    "c2/v4": {"dram_b_per_seg": 57.4, "lanes_per_inst": 15.87, "warp_inst_per_seg": 79.0},
-    "c1/v2": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.97, "warp_inst_per_seg": 94.2},
-    "c1/v2/f8": {"dram_b_per_seg": 24.84, "lanes_per_inst": 12.06, "warp_inst_per_seg": 92.9},
-    "c1/v3": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.98, "warp_inst_per_seg": 94.1},
-    "c1/v4": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.97, "warp_inst_per_seg": 94.2},
-    "c1/v5": {"dram_b_per_seg": 1.66, "lanes_per_inst": 10.97, "warp_inst_per_seg": 94.2},
-    "c1/v4/f8": {"dram_b_per_seg": 24.64, "lanes_per_inst": 12.6, "warp_inst_per_seg": 95.4},
-    "c3/v3": {"dram_b_per_seg": 75.6, "lanes_per_inst": 10.67, "warp_inst_per_seg": 397.8},
-    "c3/v2": {"dram_b_per_seg": 13.86, "lanes_per_inst": 9.38, "warp_inst_per_seg": 479.7},
-    "c3/v5": {"dram_b_per_seg": 39.6, "lanes_per_inst": 8.4, "warp_inst_per_seg": 548.0},
+NCU_FIGURES = {"sha": "1acb997947d0602c", "commit": "5736bdd", "figures": {
+    "c2/v2": {"dram_b_per_seg": 57.51, "lanes_per_inst": 14.85, "warp_inst_per_seg": 71.1},
+    "c2/v2/f8": {"dram_b_per_seg": 60.89, "lanes_per_inst": 14.79, "warp_inst_per_seg": 71.4},
+    "c2/v4": {"dram_b_per_seg": 57.41, "lanes_per_inst": 15.93, "warp_inst_per_seg": 78.6},
+    "c1/v2": {"dram_b_per_seg": 1.66, "lanes_per_inst": 11.04, "warp_inst_per_seg": 93.6},
+    "c1/v2/f8": {"dram_b_per_seg": 24.99, "lanes_per_inst": 12.14, "warp_inst_per_seg": 92.5},
+    "c1/v3": {"dram_b_per_seg": 1.68, "lanes_per_inst": 11.06, "warp_inst_per_seg": 93.5},
+    "c1/v4": {"dram_b_per_seg": 1.67, "lanes_per_inst": 11.04, "warp_inst_per_seg": 93.6},
+    "c1/v5": {"dram_b_per_seg": 1.67, "lanes_per_inst": 11.04, "warp_inst_per_seg": 93.6},
+    "c1/v4/f8": {"dram_b_per_seg": 24.68, "lanes_per_inst": 12.68, "warp_inst_per_seg": 94.8},
+    "c3/v3": {"dram_b_per_seg": 75.57, "lanes_per_inst": 10.78, "warp_inst_per_seg": 389.7},
+    "c3/v2": {"dram_b_per_seg": 13.81, "lanes_per_inst": 9.39, "warp_inst_per_seg": 480.0},
+    "c3/v5": {"dram_b_per_seg": 39.51, "lanes_per_inst": 8.4, "warp_inst_per_seg": 548.1},
 }}
 
 
