@@ -129,3 +129,47 @@ def test_captured_refit(venu, oracle, cuda):
     graph.replay()
     torch.cuda.synchronize()
     assert np.array_equal(ds.export_bvh()["nodes"].view(np.uint32), want_a.view(np.uint32))
+
+
+def test_updates_beside_the_first_wide_render(venu, oracle, cuda):
+    """The 4-wide tree, built by the first render that asks for it, while another
+    thread moves the spheres: afterwards it is that of the last pose."""
+    torch = cuda
+    n, W, H, spp, depth = 20_000, 96, 54, 2, 10
+    sp = oracle.scene_random(n, 75)
+    to = _moved(sp, 5, 0.5)
+    cam = oracle.camera((60, 15, 60), (0, 0, 0), 20.0, W / H, 0.1, 10.0)
+    want = oracle.render(to, cam, W, H, spp, subframe=1, max_depth=depth, mode=pyoracle.MODE_GB300, built_from=sp)
+    dev = torch.from_numpy(to.view(np.uint8).copy()).cuda()
+    torch.cuda.synchronize()
+    for _ in range(8):
+        ds = venu.DeviceScene(sp)
+        started = threading.Event()
+        failed = []
+
+        def move():
+            s = torch.cuda.Stream()
+            try:
+                for k in range(40):
+                    ds.update_device(dev, n, stream=s)
+                    started.set()
+                s.synchronize()
+            except venu.VenuError as e:
+                failed.append(e)
+
+        th = threading.Thread(target=move)
+        th.start()
+        started.wait()
+        wf = venu.Wavefront(0, count=True)  # counting renders of variant 4 walk the 4-wide tree to the end
+        wf.set_tuning(traverse_variant=4)
+        acc = venu.new_accum(W, H)
+        side = torch.cuda.Stream()
+        wf.render(ds, cam, W, H, spp, acc, subframe=1, max_depth=depth, reset=True, stream=side)
+        side.synchronize()
+        th.join()
+        wf.stats()  # raises on a traversal error
+        assert not failed
+        wf.render(ds, cam, W, H, spp, acc, subframe=1, max_depth=depth, reset=True)
+        torch.cuda.synchronize()
+        assert np.array_equal(acc.cpu().numpy().view(np.uint32), want["accum"].view(np.uint32))
+        ds.close()

@@ -1516,6 +1516,10 @@ venu_status ensure_wide(const venu_scene* S, cudaStream_t st) {
     std::lock_guard<std::mutex> lock(S->wide_mu);
     if (S->n < 2 || S->wide) return VENU_OK;
     const auto t0 = std::chrono::steady_clock::now();
+    // after the refits called for so far, and before any that is called for from
+    // now on: those find the whole tree and refit it, too
+    std::lock_guard<std::mutex> refits(S->refit_mu);
+    if (S->refit_done) VENU_CUDA(cudaStreamWaitEvent(st, S->refit_done, 0));
     const venu_status rc = build_wide(S, st);
     S->wide_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
     if (rc != VENU_OK) {  // no half-built tree stays behind

@@ -144,9 +144,10 @@ struct venu_scene {
     venu_sphere* upload = nullptr;
     std::mutex update_mu;         // one upload at a time
     // Refits share the counters, so each waits on the device for the one before
-    // it, on whatever stream that ran (refit_done, recorded by the first).
+    // it, on whatever stream that ran (refit_done, recorded by the first).  The first
+    // build of the wide tree reads the records and waits for them as well.
     cudaEvent_t refit_done = nullptr;
-    std::mutex refit_mu;
+    mutable std::mutex refit_mu;
     float bounds[6] = {0, 0, 0, 0, 0, 0};
     uint32_t nhoist = 0;          // huge spheres tested before traversal
     int32_t hoist[4] = {0, 0, 0, 0};
